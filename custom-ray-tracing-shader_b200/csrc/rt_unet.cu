@@ -96,6 +96,17 @@ __global__ void __launch_bounds__(128) wgradKernel(const bf16* __restrict__ x, c
 }
 
 // ---- elementwise and reshaping kernels ----
+// Position of pixel p of `total` = n * h * w; 32-bit divisions where the
+// index fits (64-bit ones are a subroutine of ~70 instructions).
+struct Pixel { int x, y, n; };
+__device__ __forceinline__ Pixel pixelOf(long long p, long long total, int w, int h) {
+    if (total <= 0xFFFFFFFFll) {
+        const unsigned u = (unsigned)p, row = u / (unsigned)w;
+        return Pixel{(int)(u % (unsigned)w), (int)(row % (unsigned)h), (int)(row / (unsigned)h)};
+    }
+    const long long row = p / w;
+    return Pixel{(int)(p % w), (int)(row % h), (int)(row / h)};
+}
 __global__ void inputKernel(const float* aov, int n, int h, int w, int H, int W, bf16* x0, const int* batch,
                             const unsigned char* flips) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -125,18 +136,6 @@ __global__ void inputKernel(const float* aov, int n, int h, int w, int H, int W,
     o[0] = packed[0];
     o[1] = packed[1];
 }
-__global__ void targetKernel(const float* target, int n, int h, int w, float* out, const int* batch,
-                             const unsigned char* flips) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long total = (long long)n * h * w;
-    if (i >= total) return;
-    int X = (int)(i % w), Y = (int)((i / w) % h), b = (int)(i / ((long long)w * h));
-    int src = batch ? batch[b] : b;
-    int sx = X, sy = Y;
-    if (flips) { if (flips[b] & 1) sx = w - 1 - X; if (flips[b] & 2) sy = h - 1 - Y; }
-    const float* t = target + (((size_t)src * h + sy) * w + sx) * 3;
-    for (int c = 0; c < 3; c++) out[(size_t)i * 3 + c] = log1pf(fmaxf(t[c], 0.0f));
-}
 // 2x2 average pooling, 8 channels per thread (16-byte loads and stores).
 __global__ void poolKernel(const bf16* in, int N, int H, int W, int C, bf16* out) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -161,72 +160,224 @@ __global__ void poolKernel(const bf16* in, int N, int H, int W, int C, bf16* out
     }
     *reinterpret_cast<uint4*>(out + (size_t)p * C + c) = r;
 }
-__global__ void poolBackwardKernel(const float* dOut, int N, int H, int W, int C, float* dIn, int accumulate) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long total = (long long)N * H * W * C;
-    if (i >= total) return;
-    int c = (int)(i % C);
-    long long p = i / C;
-    int x = (int)(p % W), y = (int)((p / W) % H), n = (int)(p / ((long long)W * H));
-    float v = 0.25f * dOut[(((size_t)n * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c];
-    dIn[i] = accumulate ? dIn[i] + v : v;
-}
-// out = concat(upsample2(low), skip) along channels.
+// out = concat(upsample2(low), skip) along channels, 8 channels per thread.
+// Bound by the write of the concatenation; one element per thread (2-byte
+// accesses, two 64-bit divisions each) took 264 us for 32 x 128 x 128 x 80.
 __global__ void upConcatKernel(const bf16* low, int Cl, const bf16* skip, int Cs, int N, int H, int W, bf16* out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int C = Cl + Cs;
-    long long total = (long long)N * H * W * C;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int C = Cl + Cs, C8 = C / 8;
+    const long long total = (long long)N * H * W * C8;
     if (i >= total) return;
-    int c = (int)(i % C);
-    long long p = i / C;
-    int x = (int)(p % W), y = (int)((p / W) % H), n = (int)(p / ((long long)W * H));
-    out[i] = c < Cl ? low[(((size_t)n * (H / 2) + y / 2) * (W / 2) + x / 2) * Cl + c]
-                    : skip[(((size_t)n * H + y) * W + x) * Cs + (c - Cl)];
+    const int c = (int)(i % C8) * 8;
+    const long long p = i / C8;
+    const Pixel q = pixelOf(p, (long long)N * H * W, W, H);
+    const uint4* src = c < Cl
+        ? reinterpret_cast<const uint4*>(low + (((size_t)q.n * (H / 2) + q.y / 2) * (W / 2) + q.x / 2) * Cl + c)
+        : reinterpret_cast<const uint4*>(skip + (size_t)p * Cs + (c - Cl));
+    *reinterpret_cast<uint4*>(out + (size_t)p * C + c) = __ldg(src);
 }
-// Backward of upConcat: gradient of low (summed over 2x2) and of skip.
-__global__ void upConcatBackwardLowKernel(const float* dOut, int Cl, int Cs, int N, int H, int W, float* dLow) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int Hl = H / 2, Wl = W / 2, C = Cl + Cs;
-    long long total = (long long)N * Hl * Wl * Cl;
-    if (i >= total) return;
-    int c = (int)(i % Cl);
-    long long p = i / Cl;
-    int x = (int)(p % Wl), y = (int)((p / Wl) % Hl), n = (int)(p / ((long long)Wl * Hl));
-    const float* d = dOut + (((size_t)n * H + 2 * y) * W + 2 * x) * C + c;
-    dLow[i] = d[0] + d[C] + d[(size_t)W * C] + d[(size_t)W * C + C];
+
+// Sums of N per-thread values over a block of up to 256 threads whose lanes hold
+// the sums of GROUP interleaved owners (thread t belongs to owner t % GROUP,
+// GROUP a power of two up to 32): add[owner * N + v] receives the totals,
+// one atomic per value and block. scratch: 8 * GROUP * N floats.
+template <int N, int GROUP>
+__device__ __forceinline__ void blockSums(float (&v)[N], float* scratch, float* add) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+        for (int off = 16; off >= GROUP; off >>= 1) v[k] += __shfl_xor_sync(0xFFFFFFFFu, v[k], off);
+    if (lane < GROUP)
+#pragma unroll
+        for (int k = 0; k < N; k++) scratch[(warp * GROUP + lane) * N + k] = v[k];
+    __syncthreads();
+    for (int i = threadIdx.x; i < GROUP * N; i += blockDim.x) {
+        float s = 0.0f;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += scratch[w * GROUP * N + i];
+        if (s != 0.0f) atomicAdd(add + i, s);
+    }
+    __syncthreads();
 }
-__global__ void upConcatBackwardSkipKernel(const float* dOut, int Cl, int Cs, long long pixels, float* dSkip) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= pixels * Cs) return;
-    int c = (int)(i % Cs);
-    long long p = i / Cs;
-    dSkip[i] = dOut[p * (Cl + Cs) + Cl + c];
+
+// The training head in one pass over the last activations d (32 channels):
+// the 1x1 output layer (pred[k] = b[k] + sum_c d[c] w[c][k], channels in
+// order as in outForwardKernel), the L1 loss against log1p of the target, the
+// output layer's gradients, and the gradient at the last 3x3 layer's
+// pre-activation (BF16, masked by d > 0) with that layer's bias gradient.
+// Two lanes per pixel, 16 channels each (32-byte loads); the sums stay in
+// registers over the pixels of a thread. It replaces five passes with one
+// global atomic per warp and sum (loss 83, output layer backward 705, mask 69,
+// bias 29, target 7 us at 32 x 128 x 128 pixels). Bound by its 73 MB of
+// traffic (11 us at copy bandwidth) and its ~460 instructions per 16 pixels.
+constexpr int kHeadHalf = 16;  // channels per lane
+__global__ void __launch_bounds__(128, 3) headKernel(const bf16* d, const float* target, int n, int h, int w,
+                                                     const int* batch, const unsigned char* flips, const float* wt,
+                                                     const float* b, bf16* dPre, float* loss, float* dW, float* dB,
+                                                     float* dBias) {
+    constexpr int C = 2 * kHeadHalf;
+    __shared__ float sW[C * kOutChannels];
+    __shared__ float scratch[8 * 2 * kHeadHalf * kOutChannels];
+    for (int i = threadIdx.x; i < C * kOutChannels; i += blockDim.x) sW[i] = wt[i];
+    __syncthreads();
+    const int half = threadIdx.x & 1;
+    const float* myW = sW + half * kHeadHalf * kOutChannels;
+    const long long total = (long long)n * h * w;
+    const float count = (float)(total * kOutChannels);
+    const float step = 1.0f / count;
+    float accW[kHeadHalf * kOutChannels] = {}, accBias[kHeadHalf] = {}, accB[kOutChannels + 1] = {};
+    const float bias[kOutChannels] = {b[0], b[1], b[2]};
+    // Whole warps walk the pixels (the channel sum passes between lanes).
+    for (long long base = (long long)blockIdx.x * (blockDim.x / 2); base < total;
+         base += (long long)gridDim.x * (blockDim.x / 2)) {
+        const long long p = base + (threadIdx.x >> 1);
+        const bool valid = p < total;
+        uint4 q[2] = {};
+        float t[kOutChannels] = {0.0f, 0.0f, 0.0f};
+        if (valid) {
+            const uint4* src = reinterpret_cast<const uint4*>(d + (size_t)p * C + half * kHeadHalf);
+            q[0] = __ldg(src);
+            q[1] = __ldg(src + 1);
+            const Pixel at = pixelOf(p, total, w, h);
+            int sx = at.x, sy = at.y;
+            if (flips) {
+                const unsigned char f = flips[at.n];
+                if (f & 1) sx = w - 1 - sx;
+                if (f & 2) sy = h - 1 - sy;
+            }
+            const float* tp = target + (((size_t)(batch ? batch[at.n] : at.n) * h + sy) * w + sx) * kOutChannels;
+            for (int k = 0; k < kOutChannels; k++) t[k] = log1pf(fmaxf(tp[k], 0.0f));
+        }
+        float x[kHeadHalf];
+        const bf16* e = reinterpret_cast<const bf16*>(q);
+#pragma unroll
+        for (int j = 0; j < kHeadHalf; j++) x[j] = __bfloat162float(e[j]);
+        // Channels 0-15 on the even lane, then 16-31 on the odd one.
+        float s[kOutChannels] = {bias[0], bias[1], bias[2]};
+#pragma unroll
+        for (int part = 0; part < 2; part++) {
+            if (part == 1)
+                for (int k = 0; k < kOutChannels; k++) s[k] = __shfl_xor_sync(0xFFFFFFFFu, s[k], 1);
+#pragma unroll
+            for (int j = 0; j < kHeadHalf; j++)
+#pragma unroll
+                for (int k = 0; k < kOutChannels; k++) s[k] += x[j] * myW[j * kOutChannels + k];
+        }
+        float g[kOutChannels];
+#pragma unroll
+        for (int k = 0; k < kOutChannels; k++) {
+            const float pred = __shfl_sync(0xFFFFFFFFu, s[k], (threadIdx.x & 31) | 1);
+            const float diff = pred - t[k];
+            g[k] = !valid ? 0.0f : diff > 0.0f ? step : (diff < 0.0f ? -step : 0.0f);
+            if (valid && half == 0) {
+                accB[k] += g[k];
+                accB[kOutChannels] += fabsf(diff);
+            }
+        }
+        uint4 o[2];
+        bf16* oe = reinterpret_cast<bf16*>(o);
+#pragma unroll
+        for (int j = 0; j < kHeadHalf; j++) {
+            float dd = 0.0f;
+#pragma unroll
+            for (int k = 0; k < kOutChannels; k++) {
+                accW[j * kOutChannels + k] += x[j] * g[k];
+                dd += g[k] * myW[j * kOutChannels + k];
+            }
+            oe[j] = __float2bfloat16(x[j] > 0.0f ? dd : 0.0f);
+            accBias[j] += __bfloat162float(oe[j]);
+        }
+        if (valid) {
+            uint4* dst = reinterpret_cast<uint4*>(dPre + (size_t)p * C + half * kHeadHalf);
+            dst[0] = o[0];
+            dst[1] = o[1];
+        }
+    }
+    accB[kOutChannels] /= count;
+    blockSums<kHeadHalf * kOutChannels, 2>(accW, scratch, dW);
+    blockSums<kHeadHalf, 2>(accBias, scratch, dBias);
+    float onlyB[kOutChannels] = {accB[0], accB[1], accB[2]}, onlyLoss[1] = {accB[kOutChannels]};
+    blockSums<kOutChannels, 1>(onlyB, scratch, dB);
+    blockSums<1, 1>(onlyLoss, scratch, loss);
 }
-__global__ void reluMaskKernel(const float* dY, const bf16* y, long long count, bf16* dPre) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    dPre[i] = __float2bfloat16(__bfloat162float(y[i]) > 0.0f ? dY[i] : 0.0f);
+
+// Gradient at a layer's pre-activation (BF16, masked by its output y > 0) and
+// its bias gradient, from the FP32 gradient of its output, which is
+//   KIND 0  dOut itself (C channels per pixel);
+//   KIND 1  the upsampled half of a decoder's input gradient: the sum of the
+//           2x2 pixels of dOut's first C channels (dOut: Cd channels, 2H x 2W);
+//   KIND 2  the skip half (channels Cd - C ... of dOut) plus a quarter of the
+//           pooled level's gradient dPool (H/2 x W/2 x C).
+// Eight channels per thread (32-byte FP32 loads, 16-byte BF16 ones); a
+// thread keeps its channels over its pixels, so the bias sums stay in
+// registers until the block's end. Bound by memory traffic: one pass over
+// dOut, y and dPre in place of one pass per operation with an element per
+// thread (32 x 128 x 128 x 32 channels: mask 69 + bias 29 us, pool backward
+// 102 and skip copy 57).
+template <int KIND>
+__global__ void __launch_bounds__(256) preGradKernel(const float* dOut, int Cd, const float* dPool, const bf16* y,
+                                                     int N, int H, int W, int C, bf16* dPre, float* db) {
+    extern __shared__ float sums[];  // [slots][C]
+    const int C8 = C / 8, slots = blockDim.x / C8;
+    const int cg = threadIdx.x % C8, slot = threadIdx.x / C8;
+    const long long total = (long long)N * H * W;
+    float acc[8] = {};
+    if (slot < slots) {
+        for (long long p = (long long)blockIdx.x * slots + slot; p < total; p += (long long)gridDim.x * slots) {
+            const uint4 yq = __ldg(reinterpret_cast<const uint4*>(y + (size_t)p * C) + cg);
+            float v[8];
+            auto load = [&](const float* src, float (&to)[8]) {
+                const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+                to[0] = a.x; to[1] = a.y; to[2] = a.z; to[3] = a.w;
+                to[4] = b.x; to[5] = b.y; to[6] = b.z; to[7] = b.w;
+            };
+            if (KIND == 0) {
+                load(dOut + (size_t)p * C + cg * 8, v);
+            } else {
+                const Pixel q = pixelOf(p, total, W, H);
+                if (KIND == 1) {
+                    const size_t row = (size_t)(2 * W) * Cd;
+                    const float* src = dOut + ((size_t)q.n * 2 * H + 2 * q.y) * row + (size_t)(2 * q.x) * Cd + cg * 8;
+                    float b[8], c[8], d[8];
+                    load(src, v); load(src + Cd, b); load(src + row, c); load(src + row + Cd, d);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] = v[j] + b[j] + c[j] + d[j];
+                } else {
+                    float b[8];
+                    load(dOut + (size_t)p * Cd + (Cd - C) + cg * 8, v);
+                    load(dPool + (((size_t)q.n * (H / 2) + q.y / 2) * (W / 2) + q.x / 2) * C + cg * 8, b);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] = v[j] + 0.25f * b[j];
+                }
+            }
+            const bf16* ye = reinterpret_cast<const bf16*>(&yq);
+            uint4 out;
+            bf16* oe = reinterpret_cast<bf16*>(&out);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                oe[j] = __float2bfloat16(__bfloat162float(ye[j]) > 0.0f ? v[j] : 0.0f);
+                acc[j] += __bfloat162float(oe[j]);
+            }
+            *(reinterpret_cast<uint4*>(dPre + (size_t)p * C) + cg) = out;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) sums[slot * C + cg * 8 + j] = acc[j];
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+        float s = 0.0f;
+        for (int k = 0; k < slots; k++) s += sums[k * C + c];
+        if (s != 0.0f) atomicAdd(&db[c], s);
+    }
 }
-__global__ void biasGradKernel(const bf16* dPre, long long pixels, int C, float* db) {
-    int c = threadIdx.x % C;
-    int lanesPerBlock = blockDim.x / C;
-    int slot = threadIdx.x / C;
-    if (slot >= lanesPerBlock) return;
-    float s = 0.0f;
-    for (long long p = (long long)blockIdx.x * lanesPerBlock + slot; p < pixels; p += (long long)gridDim.x * lanesPerBlock)
-        s += __bfloat162float(dPre[p * C + c]);
-    atomicAdd(&db[c], s);
-}
-// K-major copy for the forward convolution: wT[tap][co][ci] = w[tap][ci][co].
-__global__ void transposeKernel(const bf16* w, int Cin, int Cout, bf16* out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 9 * Cin * Cout) return;
-    int ci = i % Cin, co = (i / Cin) % Cout, tap = i / (Cin * Cout);
-    out[i] = w[((size_t)tap * Cin + ci) * Cout + co];
-}
-__global__ void toBf16Kernel(const float* in, size_t count, bf16* out) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) out[i] = __float2bfloat16(in[i]);
+template <int KIND>
+cudaError_t launchPreGrad(const float* dOut, int Cd, const float* dPool, const bf16* y, int N, int H, int W, int C,
+                          bf16* dPre, float* db, cudaStream_t s) {
+    const int slots = 256 / (C / 8);
+    const long long blocks = ((long long)N * H * W + slots - 1) / slots;
+    preGradKernel<KIND><<<(int)std::min<long long>(blocks, 148 * 8), 256, sizeof(float) * slots * C, s>>>(
+        dOut, Cd, dPool, y, N, H, W, C, dPre, db);
+    return cudaGetLastError();
 }
 // 1x1 output layer, forward: pred[p][k] = b[k] + sum_c d[p][c] w[c][k].
 __global__ void outForwardKernel(const bf16* d, long long pixels, int C, const float* w, const float* b, float* pred) {
@@ -244,50 +395,51 @@ __global__ void outForwardKernel(const bf16* d, long long pixels, int C, const f
     }
     for (int k = 0; k < kOutChannels; k++) pred[p * kOutChannels + k] = s[k];
 }
-// L1 loss in log space: loss += |pred - t| / count; dPred = sign / count.
-__global__ void lossKernel(const float* pred, const float* t, long long count, float* dPred, float* loss) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (i < count) {
-        float d = pred[i] - t[i];
-        l = fabsf(d);
-        dPred[i] = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f)) / (float)count;
-    }
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (float)count);
-}
-// 1x1 output layer, backward.
-__global__ void outBackwardKernel(const bf16* d, const float* dPred, long long pixels, int C, const float* w,
-                                  float* dW, float* dB, float* dD) {
-    long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float g[kOutChannels] = {0, 0, 0};
-    if (p < pixels)
-        for (int k = 0; k < kOutChannels; k++) g[k] = dPred[p * kOutChannels + k];
-    for (int k = 0; k < kOutChannels; k++) {
-        float v = g[k];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-        if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(&dB[k], v);
-    }
-    for (int c = 0; c < C; c++) {
-        float x = p < pixels ? __bfloat162float(d[p * C + c]) : 0.0f;
-        float dd = 0.0f;
-        for (int k = 0; k < kOutChannels; k++) {
-            float v = x * g[k];
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-            if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(&dW[c * kOutChannels + k], v);
-            dd += g[k] * w[c * kOutChannels + k];
+// The parameters' BF16 copies, after an Adam step when ADAM: wbf in the flat
+// layout, wT K-major per 3x3 layer (wT[tap][co][ci] = w[tap][ci][co]). A block
+// owns 16 input channels of one tap of one layer (16 * cout consecutive
+// parameters, transposed through shared memory into 32-byte runs of wT), or a
+// layer's bias, or the output layer. One launch of ~830 blocks replaces Adam,
+// the conversion and 18 transposes (73 us, launch-bound).
+struct WeightTable {
+    int blocks[19];               // first block of each layer's entries (taps x cin / 16, then its bias)
+    int cin[19], cout[19];
+    unsigned wOffset[19], bOffset[19];
+    int total;                    // blocks in all
+};
+template <bool ADAM>
+__global__ void __launch_bounds__(128) weightsKernel(const WeightTable T, float* p, const float* g, float* m, float* v,
+                                                     float lr, float b1, float b2, float eps, float c1, float c2,
+                                                     bf16* wbf, bf16* wT) {
+    __shared__ bf16 tile[16 * 129];  // [ci][co], padded against bank conflicts
+    int l = 0;
+    while (l < 18 && (int)blockIdx.x >= T.blocks[l + 1]) l++;
+    const int cin = T.cin[l], cout = T.cout[l], part = (int)blockIdx.x - T.blocks[l];
+    const int groups = l < 18 ? 9 * (cin / 16) : 0;
+    const bool transposed = part < groups;
+    const size_t first = transposed ? T.wOffset[l] + (size_t)part * 16 * cout : l < 18 ? T.bOffset[l] : T.wOffset[l];
+    const int count = transposed ? 16 * cout : l < 18 ? cout : cin * cout + cout;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        const size_t k = first + i;
+        float x = p[k];
+        if (ADAM) {
+            const float gi = g[k];
+            const float mi = b1 * m[k] + (1.0f - b1) * gi, vi = b2 * v[k] + (1.0f - b2) * gi * gi;
+            m[k] = mi;
+            v[k] = vi;
+            x -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+            p[k] = x;
         }
-        if (p < pixels) dD[p * C + c] = dd;
+        const bf16 h = __float2bfloat16(x);
+        wbf[k] = h;
+        if (transposed) tile[i / cout * 129 + i % cout] = h;
     }
-}
-__global__ void adamKernel(float* p, const float* g, float* m, float* v, size_t count, float lr, float b1, float b2,
-                           float eps, float c1, float c2) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi; v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    if (!transposed) return;
+    __syncthreads();
+    const int tap = part / (cin / 16), ci0 = part % (cin / 16) * 16;
+    bf16* out = wT + T.wOffset[l] + (size_t)tap * cin * cout + ci0;
+    for (int i = threadIdx.x; i < 16 * cout; i += blockDim.x)
+        out[(size_t)(i / 16) * cin + i % 16] = tile[i % 16 * 129 + i / 16];
 }
 // Network output (log space, padded frame) to linear radiance (w x h x 3).
 // Network input straight from the running sums: the AOVs of RtxReadAovs
@@ -392,12 +544,10 @@ struct Unet::Activations {
     bf16* upWeights[4] = {};
     bf16* skipWeights[4] = {};
     float* pred = nullptr;   // network output, log space
-    float* target = nullptr; // log-space target
-    float* dPred = nullptr;
-    float* dAct[18] = {};    // fp32 gradients of layer outputs
-    float* dCat[4] = {};
-    float* dPool[4] = {};
-    bf16* dPre = nullptr;    // scratch: gradient at the pre-activation, bf16
+    float* dAct[18] = {};    // fp32 gradients of the outputs of each level's first layers (even k)
+    float* dCat[4] = {};     // of the decoders' inputs
+    float* dPool[4] = {};    // of the pooled inputs
+    bf16* dPre = nullptr;    // gradient at the current layer's pre-activation, bf16
     float* loss = nullptr;
     int* batch = nullptr;
     unsigned char* flips = nullptr;
@@ -483,12 +633,26 @@ Unet::~Unet() {
     if (stream_) cudaStreamDestroy(stream_);
 }
 
-cudaError_t Unet::syncWeights(cudaStream_t s) {
-    toBf16Kernel<<<blocksFor((long long)params_, 256), 256, 0, s>>>(master_, params_, wbf_);
-    for (size_t l = 0; l + 1 < layers_.size(); l++) {
-        const UnetLayer& L = layers_[l];
-        transposeKernel<<<blocksFor(9LL * L.cin * L.cout, 256), 256, 0, s>>>(wbf_ + L.wOffset, L.cin, L.cout, wT_ + L.wOffset);
+namespace {
+WeightTable weightTable(const std::vector<UnetLayer>& layers) {
+    WeightTable T{};
+    int blocks = 0;
+    for (size_t l = 0; l < layers.size(); l++) {
+        const UnetLayer& L = layers[l];
+        T.blocks[l] = blocks;
+        T.cin[l] = L.cin; T.cout[l] = L.cout;
+        T.wOffset[l] = (unsigned)L.wOffset; T.bOffset[l] = (unsigned)L.bOffset;
+        blocks += l + 1 < layers.size() ? 9 * (L.cin / 16) + 1 : 1;
     }
+    T.total = blocks;
+    return T;
+}
+}  // namespace
+
+cudaError_t Unet::syncWeights(cudaStream_t s) {
+    const WeightTable T = weightTable(layers_);
+    weightsKernel<false><<<T.total, 128, 0, s>>>(T, master_, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f,
+                                                 1.0f, wbf_, wT_);
     return cudaGetLastError();
 }
 
@@ -529,7 +693,7 @@ cudaError_t Unet::ensure(int n, int h, int w, bool training) {
     for (int k = 0; k < 18; k++) {
         int level = k < 10 ? k / 2 : 3 - (k - 10) / 2;
         if ((e = A.make(A.a[k], px(level) * layers_[k].cout)) != cudaSuccess) return e;
-        if (training && (e = A.make(A.dAct[k], px(level) * layers_[k].cout)) != cudaSuccess) return e;
+        if (training && k % 2 == 0 && (e = A.make(A.dAct[k], px(level) * layers_[k].cout)) != cudaSuccess) return e;
     }
     for (int l = 1; l <= 4; l++) {
         if ((e = A.make(A.pool[l - 1], px(l) * kWidths[l - 1])) != cudaSuccess) return e;
@@ -551,8 +715,6 @@ cudaError_t Unet::ensure(int n, int h, int w, bool training) {
     if (upHalf && (e = A.make(A.upHalf, upHalf)) != cudaSuccess) return e;
     if ((e = A.make(A.pred, px(0) * kOutChannels)) != cudaSuccess) return e;
     if (training) {
-        if ((e = A.make(A.target, px(0) * kOutChannels)) != cudaSuccess) return e;
-        if ((e = A.make(A.dPred, px(0) * kOutChannels)) != cudaSuccess) return e;
         if ((e = A.make(A.dPre, px(0) * 128)) != cudaSuccess) return e;
         if ((e = A.make(A.loss, 1)) != cudaSuccess) return e;
         if ((e = A.make(A.batch, n)) != cudaSuccess) return e;
@@ -590,7 +752,7 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
             const UnetLayer& L = layers_[k];
             if (r == 0 && training) {
                 // The weight gradient reads the concatenated input: keep it.
-                upConcatKernel<<<blocksFor((long long)n * H * W * (Cl + Cs), 256), 256, 0, s>>>(low, Cl, skip, Cs, n, H, W, A.cat[j]);
+                upConcatKernel<<<blocksFor((long long)n * H * W * ((Cl + Cs) / 8), 256), 256, 0, s>>>(low, Cl, skip, Cs, n, H, W, A.cat[j]);
                 e = convTc(A.cat[j], nullptr, 0, n, H, W, L.cin, wT_ + L.wOffset, false, master_ + L.bOffset, L.cout, A.a[k], nullptr, true, false, convError_, s);
             } else if (r == 0 && A.upWeights[j] && convPath() == 0) {
                 // Inference, two passes: the upsampled half at half
@@ -626,57 +788,50 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
     return cudaGetLastError();
 }
 
-cudaError_t Unet::backward(cudaStream_t s) {
+cudaError_t Unet::lossAndBackward(const float* targets, const int* batch, const unsigned char* flips, float* loss,
+                                  cudaStream_t s) {
     Activations& A = *act_;
     const int n = A.n;
     cudaError_t e;
-    cudaMemsetAsync(grad_, 0, sizeof(float) * params_, s);
+    if ((e = cudaMemsetAsync(grad_, 0, sizeof(float) * params_, s)) != cudaSuccess) return e;
     const UnetLayer& O = layers_[18];
-    long long pixels0 = (long long)n * A.H * A.W;
-    outBackwardKernel<<<blocksFor(pixels0, 128), 128, 0, s>>>(A.a[17], A.dPred, pixels0, O.cin, master_ + O.wOffset,
-                                                             grad_ + O.wOffset, grad_ + O.bOffset, A.dAct[17]);
-    // Backward through one 3x3 layer k whose output gradient is dAct[k];
-    // writes the input gradient to dIn (fp32) unless dIn is null.
-    auto layerBack = [&](int k, const bf16* input, int H, int W, float* dIn, bool accumulate) -> cudaError_t {
+    const long long pixels0 = (long long)n * A.H * A.W;
+    headKernel<<<(int)std::min<long long>(blocksFor(pixels0, 64), 148 * 3), 128, 0, s>>>(
+        A.a[17], targets, n, A.H, A.W, batch, flips, master_ + O.wOffset, master_ + O.bOffset, A.dPre, loss,
+        grad_ + O.wOffset, grad_ + O.bOffset, grad_ + layers_[17].bOffset);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // Layer k from the gradient at its pre-activation (A.dPre): its weight
+    // gradient, and its input's gradient into dIn (fp32) unless dIn is null.
+    auto layerBack = [&](int k, const bf16* input, int H, int W, float* dIn) -> cudaError_t {
         const UnetLayer& L = layers_[k];
-        long long count = (long long)n * H * W * L.cout;
-        reluMaskKernel<<<blocksFor(count, 256), 256, 0, s>>>(A.dAct[k], A.a[k], count, A.dPre);
-        int per = std::max(1, 256 / L.cout);
-        biasGradKernel<<<std::min<long long>(1024, blocksFor((long long)n * H * W, per)), per * L.cout, 0, s>>>(
-            A.dPre, (long long)n * H * W, L.cout, grad_ + L.bOffset);
         cudaError_t err = wgrad(input, A.dPre, n, H, W, L.cin, L.cout, grad_ + L.wOffset, convError_, s);
-        if (err != cudaSuccess) return err;
-        if (dIn) return convTc(A.dPre, nullptr, 0, n, H, W, L.cout, wbf_ + L.wOffset, true, nullptr, L.cin, nullptr, dIn, false, accumulate, convError_, s);
-        return cudaSuccess;
+        if (err != cudaSuccess || !dIn) return err;
+        return convTc(A.dPre, nullptr, 0, n, H, W, L.cout, wbf_ + L.wOffset, true, nullptr, L.cin, nullptr, dIn, false, false, convError_, s);
+    };
+    // The second, then the first 3x3 layer of a level (k and k - 1).
+    auto levelBack = [&](int k, const bf16* input, int H, int W, float* dIn) -> cudaError_t {
+        cudaError_t err = layerBack(k, A.a[k - 1], H, W, A.dAct[k - 1]);
+        if (err == cudaSuccess)
+            err = launchPreGrad<0>(A.dAct[k - 1], 0, nullptr, A.a[k - 1], n, H, W, layers_[k - 1].cout, A.dPre,
+                                   grad_ + layers_[k - 1].bOffset, s);
+        return err == cudaSuccess ? layerBack(k - 1, input, H, W, dIn) : err;
     };
     int k = 17;
     for (int j = 3; j >= 0; j--) {  // decoder level 3 - j, from the top (level 0) down
         int level = 3 - j, H = A.H >> level, W = A.W >> level;
-        if ((e = layerBack(k, A.a[k - 1], H, W, A.dAct[k - 1], false)) != cudaSuccess) return e;
-        k--;
-        if ((e = layerBack(k, A.cat[j], H, W, A.dCat[j], false)) != cudaSuccess) return e;
-        k--;
-        int Cl = layers_[k].cout, Cs = kWidths[level];  // layers_[k]: the layer below (its output was upsampled)
-        upConcatBackwardLowKernel<<<blocksFor((long long)n * (H / 2) * (W / 2) * Cl, 256), 256, 0, s>>>(
-            A.dCat[j], Cl, Cs, n, H, W, A.dAct[k]);
-        // skip gradient into the encoder output of this level (dAct[2*level+1]) — set here, pooled part added below
-        upConcatBackwardSkipKernel<<<blocksFor((long long)n * H * W * Cs, 256), 256, 0, s>>>(
-            A.dCat[j], Cl, Cs, (long long)n * H * W, A.dAct[2 * level + 1]);
+        if ((e = levelBack(k, A.cat[j], H, W, A.dCat[j])) != cudaSuccess) return e;
+        k -= 2;  // the layer below, whose output was upsampled; the skip half waits in dCat for the encoder
+        if ((e = launchPreGrad<1>(A.dCat[j], layers_[k + 1].cin, nullptr, A.a[k], n, H / 2, W / 2, layers_[k].cout, A.dPre,
+                                  grad_ + layers_[k].bOffset, s)) != cudaSuccess) return e;
     }
     // Bottleneck and encoder: k = 9 down to 0.
-    for (int l = 4; l >= 0; l--) {
+    for (int l = 4; l >= 0; l--, k -= 2) {
         int H = A.H >> l, W = A.W >> l;
-        const bf16* in1 = l == 0 ? A.x0 : A.pool[l - 1];
-        // second conv of level l: input a[2l], output a[2l+1]
-        if ((e = layerBack(2 * l + 1, A.a[2 * l], H, W, A.dAct[2 * l], false)) != cudaSuccess) return e;
-        // first conv of level l: input in1
-        if ((e = layerBack(2 * l, in1, H, W, l == 0 ? nullptr : A.dPool[l - 1], false)) != cudaSuccess) return e;
-        if (l > 0) {
-            int C = kWidths[l - 1];
-            // encoder output of level l-1 receives the pooled gradient plus its skip gradient
-            poolBackwardKernel<<<blocksFor((long long)n * H * 2 * W * 2 * C, 256), 256, 0, s>>>(
-                A.dPool[l - 1], n, H * 2, W * 2, C, A.dAct[2 * (l - 1) + 1], 1);
-        }
+        if ((e = levelBack(k, l == 0 ? A.x0 : A.pool[l - 1], H, W, l == 0 ? nullptr : A.dPool[l - 1])) != cudaSuccess) return e;
+        // The encoder output of level l - 1 receives the pooled gradient and its skip gradient.
+        if (l > 0 && (e = launchPreGrad<2>(A.dCat[4 - l], layers_[10 + 2 * (4 - l)].cin, A.dPool[l - 1], A.a[k - 2], n, H * 2,
+                                           W * 2, kWidths[l - 1], A.dPre, grad_ + layers_[k - 2].bOffset, s)) != cudaSuccess)
+            return e;
     }
     return cudaGetLastError();
 }
@@ -694,12 +849,8 @@ cudaError_t Unet::lossAndGradient(const float* aovs, const float* targets, int n
     cudaMemcpyAsync(dA, aovs, sizeof(float) * px * kInputChannels, cudaMemcpyHostToDevice, stream_);
     cudaMemcpyAsync(dT, targets, sizeof(float) * px * 3, cudaMemcpyHostToDevice, stream_);
     inputKernel<<<blocksFor((long long)px, 256), 256, 0, stream_>>>(dA, n, h, w, A.H, A.W, A.x0, nullptr, nullptr);
-    targetKernel<<<blocksFor((long long)px, 256), 256, 0, stream_>>>(dT, n, h, w, A.target, nullptr, nullptr);
     cudaMemsetAsync(A.loss, 0, sizeof(float), stream_);
-    if ((e = forward(stream_, true)) == cudaSuccess) {
-        lossKernel<<<blocksFor((long long)px * 3, 256), 256, 0, stream_>>>(A.pred, A.target, (long long)px * 3, A.dPred, A.loss);
-        e = backward(stream_);
-    }
+    if ((e = forward(stream_, true, false)) == cudaSuccess) e = lossAndBackward(dT, nullptr, nullptr, A.loss, stream_);
     if (e == cudaSuccess) e = cudaMemcpyAsync(loss, A.loss, sizeof(float), cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess && grads) e = cudaMemcpyAsync(grads, grad_, sizeof(float) * params_, cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
@@ -729,20 +880,20 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     if ((e = cudaMalloc(&dLosses, sizeof(float) * std::max(steps, 1))) != cudaSuccess) { cudaFree(dA); cudaFree(dT); return e; }
     cudaMemsetAsync(dLosses, 0, sizeof(float) * std::max(steps, 1), stream_);
     const size_t bpx = (size_t)batch * h * w;
+    const WeightTable table = weightTable(layers_);
     for (int step = 0; step < steps && e == cudaSuccess; step++) {
         for (int b = 0; b < batch; b++) { idx[b] = (int)(rng() % (unsigned)count); flips[b] = (unsigned char)(rng() & 3u); }
         cudaMemcpyAsync(A.batch, idx.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, stream_);
         cudaMemcpyAsync(A.flips, flips.data(), batch, cudaMemcpyHostToDevice, stream_);
         inputKernel<<<blocksFor((long long)bpx, 256), 256, 0, stream_>>>(dA, batch, h, w, A.H, A.W, A.x0, A.batch, A.flips);
-        targetKernel<<<blocksFor((long long)bpx, 256), 256, 0, stream_>>>(dT, batch, h, w, A.target, A.batch, A.flips);
-        if ((e = forward(stream_, true)) != cudaSuccess) break;
-        lossKernel<<<blocksFor((long long)bpx * 3, 256), 256, 0, stream_>>>(A.pred, A.target, (long long)bpx * 3, A.dPred, dLosses + step);
-        if ((e = backward(stream_)) != cudaSuccess) break;
+        if ((e = forward(stream_, true, false)) != cudaSuccess) break;
+        if ((e = lossAndBackward(dT, A.batch, A.flips, dLosses + step, stream_)) != cudaSuccess) break;
         adamStep_++;
         const float b1 = 0.9f, b2 = 0.999f;
         float c1 = 1.0f - std::pow(b1, (float)adamStep_), c2 = 1.0f - std::pow(b2, (float)adamStep_);
-        adamKernel<<<blocksFor((long long)params_, 256), 256, 0, stream_>>>(master_, grad_, adamM_, adamV_, params_, lr, b1, b2, 1e-8f, c1, c2);
-        if ((e = syncWeights(stream_)) != cudaSuccess) break;
+        weightsKernel<true><<<table.total, 128, 0, stream_>>>(table, master_, grad_, adamM_, adamV_, lr, b1, b2, 1e-8f, c1,
+                                                              c2, wbf_, wT_);
+        if ((e = cudaGetLastError()) != cudaSuccess) break;
         // The tiny host copies above wait for the stream; keep them ordered.
         if ((step & 63) == 63) e = cudaStreamSynchronize(stream_);
     }

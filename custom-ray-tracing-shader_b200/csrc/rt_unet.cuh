@@ -69,7 +69,11 @@ private:
     // *headDone tells whether it was (else A.a[17] holds that layer's output).
     cudaError_t forward(cudaStream_t stream, bool training, bool outputLayer = true, const ConvHead* head = nullptr,
                         bool* headDone = nullptr);
-    cudaError_t backward(cudaStream_t stream);
+    // Loss and gradients after a training forward pass: targets (linear
+    // radiance) of crops batch[i] flipped by flips[i] (null: crop i as it is);
+    // the loss is added to *loss.
+    cudaError_t lossAndBackward(const float* targets, const int* batch, const unsigned char* flips, float* loss,
+                                cudaStream_t stream);
     cudaError_t syncWeights(cudaStream_t stream);
 
     std::vector<UnetLayer> layers_;

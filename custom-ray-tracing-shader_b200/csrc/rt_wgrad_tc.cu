@@ -2,26 +2,35 @@
 // tensor cores: dw[tap][ci][co] += sum over pixels p of
 // x[p + off(tap)][ci] * dy[p][co], with x and dy NHWC BF16 and dw FP32.
 //
-// Per tap this is a GEMM whose K is the pixels. Both operands are staged by
-// TMA as planes of 8 channels x pixels x 16 bytes (one image row segment of
-// 128 output pixels per stage: x with a one-pixel halo, dy without), which
-// is the MN-major no-swizzle operand layout: core matrices of 8 pixels (K)
-// x 8 channels (M or N), K groups 128 bytes apart (LBO), channel groups one
-// plane apart (SBO). The horizontal tap offset is a 16-byte shift of x's
-// start address, so a block handles one tap row dy and keeps the three dx
-// taps in three tensor-memory accumulators over its whole range of row
-// segments (split K), then adds them to dw with FP32 atomics.
+// Per tap this is a GEMM whose K is the pixels. An image row segment of up
+// to 128 pixels is staged by TMA as slabs of 16, 32 or 64 channels (the
+// widest dividing the channel count) with the 32-, 64- or 128-byte swizzle:
+// pixel rows of 2 x width bytes, which is the MN-major swizzled operand
+// layout (K groups of 8 pixels 16 x width bytes apart, SBO; channel groups a
+// slab apart, LBO). The column tap dx is a shift of x's start address by
+// pixel rows.
 //
-// M is 128 rows of one operand and N the channels of the other: M = input
-// channels (a block of 128 of them) when cin >= cout, else M = output
-// channels; the smaller channel count is N, so the padding of M to 128 rows
-// costs the least. Rows beyond the real channels read stale staging planes
-// and are dropped (a row of D depends on its row of A only).
+// The three row taps are stacked along M: the slabs of x's rows y - 1, y and
+// y + 1 follow each other in shared memory, so M runs over (dy, ci) in blocks
+// of 128 rows, N over the output channels, and one pass over a dY row feeds
+// all nine taps: ceil(3 cin / 128) blocks x 3 column taps of accumulators in
+// tensor memory. (One block per row tap, each padding its cin rows to M =
+// 128 and staging x and dY again as planes of 8 channels, took 125 us for
+// 32 -> 32 channels at 32 x 128 x 128 pixels; this form 31 us. Its floors:
+// 67 MB of operands, 10 us; 4096 rows x 24 MMAs of ~42 cycles, 15 us.)
+// Where the accumulators pass 512 columns, blocks of the grid take slices of
+// the M blocks. Split K over the blocks; each adds its accumulators to dw
+// with 16-byte FP32 reductions at the end. Rows of the last M block beyond 3 cin
+// read the next staged row and are dropped (a row of D depends on its row of
+// A only).
 //
-// Roles: warp 0 issues the TMA loads into a ring of stages, warp 1 issues
-// the MMAs (24 per stage: 3 dx taps x 8 K steps of 16 pixels) and owns the
-// tensor memory, warps 2-5 drain the accumulators at the end. Waits are
-// bounded as in rt_conv_pipe.cu.
+// Segments are as wide as the image rounded up to 16 pixels (at most 128), so the narrow
+// deep levels do no work for padding; a stage holds `rows` dY rows and
+// rows + 2 x rows.
+//
+// Roles: warp 0 issues the TMA loads into two or more stages, warp 1 issues
+// the MMAs and owns the tensor memory, warps 2-5 drain the accumulators at
+// the end. Waits are bounded as in rt_conv_pipe.cu.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -38,24 +47,30 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kM = 128;                 // pixels per row segment (K per stage)
-constexpr int kHaloPx = kM + 2;
-constexpr uint32_t kXPlane = 2176;      // 130 pixels x 16 bytes, padded to 128 bytes
-constexpr uint32_t kDPlane = kM * 16;   // 2,048
+constexpr int kM = 128;                 // rows of an M block, and the most pixels per row segment
 constexpr int kThreads = 192;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 4;
+constexpr int kMaxRows = 8;             // dY rows per stage
 constexpr uint32_t kHeader = 1024;
+constexpr uint32_t kSmemMax = 227u * 1024u;
+
+// Bytes of a staged row slab of `s` channels x px pixels, on a boundary of
+// the swizzle pattern (8 pixel rows).
+__host__ __device__ constexpr uint32_t slabBytes(int px, int s) {
+    return ((uint32_t)px * 2u * (uint32_t)s + 16u * (uint32_t)s - 1u) & ~(16u * (uint32_t)s - 1u);
+}
+inline int slabChannels(int c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
 
 struct WgradArgs {
-    int n, h, w, cin, cout;
-    int tilesPerRow, segments, segPerBlock;
-    int mIsX;            // 1: M = input channels (from mBase), N = output channels; 0: M = output, N = input
-    int mBase;           // first input channel of the M block (M = input channels)
-    int mValid, nDim;
-    int xPlanes, dPlanes;          // planes loaded per stage
-    uint32_t xBytes, stageBytes;   // staging of x (16 or xPlanes planes) and of a whole stage
+    int h, w, cin, cout;
+    int px;                        // pixels per segment (K per row): 16..128, a multiple of 16
+    int tilesPerRow, strips, units, rows;
+    int xSlabs, dSlabs;            // slabs per row
+    uint32_t xSlab, dSlab;         // bytes of one
+    uint32_t xBytes, stageBytes;   // x part of a stage, and the whole stage
     int stages;
-    uint32_t accCols, tmemCols;
+    int blocksPerSlice, mBlocks;   // M blocks of 128 rows per grid slice, and in all
+    uint32_t tmemCols;
     float* dw;
     int* errorFlag;
     unsigned long long waitLimitNs;
@@ -148,7 +163,51 @@ __device__ __forceinline__ void tmemLoad16(uint32_t taddr, uint32_t (&r)[16]) {
 __host__ __device__ constexpr uint32_t idescMnMajor(int m, int n) {
     return ummaInstrDescBf16(m, n) | (1u << 15) | (1u << 16);
 }
+// MN-major swizzled operand descriptor of slabs of S channels, `slab` bytes
+// apart (layout type in bits 61-63: 6 = 32-byte, 4 = 64-byte, 2 = 128-byte).
+template <int S>
+__device__ __forceinline__ uint64_t slabDescriptor(uint32_t addr, uint32_t slab) {
+    return ummaSmemDesc(addr, slab, 16u * S) | ((uint64_t)(S == 16 ? 6 : S == 32 ? 4 : 2) << 61);
+}
 
+// The MMAs of one dY row and one M block: 3 column taps x KK steps of 16
+// pixels, descriptors as compile-time offsets from two bases (one thread
+// issues; computing descriptors per MMA is several times slower than the
+// tensor pipe).
+template <int SX, int SD, int KK>
+__device__ __forceinline__ void issueRow(uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
+                                         uint32_t first) {
+#pragma unroll
+    for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+        for (int kk = 0; kk < KK; kk++)
+            mma(acc + (uint32_t)dx * accStep, x + (uint64_t)(dx * (SX / 8) + kk * 2 * SX), d + (uint64_t)(kk * 2 * SD),
+                idesc, (first || kk > 0) ? 1u : 0u);
+}
+template <int SX, int SD>
+__device__ __forceinline__ void issueRowK(int kk, uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
+                                          uint32_t first) {
+    switch (kk) {
+        case 1: issueRow<SX, SD, 1>(acc, accStep, x, d, idesc, first); break;
+        case 2: issueRow<SX, SD, 2>(acc, accStep, x, d, idesc, first); break;
+        case 3: issueRow<SX, SD, 3>(acc, accStep, x, d, idesc, first); break;
+        case 4: issueRow<SX, SD, 4>(acc, accStep, x, d, idesc, first); break;
+        case 5: issueRow<SX, SD, 5>(acc, accStep, x, d, idesc, first); break;
+        case 6: issueRow<SX, SD, 6>(acc, accStep, x, d, idesc, first); break;
+        case 7: issueRow<SX, SD, 7>(acc, accStep, x, d, idesc, first); break;
+        default: issueRow<SX, SD, 8>(acc, accStep, x, d, idesc, first); break;
+    }
+}
+
+// Unit u: image, first pixel and first row, and its dY rows.
+struct Unit { int img, x0, y0, rows; };
+__device__ __forceinline__ Unit unitOf(const WgradArgs& a, int u) {
+    const int strip = u % a.strips, xt = (u / a.strips) % a.tilesPerRow, img = u / (a.strips * a.tilesPerRow);
+    const int y0 = strip * a.rows;
+    return Unit{img, xt * a.px, y0, min(a.rows, a.h - y0)};
+}
+
+template <int SX, int SD>
 __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant__ CUtensorMap xMap,
                                                          const __grid_constant__ CUtensorMap dMap, WgradArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -157,11 +216,14 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
     volatile int* abortFlag = reinterpret_cast<volatile int*>(smem + Header::abort);
     const uint32_t stage0 = base + kHeader;
     const int S = a.stages;
-    const int dy = blockIdx.y;
-    const int mBase = a.mBase;
-    const long long seg0 = (long long)blockIdx.x * a.segPerBlock;
-    const long long seg1 = seg0 + a.segPerBlock < a.segments ? seg0 + a.segPerBlock : (long long)a.segments;
     const uint64_t limit = a.waitLimitNs;
+    if (base & 1023u) {  // swizzled slabs need an aligned base: report, touch nothing
+        if (threadIdx.x == 0) atomicExch(a.errorFlag, 1);
+        return;
+    }
+    // This block's M blocks, and the slabs of the stacked rows they cover.
+    const int b0 = (int)blockIdx.y * a.blocksPerSlice, b1 = min(a.mBlocks, b0 + a.blocksPerSlice);
+    const int slab0 = b0 * (kM / SX), slab1 = min(b1 * (kM / SX), 3 * a.xSlabs);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
@@ -185,24 +247,38 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + Header::tmemSlot);
 
     if (warp == 0) {
-        // ---- producer: one stage per row segment ----
-        long long k = 0;
+        // ---- producer: one stage per unit ----
+        int k = 0;
         bool ok = true;
-        for (long long s = seg0; s < seg1; s++, k++) {
-            const int st = (int)(k % S);
+        for (int u = (int)blockIdx.x; u < a.units; u += (int)gridDim.x, k++) {
+            const int st = k % S;
             if (!waitPhaseWarp(base + Header::empty + 8 * st, (uint32_t)(((k / S) & 1) ^ 1), abortFlag, limit)) { ok = false; break; }
             if (lane == 0) {
-                const int xt = (int)(s % a.tilesPerRow);
-                const long long row = s / a.tilesPerRow;
-                const int y = (int)(row % a.h), img = (int)(row / a.h), x0 = xt * kM;
+                const Unit U = unitOf(a, u);
                 const uint32_t fb = base + Header::full + 8 * st;
                 const uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
-                barExpectTx(fb, (uint32_t)a.xPlanes * kHaloPx * 16u + (uint32_t)a.dPlanes * kDPlane);
-                const int xc0 = a.mIsX ? mBase : 0;
-                for (int g = 0; g < a.xPlanes; g++)
-                    tmaLoad4(xs + (uint32_t)g * kXPlane, &xMap, xc0 + g * 8, x0 - 1, y + dy - 1, img, fb);
-                for (int g = 0; g < a.dPlanes; g++)
-                    tmaLoad4(ds + (uint32_t)g * kDPlane, &dMap, g * 8, x0, y, img, fb);
+                // Staged row j (image row y0 - 1 + j) slab c is slab (j - r) xSlabs
+                // + c of dY row r's stack: loaded when some r's M blocks cover it.
+                auto needed = [&](int j, int c) {
+                    const int rLo = max(0, j - 2), rHi = min(U.rows - 1, j);
+                    for (int r = rLo; r <= rHi; r++) {
+                        const int q = (j - r) * a.xSlabs + c;
+                        if (q >= slab0 && q < slab1) return true;
+                    }
+                    return false;
+                };
+                uint32_t boxes = 0;
+                for (int j = 0; j < U.rows + 2; j++)
+                    for (int c = 0; c < a.xSlabs; c++) boxes += needed(j, c) ? 1u : 0u;
+                barExpectTx(fb, boxes * (uint32_t)(a.px + 2) * 2u * SX + (uint32_t)(U.rows * a.dSlabs * a.px) * 2u * SD);
+                for (int r = 0; r < U.rows; r++)
+                    for (int c = 0; c < a.dSlabs; c++)
+                        tmaLoad4(ds + (uint32_t)(r * a.dSlabs + c) * a.dSlab, &dMap, c * SD, U.x0, U.y0 + r, U.img, fb);
+                for (int j = 0; j < U.rows + 2; j++)
+                    for (int c = 0; c < a.xSlabs; c++)
+                        if (needed(j, c))
+                            tmaLoad4(xs + (uint32_t)(j * a.xSlabs + c) * a.xSlab, &xMap, c * SX, U.x0 - 1, U.y0 - 1 + j,
+                                     U.img, fb);
             }
             __syncwarp();
         }
@@ -210,44 +286,32 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         // Every issued load lands before the block exits (latest phase of
         // each of the last S stages).
         if (lane == 0)
-            for (long long e = k > S ? k - S : 0; e < k; e++)
-                pollPhase(base + Header::full + 8 * (int)(e % S), (uint32_t)((e / S) & 1), limit);
+            for (int e = k > S ? k - S : 0; e < k; e++)
+                pollPhase(base + Header::full + 8 * (e % S), (uint32_t)((e / S) & 1), limit);
         __syncwarp();
     } else if (warp == 1) {
         // ---- MMA issuer ----
         if (lane == 0) {
             bool ok = true;
-            const uint32_t idesc = idescMnMajor(kM, a.nDim);
-            // Stage and phase as running counters; descriptors as compile-
-            // time offsets from two per-stage bases (a single issuing
-            // thread that computes descriptors per MMA issues several
-            // times slower than the tensor pipe runs).
-            long long k = 0;
-            int st = 0;
-            uint32_t parity = 0;
-            for (long long s = seg0; s < seg1 && ok; s++, k++) {
+            const uint32_t idesc = idescMnMajor(kM, a.cout);
+            const uint32_t cols = (uint32_t)a.cout;
+            int k = 0, st = 0;
+            uint32_t parity = 0, started = 0;
+            for (int u = (int)blockIdx.x; u < a.units && ok; u += (int)gridDim.x, k++) {
                 ok = waitPhase(base + Header::full + 8 * st, parity, abortFlag, limit);
                 if (!ok) break;
                 tcFenceAfter();
-                const uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
-                // 16 pixels per MMA: 2 core-matrix groups of 8 along K (LBO = 128 bytes),
-                // next 16 pixels 256 bytes on; tap dx one pixel (16 bytes) on.
-                const uint64_t xBase = ummaSmemDesc(xs, 128u, kXPlane), dBase = ummaSmemDesc(ds, 128u, kDPlane);
-                const uint32_t first = k > 0 ? 1u : 0u;
-                if (a.mIsX) {
-#pragma unroll
-                    for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                        for (int kk = 0; kk < kM / 16; kk++)
-                            mma(tmem + (uint32_t)dx * a.accCols, xBase + (uint64_t)(dx + 16 * kk), dBase + (uint64_t)(16 * kk),
-                                idesc, (first || kk > 0) ? 1u : 0u);
-                } else {
-#pragma unroll
-                    for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                        for (int kk = 0; kk < kM / 16; kk++)
-                            mma(tmem + (uint32_t)dx * a.accCols, dBase + (uint64_t)(16 * kk), xBase + (uint64_t)(dx + 16 * kk),
-                                idesc, (first || kk > 0) ? 1u : 0u);
+                const int rows = unitOf(a, u).rows;
+                uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
+                for (int r = 0; r < rows; r++) {
+                    const uint64_t dDesc = slabDescriptor<SD>(ds, a.dSlab);
+                    for (int b = b0; b < b1; b++)
+                        issueRowK<SX, SD>(a.px / 16, tmem + (uint32_t)(b - b0) * 3u * cols, cols,
+                                          slabDescriptor<SX>(xs + (uint32_t)(b * (kM / SX)) * a.xSlab, a.xSlab), dDesc, idesc,
+                                          started);
+                    started = 1u;
+                    xs += (uint32_t)a.xSlabs * a.xSlab;
+                    ds += (uint32_t)a.dSlabs * a.dSlab;
                 }
                 commit(base + Header::empty + 8 * st);
                 if (++st == S) { st = 0; parity ^= 1u; }
@@ -255,8 +319,8 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
             if (ok) {
                 commit(base + Header::done);
                 // The releases' arrivals land before shared memory goes away.
-                for (long long e = k > S ? k - S : 0; e < k; e++)
-                    pollPhase(base + Header::empty + 8 * (int)(e % S), (uint32_t)((e / S) & 1), limit);
+                for (int e = k > S ? k - S : 0; e < k; e++)
+                    pollPhase(base + Header::empty + 8 * (e % S), (uint32_t)((e / S) & 1), limit);
             } else {
                 *abortFlag = 1;
                 commit(base + Header::drain);
@@ -265,25 +329,25 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         }
         __syncwarp();
     } else {
-        // ---- epilogue: add the three accumulators to dw ----
+        // ---- epilogue: add the accumulators to dw ----
         const int quarter = warp & 3;
         const bool ok = waitPhaseWarp(base + Header::done, 0u, abortFlag, limit);
-        if (ok && seg1 > seg0) {
+        if (ok && (int)blockIdx.x < a.units) {
             tcFenceAfter();
-            const int r = quarter * 32 + lane;  // accumulator row of this thread
-            for (int dx = 0; dx < 3; dx++) {
-                const int tap = dy * 3 + dx;
-                for (int c = 0; c < a.nDim; c += 16) {
-                    uint32_t v[16];
-                    tmemLoad16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)dx * a.accCols + (uint32_t)c, v);
-                    if (r >= a.mValid) continue;
+            for (int b = b0; b < b1; b++) {
+                const int q = b * kM + quarter * 32 + lane;  // (dy, ci) of this thread's accumulator row
+                const int dy = q / a.cin, ci = q % a.cin;
+                for (int dx = 0; dx < 3; dx++) {
+                    float* out = a.dw + ((size_t)(dy * 3 + dx) * a.cin + ci) * a.cout;
+                    for (int c = 0; c < a.cout; c += 16) {
+                        uint32_t v[16];
+                        tmemLoad16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(((b - b0) * 3 + dx) * a.cout + c), v);
+                        if (dy > 2) continue;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        const float f = __uint_as_float(v[j]);
-                        if (f == 0.0f) continue;
-                        const int ci = a.mIsX ? mBase + r : c + j;
-                        const int co = a.mIsX ? c + j : r;
-                        atomicAdd(a.dw + ((size_t)tap * a.cin + ci) * a.cout + co, f);
+                        for (int j = 0; j < 16; j += 4)
+                            atomicAdd(reinterpret_cast<float4*>(out + c + j),
+                                      make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                  __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
                     }
                 }
             }
@@ -312,86 +376,112 @@ PFN_cuTensorMapEncodeTiled_v12000 encodeTiled() {
     return fn;
 }
 
-bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, int c, uint32_t boxPixels) {
+// Boxes of one slab of `slab` channels x boxPixels of one row, swizzled;
+// zero fill outside the image.
+bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, int c, int slab, uint32_t boxPixels) {
     auto fn = encodeTiled();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
     const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-    const cuuint32_t box[4] = {8, boxPixels, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)slab, boxPixels, 1, 1};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
+    const CUtensorMapSwizzle swizzle = slab == 16   ? CU_TENSOR_MAP_SWIZZLE_32B
+                                       : slab == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                    : CU_TENSOR_MAP_SWIZZLE_128B;
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(ptr), dims, strides, box, elem,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int SX, int SD>
+cudaError_t launch(const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid, uint32_t smemBytes,
+                   cudaStream_t stream) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel<SX, SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    wgradTcKernel<SX, SD><<<grid, kThreads, smemBytes, stream>>>(xMap, dMap, a);
+    return cudaGetLastError();
+}
+template <int SX>
+cudaError_t launchD(int sd, const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid,
+                    uint32_t smemBytes, cudaStream_t stream) {
+    return sd == 64   ? launch<SX, 64>(xMap, dMap, a, grid, smemBytes, stream)
+           : sd == 32 ? launch<SX, 32>(xMap, dMap, a, grid, smemBytes, stream)
+                      : launch<SX, 16>(xMap, dMap, a, grid, smemBytes, stream);
 }
 
 }  // namespace
 
 bool wgradTcSupported(int cin, int cout) {
-    const int small = std::min(cin, cout);
-    return cin % 16 == 0 && cout % 16 == 0 && cin >= 16 && cout >= 16 && cout <= 128 && small <= 128 &&
-           cin <= 256 && 3 * small <= 512;
+    return cin % 16 == 0 && cout % 16 == 0 && cin >= 16 && cout >= 16 && cout <= 128 && cin <= 256;
 }
 
 cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin, int cout, float* dw, int* errorFlag,
                     cudaStream_t stream) {
-    if (!wgradTcSupported(cin, cout) || n < 1 || h < 1 || w < 1 || !errorFlag) return cudaErrorNotSupported;
-    CUtensorMap xMap{}, dMap{};
-    if (!makeActivationMap(&xMap, x, n, h, w, cin, kHaloPx) || !makeActivationMap(&dMap, dy, n, h, w, cout, kM))
+    if (!wgradTcSupported(cin, cout) || n < 1 || h < 1 || w < 1 || !errorFlag || (reinterpret_cast<uintptr_t>(dw) & 15))
         return cudaErrorNotSupported;
+    const int sx = slabChannels(cin), sd = slabChannels(cout);
     WgradArgs a{};
-    a.n = n; a.h = h; a.w = w; a.cin = cin; a.cout = cout;
-    a.tilesPerRow = (w + kM - 1) / kM;
-    a.segments = n * h * a.tilesPerRow;
-    a.mIsX = cin >= cout ? 1 : 0;
-    const int mBlocks = a.mIsX ? (cin + kM - 1) / kM : 1;
-    // M operand: 16 planes staged (rows beyond the channels read stale
-    // planes and are dropped); N operand: its channels.
-    a.nDim = a.mIsX ? cout : cin;
-    a.xPlanes = a.mIsX ? std::min(16, cin / 8) : cin / 8;  // the last M block may hold fewer (set per block below)
-    a.dPlanes = cout / 8;
-    const uint32_t xStaged = a.mIsX ? 16u : (uint32_t)(cin / 8);
-    const uint32_t dStaged = a.mIsX ? (uint32_t)(cout / 8) : 16u;
-    a.xBytes = xStaged * kXPlane;
-    a.stageBytes = a.xBytes + dStaged * kDPlane;
-    a.accCols = (uint32_t)a.nDim;
+    a.h = h; a.w = w; a.cin = cin; a.cout = cout;
+    a.xSlabs = cin / sx; a.dSlabs = cout / sd;
+    a.mBlocks = (3 * cin + kM - 1) / kM;
+    // As many M blocks per grid slice as 512 columns of accumulators hold,
+    // evenly over the slices.
+    const int fit = std::min(a.mBlocks, 512 / (3 * cout));
+    if (fit < 1) return cudaErrorNotSupported;
+    const int slices = (a.mBlocks + fit - 1) / fit;
+    a.blocksPerSlice = (a.mBlocks + slices - 1) / slices;
     a.tmemCols = 32;
-    while (a.tmemCols < 3u * a.accCols) a.tmemCols <<= 1;
-    a.dw = dw;
-    a.errorFlag = errorFlag;
-    a.waitLimitNs = 1000000000ull;
-    a.stages = 2;
-    while (a.stages < kMaxStages && kHeader + (uint32_t)(a.stages + 1) * a.stageBytes <= 200u * 1024u) a.stages++;
-    const uint32_t smemBytes = kHeader + (uint32_t)a.stages * a.stageBytes;
-    if (smemBytes > 227u * 1024u) return cudaErrorNotSupported;
-    a.mValid = a.mIsX ? std::min(kM, cin) : cout;
+    while (a.tmemCols < (uint32_t)(a.blocksPerSlice * 3 * cout)) a.tmemCols <<= 1;
     int sms = 0, device = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int perSm = std::max(1, std::min((int)(228u * 1024u / (smemBytes + 1024u)), (int)(512u / a.tmemCols)));
-    const long long want = (long long)std::max(1, sms) * perSm * 2;
-    const int splits = (int)std::max(1ll, std::min<long long>(a.segments, want / (3ll * mBlocks)));
-    a.segPerBlock = (a.segments + splits - 1) / splits;
-    const int grid = (a.segments + a.segPerBlock - 1) / a.segPerBlock;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    // M blocks of 128 input channels (224 = 128 + 96), one launch each.
-    for (int mb = 0; mb < mBlocks; mb++) {
-        WgradArgs b = a;
-        if (a.mIsX) {
-            const int channels = std::min(kM, cin - mb * kM);
-            b.mBase = mb * kM;
-            b.xPlanes = channels / 8;
-            b.mValid = channels;
+    const int splits = std::max(1, std::max(1, sms) / slices);
+    // Segment width and rows per stage: two stages have to fit; the busiest
+    // block's staged rows (each unit costs its rows and about one row's
+    // latency) decide. Segments of 128 pixels fit up to about 100 channels in
+    // all, wide layers on wide images take narrower ones.
+    long long bestCost = -1, bestUnits = 0;
+    for (int px = std::min(kM, (w + 15) / 16 * 16), next = 0; px >= 16; px = next) {
+        next = px > 64 ? 64 : px > 32 ? 32 : px > 16 ? 16 : 0;
+        const uint32_t xSlab = slabBytes(px + 2, sx), dSlab = slabBytes(px, sd);
+        const int tiles = (w + px - 1) / px;
+        // A stage: rows + 2 rows of x, then the dY rows. The last M block may
+        // read past the stacked rows, at most `over` bytes past x's part.
+        const uint32_t over = (uint32_t)(a.mBlocks * (kM / sx) - 3 * a.xSlabs) * xSlab;
+        for (int rows = 1; rows <= std::min(kMaxRows, h); rows++) {
+            const uint32_t xPart = ((uint32_t)((rows + 2) * a.xSlabs) * xSlab + 1023u) & ~1023u;
+            const uint32_t stage = (xPart + std::max(over, (uint32_t)(rows * a.dSlabs) * dSlab) + 1023u) & ~1023u;
+            if (kHeader + 2u * stage > kSmemMax) break;
+            const long long strips = (h + rows - 1) / rows, units = (long long)n * tiles * strips;
+            const long long cost = (units + splits - 1) / splits * (rows + 1) * (px + 16);
+            if (units > 0x7FFFFFFFll || (bestCost >= 0 && cost > bestCost)) continue;
+            bestCost = cost;
+            bestUnits = units;
+            a.px = px; a.rows = rows;
+            a.tilesPerRow = tiles; a.strips = (int)strips; a.units = (int)units;
+            a.xSlab = xSlab; a.dSlab = dSlab;
+            a.xBytes = xPart; a.stageBytes = stage;
         }
-        wgradTcKernel<<<dim3(grid, 3, 1), kThreads, smemBytes, stream>>>(xMap, dMap, b);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    if (bestCost < 0) return cudaErrorNotSupported;
+    a.stages = 2;
+    while (a.stages < kMaxStages && kHeader + (uint32_t)(a.stages + 1) * a.stageBytes <= kSmemMax) a.stages++;
+    a.dw = dw;
+    a.errorFlag = errorFlag;
+    a.waitLimitNs = 1000000000ull;
+    CUtensorMap xMap{}, dMap{};
+    if (!makeActivationMap(&xMap, x, n, h, w, cin, sx, (uint32_t)(a.px + 2)) ||
+        !makeActivationMap(&dMap, dy, n, h, w, cout, sd, (uint32_t)a.px))
+        return cudaErrorNotSupported;
+    const dim3 grid((unsigned)std::min<long long>(splits, bestUnits), (unsigned)slices);
+    const uint32_t smemBytes = kHeader + (uint32_t)a.stages * a.stageBytes;
+    return sx == 64   ? launchD<64>(sd, xMap, dMap, a, grid, smemBytes, stream)
+           : sx == 32 ? launchD<32>(sd, xMap, dMap, a, grid, smemBytes, stream)
+                      : launchD<16>(sd, xMap, dMap, a, grid, smemBytes, stream);
 }
 
 }  // namespace rt

@@ -538,12 +538,15 @@ __global__ void __launch_bounds__(pipeThreads(ISS, EPI), ISS > 1 ? 1 : (COUT <= 
                      "r"(a.tmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+        // The next kernel in the stream may start its own setup now, and not
+        // before this block holds its tensor memory: a block of the next
+        // kernel on the same SM could take the columns first and keep them
+        // while it waits for this kernel.
+        asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     }
-    // Programmatic dependent launch (the host launches with it): the next
-    // kernel in the stream may start its own setup now; this block waits for
-    // the previous kernel to complete before any other read of global memory
-    // (input rows, bias, addend, the accumulated output).
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    // Programmatic dependent launch (the host launches with it): this block
+    // waits for the previous kernel to complete before any other read of
+    // global memory (input rows, bias, addend, the accumulated output).
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     float* sBias = reinterpret_cast<float*>(smem + Header::bias);
     for (int c = threadIdx.x; c < COUT; c += blockDim.x) sBias[c] = a.bias ? a.bias[nBase + c] : 0.0f;

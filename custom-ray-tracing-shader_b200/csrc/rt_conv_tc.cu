@@ -514,6 +514,24 @@ bool upsampledSplitSupported(int cin, int cout, int lowChannels) {
            convPipePreferred(cin - lowChannels, cout, 0);
 }
 
+namespace {
+// How the single-role kernel takes a layer: its input channels per chunk, and
+// whether it keeps the weights resident and walks a ring of rows.
+// Weights stay in shared memory when they fit beside two halo stages;
+// the chunk is the largest multiple of 16 dividing cin that still fits
+// (one chunk per tile where possible: fewer rounds of staging). Otherwise
+// weights and halo are staged per 16-channel chunk.
+struct SingleRoleForm { int kc, resident, ring; };
+constexpr uint32_t kHaloPerChannel = 3u * kHaloW * 2u;
+SingleRoleForm singleRoleForm(int cin, int cout) {
+    const uint32_t fullWeights = 9u * (uint32_t)cin * (uint32_t)cout * 2u;
+    if (kHeaderBytes + fullWeights + 4u * kHaloW * 2u * (uint32_t)cin <= 220u * 1024u) return {cin, 1, 1};
+    for (int kc = cin; kc >= 16; kc -= 16)
+        if (cin % kc == 0 && kHeaderBytes + fullWeights + 2u * kHaloPerChannel * (uint32_t)kc <= 220u * 1024u) return {kc, 1, 0};
+    return {16, 0, 0};
+}
+}  // namespace
+
 cudaError_t convTc(const bf16* in, const bf16* low, int lowChannels, int n, int h, int w, int cin,
                    const bf16* weights, bool reverseTaps, const float* bias, int cout, bf16* outB, float* outF,
                    bool relu, bool accumulate, int* errorFlag, cudaStream_t stream, const bf16* upAddend,
@@ -525,9 +543,22 @@ cudaError_t convTc(const bf16* in, const bf16* low, int lowChannels, int n, int 
         if (e == cudaSuccess) g_pipeLaunches++;
         return e;
     }
+    // Narrow images: the kernel whose tiles span rows, accumulating in the
+    // order of the kernel below that would take the layer.
+    const bool piped = convPipePreferred(cin, cout, low ? lowChannels : 0);
+    if (g_convPath.load() == 0 && !g_convPipeReference.load() && !low && w <= kNarrowWidth) {
+        const int kc = piped ? cin : singleRoleForm(cin, cout).kc;
+        cudaError_t e = kc != cin && kc != 16 ? cudaErrorNotSupported
+                                              : convNarrow(in, n, h, w, cin, weights, reverseTaps, bias, cout, outB, outF, relu,
+                                                           accumulate, kc != cin, errorFlag, stream);
+        if (e != cudaErrorNotSupported) {
+            g_pipeLaunches++;
+            return e;
+        }
+    }
     // The warp-specialised TMA form where its shared memory allows (see
     // rt_conv_pipe.cu); this kernel for the layers with the largest weights.
-    if (g_convPath.load() == 0 && convPipePreferred(cin, cout, low ? lowChannels : 0)) {
+    if (g_convPath.load() == 0 && piped) {
         cudaError_t e = convPipe(in, low, lowChannels, n, h, w, cin, weights, reverseTaps, bias, cout, outB, outF,
                                  relu, accumulate, errorFlag, stream);
         if (e != cudaErrorNotSupported) {
@@ -559,36 +590,13 @@ cudaError_t convTc(const bf16* in, const bf16* low, int lowChannels, int n, int 
     a.tilesPerRow = (w + kTileM - 1) / kTileM;
     a.tiles = n * h * a.tilesPerRow;
     a.errorFlag = errorFlag;
-    // Weights stay in shared memory when they fit beside two halo stages;
-    // the chunk is the largest multiple of 16 dividing cin that still fits
-    // (one chunk per tile where possible: fewer rounds of staging). Otherwise
-    // weights and halo are staged per 16-channel chunk.
-    const uint32_t fullWeights = 9u * (uint32_t)cin * (uint32_t)cout * 2u;
-    const uint32_t haloPerChannel = 3u * kHaloW * 2u;
-    const uint32_t ringBytes = 4u * kHaloW * 2u * (uint32_t)cin;
-    a.resident = 0;
-    a.ring = kHeaderBytes + fullWeights + ringBytes <= 220u * 1024u;
-    for (int kc = a.ring ? 16 : cin; kc >= 16; kc -= 16) {
-        if (cin % kc) continue;
-        if (kHeaderBytes + fullWeights + 2u * haloPerChannel * (uint32_t)kc <= 220u * 1024u) {
-            a.kc = kc;
-            a.resident = 1;
-            break;
-        }
-    }
-    if (a.ring) {
-        a.kc = cin;
-        a.resident = 1;
-        a.weightBytes = fullWeights;
-        a.haloBytes = ringBytes / 2u;  // the ring takes the two halo stages' room
-    } else if (a.resident) {
-        a.weightBytes = fullWeights;
-        a.haloBytes = haloPerChannel * (uint32_t)a.kc;
-    } else {
-        a.kc = 16;
-        a.weightBytes = 2u * 9u * 16u * (uint32_t)cout * 2u;
-        a.haloBytes = haloPerChannel * (uint32_t)a.kc;
-    }
+    const SingleRoleForm form = singleRoleForm(cin, cout);
+    a.kc = form.kc;
+    a.resident = form.resident;
+    a.ring = form.ring;
+    // The ring takes the two halo stages' room.
+    a.haloBytes = form.ring ? 2u * kHaloW * 2u * (uint32_t)cin : kHaloPerChannel * (uint32_t)a.kc;
+    a.weightBytes = 9u * (uint32_t)(form.resident ? cin : 2 * 16) * (uint32_t)cout * 2u;
     const uint32_t smemBytes = kHeaderBytes + a.weightBytes + 2u * a.haloBytes;
     if (smemBytes > kMaxSmem) return cudaErrorInvalidValue;
     a.accCols = 32;

@@ -149,6 +149,18 @@ cudaError_t convPipe(const __nv_bfloat16* in, const __nv_bfloat16* low, int lowC
                      cudaStream_t stream, const ConvPipeTest* test = nullptr,
                      const __nv_bfloat16* upAddend = nullptr, const ConvHead* head = nullptr, bool planarOut = false);
 
+// The same convolution on images of up to kNarrowWidth pixels (rt_conv_narrow
+// .cu): tiles of 128 positions over several rows. chunked: products
+// accumulated in chunks of 16 input channels (the single-role kernel's order
+// for layers whose weights it stages in chunks), else tap by tap. Returns
+// cudaErrorNotSupported (before any launch) for shapes it does not take.
+// Above 64 pixels a row-wide tile of 128 is more than half full and the
+// pipelined kernel's ring stages every row once.
+constexpr int kNarrowWidth = 64;
+cudaError_t convNarrow(const __nv_bfloat16* in, int n, int h, int w, int cin, const __nv_bfloat16* weights,
+                       bool reverseTaps, const float* bias, int cout, __nv_bfloat16* outB, float* outF, bool relu,
+                       bool accumulate, bool chunked, int* errorFlag, cudaStream_t stream);
+
 // Weight gradient on tcgen05 (rt_wgrad_tc.cu): dw[tap][ci][co] += sum_p
 // x[p + off(tap)][ci] dy[p][co] over NHWC BF16 x (cin channels) and dy (cout
 // channels), dw FP32 [9][cin][cout]. cin, cout multiples of 16, cout <= 128,

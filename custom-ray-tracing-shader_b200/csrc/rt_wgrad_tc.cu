@@ -31,16 +31,10 @@
 // Roles: warp 0 issues the TMA loads into two or more stages, warp 1 issues
 // the MMAs and owns the tensor memory, warps 2-5 drain the accumulators at
 // the end. Waits are bounded as in rt_conv_pipe.cu.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <cudaTypedefs.h>
-
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
 
-#include "rt_conv_tc.cuh"
+#include "rt_tc_ptx.cuh"
 
 namespace rt {
 namespace {
@@ -59,7 +53,6 @@ constexpr uint32_t kSmemMax = 227u * 1024u;
 __host__ __device__ constexpr uint32_t slabBytes(int px, int s) {
     return ((uint32_t)px * 2u * (uint32_t)s + 16u * (uint32_t)s - 1u) & ~(16u * (uint32_t)s - 1u);
 }
-inline int slabChannels(int c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
 
 struct WgradArgs {
     int h, w, cin, cout;
@@ -85,89 +78,16 @@ struct Header {
     static constexpr uint32_t abort = 16 * kMaxStages + 20;
 };
 
-__device__ __forceinline__ uint32_t smemAddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint64_t nowNs() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void barInit(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void barExpectTx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool barTryWait(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(1000u)
-        : "memory");
-    return done != 0;
-}
-__device__ bool waitPhase(uint32_t bar, uint32_t parity, volatile int* abortFlag, uint64_t limitNs) {
-    if (barTryWait(bar, parity)) return true;
-    const uint64_t deadline = nowNs() + limitNs;
-    for (;;) {
-        if (barTryWait(bar, parity)) return true;
-        if (*abortFlag) return false;
-        if (nowNs() > deadline) { *abortFlag = 1; return false; }
-    }
-}
-__device__ __forceinline__ bool waitPhaseWarp(uint32_t bar, uint32_t parity, volatile int* abortFlag,
-                                              uint64_t limitNs) {
-    bool ok = true;
-    if ((threadIdx.x & 31) == 0) ok = waitPhase(bar, parity, abortFlag, limitNs);
-    return __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
-}
-__device__ void pollPhase(uint32_t bar, uint32_t parity, uint64_t limitNs) {
-    const uint64_t deadline = nowNs() + limitNs;
-    while (!barTryWait(bar, parity) && nowNs() < deadline) {
-    }
-}
-__device__ __forceinline__ void tmaLoad4(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                         uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];\n" ::"r"(dst),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void tcFenceBefore() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tcFenceAfter() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void mma(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n}\n" ::"r"(tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-__device__ __forceinline__ void commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void tmemLoad16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-
 // Instruction descriptor: FP32 accumulator, BF16 A and B, both MN-major
 // (bits 15 and 16), N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t idescMnMajor(int m, int n) {
     return ummaInstrDescBf16(m, n) | (1u << 15) | (1u << 16);
 }
 // MN-major swizzled operand descriptor of slabs of S channels, `slab` bytes
-// apart (layout type in bits 61-63: 6 = 32-byte, 4 = 64-byte, 2 = 128-byte).
+// apart.
 template <int S>
 __device__ __forceinline__ uint64_t slabDescriptor(uint32_t addr, uint32_t slab) {
-    return ummaSmemDesc(addr, slab, 16u * S) | ((uint64_t)(S == 16 ? 6 : S == 32 ? 4 : 2) << 61);
+    return ummaSmemDesc(addr, slab, 16u * S) | slabLayout(S);
 }
 
 // The MMAs of one dY row and one M block: 3 column taps x KK steps of 16
@@ -341,6 +261,7 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
                     float* out = a.dw + ((size_t)(dy * 3 + dx) * a.cin + ci) * a.cout;
                     for (int c = 0; c < a.cout; c += 16) {
                         uint32_t v[16];
+                        __syncwarp();  // the load needs converged lanes; the additions below may diverge
                         tmemLoad16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(((b - b0) * 3 + dx) * a.cout + c), v);
                         if (dy > 2) continue;
 #pragma unroll
@@ -363,19 +284,6 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encodeTiled() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
 // Boxes of one slab of `slab` channels x boxPixels of one row, swizzled;
 // zero fill outside the image.
 bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, int c, int slab, uint32_t boxPixels) {
@@ -385,11 +293,8 @@ bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, i
     const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
     const cuuint32_t box[4] = {(cuuint32_t)slab, boxPixels, 1, 1};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
-    const CUtensorMapSwizzle swizzle = slab == 16   ? CU_TENSOR_MAP_SWIZZLE_32B
-                                       : slab == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                    : CU_TENSOR_MAP_SWIZZLE_128B;
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(ptr), dims, strides, box, elem,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, slabSwizzle(slab), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

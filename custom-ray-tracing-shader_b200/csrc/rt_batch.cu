@@ -395,6 +395,7 @@ struct BatchViewData {
 };
 
 struct Batch {
+    DeviceMemoryUser memory;
     std::string error;
     int device = -1;
     cudaStream_t stream = nullptr;
@@ -456,7 +457,7 @@ void dropGraph(Batch* b) {
 void freeArena(Batch* b) {
     void* owned[] = {b->aTris, b->aWide, b->aPacked, b->aLights, b->dScenes};
     for (void* p : owned)
-        if (p) cudaFree(p);
+        if (p) rt::deviceFree(p);
     b->aTris = nullptr; b->aWide = nullptr; b->aPacked = nullptr; b->aLights = nullptr; b->dScenes = nullptr;
     b->arenaReady = false;
     dropGraph(b);
@@ -465,7 +466,7 @@ void freeArena(Batch* b) {
 void freeViews(Batch* b) {
     void* owned[] = {b->dViews, b->dSum, b->dDepth, b->dPixels, b->dTiles};
     for (void* p : owned)
-        if (p) cudaFree(p);
+        if (p) rt::deviceFree(p);
     b->dViews = nullptr; b->dSum = nullptr; b->dDepth = nullptr; b->dPixels = nullptr; b->dTiles = nullptr;
     b->viewsReady = false;
     dropGraph(b);
@@ -510,7 +511,7 @@ bool buildScene(Batch* b, BatchSceneData& S) {
     cudaError_t e = buildBvh(S.dTris, S.count, b->stream, S.bvh, S.build, &why, 3, b->width, b->pieces, b->leaf);
     if (e != cudaSuccess) { S.builtWidth = 0; return failB(b, e, why); }
     void* unused[] = {S.bvh.binNodes, S.bvh.order, S.bvh.primLo, S.bvh.primHi};
-    for (void* q : unused) cudaFree(q);
+    for (void* q : unused) rt::deviceFree(q);
     S.bvh.binNodes = nullptr; S.bvh.order = nullptr; S.bvh.primLo = nullptr; S.bvh.primHi = nullptr;
     S.builtWidth = b->width;
     S.builtPieces = b->pieces;
@@ -841,11 +842,11 @@ void RtxBatchDestroy(void* p) {
     freeLanes(b);
     for (BatchSceneData& S : b->scenes) {
         freeBvh(S.bvh);
-        if (S.dTris) cudaFree(S.dTris);
+        if (S.dTris) rt::deviceFree(S.dTris);
     }
     void* owned[] = {b->dDirs, b->dPassXor, b->dSeedHash, b->dSample, b->dCounters, b->dError};
     for (void* q : owned)
-        if (q) cudaFree(q);
+        if (q) rt::deviceFree(q);
     if (b->start) cudaEventDestroy(b->start);
     if (b->stop) cudaEventDestroy(b->stop);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -873,13 +874,13 @@ int RtxBatchAddScene(void* p, const Triangle* triangles, int count) {
     S.lights.resize((size_t)up.lightCount);
     if (up.lightCount &&
         (e = cudaMemcpy(S.lights.data(), dLights, sizeof(Light) * S.lights.size(), cudaMemcpyDeviceToHost)) != cudaSuccess) {
-        cudaFree(dLights);
-        cudaFree(S.dTris);
+        rt::deviceFree(dLights);
+        rt::deviceFree(S.dTris);
         failB(b, e, "scene");
         return -1;
     }
-    cudaFree(dLights);
-    if (!buildScene(b, S)) { freeBvh(S.bvh); cudaFree(S.dTris); return -1; }
+    rt::deviceFree(dLights);
+    if (!buildScene(b, S)) { freeBvh(S.bvh); rt::deviceFree(S.dTris); return -1; }
     b->scenes.push_back(S);
     b->stats.buildMs += S.build.buildMs + S.build.collapseMs;
     b->stats.triangles += count;

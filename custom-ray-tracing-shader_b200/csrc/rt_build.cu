@@ -716,7 +716,7 @@ cudaError_t alloc(T*& p, size_t count) { return rt::deviceAlloc(reinterpret_cast
 void freeBvh(BuiltBvh& b) {
     void* owned[] = {b.binNodes, b.order, b.wideNodes, b.packedTris, b.primLo, b.primHi};
     for (void* p : owned)
-        if (p) cudaFree(p);
+        if (p) rt::deviceFree(p);
     b = BuiltBvh{};
 }
 
@@ -752,9 +752,9 @@ cudaError_t pieceMap(const SceneTri* tris, int triCount, int maxPieces, cudaStre
     if (err == cudaSuccess && ms) err = cudaEventElapsedTime(ms, t0, t1);
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
-    cudaFree(counts); cudaFree(pfx); cudaFree(sums); cudaFree(dTotal);
+    rt::deviceFree(counts); rt::deviceFree(pfx); rt::deviceFree(sums); rt::deviceFree(dTotal);
     if (err == cudaSuccess && (hostTotal < triCount || hostTotal > triCount * maxPieces)) err = cudaErrorUnknown;
-    if (err != cudaSuccess) { cudaFree(map); return err; }
+    if (err != cudaSuccess) { rt::deviceFree(map); return err; }
     if (primTri) *primTri = map;
     *total = hostTotal;
     return cudaSuccess;
@@ -782,7 +782,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         err = pieceMap(tris, triCount, pieces, stream, &primTri, &total, &pieceMs);
         if (err != cudaSuccess) { cudaEventDestroy(e0); *failure = "triangle pieces"; return err; }
         if (total == triCount) {  // no triangle is split: a tree over the triangles themselves
-            cudaFree(primTri);
+            rt::deviceFree(primTri);
             primTri = nullptr;
         }
         n = total;
@@ -796,9 +796,9 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     unsigned* flags = nullptr; unsigned* prefix = nullptr; unsigned* blockSums = nullptr; int* counters = nullptr;
     BinNode* rawNodes = nullptr; int* interior = nullptr; int* rank = nullptr; int* newIndex = nullptr;
     Job* jobs = nullptr; Job* jobsB = nullptr;
-    int* hostCounters = nullptr;
     int* levelCounts = nullptr; int* levelStartDev = nullptr; int* jobCounts = nullptr;
-    int* hostLevels = nullptr; int* hostStarts = nullptr; int* hostJobs = nullptr;
+    int hostCounters[8] = {}, hostLevels[2 * (kBinaryMaxDepth + 2 + kLevelBatch)], hostStarts[kBinaryMaxDepth + 4 + kLevelBatch];
+    int hostJobs[kStackCapacity + 2 + kLevelBatch];
     std::vector<int> levelStart;
     int nScanBlocks = blocksFor(n, kScanBlock);
 
@@ -809,14 +809,10 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     RT_TRY(alloc(bins, (size_t)taskCapacity * 3 * kBins)); RT_TRY(alloc(splits, taskCapacity));
     RT_TRY(alloc(flags, n)); RT_TRY(alloc(prefix, n)); RT_TRY(alloc(blockSums, nScanBlocks));
     RT_TRY(alloc(counters, 8)); RT_TRY(alloc(rawNodes, nodeCapacity));
-    RT_TRY(cudaMallocHost(reinterpret_cast<void**>(&hostCounters), 8 * sizeof(int)));
     {
         const int levelSlots = kBinaryMaxDepth + 2 + kLevelBatch, jobSlots = kStackCapacity + 2 + kLevelBatch;
         RT_TRY(alloc(levelCounts, 2 * levelSlots)); RT_TRY(alloc(levelStartDev, levelSlots + 2));
         RT_TRY(alloc(jobCounts, jobSlots));
-        RT_TRY(cudaMallocHost(reinterpret_cast<void**>(&hostLevels), sizeof(int) * 2 * levelSlots));
-        RT_TRY(cudaMallocHost(reinterpret_cast<void**>(&hostStarts), sizeof(int) * (levelSlots + 2)));
-        RT_TRY(cudaMallocHost(reinterpret_cast<void**>(&hostJobs), sizeof(int) * jobSlots));
     }
     // Renumbering and collapse buffers at their upper bounds (node count <=
     // nodeCapacity, wide nodes and jobs <= 2n + 8), so no allocation falls
@@ -965,15 +961,11 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     }
 done:
 #undef RT_TRY
-    cudaFree(cent); cudaFree(orderB); cudaFree(posTask); cudaFree(posTaskB); cudaFree(tasks); cudaFree(tasksB);
-    cudaFree(bins); cudaFree(splits); cudaFree(flags); cudaFree(prefix); cudaFree(blockSums); cudaFree(counters);
-    cudaFree(rawNodes); cudaFree(interior); cudaFree(rank); cudaFree(newIndex); cudaFree(jobs); cudaFree(jobsB);
-    cudaFree(primTri);
-    if (hostCounters) cudaFreeHost(hostCounters);
-    cudaFree(levelCounts); cudaFree(levelStartDev); cudaFree(jobCounts);
-    if (hostLevels) cudaFreeHost(hostLevels);
-    if (hostStarts) cudaFreeHost(hostStarts);
-    if (hostJobs) cudaFreeHost(hostJobs);
+    rt::deviceFree(cent); rt::deviceFree(orderB); rt::deviceFree(posTask); rt::deviceFree(posTaskB); rt::deviceFree(tasks); rt::deviceFree(tasksB);
+    rt::deviceFree(bins); rt::deviceFree(splits); rt::deviceFree(flags); rt::deviceFree(prefix); rt::deviceFree(blockSums); rt::deviceFree(counters);
+    rt::deviceFree(rawNodes); rt::deviceFree(interior); rt::deviceFree(rank); rt::deviceFree(newIndex); rt::deviceFree(jobs); rt::deviceFree(jobsB);
+    rt::deviceFree(primTri);
+    rt::deviceFree(levelCounts); rt::deviceFree(levelStartDev); rt::deviceFree(jobCounts);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (e2) cudaEventDestroy(e2);

@@ -22,14 +22,30 @@ namespace rt {
 constexpr float kPi = 3.14159265358979323846f;
 
 // ---- device allocation ----
-// The renderer's device allocations go through deviceAlloc, so a test can
-// make the n-th next one fail on the host, as an out-of-memory cudaMalloc
-// would, without touching the GPU (RtxDebugFailAllocation).
+// The library's device allocations go through deviceAlloc and deviceFree
+// (rt_memory.cu). Freed blocks are kept, up to a bound per device, for later
+// allocations of about their size, and handed out again only after a device
+// synchronisation that follows the free, so any stream may use them (freeing
+// waits for the device with cudaFree as well). The cache is given back when
+// the last DeviceMemoryUser (session, batch, network) goes, at RtShutdown, and
+// when the device runs out of memory. Safe with several threads and devices.
+// setFailAllocation makes the n-th next allocation fail on the host, as an
+// out-of-memory cudaMalloc would, without touching the GPU
+// (RtxDebugFailAllocation).
 cudaError_t deviceAllocBytes(void** p, size_t bytes);
 template <class T>
 inline cudaError_t deviceAlloc(T** p, size_t bytes) {
     return deviceAllocBytes(reinterpret_cast<void**>(p), bytes);
 }
+void deviceFree(void* p);
+void trimDeviceMemory();
+void setFailAllocation(int n);
+struct DeviceMemoryUser {
+    DeviceMemoryUser();
+    ~DeviceMemoryUser();
+    DeviceMemoryUser(const DeviceMemoryUser&) = delete;
+    DeviceMemoryUser& operator=(const DeviceMemoryUser&) = delete;
+};
 
 // ---- portable bit helpers (device intrinsics, host builtins) ----
 RT_HD unsigned popc(unsigned x) {

@@ -366,7 +366,7 @@ void freeWavefront(WavefrontBuffers& b) {
     void* owned[] = {b.pathA, b.pathB, b.pathC, b.radiance, b.albedo, b.normal, b.hits, b.queue[0], b.queue[1],
                      b.shadowRay, b.shadowDir, b.shadowContrib, b.counts};
     for (void* p : owned)
-        if (p) cudaFree(p);
+        if (p) rt::deviceFree(p);
     b = WavefrontBuffers{};
 }
 

@@ -48,26 +48,13 @@ constexpr int kDefaultTraversalLeaf = 2;
 
 // A denoising network with its last error message (RtxUnet* entry points).
 struct UnetHandle {
+    rt::DeviceMemoryUser memory;
     rt::Unet net;
     std::string error;
     explicit UnetHandle(unsigned seed) : net(seed) {}
 };
 
 namespace rt {
-// Countdown of RtxDebugFailAllocation: when it reaches the call that brings
-// it from 1 to 0, that allocation fails without calling cudaMalloc.
-static std::atomic<long long> g_failAllocationIn{0};
-cudaError_t deviceAllocBytes(void** p, size_t bytes) {
-    long long n = g_failAllocationIn.load();
-    while (n > 0 && !g_failAllocationIn.compare_exchange_weak(n, n - 1)) {
-    }
-    if (n == 1) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
-    return cudaMalloc(p, bytes);
-}
-
 // The sampler's direction numbers: cuRAND's JOEKUO6 table, fetched at run
 // time like the reference (sampling.cuh:10), 260 dimensions x 32 words.
 const unsigned* hostSobolDirections(std::string& error) {
@@ -81,6 +68,7 @@ const unsigned* hostSobolDirections(std::string& error) {
 namespace {
 
 struct Session {
+    DeviceMemoryUser memory;
     std::string hostError;
     cudaError_t error = cudaSuccess;
     bool ready = false;
@@ -197,7 +185,7 @@ void releaseScene(Session* s) {
     void* owned[] = {s->dTris, s->dLights, s->dDirs, s->dPassXor, s->dSeedHash, s->dSum, s->dDepth, s->dPixels,
                      s->dCounters, s->dError, s->dDenoise};
     for (void* p : owned)
-        if (p) cudaFree(p);
+        if (p) rt::deviceFree(p);
     s->dTris = nullptr; s->dLights = nullptr; s->dDirs = nullptr; s->dPassXor = nullptr; s->dSeedHash = nullptr;
     s->dSum = nullptr; s->dDepth = nullptr; s->dPixels = nullptr; s->dCounters = nullptr; s->dError = nullptr;
     s->dDenoise = nullptr;
@@ -445,24 +433,28 @@ const char* RtLastError(void* p) {
     if (s && !s->hostError.empty()) return s->hostError.c_str();
     return cudaGetErrorString(s ? s->error : cudaErrorInvalidValue);
 }
-void RtShutdown(void* p) {
-    Session* s = static_cast<Session*>(p);
-    if (!s) return;
+static void releaseSession(Session* s) {
     // Releasing on another device than the scene's would free nothing; the
     // attempt goes on regardless so the session is left empty.
     if (s->device >= 0 && s->stream) (void)useDevice(s);
     releaseScene(s);
     s->hostError.clear();
 }
+void RtShutdown(void* p) {
+    Session* s = static_cast<Session*>(p);
+    if (!s) return;
+    releaseSession(s);
+    rt::trimDeviceMemory();  // the caller gives the scene up: so does the cache
+}
 void RtDestroy(void* p) {
     Session* s = static_cast<Session*>(p);
-    if (s) { RtShutdown(s); delete s; }
+    if (s) { releaseSession(s); delete s; }
 }
 
 int RtInitialize(void* p, const Triangle* triangles, int count, int width, int height) {
     Session* s = static_cast<Session*>(p);
     if (!s) return 0;
-    RtShutdown(s);
+    releaseSession(s);  // its blocks are kept for the new scene's
     if (!triangles || count <= 0 || width <= 0 || height <= 0 || width > 4096 || height > 4096) {
         s->hostError = "RtInitialize: need triangles, count > 0 and 1 <= width, height <= 4096";
         s->error = cudaErrorInvalidValue;
@@ -513,7 +505,7 @@ int RtInitialize(void* p, const Triangle* triangles, int count, int width, int h
         e = buildBvh(s->dTris, count, s->stream, s->pieceBvh, s->pieceBuild, &why, 3, 8, s->pieces, s->traversalLeaf);
         if (e == cudaSuccess) {
             void* unused[] = {s->pieceBvh.binNodes, s->pieceBvh.order, s->pieceBvh.primLo, s->pieceBvh.primHi};
-            for (void* q : unused) cudaFree(q);
+            for (void* q : unused) rt::deviceFree(q);
             s->pieceBvh.binNodes = nullptr; s->pieceBvh.order = nullptr;
             s->pieceBvh.primLo = nullptr; s->pieceBvh.primHi = nullptr;
         }
@@ -638,7 +630,7 @@ int RtxQueryRays(void* p, const RtxQuery* queries, int count, int any, RtxHit* h
     if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), dh, sizeof(float4) * (size_t)count, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, s->dError, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    cudaFree(dq); cudaFree(dh);
+    rt::deviceFree(dq); rt::deviceFree(dh);
     if (e != cudaSuccess) { fail(s, e); return 0; }
     if (overflow) { s->hostError = "BVH traversal stack overflow"; return 0; }
     for (int i = 0; i < count; i++) {
@@ -669,7 +661,7 @@ int RtxSobolSamples(const unsigned* pixel, const unsigned* sample, const unsigne
     if (e == cudaSuccess) e = cudaMemcpy(dseed, seed, sizeof(unsigned) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launchSobolSamples(dd, dp, ds, dseed, count, ndim, dout, 0);
     if (e == cudaSuccess) e = cudaMemcpy(out, dout, sizeof(float) * n * ndim, cudaMemcpyDeviceToHost);
-    cudaFree(dd); cudaFree(dp); cudaFree(ds); cudaFree(dseed); cudaFree(dout);
+    rt::deviceFree(dd); rt::deviceFree(dp); rt::deviceFree(ds); rt::deviceFree(dseed); rt::deviceFree(dout);
     return e == cudaSuccess ? 1 : 0;
 }
 
@@ -820,7 +812,7 @@ int RtxUnetInfer(void* p, const float* aovs, int h, int w, float* radiance) {
     if (e == cudaSuccess) e = u->net.inferDevice(dIn, h, w, dOut, 0, why);
     if (e == cudaSuccess) e = cudaMemcpy(radiance, dOut, sizeof(float) * px * 3, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = u->net.checkConvolutions(why);
-    cudaFree(dIn); cudaFree(dOut);
+    rt::deviceFree(dIn); rt::deviceFree(dOut);
     return unetResult(u, e, why);
 }
 int RtxUnetSave(void* p, const char* path, int optimizerState) {
@@ -920,7 +912,7 @@ int RtxConvLaunchCounts(long long* pipelined, long long* singleRole) {
 
 int RtxDebugFailAllocation(int n) {
     if (n < 0) return 0;
-    rt::g_failAllocationIn.store(n);
+    rt::setFailAllocation(n);
     return 1;
 }
 

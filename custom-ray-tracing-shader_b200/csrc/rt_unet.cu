@@ -554,12 +554,12 @@ struct Unet::Activations {
     std::vector<void*> owned;
     template <class T>
     cudaError_t make(T*& p, size_t count) {
-        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), sizeof(T) * std::max<size_t>(count, 1));
+        cudaError_t e = rt::deviceAlloc(&p, sizeof(T) * std::max<size_t>(count, 1));
         if (e == cudaSuccess) owned.push_back(p);
         return e;
     }
     ~Activations() {
-        for (void* p : owned) cudaFree(p);
+        for (void* p : owned) rt::deviceFree(p);
     }
 };
 
@@ -609,13 +609,13 @@ Unet::Unet(unsigned seed) {
             host[L.wOffset + i] = v;
         }
     }
-    cudaMalloc(&master_, sizeof(float) * params_);
-    cudaMalloc(&grad_, sizeof(float) * params_);
-    cudaMalloc(&adamM_, sizeof(float) * params_);
-    cudaMalloc(&adamV_, sizeof(float) * params_);
-    cudaMalloc(&wbf_, sizeof(bf16) * params_);
-    cudaMalloc(&wT_, sizeof(bf16) * params_);
-    cudaMalloc(&convError_, sizeof(int));
+    rt::deviceAlloc(&master_, sizeof(float) * params_);
+    rt::deviceAlloc(&grad_, sizeof(float) * params_);
+    rt::deviceAlloc(&adamM_, sizeof(float) * params_);
+    rt::deviceAlloc(&adamV_, sizeof(float) * params_);
+    rt::deviceAlloc(&wbf_, sizeof(bf16) * params_);
+    rt::deviceAlloc(&wT_, sizeof(bf16) * params_);
+    rt::deviceAlloc(&convError_, sizeof(int));
     // Every copy and fill goes through stream_: it is non-blocking, so it is
     // not ordered after work on the legacy default stream.
     cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
@@ -629,7 +629,7 @@ Unet::Unet(unsigned seed) {
 
 Unet::~Unet() {
     delete act_;
-    cudaFree(master_); cudaFree(grad_); cudaFree(adamM_); cudaFree(adamV_); cudaFree(wbf_); cudaFree(wT_); cudaFree(convError_);
+    rt::deviceFree(master_); rt::deviceFree(grad_); rt::deviceFree(adamM_); rt::deviceFree(adamV_); rt::deviceFree(wbf_); rt::deviceFree(wT_); rt::deviceFree(convError_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -844,8 +844,8 @@ cudaError_t Unet::lossAndGradient(const float* aovs, const float* targets, int n
     Activations& A = *act_;
     float *dA = nullptr, *dT = nullptr;
     size_t px = (size_t)n * h * w;
-    if ((e = cudaMalloc(&dA, sizeof(float) * px * kInputChannels)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&dT, sizeof(float) * px * 3)) != cudaSuccess) { cudaFree(dA); return e; }
+    if ((e = rt::deviceAlloc(&dA, sizeof(float) * px * kInputChannels)) != cudaSuccess) return e;
+    if ((e = rt::deviceAlloc(&dT, sizeof(float) * px * 3)) != cudaSuccess) { rt::deviceFree(dA); return e; }
     cudaMemcpyAsync(dA, aovs, sizeof(float) * px * kInputChannels, cudaMemcpyHostToDevice, stream_);
     cudaMemcpyAsync(dT, targets, sizeof(float) * px * 3, cudaMemcpyHostToDevice, stream_);
     inputKernel<<<blocksFor((long long)px, 256), 256, 0, stream_>>>(dA, n, h, w, A.H, A.W, A.x0, nullptr, nullptr);
@@ -855,7 +855,7 @@ cudaError_t Unet::lossAndGradient(const float* aovs, const float* targets, int n
     if (e == cudaSuccess && grads) e = cudaMemcpyAsync(grads, grad_, sizeof(float) * params_, cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
     if (e == cudaSuccess) e = checkConvolutions(error);
-    cudaFree(dA); cudaFree(dT);
+    rt::deviceFree(dA); rt::deviceFree(dT);
     return e;
 }
 
@@ -868,8 +868,8 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     Activations& A = *act_;
     float *dA = nullptr, *dT = nullptr;
     size_t px = (size_t)count * h * w;
-    if ((e = cudaMalloc(&dA, sizeof(float) * px * kInputChannels)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&dT, sizeof(float) * px * 3)) != cudaSuccess) { cudaFree(dA); return e; }
+    if ((e = rt::deviceAlloc(&dA, sizeof(float) * px * kInputChannels)) != cudaSuccess) return e;
+    if ((e = rt::deviceAlloc(&dT, sizeof(float) * px * 3)) != cudaSuccess) { rt::deviceFree(dA); return e; }
     cudaMemcpyAsync(dA, aovs, sizeof(float) * px * kInputChannels, cudaMemcpyHostToDevice, stream_);
     cudaMemcpyAsync(dT, targets, sizeof(float) * px * 3, cudaMemcpyHostToDevice, stream_);
     std::mt19937 rng(seed);
@@ -877,7 +877,7 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     std::vector<unsigned char> flips(batch);
     std::vector<float> lossHost(steps, 0.0f);
     float* dLosses = nullptr;
-    if ((e = cudaMalloc(&dLosses, sizeof(float) * std::max(steps, 1))) != cudaSuccess) { cudaFree(dA); cudaFree(dT); return e; }
+    if ((e = rt::deviceAlloc(&dLosses, sizeof(float) * std::max(steps, 1))) != cudaSuccess) { rt::deviceFree(dA); rt::deviceFree(dT); return e; }
     cudaMemsetAsync(dLosses, 0, sizeof(float) * std::max(steps, 1), stream_);
     const size_t bpx = (size_t)batch * h * w;
     const WeightTable table = weightTable(layers_);
@@ -900,7 +900,7 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     if (e == cudaSuccess && losses) e = cudaMemcpyAsync(losses, dLosses, sizeof(float) * steps, cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
     if (e == cudaSuccess) e = checkConvolutions(error);
-    cudaFree(dA); cudaFree(dT); cudaFree(dLosses);
+    rt::deviceFree(dA); rt::deviceFree(dT); rt::deviceFree(dLosses);
     return e;
 }
 

@@ -197,7 +197,7 @@ cudaError_t uploadScene(const void* triangles, int count, cudaStream_t stream, S
         RT_TRY(cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream));
         RT_TRY(cudaStreamSynchronize(stream));
         if (!hostCounters[1]) break;
-        cudaFree(table); cudaFree(slotIndex); cudaFree(values);
+        rt::deviceFree(table); rt::deviceFree(slotIndex); rt::deviceFree(values);
         table = nullptr; slotIndex = nullptr; values = nullptr;
         if ((unsigned long long)cap * 4 > (1ull << 31)) { error = "too many distinct colour values"; e = cudaErrorInvalidValue; goto done; }
         cap *= 4;
@@ -241,11 +241,11 @@ cudaError_t uploadScene(const void* triangles, int count, cudaStream_t stream, S
     R.lightArea = area;
 #undef RT_TRY
 done:
-    cudaFree(table); cudaFree(slotIndex); cudaFree(values); cudaFree(counters); cudaFree(blockCounts);
-    cudaFree(decoded); cudaFree(emitterArea); cudaFree(emitterTri);
+    rt::deviceFree(table); rt::deviceFree(slotIndex); rt::deviceFree(values); rt::deviceFree(counters); rt::deviceFree(blockCounts);
+    rt::deviceFree(decoded); rt::deviceFree(emitterArea); rt::deviceFree(emitterTri);
     if (e != cudaSuccess) {
-        cudaFree(dTris);
-        cudaFree(dLights);
+        rt::deviceFree(dTris);
+        rt::deviceFree(dLights);
         if (error.empty()) error = std::string("scene upload: ") + cudaGetErrorString(e);
         return e;
     }

@@ -92,6 +92,85 @@ RT_HD float quantum(unsigned w, unsigned b) {
 #endif
 }
 
+#ifdef __CUDA_ARCH__
+// Two floats in one 64-bit register pair and their packed arithmetic (one
+// instruction for both, each rounded like the scalar operation).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Plane distances q * a + b of children b0 and b0 + 1 (bytes of w).
+__device__ __forceinline__ unsigned long long planes2(unsigned w, unsigned b0, unsigned long long a, unsigned long long b) {
+    const unsigned long long q = pack2(__uint_as_float(__byte_perm(w, 0x4B000000u, b0 | 0x7440u)),
+                                       __uint_as_float(__byte_perm(w, 0x4B000000u, (b0 + 1u) | 0x7440u)));
+    return fma2(add2(q, pack2(-8388608.0f, -8388608.0f)), a, b);
+}
+// intersectWideNode for rays without axis-parallel components (parMask 0):
+// the same operations, two children per packed instruction, and the meta
+// bytes of four children decoded at once (Ylitie, Karras and Laine 2017).
+// About 230 instructions against 300 for one child at a time; traversal
+// issues 70% of its cycles, so they are what it is bound by.
+__device__ __forceinline__ unsigned wideNodeMask(const uint4& w0, const uint4& w1, const uint4& w2, const uint4& w3,
+                                                 const uint4& w4, const RaySetup& r, float tmax) {
+    const float sx = bitsToFloat((w0.w & 0xFFu) << 23), sy = bitsToFloat(((w0.w >> 8) & 0xFFu) << 23),
+                sz = bitsToFloat(((w0.w >> 16) & 0xFFu) << 23);
+    const float ax = sx * r.inv.x, ay = sy * r.inv.y, az = sz * r.inv.z;
+    const float bx = (bitsToFloat(w0.x) - r.o.x) * r.inv.x, by = (bitsToFloat(w0.y) - r.o.y) * r.inv.y,
+                bz = (bitsToFloat(w0.z) - r.o.z) * r.inv.z;
+    const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+    const unsigned long long bx2 = pack2(bx, bx), by2 = pack2(by, by), bz2 = pack2(bz, bz);
+    const bool nx = r.inv.x < 0.0f, ny = r.inv.y < 0.0f, nz = r.inv.z < 0.0f;
+    const unsigned oct4 = r.octInv * 0x01010101u;
+    unsigned mask = 0;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const unsigned loX = half ? w2.y : w2.x, hiX = half ? w3.w : w3.z;
+        const unsigned loY = half ? w2.w : w2.z, hiY = half ? w4.y : w4.x;
+        const unsigned loZ = half ? w3.y : w3.x, hiZ = half ? w4.w : w4.z;
+        const unsigned nearX = nx ? hiX : loX, farX = nx ? loX : hiX;
+        const unsigned nearY = ny ? hiY : loY, farY = ny ? loY : hiY;
+        const unsigned nearZ = nz ? hiZ : loZ, farZ = nz ? loZ : hiZ;
+        // Interior children are the meta bytes with bits 3 and 4 set; their
+        // bit positions are flipped into the ray's front-to-back order.
+        const unsigned meta4 = half ? w1.w : w1.z;
+        const unsigned inner4 = ((meta4 & (meta4 << 1)) >> 4 & 0x01010101u) * 255u;
+        const unsigned index4 = (meta4 ^ (oct4 & inner4)) & 0x1F1F1F1Fu, bits4 = (meta4 >> 5) & 0x07070707u;
+#pragma unroll
+        for (unsigned b = 0; b < 4; b += 2) {
+            float tn[3][2], tf[3][2];
+            unpack2(planes2(nearX, b, ax2, bx2), tn[0][0], tn[0][1]);
+            unpack2(planes2(nearY, b, ay2, by2), tn[1][0], tn[1][1]);
+            unpack2(planes2(nearZ, b, az2, bz2), tn[2][0], tn[2][1]);
+            unpack2(planes2(farX, b, ax2, bx2), tf[0][0], tf[0][1]);
+            unpack2(planes2(farY, b, ay2, by2), tf[1][0], tf[1][1]);
+            unpack2(planes2(farZ, b, az2, bz2), tf[2][0], tf[2][1]);
+#pragma unroll
+            for (unsigned c = 0; c < 2; c++) {
+                const float tmin = fmaxf(fmaxf(tn[0][c], tn[1][c]), fmaxf(tn[2][c], 0.0f));
+                const float tmaxc = fminf(fminf(tf[0][c], tf[1][c]), fminf(tf[2][c], tmax));
+                const unsigned bits = (bits4 >> (8 * (b + c))) & 0xFFu, index = (index4 >> (8 * (b + c))) & 0xFFu;
+                if (tmin <= tmaxc) mask |= bits << index;
+            }
+        }
+    }
+    return mask;
+}
+#endif
+
 // Tests the eight child boxes of a wide node against [0, tmax]. Returns the
 // node's hit mask: bits 24-31 interior children (octant-ordered), bits 0-23
 // triangles relative to triBase. Also returns childBase/triBase/imask.
@@ -103,6 +182,14 @@ RT_HD unsigned intersectWideNode(const uint4* node, const RaySetup& r, float tma
                                  unsigned& triBase, unsigned& imask) {
     uint4 w0 = loadVec(node + 0), w1 = loadVec(node + 1), w2 = loadVec(node + 2), w3 = loadVec(node + 3),
           w4 = loadVec(node + 4);
+#ifdef __CUDA_ARCH__
+    if (r.parMask == 0u) {
+        imask = w0.w >> 24;
+        childBase = w1.x;
+        triBase = w1.y;
+        return wideNodeMask(w0, w1, w2, w3, w4, r, tmax);
+    }
+#endif
     float px = bitsToFloat(w0.x), py = bitsToFloat(w0.y), pz = bitsToFloat(w0.z);
     float sx = bitsToFloat((w0.w & 0xFFu) << 23), sy = bitsToFloat(((w0.w >> 8) & 0xFFu) << 23),
           sz = bitsToFloat(((w0.w >> 16) & 0xFFu) << 23);

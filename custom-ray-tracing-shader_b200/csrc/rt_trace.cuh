@@ -25,42 +25,15 @@ namespace rt {
 constexpr int kSharedStack = 8;
 constexpr int kTraceBlock = 128;
 
-// Per-lane traversal state.
+// Per-lane traversal state in registers. The ray's origin and direction for
+// triangle tests and its best hit live in WarpTriangles, where any lane of
+// the warp may test for it; tmax mirrors the best hit's distance.
 struct LaneRay {
     RaySetup r;
-    Hit hit;
+    float tmax;
     uint2 group, triGroup;
     int top;
 };
-
-// root: index of the ray's root node (0 for a single scene; the scene's
-// first node when several scenes share one node array).
-__device__ __forceinline__ void laneStart(LaneRay& L, float3 o, float3 d, float limit, unsigned root) {
-    L.r = setupRay(o, d);
-    L.hit = Hit{-1, limit, 0.0f, 0.0f};
-    L.group = make_uint2(root, 0x80000000u);
-    L.triGroup = make_uint2(0u, 0u);
-    L.top = 0;
-}
-
-// Triangle step: tests the highest pending triangle of the lane's group.
-// Returns true when an any-hit query is answered.
-template <bool ANY>
-__device__ __forceinline__ bool triangleStep(LaneRay& L, const float4* tris) {
-    int bit = 31 - __clz(L.triGroup.y);
-    L.triGroup.y &= ~(1u << bit);
-    const float4* t = tris + (size_t)(L.triGroup.x + (unsigned)bit) * 3;
-    float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
-    float u, v, dist = intersectTriangle(L.r.o, L.r.d, a, b, c, u, v);
-    if (dist > 0) {
-        int index = __float_as_int(c.z);
-        if (dist < L.hit.distance || (dist == L.hit.distance && index < L.hit.index)) {
-            L.hit.index = index; L.hit.distance = dist; L.hit.u = u; L.hit.v = v;
-            if (ANY) return true;
-        }
-    }
-    return false;
-}
 
 // Node step, taken when the lane has no pending triangles: pops an entry if
 // the current group has no interior children left, then visits one child
@@ -85,34 +58,28 @@ __device__ __forceinline__ bool nodeStep(LaneRay& L, const uint4* nodes, uint2* 
         L.top++;
     }
     unsigned childBase, triBase, imask;
-    unsigned mask = intersectWideNode(nodes + (size_t)child * 5, L.r, L.hit.distance, childBase, triBase, imask);
+    unsigned mask = intersectWideNode(nodes + (size_t)child * 5, L.r, L.tmax, childBase, triBase, imask);
     L.group = make_uint2(childBase, (mask & 0xFF000000u) | imask);
     L.triGroup = make_uint2(triBase, mask & 0x00FFFFFFu);
     return false;
 }
 
-// Per-warp shared scratch of the cooperative triangle phase.
+// Per-warp shared state of the cooperative triangle phase: the rays in flight
+// (written when a lane fetches one) and each round's pending triangles.
+// 1,888 bytes per warp: with the stacks a block of 4 warps takes 15,744
+// bytes, so that 8 blocks stay within 132 KB of the SM's storage and leave
+// the rest to L1.
 struct WarpTriangles {
     float4 origin[32];              // each lane's ray origin
     float4 dir[32];                 // each lane's ray direction
     unsigned long long best[32];    // (distance bits << 32 | index) of each lane's best hit
     float2 uv[32];                  // barycentrics of that hit
-    unsigned end[32];               // inclusive prefix sum of pending triangle counts
     uint2 group[32];                // each lane's pending triangle group
+    unsigned short start[32];       // exclusive prefix sum of pending triangle counts
+    unsigned char owner[32];        // lanes with pending triangles, in lane order
 };
 constexpr size_t traceSharedBytes(int block) {
     return sizeof(uint2) * kSharedStack * block + sizeof(WarpTriangles) * (block / 32);
-}
-
-// Position of the k-th (0-based) set bit of m; m has more than k set bits.
-__device__ __forceinline__ unsigned selectBit(unsigned m, unsigned k) {
-    unsigned pos = 0;
-#pragma unroll
-    for (unsigned width = 16; width > 0; width >>= 1) {
-        unsigned low = __popc(m & ((1u << width) - 1u));
-        if (k >= low) { k -= low; m >>= width; pos += width; }
-    }
-    return pos;
 }
 
 // Key ordering hits like the reference's acceptance rule (renderer.cu:153):
@@ -125,45 +92,66 @@ __device__ __forceinline__ unsigned long long hitKey(float distance, int index) 
     return ((unsigned long long)__float_as_uint(distance) << 32) | (unsigned)(index < 0 ? 0 : index);
 }
 
+// root: index of the ray's root node (0 for a single scene; the scene's
+// first node when several scenes share one node array).
+__device__ __forceinline__ void laneStart(LaneRay& L, float3 o, float3 d, float limit, unsigned root, WarpTriangles& W,
+                                          unsigned lane) {
+    L.r = setupRay(o, d);
+    L.tmax = limit;
+    L.group = make_uint2(root, 0x80000000u);
+    L.triGroup = make_uint2(0u, 0u);
+    L.top = 0;
+    W.origin[lane] = make_float4(o.x, o.y, o.z, 0.0f);
+    W.dir[lane] = make_float4(d.x, d.y, d.z, 0.0f);
+    W.best[lane] = hitKey(limit, -1);
+    W.uv[lane] = make_float2(0.0f, 0.0f);
+}
+
 // Cooperative triangle phase: the warp's pending triangles (all lanes' groups)
 // are dealt out one per lane per iteration; each candidate hit is merged into
 // its ray's best with a shared-memory 64-bit atomicMin on hitKey. The result
 // is the minimum over the same candidate set as testing them one by one, so
-// it equals the sequential outcome. Returns true for a lane whose any-hit
-// query is answered.
-template <bool ANY>
+// it equals the sequential outcome. Returns true for a lane whose best hit
+// changed (any-hit: the query is answered).
+//
+// Dealing: counts are below 32, so their prefix sums come from one ballot per
+// bit of the counts; of a round's work items, item w belongs to the last
+// owner whose first item is at or before w, found from the mask of first
+// items by a population count.
 __device__ __forceinline__ bool warpTrianglePhase(LaneRay& L, bool busy, const float4* tris, WarpTriangles& W,
-                                                  unsigned lane) {
+                                                  unsigned lane, unsigned below) {
+    const unsigned full = 0xFFFFFFFFu;
     const unsigned count = busy ? __popc(L.triGroup.y) : 0u;
-    unsigned incl = count;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        unsigned v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-        if ((int)lane >= off) incl += v;
+    const unsigned pending = __ballot_sync(full, count != 0u);
+    if (pending == 0u) return false;
+    const unsigned b0 = __ballot_sync(full, count & 1u), b1 = __ballot_sync(full, count & 2u),
+                   b2 = __ballot_sync(full, count & 4u);
+    unsigned excl = __popc(b0 & below) + 2u * __popc(b1 & below) + 4u * __popc(b2 & below);
+    unsigned total = __popc(b0) + 2u * __popc(b1) + 4u * __popc(b2);
+    if (__any_sync(full, count > 7u)) {
+        const unsigned b3 = __ballot_sync(full, count & 8u), b4 = __ballot_sync(full, count & 16u);
+        excl += 8u * __popc(b3 & below) + 16u * __popc(b4 & below);
+        total += 8u * __popc(b3) + 16u * __popc(b4);
     }
-    const unsigned total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    if (total == 0u) return false;
-    const unsigned long long key0 = busy ? hitKey(L.hit.distance, L.hit.index) : ~0ull;
-    W.origin[lane] = make_float4(L.r.o.x, L.r.o.y, L.r.o.z, 0.0f);
-    W.dir[lane] = make_float4(L.r.d.x, L.r.d.y, L.r.d.z, 0.0f);
-    W.best[lane] = key0;
-    W.end[lane] = incl;
-    W.group[lane] = busy ? L.triGroup : make_uint2(0u, 0u);
+    if (count) {
+        W.group[lane] = L.triGroup;
+        W.start[lane] = (unsigned short)excl;
+        W.owner[__popc(pending & below)] = (unsigned char)lane;
+    }
     __syncwarp();
+    unsigned before = 0u;  // owners whose first item lies before this iteration's items
     for (unsigned base = 0; base < total; base += 32u) {
-        const unsigned w = base + lane;
+        const unsigned first = excl - base;
+        const unsigned heads = __reduce_or_sync(full, count && first < 32u ? 1u << first : 0u);
         unsigned long long key = ~0ull;
         unsigned owner = 0;
         float u = 0.0f, v = 0.0f;
-        if (w < total) {
-            unsigned pos = 0;
-#pragma unroll
-            for (unsigned step = 16; step > 0; step >>= 1)
-                if (W.end[pos + step - 1] <= w) pos += step;
-            owner = pos;
+        if (base + lane < total) {
+            owner = W.owner[before + __popc(heads & (below | (1u << lane))) - 1u];
             const uint2 g = W.group[owner];
-            const unsigned bit = selectBit(g.y, w - (W.end[owner] - __popc(g.y)));
-            const float4* t = tris + (size_t)(g.x + bit) * 3;
+            unsigned m = g.y;
+            for (unsigned skip = base + lane - W.start[owner]; skip; skip--) m &= m - 1u;
+            const float4* t = tris + (size_t)(g.x + (unsigned)(__ffs(m) - 1)) * 3;
             float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
             float4 o4 = W.origin[owner], d4 = W.dir[owner];
             float dist = intersectTriangle(v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z), a, b, c, u, v);
@@ -172,24 +160,21 @@ __device__ __forceinline__ bool warpTrianglePhase(LaneRay& L, bool busy, const f
                 if (k < W.best[owner]) { atomicMin(&W.best[owner], k); key = k; }
             }
         }
+        before += __popc(heads);
         __syncwarp();
         if (key != ~0ull && W.best[owner] == key) W.uv[owner] = make_float2(u, v);
         __syncwarp();
     }
-    bool answered = false;
-    if (busy) {
-        const unsigned long long b = W.best[lane];
-        if (b != key0) {
-            L.hit.distance = __uint_as_float((unsigned)(b >> 32));
-            L.hit.index = (int)(unsigned)(b & 0xFFFFFFFFull);
-            const float2 uv = W.uv[lane];
-            L.hit.u = uv.x; L.hit.v = uv.y;
-            answered = ANY;
-        }
+    bool changed = false;
+    if (count) {
+        // A first hit lies below the limit; a later one at an equal distance
+        // (a smaller index) changes nothing here.
+        const float distance = __uint_as_float((unsigned)(W.best[lane] >> 32));
+        changed = distance < L.tmax;
+        L.tmax = distance;
         L.triGroup.y = 0u;
     }
-    __syncwarp();
-    return answered;
+    return changed;
 }
 
 // Persistent query loop over `count` rays of an IO object providing
@@ -218,7 +203,13 @@ __device__ __forceinline__ void persistentTrace(IO& io, int count, const uint4* 
     const unsigned below = (1u << lane) - 1u;
     LaneRay L;
     int k = -1, overflow = 0;
-    bool drained = false;
+    bool drained = false, hit = false;
+    // The lane's finished query: its best hit, or none within the limit.
+    auto finish = [&]() {
+        const unsigned long long b = W.best[lane];
+        const float2 uv = W.uv[lane];
+        io.store(k, Hit{hit ? (int)(unsigned)(b & 0xFFFFFFFFull) : -1, __uint_as_float((unsigned)(b >> 32)), uv.x, uv.y});
+    };
     unsigned finished = 0;
     for (;;) {
         if (!drained) {
@@ -236,8 +227,9 @@ __device__ __forceinline__ void persistentTrace(IO& io, int count, const uint4* 
                         unsigned root = 0;
                         io.load(mine, o, d, limit, root);
                         if (limit > 0.0f) {
-                            laneStart(L, o, d, limit, root);
+                            laneStart(L, o, d, limit, root, W, lane);
                             k = mine;
+                            hit = false;
                         } else {
                             // No distance can be accepted (limit <= 0 or NaN):
                             // the reference's answer is "no hit" at once.
@@ -251,13 +243,9 @@ __device__ __forceinline__ void persistentTrace(IO& io, int count, const uint4* 
         if (!__any_sync(0xFFFFFFFFu, k >= 0)) break;
         const int threshold = drained ? 1 : refill;
         for (;;) {
-            if (warpTrianglePhase<ANY>(L, k >= 0, tris, W, lane)) {
-                io.store(k, L.hit);
-                k = -1;
-                finished++;
-            }
-            if (k >= 0 && nodeStep(L, nodes, sstack, stride, lstack, overflow, stackLimit)) {
-                io.store(k, L.hit);
+            if (warpTrianglePhase(L, k >= 0, tris, W, lane, below)) hit = true;
+            if (k >= 0 && ((ANY && hit) || nodeStep(L, nodes, sstack, stride, lstack, overflow, stackLimit))) {
+                finish();
                 k = -1;
                 finished++;
             }

@@ -30,6 +30,7 @@
 #include "rt_render.cuh"
 #include "rt_trace.cuh"
 #include "rt_upload.cuh"
+#include "rt_wavefront.cuh"
 
 namespace rt {
 namespace {
@@ -90,6 +91,7 @@ __global__ void batchSobolKernel(const unsigned* dirs, const unsigned* sample, i
 }
 
 __global__ void batchGenerateKernel(BatchWave A, WavefrontBuffers B) {
+    initCounts(B, A.n);
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= A.n) return;
     const unsigned g = batchPixel(A, p);
@@ -99,59 +101,47 @@ __global__ void batchGenerateKernel(BatchWave A, WavefrontBuffers B) {
     const int x = (int)(local % (unsigned)V.w), y = (int)(local / (unsigned)V.w);
     Sampler rng{A.F.passXor + batchRow(A, p) * kSobolDims, A.F.seedHash, local, 0u};
     PathState st = startPath(V.cam, A.F.set, x, y, V.w, V.h, rng);
-    B.pathA[p] = make_float4(st.origin.x, st.origin.y, st.origin.z, 0.0f);
-    B.pathB[p] = make_float4(st.dir.x, st.dir.y, st.dir.z, __int_as_float(v));
-    B.pathC[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    B.radiance[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.albedo[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.normal[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.queue[0][p] = p;
-    if (p == 0) { B.counts[0] = A.n; B.counts[1] = 0; B.counts[2] = 0; }
+    storeStart(B, p, st, __int_as_float(v));
 }
 
 // Closest hit for every queued path; each ray starts at its scene's root.
 struct BatchExtendIO {
-    const int* queue;
+    const int* queue;  // null: every path
     const float4 *pathA, *pathB;
     float4* hits;
     const BatchView* views;
     const BatchScene* scenes;
+    __device__ int path(int k) const { return queue ? queue[k] : k; }
     __device__ void load(int k, float3& o, float3& d, float& limit, unsigned& root) const {
-        int p = queue[k];
+        int p = path(k);
         float4 a = pathA[p], b = pathB[p];
         o = v3(a.x, a.y, a.z); d = v3(b.x, b.y, b.z); limit = 1e30f;
         root = scenes[views[__float_as_int(b.w)].scene].root;
     }
     __device__ void store(int k, const Hit& h) const {
-        hits[queue[k]] = make_float4(h.distance, h.u, h.v, __int_as_float(h.index));
+        hits[path(k)] = make_float4(h.distance, h.u, h.v, __int_as_float(h.index));
     }
 };
 // Traversal kernels are compiled for 1,024 resident threads per SM (64
 // registers), as the single-scene ones.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batchExtendKernel(const uint4* wide, const float4* packed,
-                                                           WavefrontBuffers B, int q, const BatchView* views,
+                                                           WavefrontBuffers B, int bounce, const BatchView* views,
                                                            const BatchScene* scenes, unsigned long long* counter,
                                                            int* errorFlag, int refill) {
-    BatchExtendIO io{B.queue[q], B.pathA, B.pathB, B.hits, views, scenes};
-    persistentTrace<false>(io, B.counts[q], wide, packed, &B.counts[3], counter, errorFlag, kStackCapacity, refill);
+    BatchExtendIO io{bounceQueue(B, bounce), B.pathA, B.pathB, B.hits, views, scenes};
+    int* c = bounceCounts(B, bounce);
+    persistentTrace<false>(io, c[kLive], wide, packed, &c[kExtendFetch], counter, errorFlag, kStackCapacity, refill);
 }
 
-// Appends to a queue with one atomic per warp.
-__device__ __forceinline__ int warpAppend(int* counter, bool want) {
-    unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
-    if (!mask) return -1;
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xFFFFFFFFu, base, leader);
-    return want ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
-}
-
-__global__ void batchShadeKernel(BatchWave A, WavefrontBuffers B, int q, int bounce) {
-    int count = B.counts[q];
-    int nq = q ^ 1;
+// Blocks as shadeKernel's (rt_render.cu).
+constexpr int kBatchShadeBlock = 128, kBatchShadePerSm = 6;
+__global__ void __launch_bounds__(kBatchShadeBlock, kBatchShadePerSm) batchShadeKernel(BatchWave A, WavefrontBuffers B, int bounce) {
+    int* c = bounceCounts(B, bounce);
+    const int count = c[kLive];
+    const bool first = bounce == 0;
+    const int* queue = bounceQueue(B, bounce);
+    int* next = B.queue[(bounce + 1) & 1];
     int stride = gridDim.x * blockDim.x;
     int limit = ((count + 31) / 32) * 32;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < limit; k += stride) {
@@ -161,44 +151,26 @@ __global__ void batchShadeKernel(BatchWave A, WavefrontBuffers B, int q, int bou
         unsigned root = 0;
         ShadowRequest req;
         if (valid) {
-            p = B.queue[q][k];
-            float4 a = B.pathA[p], b = B.pathB[p], c = B.pathC[p], rad = B.radiance[p], hv = B.hits[p];
+            p = queue ? queue[k] : k;
+            float4 b = B.pathB[p], hv = B.hits[p];
             const int v = __float_as_int(b.w);
             const BatchView& V = A.F.views[v];
             const BatchScene& S = A.F.scenes[V.scene];
             root = S.root;
-            PathState st;
-            st.origin = v3(a.x, a.y, a.z); st.prevPdf = a.w;
-            st.dir = v3(b.x, b.y, b.z);
-            st.throughput = v3(c.x, c.y, c.z);
-            st.radiance = v3(rad.x, rad.y, rad.z); st.covered = __float_as_uint(rad.w);
-            float4 al = B.albedo[p], no = B.normal[p];
-            st.albedo = v3(al.x, al.y, al.z); st.normal = v3(no.x, no.y, no.z);
-            st.depth = al.w;
+            PathState st = loadPath(B, p, first, B.pathA[p], b);
+            const float3 before = st.radiance;
             Hit h{__float_as_int(hv.w), hv.x, hv.y, hv.z};
             const unsigned local = batchPixel(A, p) - V.pixelStart;
             Sampler rng{A.F.passXor + batchRow(A, p) * kSobolDims, A.F.seedHash, local, 4u + 8u * (unsigned)bounce};
             unsigned f = shadeBounce(S.view, A.F.set, bounce, st, h, rng, req);
             cont = (f & kContinue) != 0;
             shadow = (f & kShadow) != 0;
-            B.pathA[p] = make_float4(st.origin.x, st.origin.y, st.origin.z, st.prevPdf);
-            B.pathB[p] = make_float4(st.dir.x, st.dir.y, st.dir.z, __int_as_float(v));
-            B.pathC[p] = make_float4(st.throughput.x, st.throughput.y, st.throughput.z, 0.0f);
-            B.radiance[p] = make_float4(st.radiance.x, st.radiance.y, st.radiance.z, __uint_as_float(st.covered));
-            if (bounce == 0) {
-                B.albedo[p] = make_float4(st.albedo.x, st.albedo.y, st.albedo.z, st.depth);
-                B.normal[p] = make_float4(st.normal.x, st.normal.y, st.normal.z, 0.0f);
-            }
+            storePath(B, p, first, st, before, cont, __int_as_float(v));
         }
-        int slot = warpAppend(&B.counts[nq], cont);
-        if (slot >= 0) B.queue[nq][slot] = p;
-        int sslot = warpAppend(&B.counts[2], shadow);
-        if (sslot >= 0) {
-            B.shadowRay[sslot] = make_float4(req.origin.x, req.origin.y, req.origin.z, req.limit);
-            B.shadowDir[sslot] = make_float4(req.dir.x, req.dir.y, req.dir.z, __int_as_float(p));
-            B.shadowContrib[sslot] =
-                make_float4(req.contribution.x, req.contribution.y, req.contribution.z, __uint_as_float(root));
-        }
+        int slot = warpAppend(&c[kCountStride + kLive], cont);
+        if (slot >= 0) next[slot] = p;
+        int sslot = warpAppend(&c[kShadowRays], shadow);
+        if (sslot >= 0) storeShadow(B, sslot, req, p, __uint_as_float(root));
     }
 }
 
@@ -220,34 +192,28 @@ struct BatchShadowIO {
 };
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batchShadowKernel(const uint4* wide, const float4* packed,
-                                                           WavefrontBuffers B, unsigned long long* counter,
+                                                           WavefrontBuffers B, int bounce, unsigned long long* counter,
                                                            int* errorFlag, int refill) {
     BatchShadowIO io{B.shadowRay, B.shadowDir, B.shadowContrib, B.radiance};
-    persistentTrace<true>(io, B.counts[2], wide, packed, &B.counts[4], counter, errorFlag, kStackCapacity, refill);
+    int* c = bounceCounts(B, bounce);
+    persistentTrace<true>(io, c[kShadowRays], wide, packed, &c[kShadowFetch], counter, errorFlag, kStackCapacity, refill);
 }
 
-__global__ void batchResetQueuesKernel(WavefrontBuffers B, int q) {
-    if (threadIdx.x == 0) { B.counts[q ^ 1] = 0; B.counts[2] = 0; B.counts[3] = 0; B.counts[4] = 0; }
-}
-
-// Adds paths [firstPath, firstPath + count) of the wave (all of one sample
-// row) to their pixels; the rows of a wave are added by successive launches.
-__global__ void batchAccumulateKernel(BatchWave A, WavefrontBuffers B, int firstPath, int count) {
-    int p = firstPath + blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= firstPath + count) return;
-    const size_t i = batchPixel(A, p);
-    const int row = batchRow(A, p);
+// Adds the wave's paths to their pixels, one thread per pixel in sample order
+// (see accumulateKernel in rt_render.cu).
+__global__ void batchAccumulateKernel(BatchWave A, WavefrontBuffers B) {
+    const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= min((unsigned)A.n, A.pixels)) return;
+    const size_t i = batchPixel(A, (int)j);
+    const int row0 = batchRow(A, (int)j);
     const unsigned sample0 = *A.F.sample;
-    const bool first = row == 0 && sample0 == 0;
+    const bool first = row0 == 0 && sample0 == 0;
     Accum total = first ? Accum{v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0), 0u} : A.F.sums[i];
     float depthTotal = first ? 0.0f : A.F.depthSums[i];
-    float4 rad = B.radiance[p], al = B.albedo[p], no = B.normal[p];
-    PathState st;
-    st.radiance = v3(rad.x, rad.y, rad.z); st.covered = __float_as_uint(rad.w);
-    st.albedo = v3(al.x, al.y, al.z); st.normal = v3(no.x, no.y, no.z);
-    addPath(total, st);
+    int row = row0 - 1;
+    for (long long p = j; p < A.n; p += A.pixels, row++) addStored(B, (int)p, total, depthTotal);
     A.F.sums[i] = total;
-    A.F.depthSums[i] = depthTotal + al.w;
+    A.F.depthSums[i] = depthTotal;
     if (row == A.F.set.raysPerPixel - 1)
         A.F.pixels[i] = displayPixel(total, sample0 + (unsigned)A.F.set.raysPerPixel, A.F.set.exposure);
 }
@@ -358,17 +324,17 @@ template <int BLOCK> int TraceLaunch<BLOCK>::extendBlocks = 0;
 template <int BLOCK> int TraceLaunch<BLOCK>::shadowBlocks = 0;
 
 template <int BLOCK>
-void launchTraversal(bool shadow, const uint4* wide, const float4* packed, const WavefrontBuffers& B, int q,
+void launchTraversal(bool shadow, const uint4* wide, const float4* packed, const WavefrontBuffers& B, int bounce,
                      const BatchView* views, const BatchScene* scenes, unsigned long long* counter, int* errorFlag,
                      int refill, cudaStream_t stream) {
     TraceLaunch<BLOCK>::configure();
     const size_t smem = traceSharedBytes(BLOCK);
     if (shadow)
-        batchShadowKernel<BLOCK><<<TraceLaunch<BLOCK>::shadowBlocks, BLOCK, smem, stream>>>(wide, packed, B, counter,
+        batchShadowKernel<BLOCK><<<TraceLaunch<BLOCK>::shadowBlocks, BLOCK, smem, stream>>>(wide, packed, B, bounce, counter,
                                                                                             errorFlag, refill);
     else
         batchExtendKernel<BLOCK><<<TraceLaunch<BLOCK>::extendBlocks, BLOCK, smem, stream>>>(
-            wide, packed, B, q, views, scenes, counter, errorFlag, refill);
+            wide, packed, B, bounce, views, scenes, counter, errorFlag, refill);
 }
 
 }  // namespace
@@ -404,6 +370,7 @@ struct Batch {
     std::vector<BatchViewData> views;
     // Arenas of all scenes and the tables the kernels read.
     SceneTri* aTris = nullptr;
+    float4* aShade = nullptr;  // aTris on 128-byte boundaries (SceneView::shade)
     uint4* aWide = nullptr;
     float4* aPacked = nullptr;
     Light* aLights = nullptr;
@@ -455,10 +422,10 @@ void dropGraph(Batch* b) {
 }
 
 void freeArena(Batch* b) {
-    void* owned[] = {b->aTris, b->aWide, b->aPacked, b->aLights, b->dScenes};
+    void* owned[] = {b->aTris, b->aShade, b->aWide, b->aPacked, b->aLights, b->dScenes};
     for (void* p : owned)
         if (p) rt::deviceFree(p);
-    b->aTris = nullptr; b->aWide = nullptr; b->aPacked = nullptr; b->aLights = nullptr; b->dScenes = nullptr;
+    b->aTris = nullptr; b->aShade = nullptr; b->aWide = nullptr; b->aPacked = nullptr; b->aLights = nullptr; b->dScenes = nullptr;
     b->arenaReady = false;
     dropGraph(b);
 }
@@ -541,6 +508,7 @@ bool ensureArena(Batch* b) {
     }
     cudaError_t e;
     if ((e = rt::deviceAlloc(&b->aTris, sizeof(SceneTri) * tris)) != cudaSuccess) return failB(b, e, "arena");
+    if ((e = rt::deviceAlloc(&b->aShade, sizeof(float4) * 8 * tris)) != cudaSuccess) return failB(b, e, "arena");
     if ((e = rt::deviceAlloc(&b->aWide, sizeof(uint4) * 5 * nodes)) != cudaSuccess) return failB(b, e, "arena");
     if ((e = rt::deviceAlloc(&b->aPacked, sizeof(float4) * 3 * packedCount)) != cudaSuccess) return failB(b, e, "arena");
     if ((e = rt::deviceAlloc(&b->aLights, sizeof(Light) * std::max<size_t>(lights, 1))) != cudaSuccess) return failB(b, e, "arena");
@@ -563,9 +531,10 @@ bool ensureArena(Batch* b) {
         if ((e = cudaGetLastError()) != cudaSuccess) return failB(b, e);
         for (const Light& L : S.lights) allLights.push_back(Light{L.triangle + (int)S.triBase, L.cumulativeArea});
         SceneView view{b->aTris, b->aWide, b->aPacked, b->aLights + S.lightBase, (int)S.lights.size(), S.lightArea,
-                       S.build.wideDepth, b->environmentMode, b->environment};
+                       S.build.wideDepth, b->environmentMode, b->environment, kStackCapacity, 0u, b->aShade};
         table.push_back(BatchScene{view, S.nodeBase});
     }
+    if ((e = padTriangles(b->aTris, tris, b->aShade, b->stream)) != cudaSuccess) return failB(b, e);
     if (!allLights.empty() &&
         (e = cudaMemcpyAsync(b->aLights, allLights.data(), sizeof(Light) * allLights.size(), cudaMemcpyHostToDevice,
                              b->stream)) != cudaSuccess) return failB(b, e);
@@ -705,7 +674,7 @@ cudaError_t enqueueFrame(Batch* b, const Settings& set, int* launches) {
         return cudaGetLastError();
     }
     const int cap = b->wave.capacity;
-    const int shadeBlocks = deviceSms() * (2048 / 256);
+    const int shadeBlocks = deviceSms() * kBatchShadePerSm;
     if (nLanes > 1) {
         if ((e = cudaEventRecord(b->fork, main)) != cudaSuccess) return e;
         for (int k = 1; k < nLanes; k++)
@@ -720,36 +689,27 @@ cudaError_t enqueueFrame(Batch* b, const Settings& set, int* launches) {
             BatchWave A{F, start, (unsigned)b->pixels, (int)std::min<unsigned long long>((unsigned long long)cap, total - start)};
             batchGenerateKernel<<<blocksFor(A.n, 256), 256, 0, s>>>(A, W);
             n++;
-            int q = 0;
             for (int bounce = 0; bounce < set.maxBounces; bounce++) {
-                batchResetQueuesKernel<<<1, 32, 0, s>>>(W, q);
                 unsigned long long* rays = &b->dCounters[bounce == 0 ? 0 : 1];
                 switch (b->block) {
-                    case 64: launchTraversal<64>(false, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
-                    case 256: launchTraversal<256>(false, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
-                    default: launchTraversal<128>(false, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
+                    case 64: launchTraversal<64>(false, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
+                    case 256: launchTraversal<256>(false, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
+                    default: launchTraversal<128>(false, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, rays, b->dError, b->refill, s); break;
                 }
-                batchShadeKernel<<<shadeBlocks, 256, 0, s>>>(A, W, q, bounce);
+                batchShadeKernel<<<shadeBlocks, kBatchShadeBlock, 0, s>>>(A, W, bounce);
                 unsigned long long* shadowRays = &b->dCounters[2];
                 switch (b->block) {
-                    case 64: launchTraversal<64>(true, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
-                    case 256: launchTraversal<256>(true, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
-                    default: launchTraversal<128>(true, b->aWide, b->aPacked, W, q, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
+                    case 64: launchTraversal<64>(true, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
+                    case 256: launchTraversal<256>(true, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
+                    default: launchTraversal<128>(true, b->aWide, b->aPacked, W, bounce, b->dViews, b->dScenes, shadowRays, b->dError, b->refill, s); break;
                 }
-                n += 4;
-                q ^= 1;
+                n += 3;
             }
             // Samples of a pixel are added in sample order, whichever lane
             // ran the previous wave.
             if (nLanes > 1 && wave > 0 && (e = cudaStreamWaitEvent(s, b->accumulated, 0)) != cudaSuccess) return e;
-            for (int first = 0; first < A.n;) {
-                const long long rowEnd = (long long)((A.start + (unsigned)first) / b->pixels + 1) * (long long)b->pixels -
-                                         (long long)A.start;
-                const int count = (int)std::min<long long>(rowEnd, A.n) - first;
-                batchAccumulateKernel<<<blocksFor(count, 256), 256, 0, s>>>(A, W, first, count);
-                first += count;
-                n++;
-            }
+            batchAccumulateKernel<<<blocksFor(std::min<long long>(A.n, (long long)b->pixels), 256), 256, 0, s>>>(A, W);
+            n++;
             if (nLanes > 1 && (e = cudaEventRecord(b->accumulated, s)) != cudaSuccess) return e;
         }
     }

@@ -74,7 +74,37 @@ struct SceneView {
     float3 environment;      // the constant radiance of mode 1
     int stackLimit = kStackCapacity;  // traversal stack entries before the overflow error
     unsigned root = 0;                // root node of the scene's wide tree (its first node in a batch arena)
+    const float4* shade = nullptr;    // device: tris on 128-byte boundaries, 8 float4 each (padTriangles)
 };
+
+// Triangle i of the scene. Shading threads read scattered triangles: on the
+// device they come from the 128-byte records as up to eight 16-byte loads (the
+// ABI's 116-byte records allow 4-byte loads only, about 27 per hit).
+RT_HD SceneTri sceneTriangle(const SceneView& sc, int i) {
+#ifdef __CUDA_ARCH__
+    const float4* r = sc.shade + (size_t)i * 8;
+    float4 q[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) q[k] = __ldg(r + k);
+    SceneTri t;
+    t.origin = v3(q[0].x, q[0].y, q[0].z);
+    t.edge1 = v3(q[0].w, q[1].x, q[1].y);
+    t.edge2 = v3(q[1].z, q[1].w, q[2].x);
+    t.color = v3(q[2].y, q[2].z, q[2].w);
+    t.emission = q[3].x;
+    t.oneSided = __float_as_int(q[3].y);
+    t.normal0 = v3(q[3].z, q[3].w, q[4].x);
+    t.normal1 = v3(q[4].y, q[4].z, q[4].w);
+    t.normal2 = v3(q[5].x, q[5].y, q[5].z);
+    t.mesh = __float_as_int(q[5].w);
+    t.specularColor = v3(q[6].x, q[6].y, q[6].z);
+    t.smoothness = q[6].w;
+    t.specularProbability = q[7].x;
+    return t;
+#else
+    return sc.tris[i];
+#endif
+}
 
 // ---- BRDF and sky (renderer.cu:181-196) ----
 RT_HD float phongExponent(const SceneTri& t) {
@@ -158,7 +188,7 @@ RT_HD unsigned shadeBounce(const SceneView& sc, const Settings& set, int bounce,
         if (bounce > 0) st.radiance = add(st.radiance, mul(st.throughput, environmentRadiance(sc, st.dir, set.skyStrength)));
         return 0;
     }
-    const SceneTri& t = sc.tris[hit.index];
+    const SceneTri t = sceneTriangle(sc, hit.index);
     float3 g = normalize(cross(t.edge1, t.edge2));
     if (dot(g, st.dir) > 0) g = scale(g, -1.0f);
     if (bounce == 0) {
@@ -194,7 +224,7 @@ RT_HD unsigned shadeBounce(const SceneView& sc, const Settings& set, int bounce,
             if (pick >= sc.lights[mid].cumulativeArea) l = mid + 1;
             else hi = mid;
         }
-        const SceneTri& L = sc.tris[sc.lights[l].triangle];
+        const SceneTri L = sceneTriangle(sc, sc.lights[l].triangle);
         float root = sqrtf(rng(1)), v = rng(2);
         float3 target = add(L.origin, add(scale(L.edge1, root * (1.0f - v)), scale(L.edge2, root * v)));
         float3 off = sub(target, st.origin);

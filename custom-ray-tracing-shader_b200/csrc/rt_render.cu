@@ -12,10 +12,12 @@
 //  - one kernel per pixel (megakernel), the reference's launch shape with the
 //    same traversal and shading code.
 // Traversal stacks live in shared memory, one column per thread.
+#include <algorithm>
 #include <vector>
 
 #include "rt_render.cuh"
 #include "rt_trace.cuh"
+#include "rt_wavefront.cuh"
 
 namespace rt {
 namespace {
@@ -76,58 +78,49 @@ __device__ __forceinline__ int waveRow(const WaveArgs& A, int p) { return (A.sta
 __device__ __forceinline__ int wavePixel(const WaveArgs& A, int p) { return (A.start + p) % (A.L.w * A.L.h); }
 
 __global__ void generateKernel(WaveArgs A, WavefrontBuffers B) {
+    initCounts(B, A.n);
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= A.n) return;
     int pix = wavePixel(A, p);
     int x = pix % A.L.w, y = pix / A.L.w;
     Sampler rng{A.L.passXor + waveRow(A, p) * kSobolDims, A.L.seedHash, (unsigned)pix, 0u};
     PathState st = startPath(A.L.cam, A.L.set, x, y, A.L.w, A.L.h, rng);
-    B.pathA[p] = make_float4(st.origin.x, st.origin.y, st.origin.z, 0.0f);
-    B.pathB[p] = make_float4(st.dir.x, st.dir.y, st.dir.z, 0.0f);
-    B.pathC[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    B.radiance[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.albedo[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.normal[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.queue[0][p] = p;
-    if (p == 0) { B.counts[0] = A.n; B.counts[1] = 0; B.counts[2] = 0; }
+    storeStart(B, p, st, 0.0f);
 }
 
 // Closest hit for every queued path (persistent, dynamic fetch).
 struct ExtendIO {
-    const int* queue;
+    const int* queue;  // null: every path
     const float4 *pathA, *pathB;
     float4* hits;
+    __device__ int path(int k) const { return queue ? queue[k] : k; }
     __device__ void load(int k, float3& o, float3& d, float& limit, unsigned&) const {
-        int p = queue[k];
+        int p = path(k);
         float4 a = pathA[p], b = pathB[p];
         o = v3(a.x, a.y, a.z); d = v3(b.x, b.y, b.z); limit = 1e30f;
     }
     __device__ void store(int k, const Hit& h) const {
-        hits[queue[k]] = make_float4(h.distance, h.u, h.v, __int_as_float(h.index));
+        hits[path(k)] = make_float4(h.distance, h.u, h.v, __int_as_float(h.index));
     }
 };
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) extendKernel(const uint4* wide, const float4* packed, WavefrontBuffers B,
-                                                            int q, unsigned long long* counter, int* errorFlag,
+                                                            int bounce, unsigned long long* counter, int* errorFlag,
                                                             int stackLimit, int refill) {
-    ExtendIO io{B.queue[q], B.pathA, B.pathB, B.hits};
-    persistentTrace<false>(io, B.counts[q], wide, packed, &B.counts[3], counter, errorFlag, stackLimit, refill);
+    ExtendIO io{bounceQueue(B, bounce), B.pathA, B.pathB, B.hits};
+    int* c = bounceCounts(B, bounce);
+    persistentTrace<false>(io, c[kLive], wide, packed, &c[kExtendFetch], counter, errorFlag, stackLimit, refill);
 }
 
-// Appends to a queue with one atomic per warp.
-__device__ __forceinline__ int warpAppend(int* counter, bool want) {
-    unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
-    if (!mask) return -1;
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xFFFFFFFFu, base, leader);
-    return want ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
-}
-
-__global__ void shadeKernel(WaveArgs A, WavefrontBuffers B, int q, int bounce) {
-    int count = B.counts[q];
-    int nq = q ^ 1;
+// Shading blocks: 6 of 128 threads per SM (80 registers; left alone the kernel
+// takes 92 and 2 blocks of 256 fit). On the 1M-triangle pass 33.9 ms at 2 x
+// 256, 33.4 at 5 x 128, 33.1 at 6 x 128, 33.3 at 8 x 128.
+constexpr int kShadeBlock = 128, kShadePerSm = 6;
+__global__ void __launch_bounds__(kShadeBlock, kShadePerSm) shadeKernel(WaveArgs A, WavefrontBuffers B, int bounce) {
+    int* c = bounceCounts(B, bounce);
+    const int count = c[kLive];
+    const bool first = bounce == 0;
+    const int* queue = bounceQueue(B, bounce);
+    int* next = B.queue[(bounce + 1) & 1];
     int stride = gridDim.x * blockDim.x;
     int limit = ((count + 31) / 32) * 32;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < limit; k += stride) {
@@ -136,39 +129,22 @@ __global__ void shadeKernel(WaveArgs A, WavefrontBuffers B, int q, int bounce) {
         int p = 0;
         ShadowRequest req;
         if (valid) {
-            p = B.queue[q][k];
-            float4 a = B.pathA[p], b = B.pathB[p], c = B.pathC[p], rad = B.radiance[p], hv = B.hits[p];
-            PathState st;
-            st.origin = v3(a.x, a.y, a.z); st.prevPdf = a.w;
-            st.dir = v3(b.x, b.y, b.z);
-            st.throughput = v3(c.x, c.y, c.z);
-            st.radiance = v3(rad.x, rad.y, rad.z); st.covered = __float_as_uint(rad.w);
-            float4 al = B.albedo[p], no = B.normal[p];
-            st.albedo = v3(al.x, al.y, al.z); st.normal = v3(no.x, no.y, no.z);
-            st.depth = al.w;
+            p = queue ? queue[k] : k;
+            float4 hv = B.hits[p];
+            PathState st = loadPath(B, p, first, B.pathA[p], B.pathB[p]);
+            const float3 before = st.radiance;
             Hit h{__float_as_int(hv.w), hv.x, hv.y, hv.z};
             Sampler rng{A.L.passXor + waveRow(A, p) * kSobolDims, A.L.seedHash, (unsigned)wavePixel(A, p),
                         4u + 8u * (unsigned)bounce};
             unsigned f = shadeBounce(A.L.scene, A.L.set, bounce, st, h, rng, req);
             cont = (f & kContinue) != 0;
             shadow = (f & kShadow) != 0;
-            B.pathA[p] = make_float4(st.origin.x, st.origin.y, st.origin.z, st.prevPdf);
-            B.pathB[p] = make_float4(st.dir.x, st.dir.y, st.dir.z, 0.0f);
-            B.pathC[p] = make_float4(st.throughput.x, st.throughput.y, st.throughput.z, 0.0f);
-            B.radiance[p] = make_float4(st.radiance.x, st.radiance.y, st.radiance.z, __uint_as_float(st.covered));
-            if (bounce == 0) {
-                B.albedo[p] = make_float4(st.albedo.x, st.albedo.y, st.albedo.z, st.depth);
-                B.normal[p] = make_float4(st.normal.x, st.normal.y, st.normal.z, 0.0f);
-            }
+            storePath(B, p, first, st, before, cont, 0.0f);
         }
-        int slot = warpAppend(&B.counts[nq], cont);
-        if (slot >= 0) B.queue[nq][slot] = p;
-        int sslot = warpAppend(&B.counts[2], shadow);
-        if (sslot >= 0) {
-            B.shadowRay[sslot] = make_float4(req.origin.x, req.origin.y, req.origin.z, req.limit);
-            B.shadowDir[sslot] = make_float4(req.dir.x, req.dir.y, req.dir.z, __int_as_float(p));
-            B.shadowContrib[sslot] = make_float4(req.contribution.x, req.contribution.y, req.contribution.z, 0.0f);
-        }
+        int slot = warpAppend(&c[kCountStride + kLive], cont);
+        if (slot >= 0) next[slot] = p;
+        int sslot = warpAppend(&c[kShadowRays], shadow);
+        if (sslot >= 0) storeShadow(B, sslot, req, p, 0.0f);
     }
 }
 
@@ -189,34 +165,30 @@ struct ShadowIO {
     }
 };
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) shadowKernel(const uint4* wide, const float4* packed, WavefrontBuffers B,
-                                                            unsigned long long* counter, int* errorFlag,
+                                                            int bounce, unsigned long long* counter, int* errorFlag,
                                                             int stackLimit, int refill) {
     ShadowIO io{B.shadowRay, B.shadowDir, B.shadowContrib, B.radiance};
-    persistentTrace<true>(io, B.counts[2], wide, packed, &B.counts[4], counter, errorFlag, stackLimit, refill);
+    int* c = bounceCounts(B, bounce);
+    persistentTrace<true>(io, c[kShadowRays], wide, packed, &c[kShadowFetch], counter, errorFlag, stackLimit, refill);
 }
 
-__global__ void resetQueuesKernel(WavefrontBuffers B, int q) {
-    if (threadIdx.x == 0) { B.counts[q ^ 1] = 0; B.counts[2] = 0; B.counts[3] = 0; B.counts[4] = 0; }
-}
-
-// Adds paths [first, first + count) of the wave (all of one sample row) to
-// their pixels' sums; the rows of a wave are added by successive launches, so
-// each pixel's samples are added in sample order.
-__global__ void accumulateKernel(WaveArgs A, WavefrontBuffers B, int firstPath, int count) {
-    int p = firstPath + blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= firstPath + count) return;
-    size_t i = (size_t)wavePixel(A, p);
-    const int row = waveRow(A, p);
-    const bool first = row == 0 && A.L.sample0 == 0;
+// Adds the wave's paths to their pixels' sums. A thread owns the pixel of
+// path j < pixels and adds its paths j, j + pixels, ... in order, so each
+// pixel's samples are added in sample order and its sums are read and written
+// once per wave (88 bytes, not once per sample row).
+__global__ void accumulateKernel(WaveArgs A, WavefrontBuffers B) {
+    const int pixels = A.L.w * A.L.h;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= min(A.n, pixels)) return;
+    const size_t i = (size_t)wavePixel(A, j);
+    const int row0 = waveRow(A, j);
+    const bool first = row0 == 0 && A.L.sample0 == 0;
     Accum total = first ? Accum{v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0), 0u} : A.L.sums[i];
     float depthTotal = first ? 0.0f : A.L.depthSums[i];
-    float4 rad = B.radiance[p], al = B.albedo[p], no = B.normal[p];
-    PathState st;
-    st.radiance = v3(rad.x, rad.y, rad.z); st.covered = __float_as_uint(rad.w);
-    st.albedo = v3(al.x, al.y, al.z); st.normal = v3(no.x, no.y, no.z);
-    addPath(total, st);
+    int row = row0 - 1;
+    for (long long p = j; p < A.n; p += pixels, row++) addStored(B, (int)p, total, depthTotal);
     A.L.sums[i] = total;
-    A.L.depthSums[i] = depthTotal + al.w;
+    A.L.depthSums[i] = depthTotal;
     if (row == A.L.set.raysPerPixel - 1)
         A.L.pixels[i] = displayPixel(total, A.L.sample0 + (unsigned)A.L.set.raysPerPixel, A.L.set.exposure);
 }
@@ -332,10 +304,6 @@ int smCount() {
     }
     return sms;
 }
-int persistentBlocks(int blockSize) {
-    int perSm = 2048 / blockSize;
-    return smCount() * (perSm > 0 ? perSm : 1);
-}
 // Resident blocks of a traversal kernel, for a grid of exactly one wave.
 template <class K>
 int traceBlocks(K kernel, size_t smem) {
@@ -357,7 +325,7 @@ cudaError_t allocWavefront(WavefrontBuffers& b, int capacity) {
     RT_ALLOC(b.radiance, n); RT_ALLOC(b.albedo, n); RT_ALLOC(b.normal, n); RT_ALLOC(b.hits, n);
     RT_ALLOC(b.queue[0], n); RT_ALLOC(b.queue[1], n);
     RT_ALLOC(b.shadowRay, n); RT_ALLOC(b.shadowDir, n); RT_ALLOC(b.shadowContrib, n);
-    RT_ALLOC(b.counts, 8);
+    RT_ALLOC(b.counts, kWaveCounts);
 #undef RT_ALLOC
     b.capacity = capacity;
     return cudaSuccess;
@@ -401,7 +369,7 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const Tr
     const size_t smem = kTraceSmem;
     const int stackLimit = tuning.stackLimit;
     const int refill = tuning.refill;
-    int shadeBlocks = persistentBlocks(256);
+    const int shadeBlocks = smCount() * kShadePerSm;
     int pixels = L.w * L.h;
     int n = 0;
     static thread_local std::vector<cudaEvent_t> pool;
@@ -436,35 +404,26 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const Tr
             WaveArgs A{L, start, total - start < B.capacity ? total - start : B.capacity};
             generateKernel<<<blocks(A.n, 256), 256, 0, ws>>>(A, W);
             n++;
-            int q = 0;
             for (int bounce = 0; bounce < L.set.maxBounces; bounce++) {
-                resetQueuesKernel<<<1, 32, 0, ws>>>(W, q);
                 Mark m{nullptr, nullptr, bounce == 0 ? 0 : 1};
                 if (timing) { m.a = event(ev++); m.b = event(ev++); cudaEventRecord(m.a, ws); }
-                extendKernel<<<extendBlocks, kTraceBlock, smem, ws>>>(L.scene.wide, L.scene.packed, W, q,
+                extendKernel<<<extendBlocks, kTraceBlock, smem, ws>>>(L.scene.wide, L.scene.packed, W, bounce,
                                                                       &L.counters[bounce == 0 ? 0 : 1], L.errorFlag,
                                                                       stackLimit, refill);
                 if (timing) { cudaEventRecord(m.b, ws); marks.push_back(m); }
-                shadeKernel<<<shadeBlocks, 256, 0, ws>>>(A, W, q, bounce);
+                shadeKernel<<<shadeBlocks, kShadeBlock, 0, ws>>>(A, W, bounce);
                 Mark s{nullptr, nullptr, 2};
                 if (timing) { s.a = event(ev++); s.b = event(ev++); cudaEventRecord(s.a, ws); }
-                shadowKernel<<<shadowBlocks, kTraceBlock, smem, ws>>>(L.scene.wide, L.scene.packed, W, &L.counters[2],
-                                                                      L.errorFlag, stackLimit, refill);
+                shadowKernel<<<shadowBlocks, kTraceBlock, smem, ws>>>(L.scene.wide, L.scene.packed, W, bounce,
+                                                                      &L.counters[2], L.errorFlag, stackLimit, refill);
                 if (timing) { cudaEventRecord(s.b, ws); marks.push_back(s); }
-                n += 4;
-                q ^= 1;
+                n += 3;
             }
             // Samples of a pixel are added in sample order: after the
             // previous wave's accumulation, whichever lane ran it.
-            // Within the wave, one launch per sample row it covers.
             if (two && wave > 0) cudaStreamWaitEvent(ws, overlap->accumulated, 0);
-            for (int first = 0; first < A.n;) {
-                const int rowEnd = ((A.start + first) / pixels + 1) * pixels - A.start;
-                const int count = (rowEnd < A.n ? rowEnd : A.n) - first;
-                accumulateKernel<<<blocks(count, 256), 256, 0, ws>>>(A, W, first, count);
-                first += count;
-                n++;
-            }
+            accumulateKernel<<<blocks(std::min(A.n, pixels), 256), 256, 0, ws>>>(A, W);
+            n++;
             if (two) cudaEventRecord(overlap->accumulated, ws);
         }
     }

@@ -28,17 +28,17 @@ struct RenderLaunch {
 struct WavefrontBuffers {
     int capacity = 0;
     float4* pathA = nullptr;     // origin.xyz, prevPdf
-    float4* pathB = nullptr;     // dir.xyz, pixel index (bits)
-    float4* pathC = nullptr;     // throughput.xyz, sample row r (bits)
+    float4* pathB = nullptr;     // dir.xyz, the batch's view (bits)
+    float4* pathC = nullptr;     // throughput.xyz
     float4* radiance = nullptr;  // radiance.xyz, covered (bits)
-    float4* albedo = nullptr;    // albedo.xyz
+    float4* albedo = nullptr;    // albedo.xyz, first-hit distance
     float4* normal = nullptr;    // normal.xyz
-    float4* hits = nullptr;      // per queue slot: distance, u, v, index (bits)
+    float4* hits = nullptr;      // distance, u, v, index (bits)
     int* queue[2] = {nullptr, nullptr};   // active path ids, ping-pong
     float4* shadowRay = nullptr;      // origin.xyz, limit
     float4* shadowDir = nullptr;      // dir.xyz, path id (bits)
     float4* shadowContrib = nullptr;  // contribution.xyz
-    int* counts = nullptr;            // [0..1] queue sizes, [2] shadow queue size, [3..4] fetch counters
+    int* counts = nullptr;            // queue sizes and fetch positions per bounce (rt_wavefront.cuh)
 };
 
 // Speed-only knobs of the persistent traversal kernels.

@@ -90,6 +90,7 @@ struct Session {
     cudaStream_t stream = nullptr;
     cudaEvent_t start = nullptr, stop = nullptr;
     SceneTri* dTris = nullptr;
+    float4* dShade = nullptr;     // dTris on 128-byte boundaries (SceneView::shade)
     Light* dLights = nullptr;
     unsigned* dDirs = nullptr;
     unsigned* dPassXor = nullptr;
@@ -182,11 +183,11 @@ void releaseScene(Session* s) {
     s->pieceBuild = BuildResult{};
     freeWavefront(s->wave);
     releaseOverlap(s);
-    void* owned[] = {s->dTris, s->dLights, s->dDirs, s->dPassXor, s->dSeedHash, s->dSum, s->dDepth, s->dPixels,
+    void* owned[] = {s->dTris, s->dShade, s->dLights, s->dDirs, s->dPassXor, s->dSeedHash, s->dSum, s->dDepth, s->dPixels,
                      s->dCounters, s->dError, s->dDenoise};
     for (void* p : owned)
         if (p) rt::deviceFree(p);
-    s->dTris = nullptr; s->dLights = nullptr; s->dDirs = nullptr; s->dPassXor = nullptr; s->dSeedHash = nullptr;
+    s->dTris = nullptr; s->dShade = nullptr; s->dLights = nullptr; s->dDirs = nullptr; s->dPassXor = nullptr; s->dSeedHash = nullptr;
     s->dSum = nullptr; s->dDepth = nullptr; s->dPixels = nullptr; s->dCounters = nullptr; s->dError = nullptr;
     s->dDenoise = nullptr;
     if (s->start) cudaEventDestroy(s->start);
@@ -221,7 +222,7 @@ bool validSettings(const RenderSettings* st) {
 
 SceneView deviceView(Session* s) {
     return SceneView{s->dTris, travWide(s), travPacked(s), s->dLights, s->lightCount, s->lightArea,
-                     travBuild(s).wideDepth, s->environmentMode, s->environment, s->tuning.stackLimit};
+                     travBuild(s).wideDepth, s->environmentMode, s->environment, s->tuning.stackLimit, 0u, s->dShade};
 }
 
 // Paths per wave: RTX_TUNE_PATHS_IN_FLIGHT (default kDefaultPathsInFlight),
@@ -482,6 +483,8 @@ int RtInitialize(void* p, const Triangle* triangles, int count, int width, int h
     s->triCount = count;
     s->lightCount = s->upload.lightCount;
     s->lightArea = s->upload.lightArea;
+    RT_CHECK(rt::deviceAlloc(&s->dShade, sizeof(float4) * 8 * (size_t)count));
+    RT_CHECK(padTriangles(s->dTris, (size_t)count, s->dShade, s->stream));
     RT_CHECK(rt::deviceAlloc(&s->dDirs, sizeof(unsigned) * kSobolDims * 32));
     RT_CHECK(cudaMemcpyAsync(s->dDirs, dirs, sizeof(unsigned) * kSobolDims * 32, cudaMemcpyHostToDevice, s->stream));
     RT_CHECK(rt::deviceAlloc(&s->dPassXor, sizeof(unsigned) * 16 * kSobolDims));

@@ -42,10 +42,8 @@ __device__ __forceinline__ bool nodeStep(LaneRay& L, const uint4* nodes, uint2* 
                                          int& overflow, int stackLimit) {
     if (L.group.y <= 0x00FFFFFFu) {
         if (L.top == 0) return true;
-        L.top--;
-        uint2 g = L.top < kSharedStack ? sstack[L.top * stride] : lstack[L.top - kSharedStack];
-        if (g.y <= 0x00FFFFFFu) { L.triGroup = g; L.group = make_uint2(0u, 0u); return false; }
-        L.group = g;
+        L.top--;  // only groups with interior children are pushed
+        L.group = L.top < kSharedStack ? sstack[L.top * stride] : lstack[L.top - kSharedStack];
     }
     int bit = 31 - __clz(L.group.y & 0xFF000000u);
     L.group.y &= ~(1u << bit);

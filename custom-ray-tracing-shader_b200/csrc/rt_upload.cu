@@ -155,6 +155,16 @@ __global__ void cumulativeAreaKernel(const int* emitterTri, const float* emitter
     if (lane == 0) *totalArea = carry;
 }
 
+__global__ void padTrianglesKernel(const SceneTri* tris, size_t count, float4* out) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count * 8) return;
+    constexpr int kWords = (int)sizeof(SceneTri) / 4;
+    const float* w = reinterpret_cast<const float*>(tris + i / 8);
+    const int k = (int)(i % 8) * 4;
+    out[i] = make_float4(w[k], k + 1 < kWords ? w[k + 1] : 0.0f, k + 2 < kWords ? w[k + 2] : 0.0f,
+                         k + 3 < kWords ? w[k + 3] : 0.0f);
+}
+
 inline int gridFor(long long n, int block) { return (int)((n + block - 1) / block); }
 
 }  // namespace
@@ -253,6 +263,11 @@ done:
     *dLightsOut = dLights;
     R.ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return cudaSuccess;
+}
+
+cudaError_t padTriangles(const SceneTri* tris, size_t count, float4* out, cudaStream_t stream) {
+    padTrianglesKernel<<<gridFor((long long)count * 8, kBlock), kBlock, 0, stream>>>(tris, count, out);
+    return cudaGetLastError();
 }
 
 }  // namespace rt

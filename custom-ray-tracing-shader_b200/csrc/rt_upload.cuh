@@ -38,4 +38,8 @@ struct UploadResult {
 cudaError_t uploadScene(const void* triangles, int count, cudaStream_t stream, SceneTri** dTris, Light** dLights,
                         UploadResult& result, std::string& error);
 
+// The shading copy of prepared triangles (SceneView::shade): the same words
+// on 128-byte boundaries, 8 float4 per triangle.
+cudaError_t padTriangles(const SceneTri* tris, size_t count, float4* out, cudaStream_t stream);
+
 }  // namespace rt

@@ -29,9 +29,21 @@ constexpr int kTileX = 16, kTileY = 8, kMegaBlock = kTileX * kTileY;
 // registers) 2,841 Mrays/s, 7 (72) 2,972, 8 (64) 3,003.
 constexpr int kTraceMinBlocks = 8;
 
+// Programmatic dependent launch of a pass's stages (launchStage): a stage lets
+// the next one's blocks start as its own leave the SMs and waits for the
+// previous stage before it touches memory.
+__device__ __forceinline__ void stageBegin() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// Sampler tables of the pass; zeroes its ray counters and error flag (status:
+// kStatusWords words).
 __global__ void sobolTablesKernel(const unsigned* dirs, unsigned sample0, int rpp, unsigned seed, unsigned* passXor,
-                                  unsigned* seedHash) {
+                                  unsigned* seedHash, unsigned long long* status) {
+    stageBegin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kStatusWords) status[i] = 0ull;
     int passEntries = rpp * kSobolDims;
     if (i < passEntries) {
         int r = i / kSobolDims, d = i % kSobolDims;
@@ -78,6 +90,7 @@ __device__ __forceinline__ int waveRow(const WaveArgs& A, int p) { return (A.sta
 __device__ __forceinline__ int wavePixel(const WaveArgs& A, int p) { return (A.start + p) % (A.L.w * A.L.h); }
 
 __global__ void generateKernel(WaveArgs A, WavefrontBuffers B) {
+    stageBegin();
     initCounts(B, A.n);
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= A.n) return;
@@ -106,6 +119,7 @@ struct ExtendIO {
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) extendKernel(const uint4* wide, const float4* packed, WavefrontBuffers B,
                                                             int bounce, unsigned long long* counter, int* errorFlag,
                                                             int stackLimit, int refill) {
+    stageBegin();
     ExtendIO io{bounceQueue(B, bounce), B.pathA, B.pathB, B.hits};
     int* c = bounceCounts(B, bounce);
     persistentTrace<false>(io, c[kLive], wide, packed, &c[kExtendFetch], counter, errorFlag, stackLimit, refill);
@@ -116,6 +130,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) extendKernel(con
 // 256, 33.4 at 5 x 128, 33.1 at 6 x 128, 33.3 at 8 x 128.
 constexpr int kShadeBlock = 128, kShadePerSm = 6;
 __global__ void __launch_bounds__(kShadeBlock, kShadePerSm) shadeKernel(WaveArgs A, WavefrontBuffers B, int bounce) {
+    stageBegin();
     int* c = bounceCounts(B, bounce);
     const int count = c[kLive];
     const bool first = bounce == 0;
@@ -167,9 +182,31 @@ struct ShadowIO {
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) shadowKernel(const uint4* wide, const float4* packed, WavefrontBuffers B,
                                                             int bounce, unsigned long long* counter, int* errorFlag,
                                                             int stackLimit, int refill) {
+    stageBegin();
     ShadowIO io{B.shadowRay, B.shadowDir, B.shadowContrib, B.radiance};
     int* c = bounceCounts(B, bounce);
     persistentTrace<true>(io, c[kShadowRays], wide, packed, &c[kShadowFetch], counter, errorFlag, stackLimit, refill);
+}
+
+// The light samples of a bounce and the closest hits of the next in one
+// launch (they are independent: one adds to the paths' radiance, the other
+// reads their rays and writes hits): the warps that finish the closest hits
+// early go on with the shadow rays instead of idling through the launch's
+// drain, and a bounce is two launches instead of three.
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) shadowExtendKernel(const uint4* wide, const float4* packed,
+                                                                  WavefrontBuffers B, int bounce,
+                                                                  unsigned long long* shadowCounter,
+                                                                  unsigned long long* counter, int* errorFlag,
+                                                                  int stackLimit, int refill) {
+    stageBegin();
+    {
+        ExtendIO io{bounceQueue(B, bounce + 1), B.pathA, B.pathB, B.hits};
+        int* c = bounceCounts(B, bounce + 1);
+        persistentTrace<false>(io, c[kLive], wide, packed, &c[kExtendFetch], counter, errorFlag, stackLimit, refill);
+    }
+    ShadowIO io{B.shadowRay, B.shadowDir, B.shadowContrib, B.radiance};
+    int* c = bounceCounts(B, bounce);
+    persistentTrace<true>(io, c[kShadowRays], wide, packed, &c[kShadowFetch], shadowCounter, errorFlag, stackLimit, refill);
 }
 
 // Adds the wave's paths to their pixels' sums. A thread owns the pixel of
@@ -177,6 +214,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) shadowKernel(con
 // pixel's samples are added in sample order and its sums are read and written
 // once per wave (88 bytes, not once per sample row).
 __global__ void accumulateKernel(WaveArgs A, WavefrontBuffers B) {
+    stageBegin();
     const int pixels = A.L.w * A.L.h;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= min(A.n, pixels)) return;
@@ -314,6 +352,23 @@ int traceBlocks(K kernel, size_t smem) {
 }
 constexpr size_t kTraceSmem = traceSharedBytes(kTraceBlock);
 
+// Launches a stage; dependent: with programmatic stream serialization (see
+// stageBegin).
+template <class... P, class... A>
+void launchStage(bool dependent, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace
 
 cudaError_t allocWavefront(WavefrontBuffers& b, int capacity) {
@@ -339,9 +394,9 @@ void freeWavefront(WavefrontBuffers& b) {
 }
 
 cudaError_t buildSobolTables(const unsigned* dirs, unsigned sample0, int rpp, unsigned seed, unsigned* passXor,
-                             unsigned* seedHash, cudaStream_t stream) {
+                             unsigned* seedHash, unsigned long long* status, cudaStream_t stream) {
     int total = (rpp + 1) * kSobolDims;
-    sobolTablesKernel<<<blocks(total, 256), 256, 0, stream>>>(dirs, sample0, rpp, seed, passXor, seedHash);
+    sobolTablesKernel<<<blocks(total, 256), 256, 0, stream>>>(dirs, sample0, rpp, seed, passXor, seedHash, status);
     return cudaGetLastError();
 }
 
@@ -361,10 +416,11 @@ cudaError_t launchMegakernel(const RenderLaunch& L, cudaStream_t stream, int* la
 cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const TraceTuning& tuning, cudaStream_t stream,
                             int* launches, float* extendMs, float* shadowMs, bool timing, float* primaryMs,
                             const WaveOverlap* overlap) {
-    static int extendBlocks = 0, shadowBlocks = 0;
+    static int extendBlocks = 0, shadowBlocks = 0, bothBlocks = 0;
     if (!extendBlocks) {
-        extendBlocks = traceBlocks(extendKernel, kTraceSmem);
+        bothBlocks = traceBlocks(shadowExtendKernel, kTraceSmem);
         shadowBlocks = traceBlocks(shadowKernel, kTraceSmem);
+        extendBlocks = traceBlocks(extendKernel, kTraceSmem);
     }
     const size_t smem = kTraceSmem;
     const int stackLimit = tuning.stackLimit;
@@ -380,6 +436,12 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const Tr
         return pool[k];
     };
     size_t ev = 0;
+    const int total = pixels * L.set.raysPerPixel;  // paths of the pass (at most 4096^2 * 16 < 2^31)
+    // A pass of one wave has nothing on another lane to overlap with: its
+    // stages overlap with one another instead (dependent launches, shadow rays
+    // traced with the next bounce's closest hits), unless they are timed apart.
+    const bool single = total <= B.capacity, chained = single && !timing;
+    if (single) overlap = nullptr;
     int nLanes = overlap ? std::max(1, std::min(overlap->lanes, kMaxLanes)) : 1;
     for (int k = 1; k < nLanes; k++)
         if (!overlap->buffers[k - 1] || !overlap->streams[k - 1] || overlap->buffers[k - 1]->capacity != B.capacity)
@@ -396,14 +458,32 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const Tr
         for (int k = 1; k < nLanes; k++) cudaStreamWaitEvent(laneStream[k], overlap->fork, 0);
     }
     int wave = 0;
-    const int total = pixels * L.set.raysPerPixel;  // paths of the pass (at most 4096^2 * 16 < 2^31)
     {
         for (int start = 0; start < total; start += B.capacity, wave++) {
             WavefrontBuffers& W = *lanes[wave % nLanes];
             cudaStream_t ws = laneStream[wave % nLanes];
             WaveArgs A{L, start, total - start < B.capacity ? total - start : B.capacity};
-            generateKernel<<<blocks(A.n, 256), 256, 0, ws>>>(A, W);
+            launchStage(chained, generateKernel, blocks(A.n, 256), 256, 0, ws, A, W);
             n++;
+            if (chained) {
+                const uint4* wide = L.scene.wide;
+                const float4* packed = L.scene.packed;
+                unsigned long long* rays = L.counters;
+                launchStage(true, extendKernel, extendBlocks, kTraceBlock, smem, ws, wide, packed, W, 0, &rays[0], L.errorFlag,
+                            stackLimit, refill);
+                for (int bounce = 0; bounce < L.set.maxBounces; bounce++) {
+                    launchStage(true, shadeKernel, shadeBlocks, kShadeBlock, 0, ws, A, W, bounce);
+                    if (bounce + 1 < L.set.maxBounces)
+                        launchStage(true, shadowExtendKernel, bothBlocks, kTraceBlock, smem, ws, wide, packed, W, bounce, &rays[2],
+                                    &rays[1], L.errorFlag, stackLimit, refill);
+                    else
+                        launchStage(true, shadowKernel, shadowBlocks, kTraceBlock, smem, ws, wide, packed, W, bounce, &rays[2],
+                                    L.errorFlag, stackLimit, refill);
+                }
+                launchStage(true, accumulateKernel, blocks(std::min(A.n, pixels), 256), 256, 0, ws, A, W);
+                n += 2 + 2 * L.set.maxBounces;
+                break;
+            }
             for (int bounce = 0; bounce < L.set.maxBounces; bounce++) {
                 Mark m{nullptr, nullptr, bounce == 0 ? 0 : 1};
                 if (timing) { m.a = event(ev++); m.b = event(ev++); cudaEventRecord(m.a, ws); }

@@ -70,8 +70,11 @@ struct WaveOverlap {
 cudaError_t allocWavefront(WavefrontBuffers& b, int capacity);
 void freeWavefront(WavefrontBuffers& b);
 
+// status: kStatusWords words that the table kernel zeroes, four ray counters
+// (RenderLaunch::counters) and the error flag.
+constexpr int kStatusWords = 5;
 cudaError_t buildSobolTables(const unsigned* dirs, unsigned sample0, int rpp, unsigned seed, unsigned* passXor,
-                             unsigned* seedHash, cudaStream_t stream);
+                             unsigned* seedHash, unsigned long long* status, cudaStream_t stream);
 // One kernel per path: returns the number of kernel launches in *launches.
 cudaError_t launchMegakernel(const RenderLaunch& L, cudaStream_t stream, int* launches);
 // Wavefront: generate -> (extend -> shade -> shadow)* per wave. Timing of the

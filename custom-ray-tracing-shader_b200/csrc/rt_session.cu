@@ -98,7 +98,7 @@ struct Session {
     Accum* dSum = nullptr;
     float* dDepth = nullptr;      // running sums of first-hit distance (added AOV)
     uchar4* dPixels = nullptr;
-    unsigned long long* dCounters = nullptr;
+    unsigned long long* dCounters = nullptr;  // kStatusWords words, the last holding *dError and a query's fetch position
     int* dError = nullptr;
     float4* dDenoise = nullptr;
     BuiltBvh bvh;          // the reference's binary tree (RtBvhInfo, RtxExportBvh) and its wide collapse
@@ -184,7 +184,7 @@ void releaseScene(Session* s) {
     freeWavefront(s->wave);
     releaseOverlap(s);
     void* owned[] = {s->dTris, s->dShade, s->dLights, s->dDirs, s->dPassXor, s->dSeedHash, s->dSum, s->dDepth, s->dPixels,
-                     s->dCounters, s->dError, s->dDenoise};
+                     s->dCounters, s->dDenoise};
     for (void* p : owned)
         if (p) rt::deviceFree(p);
     s->dTris = nullptr; s->dShade = nullptr; s->dLights = nullptr; s->dDirs = nullptr; s->dPassXor = nullptr; s->dSeedHash = nullptr;
@@ -277,9 +277,7 @@ bool renderDevice(Session* s, const CameraData* camera, const RenderSettings* se
     // integrator's kernels.
     if (s->integrator != 1 && !ensureWave(s, set.raysPerPixel)) return false;
     if ((e = cudaEventRecord(s->start, s->stream)) != cudaSuccess) return fail(s, e);
-    if ((e = buildSobolTables(s->dDirs, s->samples, set.raysPerPixel, set.seed, s->dPassXor, s->dSeedHash, s->stream)) != cudaSuccess) return fail(s, e);
-    if ((e = cudaMemsetAsync(s->dCounters, 0, 4 * sizeof(unsigned long long), s->stream)) != cudaSuccess) return fail(s, e);
-    if ((e = cudaMemsetAsync(s->dError, 0, sizeof(int), s->stream)) != cudaSuccess) return fail(s, e);
+    if ((e = buildSobolTables(s->dDirs, s->samples, set.raysPerPixel, set.seed, s->dPassXor, s->dSeedHash, s->dCounters, s->stream)) != cudaSuccess) return fail(s, e);
     RenderLaunch L{deviceView(s), cam, set, s->width, s->height, s->samples, s->dPassXor, s->dSeedHash,
                    s->dSum, s->dDepth, s->dPixels, s->dCounters, s->dError};
     int launches = 0;
@@ -292,13 +290,11 @@ bool renderDevice(Session* s, const CameraData* camera, const RenderSettings* se
     }
     if (e != cudaSuccess) return fail(s, e);
     if ((e = cudaEventRecord(s->stop, s->stream)) != cudaSuccess) return fail(s, e);
-    if ((e = cudaEventSynchronize(s->stop)) != cudaSuccess) return fail(s, e);
+    unsigned long long counters[kStatusWords];
+    if ((e = cudaMemcpyAsync(counters, s->dCounters, sizeof(counters), cudaMemcpyDeviceToHost, s->stream)) != cudaSuccess) return fail(s, e);
+    if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return fail(s, e);
     if ((e = cudaEventElapsedTime(computeMs, s->start, s->stop)) != cudaSuccess) return fail(s, e);
-    unsigned long long counters[4];
-    int overflow = 0;
-    if ((e = cudaMemcpy(counters, s->dCounters, sizeof(counters), cudaMemcpyDeviceToHost)) != cudaSuccess) return fail(s, e);
-    if ((e = cudaMemcpy(&overflow, s->dError, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess) return fail(s, e);
-    if (overflow) return fail(s, cudaErrorUnknown, "BVH traversal stack overflow");
+    if ((int)counters[kStatusWords - 1]) return fail(s, cudaErrorUnknown, "BVH traversal stack overflow");
     s->stats.primaryRays = counters[0];
     s->stats.secondaryRays = counters[1];
     s->stats.shadowRays = counters[2];
@@ -492,8 +488,8 @@ int RtInitialize(void* p, const Triangle* triangles, int count, int width, int h
     RT_CHECK(rt::deviceAlloc(&s->dSum, sizeof(Accum) * (size_t)width * height));
     RT_CHECK(rt::deviceAlloc(&s->dDepth, sizeof(float) * (size_t)width * height));
     RT_CHECK(rt::deviceAlloc(&s->dPixels, sizeof(uchar4) * (size_t)width * height));
-    RT_CHECK(rt::deviceAlloc(&s->dCounters, 4 * sizeof(unsigned long long)));
-    RT_CHECK(rt::deviceAlloc(&s->dError, 2 * sizeof(int)));
+    RT_CHECK(rt::deviceAlloc(&s->dCounters, kStatusWords * sizeof(unsigned long long)));
+    s->dError = reinterpret_cast<int*>(s->dCounters + kStatusWords - 1);
     const char* why = nullptr;
     // The tree that is traced is built here: over triangle pieces when some
     // triangle is split, else the reference's own tree. The reference's tree

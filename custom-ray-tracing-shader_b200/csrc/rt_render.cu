@@ -232,19 +232,23 @@ __global__ void accumulateKernel(WaveArgs A, WavefrontBuffers B) {
 }
 
 // ---- per-ray queries, sampler values ----
+// Rays in the caller's records (RtxQuery: origin, direction, limit, 28 bytes)
+// and hits in RtxHit's layout, so neither side of a call is repacked.
 struct QueryIO {
-    const float4* q;
+    const float* q;
     float4* out;
     __device__ void load(int k, float3& o, float3& d, float& limit, unsigned&) const {
-        float4 a = q[2 * k], b = q[2 * k + 1];
-        o = v3(a.x, a.y, a.z); d = v3(a.w, b.x, b.y); limit = b.z;
+        const float* r = q + 7 * (size_t)k;
+        o = v3(__ldg(r), __ldg(r + 1), __ldg(r + 2));
+        d = v3(__ldg(r + 3), __ldg(r + 4), __ldg(r + 5));
+        limit = __ldg(r + 6);
     }
     __device__ void store(int k, const Hit& h) const {
         out[k] = make_float4(__int_as_float(h.index), h.distance, h.u, h.v);
     }
 };
 template <bool ANY>
-__global__ void __launch_bounds__(kTraceBlock) queryKernel(const uint4* wide, const float4* packed, const float4* q,
+__global__ void __launch_bounds__(kTraceBlock) queryKernel(const uint4* wide, const float4* packed, const float* q,
                                                            int count, float4* out, int* fetch, int* errorFlag,
                                                            int stackLimit, int refill) {
     QueryIO io{q, out};
@@ -528,23 +532,22 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& B, const Tr
     return e;
 }
 
-cudaError_t launchQueries(const uint4* wide, const float4* packed, const float4* queries, int count, int any,
-                          float4* hits, int* fetch, int* errorFlag, int wideDepth, const TraceTuning& tuning,
-                          cudaStream_t stream) {
-    (void)wideDepth;
+cudaError_t launchQueries(const uint4* wide, const float4* packed, const float* queries, int count, int any,
+                          float4* hits, int* status, const TraceTuning& tuning, cudaStream_t stream) {
     const int stackLimit = tuning.stackLimit;
     const int refill = tuning.refill;
-    cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(int), stream);
+    int *errorFlag = status, *fetch = status + 1;
+    cudaError_t e = cudaMemsetAsync(status, 0, 2 * sizeof(int), stream);
     if (e != cudaSuccess) return e;
-    if (any) {
-        static int blocks = traceBlocks(queryKernel<true>, kTraceSmem);
-        queryKernel<true><<<blocks, kTraceBlock, kTraceSmem, stream>>>(wide, packed, queries, count, hits, fetch, errorFlag,
-                                                                      stackLimit, refill);
-    } else {
-        static int blocks = traceBlocks(queryKernel<false>, kTraceSmem);
-        queryKernel<false><<<blocks, kTraceBlock, kTraceSmem, stream>>>(wide, packed, queries, count, hits, fetch, errorFlag,
-                                                                       stackLimit, refill);
-    }
+    // Up to four warps' worth of rays per SM run as blocks of one warp, spread
+    // over the SMs (4,096 rays: 128 SMs of one warp instead of 32 of four);
+    // more rays in blocks of 128, one wave of resident blocks at most.
+    const int block = count <= smCount() * kTraceBlock ? 32 : kTraceBlock;
+    const size_t smem = traceSharedBytes(block);
+    static int mostAny = traceBlocks(queryKernel<true>, kTraceSmem), most = traceBlocks(queryKernel<false>, kTraceSmem);
+    const int want = blocks(count, block), grid = block == 32 ? want : std::min(any ? mostAny : most, want);
+    (any ? queryKernel<true> : queryKernel<false>)<<<grid, block, smem, stream>>>(wide, packed, queries, count, hits, fetch,
+                                                                                 errorFlag, stackLimit, refill);
     return cudaGetLastError();
 }
 

@@ -83,10 +83,10 @@ cudaError_t launchWavefront(const RenderLaunch& L, WavefrontBuffers& b, const Tr
                             int* launches, float* extendMs, float* shadowMs, bool timing,
                             float* primaryMs = nullptr, const WaveOverlap* overlap = nullptr);
 
-// fetch: one device int of scratch (the work counter of the persistent kernel).
-cudaError_t launchQueries(const uint4* wide, const float4* packed, const float4* queries /*2 per query*/, int count,
-                          int any, float4* hits, int* fetch, int* errorFlag, int wideDepth, const TraceTuning& tuning,
-                          cudaStream_t stream);
+// queries: count records of 7 floats (RtxQuery); hits: RtxHit records; status:
+// two device ints, zeroed here: the error flag and the fetch position.
+cudaError_t launchQueries(const uint4* wide, const float4* packed, const float* queries, int count, int any,
+                          float4* hits, int* status, const TraceTuning& tuning, cudaStream_t stream);
 cudaError_t launchSobolSamples(const unsigned* dirs, const unsigned* pixel, const unsigned* sample, const unsigned* seed,
                                int count, int ndim, float* out, cudaStream_t stream);
 // Denoise: prepare guides from the running sums, filter, tonemap into pixels.

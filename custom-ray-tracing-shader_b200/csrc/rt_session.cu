@@ -611,32 +611,23 @@ int RtxQueryRays(void* p, const RtxQuery* queries, int count, int any, RtxHit* h
     if (!s->ready || !queries || !hits || count < 0) { s->error = cudaErrorInvalidValue; s->hostError = "RtxQueryRays: invalid arguments"; return 0; }
     if (count == 0) return 1;
     if (!useDevice(s)) return 0;
-    std::vector<float4> packed((size_t)count * 2);
-    for (int i = 0; i < count; i++) {
-        const RtxQuery& q = queries[i];
-        packed[2 * (size_t)i] = make_float4(q.origin.x, q.origin.y, q.origin.z, q.direction.x);
-        packed[2 * (size_t)i + 1] = make_float4(q.direction.y, q.direction.z, q.limit, 0.0f);
-    }
-    float4 *dq = nullptr, *dh = nullptr;
-    std::vector<float4> out((size_t)count);
+    // The records go to the device and the hits come back as they are.
+    float *dq = nullptr, *dh = nullptr;
     int overflow = 0;
-    cudaError_t e = rt::deviceAlloc(&dq, sizeof(float4) * packed.size());
-    if (e == cudaSuccess) e = rt::deviceAlloc(&dh, sizeof(float4) * (size_t)count);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dq, packed.data(), sizeof(float4) * packed.size(), cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->dError, 0, sizeof(int), s->stream);
-    if (e == cudaSuccess) e = launchQueries(travWide(s), travPacked(s), dq, count, any, dh, s->dError + 1, s->dError,
-                                            travBuild(s).wideDepth, s->tuning, s->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), dh, sizeof(float4) * (size_t)count, cudaMemcpyDeviceToHost, s->stream);
+    cudaError_t e = rt::deviceAlloc(&dq, sizeof(RtxQuery) * (size_t)count);
+    if (e == cudaSuccess) e = rt::deviceAlloc(&dh, sizeof(RtxHit) * (size_t)count);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dq, queries, sizeof(RtxQuery) * (size_t)count, cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = launchQueries(travWide(s), travPacked(s), dq, count, any, reinterpret_cast<float4*>(dh), s->dError,
+                                            s->tuning, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, s->dError, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess && !overflow) {
+        e = cudaMemcpyAsync(hits, dh, sizeof(RtxHit) * (size_t)count, cudaMemcpyDeviceToHost, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    }
     rt::deviceFree(dq); rt::deviceFree(dh);
     if (e != cudaSuccess) { fail(s, e); return 0; }
     if (overflow) { s->hostError = "BVH traversal stack overflow"; return 0; }
-    for (int i = 0; i < count; i++) {
-        int index;
-        std::memcpy(&index, &out[i].x, 4);
-        hits[i] = RtxHit{index, out[i].y, out[i].z, out[i].w};
-    }
     return 1;
 }
 
@@ -963,11 +954,10 @@ int RtxSetTuning(void* p, int key, int value) {
 namespace {
 
 constexpr int kStaticQueryRays = 16384;  // largest count one call accepts
-constexpr size_t kStaticPacked = 0;                                    // 2 float4 per ray, kernel layout
-constexpr size_t kStaticHits = 2 * (size_t)kStaticQueryRays;           // 1 float4 per ray, RtxHit layout
-constexpr size_t kStaticRaw = 3 * (size_t)kStaticQueryRays;            // caller's 28-byte RtxQuery records
-constexpr size_t kStaticCounters = kStaticRaw + (7 * (size_t)kStaticQueryRays + 3) / 4;  // work counter, error flag
-constexpr size_t kStaticFloat4s = kStaticCounters + 1;                 // 1,245,200 bytes in total
+constexpr size_t kStaticHits = 0;                                      // 1 float4 per ray, RtxHit layout
+constexpr size_t kStaticRaw = kStaticQueryRays;                        // caller's 28-byte RtxQuery records
+constexpr size_t kStaticCounters = kStaticRaw + (7 * (size_t)kStaticQueryRays + 3) / 4;  // error flag, fetch position
+constexpr size_t kStaticFloat4s = kStaticCounters + 1;                 // 720,912 bytes in total
 constexpr int kStaticMaxDevices = 64;
 
 // One copy per GPU that loads the library, held until the process exits.
@@ -996,15 +986,6 @@ float4* staticQueryScratch(int device, std::string& error) {
     return g_staticScratchAddress[device];
 }
 
-// 28-byte RtxQuery records -> the query kernel's two-float4 layout.
-__global__ void packStaticQueriesKernel(const float* raw, float4* packed, int count) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float* q = raw + 7 * (size_t)i;
-    packed[2 * (size_t)i] = make_float4(q[0], q[1], q[2], q[3]);
-    packed[2 * (size_t)i + 1] = make_float4(q[4], q[5], q[6], 0.0f);
-}
-
 }  // namespace
 
 extern "C" int RtxQueryRaysStatic(void* p, const RtxQuery* queries, int count, int any, RtxHit* hits) {
@@ -1026,24 +1007,16 @@ extern "C" int RtxQueryRaysStatic(void* p, const RtxQuery* queries, int count, i
     std::string why;
     float4* scratch = staticQueryScratch(s->device, why);
     if (!scratch) { s->hostError = why; return 0; }
-    float4* packed = scratch + kStaticPacked;
     float4* deviceHits = scratch + kStaticHits;
     float* raw = reinterpret_cast<float*>(scratch + kStaticRaw);
-    int* counters = reinterpret_cast<int*>(scratch + kStaticCounters);  // [0] work counter, [1] error flag
+    int* status = reinterpret_cast<int*>(scratch + kStaticCounters);  // error flag, fetch position
     int overflow = 0;
     e = cudaMemcpyAsync(raw, queries, sizeof(RtxQuery) * (size_t)count, cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) {
-        packStaticQueriesKernel<<<(count + 255) / 256, 256, 0, s->stream>>>(raw, packed, count);
-        e = cudaGetLastError();
-    }
-    // The array keeps the previous call's contents: clear the counters.
-    if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, 2 * sizeof(int), s->stream);
     if (e == cudaSuccess)
-        e = launchQueries(travWide(s), travPacked(s), packed, count, any, deviceHits, counters, counters + 1,
-                          travBuild(s).wideDepth, s->tuning, s->stream);
+        e = launchQueries(travWide(s), travPacked(s), raw, count, any, deviceHits, status, s->tuning, s->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hits, deviceHits, sizeof(RtxHit) * (size_t)count, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, counters + 1, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, status, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) { fail(s, e); return 0; }
     if (overflow) { s->hostError = "BVH traversal stack overflow"; return 0; }

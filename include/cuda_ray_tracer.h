@@ -371,7 +371,7 @@ int RtxBatchStatsGet(void* batch, RtxBatchStats* stats);
  * running beside a CUDA graph capture, latency-critical loops where
  * cudaMalloc/cudaFree would synchronise the device, hosts whose device memory
  * belongs to a pool). Rays and hits are staged in a file-scope device array
- * of 1,245,200 bytes (about 1.19 MiB) that every GPU loading the library
+ * of 720,912 bytes (about 0.69 MiB) that every GPU loading the library
  * keeps until the process exits; count may be at most 16384 per call (larger
  * counts return 0 with a message). The first call on each device looks up
  * that array's device address, so make it before any stream capture; the

@@ -275,35 +275,111 @@ __global__ void denoisePrepareKernel(const Accum* sums, unsigned samples, int co
     albedo[i] = make_float4(a.x, a.y, a.z, 0.0f);
     normal[i] = make_float4(n.x, n.y, n.z, 0.0f);
 }
-__global__ void atrousKernel(const float4* in, const float4* albedo, const float4* normal, float4* out, int w, int h,
-                             int step, float colorPhi) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const float kernel[3] = {3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
-    int i = y * w + x;
-    float4 c0 = in[i], a0 = albedo[i], n0 = normal[i];
-    if (c0.w == 0.0f) { out[i] = c0; return; }
-    float3 sum = v3(0, 0, 0);
-    float wsum = 0.0f;
-    for (int dy = -2; dy <= 2; dy++)
-        for (int dx = -2; dx <= 2; dx++) {
-            int xx = x + dx * step, yy = y + dy * step;
-            if (xx < 0 || yy < 0 || xx >= w || yy >= h) continue;
-            int j = yy * w + xx;
-            float4 c = in[j];
-            if (c.w == 0.0f) continue;
-            float4 a = albedo[j], n = normal[j];
-            float3 dc = v3(c.x - c0.x, c.y - c0.y, c.z - c0.z);
-            float3 da = v3(a.x - a0.x, a.y - a0.y, a.z - a0.z);
-            float wc = expf(-dot(dc, dc) / colorPhi);
-            float wa = expf(-dot(da, da) / 0.02f);
-            float wn = powf(fmaxf(0.0f, n.x * n0.x + n.y * n0.y + n.z * n0.z), 64.0f);
-            float wk = kernel[abs(dx)] * kernel[abs(dy)] * wc * wa * wn;
-            sum = add(sum, scale(v3(c.x, c.y, c.z), wk));
-            wsum += wk;
+// x / 0.02f, correctly rounded like the division it replaces: a quotient
+// estimate and one residual correction (Markstein 1990), exact against the
+// division for every float in [2^-100, 2^100] (checked over all of them) and
+// for 0 up to the sign; the rest take the division.
+__device__ __forceinline__ float over002(float x) {
+    const float magnitude = fabsf(x);
+    if (magnitude == 0.0f || (magnitude >= 7.88861e-31f && magnitude <= 1.26765e30f)) {
+        const float q = x * 50.0f, rest = __fmaf_rn(-q, 0.02f, x);
+        return __fmaf_rn(rest, 50.0f, q);
+    }
+    return x / 0.02f;
+}
+// Weight of a tap without its kernel factors' product order changed:
+// ((k * wc) * wa) * wn. invPhi is a power of two, so the product with it is
+// the quotient by colorPhi.
+__device__ __forceinline__ float tapWeight(float k, float4 c0, float4 a0, float4 n0, float4 c, float4 a, float4 n,
+                                           float invPhi) {
+    const float3 dc = v3(c.x - c0.x, c.y - c0.y, c.z - c0.z);
+    const float3 da = v3(a.x - a0.x, a.y - a0.y, a.z - a0.z);
+    const float wc = expf(-dot(dc, dc) * invPhi);
+    const float wa = expf(over002(-dot(da, da)));
+    const float wn = powf(fmaxf(0.0f, n.x * n0.x + n.y * n0.y + n.z * n0.z), 64.0f);
+    return k * wc * wa * wn;
+}
+// One pass of the a-trous filter: 25 taps `step` pixels apart. The pixels of
+// one residue (x mod step, y mod step) form a dense lattice on which the taps
+// are the neighbours within two, so a block takes a 32 x 16 tile of one
+// lattice with its two-point border into shared memory. A tap's weight is the
+// same seen from both ends (squares and products of the same pairs), so each
+// pair's two exponentials and its power are computed once, by the end that
+// comes first, and the 25 weighted sums read them: 14.4 evaluations per
+// pixel instead of 25. Bound by those evaluations (about 150 instructions
+// each). 1283 x 717, five passes: 695 us with one thread per pixel evaluating
+// every tap, 496 us now (85 at step 1, 117 at step 16, whose lattices of 81 x 45
+// points fill 96 x 48).
+constexpr int kAtX = 32, kAtY = 16, kAtW = kAtX + 4, kAtH = kAtY + 4, kAtOwners = kAtW * (kAtY + 2), kAtThreads = 256;
+constexpr size_t kAtrousSmem = sizeof(float4) * 3 * kAtW * kAtH + sizeof(float) * 12 * kAtOwners;
+// Index of forward offset (dx, dy): dy = 0 and dx = 1, 2; dy = 1, 2 and dx = -2 .. 2.
+__host__ __device__ constexpr int atOffset(int dx, int dy) { return dy == 0 ? dx - 1 : 2 + 5 * (dy - 1) + dx + 2; }
+__global__ void __launch_bounds__(kAtThreads) atrousKernel(const float4* in, const float4* albedo, const float4* normal,
+                                                           float4* out, int w, int h, int step, float invPhi) {
+    extern __shared__ float4 atSmem[];
+    float4 *sc = atSmem, *sa = sc + kAtW * kAtH, *sn = sa + kAtW * kAtH;
+    float* sw = reinterpret_cast<float*>(sn + kAtW * kAtH);  // [12][kAtOwners]; below 0: no such tap
+    const int rx = blockIdx.x % step, ry = blockIdx.y % step;
+    const int gx0 = (int)(blockIdx.x / step) * kAtX - 2, gy0 = (int)(blockIdx.y / step) * kAtY - 2;
+    for (int i = threadIdx.x; i < kAtW * kAtH; i += kAtThreads) {
+        const int gx = gx0 + i % kAtW, gy = gy0 + i / kAtW;
+        const int x = gx * step + rx, y = gy * step + ry;
+        float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a = c, n = c;
+        if (gx >= 0 && gy >= 0 && x < w && y < h) {
+            const int j = y * w + x;
+            c = in[j]; a = albedo[j]; n = normal[j];
         }
-    float3 r = wsum > 0 ? scale(sum, 1.0f / wsum) : v3(c0.x, c0.y, c0.z);
-    out[i] = make_float4(r.x, r.y, r.z, c0.w);
+        sc[i] = c; sa[i] = a; sn[i] = n;
+    }
+    __syncthreads();
+    constexpr float kernel[3] = {3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
+    // Pair weights, by the pixels (owners) whose forward taps they are; a pair
+    // with neither end in the tile is not needed.
+    for (int i = threadIdx.x; i < kAtOwners; i += kAtThreads) {
+        const int lx = i % kAtW, ly = i / kAtW;
+        const bool mine = lx >= 2 && lx < kAtX + 2 && ly >= 2;
+        const float4 c0 = sc[i], a0 = sa[i], n0 = sn[i];
+#pragma unroll
+        for (int dy = 0; dy <= 2; dy++)
+#pragma unroll
+            for (int dx = -2; dx <= 2; dx++) {
+                if (dy == 0 && dx <= 0) continue;
+                const int px = lx + dx, py = ly + dy;
+                if (!mine && !(px >= 2 && px < kAtX + 2 && py >= 2 && py < kAtY + 2)) continue;
+                const int j = py * kAtW + px;
+                const float4 c = sc[j];
+                float weight = -1.0f;
+                if (c0.w != 0.0f && c.w != 0.0f)
+                    weight = tapWeight(kernel[dx < 0 ? -dx : dx] * kernel[dy], c0, a0, n0, c, sa[j], sn[j], invPhi);
+                sw[atOffset(dx, dy) * kAtOwners + i] = weight;
+            }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kAtX * kAtY; i += kAtThreads) {
+        const int lx = i % kAtX + 2, ly = i / kAtX + 2, at = ly * kAtW + lx;
+        const int x = (gx0 + lx) * step + rx, y = (gy0 + ly) * step + ry;
+        if (x >= w || y >= h) continue;
+        const float4 c0 = sc[at];
+        if (c0.w == 0.0f) { out[y * w + x] = c0; continue; }
+        float3 sum = v3(0, 0, 0);
+        float wsum = 0.0f;
+#pragma unroll
+        for (int dy = -2; dy <= 2; dy++)
+#pragma unroll
+            for (int dx = -2; dx <= 2; dx++) {
+                const bool forward = dy > 0 || (dy == 0 && dx > 0);
+                const float4 c = sc[at + dy * kAtW + dx];
+                float wk;
+                if (dx == 0 && dy == 0) wk = tapWeight(kernel[0] * kernel[0], c0, sa[at], sn[at], c0, sa[at], sn[at], invPhi);
+                else if (forward) wk = sw[atOffset(forward ? dx : 1, forward ? dy : 0) * kAtOwners + at];
+                else wk = sw[atOffset(forward ? 1 : -dx, forward ? 0 : -dy) * kAtOwners + at + dy * kAtW + dx];
+                if (wk < 0.0f) continue;
+                sum = add(sum, scale(v3(c.x, c.y, c.z), wk));
+                wsum += wk;
+            }
+        float3 r = wsum > 0 ? scale(sum, 1.0f / wsum) : v3(c0.x, c0.y, c0.z);
+        out[y * w + x] = make_float4(r.x, r.y, r.z, c0.w);
+    }
 }
 __global__ void denoisePresentKernel(const Accum* sums, const float4* color, int count, float exposure, uchar4* pixels) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -581,13 +657,17 @@ cudaError_t launchDenoise(const Accum* sums, unsigned samples, int w, int h, flo
     int count = w * h;
     float4 *color = work, *albedo = work + count, *normal = work + 2 * (size_t)count, *tmp = work + 3 * (size_t)count;
     denoisePrepareKernel<<<blocks(count, 256), 256, 0, stream>>>(sums, samples, count, color, albedo, normal);
-    dim3 block(16, 16), grid((w + 15) / 16, (h + 15) / 16);
+    cudaError_t e = cudaFuncSetAttribute(atrousKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAtrousSmem);
+    if (e != cudaSuccess) return e;
     float4 *src = color, *dst = tmp;
-    float phi = 0.5f;
+    float invPhi = 2.0f;  // colour bandwidth 0.5, halved every pass
     for (int it = 0; it < kAtrousPasses; it++) {
-        atrousKernel<<<grid, block, 0, stream>>>(src, albedo, normal, dst, w, h, 1 << it, phi);
+        const int step = 1 << it;
+        auto tiles = [&](int size, int tile) { return step * (((size + step - 1) / step + tile - 1) / tile); };
+        atrousKernel<<<dim3(tiles(w, kAtX), tiles(h, kAtY)), kAtThreads, kAtrousSmem, stream>>>(src, albedo, normal, dst, w, h,
+                                                                                              step, invPhi);
         float4* t = src; src = dst; dst = t;
-        phi *= 0.5f;
+        invPhi *= 2.0f;
     }
     denoisePresentKernel<<<blocks(count, 256), 256, 0, stream>>>(sums, src, count, exposure, pixels);
     return cudaGetLastError();

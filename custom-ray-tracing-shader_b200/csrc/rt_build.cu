@@ -42,8 +42,13 @@ constexpr int kBinPer = 8;         // positions per thread in the binning pass
 // Tasks of at most kSmallTask primitives are binned by one warp each
 // (binSmallKernel); larger ones by position blocks (binKernel).
 constexpr int kSmallTask = 2048;
-// Levels (binned SAH, or wide collapse) queued per host read of the counts.
-constexpr int kLevelBatch = 8;
+// Tasks of at most this many primitives are finished by one warp each, down to
+// their leaves (subtreeKernel).
+constexpr int kSubtree = 32;
+// Levels (binned SAH, or wide collapse) queued per host read of the counts:
+// a first batch of 8, then 4 at a time. A level without tasks costs its
+// launches only.
+constexpr int kLevelBatch = 8, kNextLevels = 4;
 
 struct Task {
     int node, first, count, depth;
@@ -51,6 +56,12 @@ struct Task {
 };
 struct BinAcc { unsigned count; float lo[3], hi[3], clo[3], chi[3]; };
 struct Split { int axis, bin, leftCount, childTask[2]; };
+// A finished subtree: its root's raw node, and its other nodes at [base, base +
+// 2 * interior) in the reference's depth-first order.
+struct Subtree { int root, base, interior; };
+// counters: [0] raw nodes, [1] (unused), [2] maximum depth, [3] error, [4]
+// subtree tasks, [5] finished blocks of a scan.
+constexpr int kCounters = 8;
 
 __device__ __forceinline__ void atomicMinFloat(float* a, float v) {
     if (v >= 0.0f) atomicMin(reinterpret_cast<int*>(a), __float_as_int(v));
@@ -74,6 +85,29 @@ __device__ __forceinline__ void growBox(float lo[3], float hi[3], const float ol
 }
 
 // ---- primitive boxes and root bounds ----
+// Grows the root's box and centroid box by a block's values (v: low, high,
+// centroid low and high of this thread's primitive): one set of atomics per
+// block of 256 threads (per warp they serialised on the root's addresses, 484
+// us for 1.3M primitives).
+__device__ __forceinline__ void growRoot(float (&v)[12], Task* root) {
+    __shared__ float part[8][12];
+    for (int off = 16; off > 0; off >>= 1)
+        for (int k = 0; k < 12; k++) {
+            float o = __shfl_xor_sync(0xFFFFFFFFu, v[k], off);
+            v[k] = ((k / 3) & 1) ? fmaxf(v[k], o) : fminf(v[k], o);
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 12; k++) part[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        const int k = threadIdx.x;
+        float x = part[0][k];
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) x = ((k / 3) & 1) ? fmaxf(x, part[w][k]) : fminf(x, part[w][k]);
+        float* at = k < 3 ? &root->lo[k] : k < 6 ? &root->hi[k - 3] : k < 9 ? &root->clo[k - 6] : &root->chi[k - 9];
+        if ((k / 3) & 1) atomicMaxFloat(at, x);
+        else atomicMinFloat(at, x);
+    }
+}
 __global__ void primBoxesKernel(const SceneTri* tris, int n, float4* plo, float4* phi, float4* cent, Task* root) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     float v[12];
@@ -97,17 +131,7 @@ __global__ void primBoxesKernel(const SceneTri* tris, int n, float4* plo, float4
         cent[i] = make_float4(ce[0], ce[1], ce[2], 0.0f);
         for (int k = 0; k < 3; k++) { v[k] = lo[k]; v[3 + k] = hi[k]; v[6 + k] = ce[k]; v[9 + k] = ce[k]; }
     }
-    for (int off = 16; off > 0; off >>= 1)
-        for (int k = 0; k < 12; k++) {
-            float o = __shfl_xor_sync(0xFFFFFFFFu, v[k], off);
-            v[k] = ((k / 3) & 1) ? fmaxf(v[k], o) : fminf(v[k], o);
-        }
-    if ((threadIdx.x & 31) == 0) {
-        for (int k = 0; k < 3; k++) {
-            atomicMinFloat(&root->lo[k], v[k]); atomicMaxFloat(&root->hi[k], v[3 + k]);
-            atomicMinFloat(&root->clo[k], v[6 + k]); atomicMaxFloat(&root->chi[k], v[9 + k]);
-        }
-    }
+    growRoot(v, root);
 }
 
 // Traversal-tree primitives: each triangle cut into `pieces` slabs along the
@@ -202,17 +226,7 @@ __global__ void splitBoxesKernel(const SceneTri* tris, const int* primTri, int n
         cent[r] = make_float4(ce[0], ce[1], ce[2], 0.0f);
         for (int k = 0; k < 3; k++) { v[k] = lo[k]; v[3 + k] = hi[k]; v[6 + k] = ce[k]; v[9 + k] = ce[k]; }
     }
-    for (int off = 16; off > 0; off >>= 1)
-        for (int k = 0; k < 12; k++) {
-            float o = __shfl_xor_sync(0xFFFFFFFFu, v[k], off);
-            v[k] = ((k / 3) & 1) ? fmaxf(v[k], o) : fminf(v[k], o);
-        }
-    if ((threadIdx.x & 31) == 0) {
-        for (int k = 0; k < 3; k++) {
-            atomicMinFloat(&root->lo[k], v[k]); atomicMaxFloat(&root->hi[k], v[3 + k]);
-            atomicMinFloat(&root->clo[k], v[6 + k]); atomicMaxFloat(&root->chi[k], v[9 + k]);
-        }
-    }
+    growRoot(v, root);
 }
 
 __global__ void iotaKernel(int* a, int n, int value0, int* b, int bValue) {
@@ -223,7 +237,7 @@ __global__ void iotaKernel(int* a, int n, int value0, int* b, int bValue) {
 // Level counts (taskCount[0] open tasks, taskCount[1] of them larger than
 // kSmallTask) live on the device, so levels are queued without the host
 // reading them: per-task kernels loop over the device count.
-__global__ void clearBinsKernel(BinAcc* bins, const int* taskCount, const Task* tasks) {
+__device__ __forceinline__ void clearBins(BinAcc* bins, const int* taskCount, const Task* tasks) {
     if (!taskCount[1]) return;
     const int count = taskCount[0] * 3 * kBins;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -233,6 +247,7 @@ __global__ void clearBinsKernel(BinAcc* bins, const int* taskCount, const Task* 
         for (int a = 0; a < 3; a++) { b.lo[a] = FLT_MAX; b.hi[a] = -FLT_MAX; b.clo[a] = FLT_MAX; b.chi[a] = -FLT_MAX; }
     }
 }
+__global__ void clearBinsKernel(BinAcc* bins, const int* taskCount, const Task* tasks) { clearBins(bins, taskCount, tasks); }
 
 __device__ __forceinline__ void accumulateBin(BinAcc* dst, float4 lo, float4 hi, float4 c) {
     atomicAdd(&dst->count, 1u);
@@ -294,12 +309,11 @@ __device__ void warpAccumulate(BinAcc* dst, float4 lo, float4 hi, float4 c) {
     if ((pending >> lane) & 1u) accumulateBin(dst, lo, hi, c);
 }
 
-// Bins every primitive of every open task. The task owning the first position
-// of a block's chunk is aggregated in shared memory; others go to global bins.
-__global__ void __launch_bounds__(kBinBlock) binKernel(const int* order, const int* posTask, const float4* cent,
-                                                       const float4* plo, const float4* phi, const Task* tasks,
-                                                       int nPos, BinAcc* bins, const int* taskCount) {
-    __shared__ BinAcc sb[3 * kBins];
+// Bins every primitive of the open tasks above kSmallTask. The task owning the
+// first position of a block's chunk is aggregated in shared memory (sb, 3 *
+// kBins); others go to global bins.
+__device__ void binLarge(const int* order, const int* posTask, const float4* cent, const float4* plo, const float4* phi,
+                         const Task* tasks, int nPos, BinAcc* bins, const int* taskCount, BinAcc* sb) {
     __shared__ int sTask;
     if (!taskCount[1]) return;  // no task above kSmallTask at this level
     int base = blockIdx.x * kBinBlock * kBinPer;
@@ -382,17 +396,23 @@ __device__ void binSmallTask(const int* order, const float4* cent, const float4*
     __syncwarp();
 }
 
-// One warp per small task: warp-private bins in shared memory (atomics only
-// within the warp), written out with plain stores, so these bins need no
-// clearing and no global atomics. Bins hold a count and minima/maxima, so the
-// order of accumulation does not change them.
-__global__ void __launch_bounds__(256) binSmallKernel(const int* order, const float4* cent, const float4* plo,
-                                                      const float4* phi, const Task* tasks, const int* taskCount,
-                                                      BinAcc* bins) {
+// The bins of a level's tasks in one launch. Blocks below largeBlocks: position
+// chunks of the large tasks. The others: one warp per small task, with
+// warp-private bins in shared memory (atomics only within the warp), written
+// out with plain stores, so these bins need no clearing and no global atomics.
+// Bins hold a count and minima/maxima, so the order of accumulation does not
+// change them.
+__global__ void __launch_bounds__(kBinBlock) binKernel(const int* order, const int* posTask, const float4* cent,
+                                                       const float4* plo, const float4* phi, const Task* tasks,
+                                                       int nPos, BinAcc* bins, const int* taskCount, int largeBlocks) {
     __shared__ BinAcc sb[8][3 * kBins];
+    if ((int)blockIdx.x < largeBlocks) {
+        binLarge(order, posTask, cent, plo, phi, tasks, nPos, bins, taskCount, sb[0]);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nTasks = taskCount[0];
-    for (int t = blockIdx.x * 8 + warp; t < nTasks; t += gridDim.x * 8)
+    const int nTasks = taskCount[0], first = (int)blockIdx.x - largeBlocks, stride = ((int)gridDim.x - largeBlocks) * 8;
+    for (int t = first * 8 + warp; t < nTasks; t += stride)
         binSmallTask(order, cent, plo, phi, tasks[t], t, bins, sb[warp], lane);
 }
 
@@ -406,8 +426,8 @@ __global__ void __launch_bounds__(256) binSmallKernel(const int* order, const fl
 // taskCount: this level's counts; nextCount: the next level's (open tasks,
 // tasks above kSmallTask); counters: 0 nodes, 2 maximum depth, 3 error.
 __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, Split* splits, BinNode* nodes,
-                          int* counters, int* nextCount, Task* nextTasks, int nodeCapacity, int taskCapacity,
-                          int leafSize) {
+                          int* counters, int* nextCount, Task* nextTasks, Task* subtrees, int nodeCapacity,
+                          int taskCapacity, int subtreeCapacity, int leafSize) {
     const unsigned full = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     int bestAxis = -1, bestBin = -1;
@@ -442,7 +462,7 @@ __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, S
     const bool split = bestAxis >= 0;
     // Children's boxes, centroid boxes and counts are unions over the bins.
     Task C[2];
-    bool open[2] = {false, false};
+    bool open[2] = {false, false}, small[2] = {false, false};  // small: finished by subtreeKernel
     if (split) {
         for (int side = 0; side < 2; side++) {
             for (int k = 0; k < 3; k++) { C[side].lo[k] = C[side].clo[k] = FLT_MAX; C[side].hi[k] = C[side].chi[k] = -FLT_MAX; }
@@ -459,6 +479,8 @@ __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, S
         for (int side = 0; side < 2; side++) {
             C[side].depth = T.depth + 1;
             open[side] = !(C[side].count <= leafSize || C[side].depth == kBinaryMaxDepth);
+            small[side] = open[side] && C[side].count <= kSubtree;
+            open[side] = open[side] && !small[side];
         }
     }
     // Maximum depth: a task's own, its children's when it splits.
@@ -478,6 +500,10 @@ __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, S
     if (lane == 0 && (open0 | open1)) taskBase = atomicAdd(&nextCount[0], __popc(open0) + __popc(open1));
     if (lane == 0 && (big0 | big1)) atomicAdd(&nextCount[1], __popc(big0) + __popc(big1));
     taskBase = __shfl_sync(full, taskBase, 0);
+    const unsigned small0 = __ballot_sync(full, small[0]), small1 = __ballot_sync(full, small[1]);
+    int subtreeBase = 0;
+    if (lane == 0 && (small0 | small1)) subtreeBase = atomicAdd(&counters[4], __popc(small0) + __popc(small1));
+    subtreeBase = __shfl_sync(full, subtreeBase, 0);
     if (!have) return;
 
     Split S;
@@ -494,9 +520,16 @@ __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, S
     C[1].first = T.first + C[0].count;
     S.leftCount = C[0].count;
     int k = taskBase + __popc(open0 & below) + __popc(open1 & below);
+    int m = subtreeBase + __popc(small0 & below) + __popc(small1 & below);
     for (int side = 0; side < 2; side++) {
         Task& c = C[side];
         c.node = child + side;
+        if (small[side]) {
+            if (m >= subtreeCapacity) atomicExch(&counters[3], 2);
+            else subtrees[m] = c;
+            m++;
+            continue;
+        }
         if (!open[side]) {
             nodes[c.node] = BinNode{v3(c.lo[0], c.lo[1], c.lo[2]), c.first, v3(c.hi[0], c.hi[1], c.hi[2]), c.count};
             continue;
@@ -509,8 +542,8 @@ __device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, S
     splits[t] = S;
 }
 __global__ void splitKernel(const Task* tasks, const int* taskCount, const BinAcc* bins, Split* splits, BinNode* nodes,
-                            int* counters, int* nextCount, Task* nextTasks, int nodeCapacity, int taskCapacity,
-                            int leafSize) {
+                            int* counters, int* nextCount, Task* nextTasks, Task* subtrees, int nodeCapacity,
+                            int taskCapacity, int subtreeCapacity, int leafSize) {
     const int nTasks = taskCount[0];
     // Whole warps walk the tasks (splitTask uses warp collectives).
     for (int base = blockIdx.x * blockDim.x; base < nTasks; base += gridDim.x * blockDim.x) {
@@ -519,41 +552,30 @@ __global__ void splitKernel(const Task* tasks, const int* taskCount, const BinAc
         Task T;
         if (have) T = tasks[t];
         else T.count = 0, T.depth = 0;
-        splitTask(have, T, t, bins, splits, nodes, counters, nextCount, nextTasks, nodeCapacity, taskCapacity,
-                  leafSize);
+        splitTask(have, T, t, bins, splits, nodes, counters, nextCount, nextTasks, subtrees, nodeCapacity, taskCapacity,
+                  subtreeCapacity, leafSize);
     }
 }
 
-__global__ void flagKernel(const int* order, const int* posTask, const float4* cent, const Task* tasks,
-                           const Split* splits, int nPos, unsigned* flags) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nPos) return;
-    int t = posTask[j];
-    unsigned f = 0;
-    if (t >= 0) {
-        Split S = splits[t];
-        if (S.axis >= 0) {
-            const Task& T = tasks[t];
-            float lo = T.clo[S.axis];
-            float s = kBins / (T.chi[S.axis] - lo);
-            float4 c = cent[order[j]];
-            float ca = S.axis == 0 ? c.x : (S.axis == 1 ? c.y : c.z);
-            f = binOf(ca, lo, s) <= S.bin ? 1u : 0u;
-        }
-    }
-    flags[j] = f;
+// 1 when position j's primitive goes to its task's left child.
+__device__ __forceinline__ unsigned leftFlag(int j, const int* order, const int* posTask, const float4* cent,
+                                             const Task* tasks, const Split* splits) {
+    const int t = posTask[j];
+    if (t < 0) return 0u;
+    const Split S = splits[t];
+    if (S.axis < 0) return 0u;
+    const Task& T = tasks[t];
+    float lo = T.clo[S.axis];
+    float s = kBins / (T.chi[S.axis] - lo);
+    float4 c = cent[order[j]];
+    float ca = S.axis == 0 ? c.x : (S.axis == 1 ? c.y : c.z);
+    return binOf(ca, lo, s) <= S.bin ? 1u : 0u;
 }
 
-// Exclusive scan, phase 1: per-block scan in place, block totals out.
-__global__ void __launch_bounds__(256) scanBlocksKernel(const unsigned* in, unsigned* data, int n, unsigned* blockSums) {
-    __shared__ unsigned warpSums[8];
-    int base = blockIdx.x * kScanBlock;
-    unsigned v[4], local = 0;
-    for (int k = 0; k < 4; k++) {
-        int j = base + threadIdx.x * 4 + k;
-        v[k] = j < n ? in[j] : 0u;
-        local += v[k];
-    }
+// Exclusive scan of 4 consecutive values per thread over a block of 256, block
+// total to *sum (thread 7's store); returns the thread's prefix.
+__device__ __forceinline__ unsigned scanBlock(const unsigned (&v)[4], unsigned* warpSums, unsigned* sum) {
+    const unsigned local = v[0] + v[1] + v[2] + v[3];
     unsigned incl = local;
     for (int off = 1; off < 32; off <<= 1) {
         unsigned o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
@@ -568,52 +590,91 @@ __global__ void __launch_bounds__(256) scanBlocksKernel(const unsigned* in, unsi
             if (threadIdx.x >= off) wi += o;
         }
         if (threadIdx.x < 8) warpSums[threadIdx.x] = wi - w;
-        if (threadIdx.x == 7) blockSums[blockIdx.x] = wi;
+        if (threadIdx.x == 7) *sum = wi;
     }
     __syncthreads();
-    unsigned run = warpSums[threadIdx.x >> 5] + incl - local;
-    for (int k = 0; k < 4; k++) {
-        int j = base + threadIdx.x * 4 + k;
-        if (j < n) data[j] = run;
-        run += v[k];
-    }
+    return warpSums[threadIdx.x >> 5] + incl - local;
 }
-// Phase 2: one block scans the block totals (exclusive, in place).
-__global__ void __launch_bounds__(1024) scanTotalsKernel(unsigned* sums, int count) {
+// Exclusive scan of the block totals, in place, by one block of 256 threads.
+__device__ void scanTotals(unsigned* sums, int count) {
     __shared__ unsigned carry;
-    __shared__ unsigned warpSums[32];
+    __shared__ unsigned warpSums[8];
+    __shared__ unsigned total;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int base = 0; base < count; base += 1024) {
-        int j = base + threadIdx.x;
-        unsigned v = j < count ? sums[j] : 0u, incl = v;
-        for (int off = 1; off < 32; off <<= 1) {
-            unsigned o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-            if ((threadIdx.x & 31) >= off) incl += o;
-        }
-        if ((threadIdx.x & 31) == 31) warpSums[threadIdx.x >> 5] = incl;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            unsigned w = warpSums[threadIdx.x], wi = w;
-            for (int off = 1; off < 32; off <<= 1) {
-                unsigned o = __shfl_up_sync(0xFFFFFFFFu, wi, off);
-                if (threadIdx.x >= off) wi += o;
-            }
-            warpSums[threadIdx.x] = wi - w;
+        unsigned v[4];
+        const int j = base + threadIdx.x * 4;
+        for (int k = 0; k < 4; k++) v[k] = j + k < count ? __ldcg(sums + j + k) : 0u;
+        unsigned run = carry + scanBlock(v, warpSums, &total);
+        for (int k = 0; k < 4; k++) {
+            if (j + k < count) sums[j + k] = run;
+            run += v[k];
         }
         __syncthreads();
-        unsigned excl = carry + warpSums[threadIdx.x >> 5] + incl - v;
-        if (j < count) sums[j] = excl;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = excl + v;
+        if (threadIdx.x == 0) carry += total;
         __syncthreads();
     }
 }
-// Phase 3 is folded into the consumer: prefix(j) = data[j] + sums[j / kScanBlock].
+// The block that finishes last scans the totals (done: zero before the launch
+// and after it). Every block of the grid calls this once its total is stored.
+__device__ void scanTotalsLast(unsigned* sums, int count, int* done) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(done, 1) == count - 1 ? 1 : 0;
+        if (last) *done = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    scanTotals(sums, count);
+}
+__global__ void __launch_bounds__(256) scanBlocksKernel(const unsigned* in, unsigned* data, int n, unsigned* blockSums,
+                                                        int* done) {
+    __shared__ unsigned warpSums[8];
+    const int j = blockIdx.x * kScanBlock + threadIdx.x * 4;
+    unsigned v[4];
+    for (int k = 0; k < 4; k++) v[k] = j + k < n ? in[j + k] : 0u;
+    unsigned run = scanBlock(v, warpSums, &blockSums[blockIdx.x]);
+    for (int k = 0; k < 4; k++) {
+        if (j + k < n) data[j + k] = run;
+        run += v[k];
+    }
+    scanTotalsLast(blockSums, (int)gridDim.x, done);
+}
+// A level's partition, first half: every position's side and the scan of the
+// sides. Also records the node count after the level's splits (the first node
+// of the next depth) and clears the bins of the next level's large tasks.
+__global__ void __launch_bounds__(256) partitionKernel(const int* order, const int* posTask, const float4* cent,
+                                                       const Task* tasks, const Split* splits, int n, unsigned* flags,
+                                                       unsigned* prefix, unsigned* blockSums, int* counters, int* levelStart,
+                                                       const int* taskCount, const int* nextCount, const Task* nextTasks,
+                                                       BinAcc* bins) {
+    __shared__ unsigned warpSums[8];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *levelStart = counters[0];
+    if (!taskCount[0]) return;  // a level past the last: nothing moves
+    clearBins(bins, nextCount, nextTasks);
+    const int j = blockIdx.x * kScanBlock + threadIdx.x * 4;
+    unsigned v[4];
+    for (int k = 0; k < 4; k++) {
+        v[k] = j + k < n ? leftFlag(j + k, order, posTask, cent, tasks, splits) : 0u;
+        if (j + k < n) flags[j + k] = v[k];
+    }
+    unsigned run = scanBlock(v, warpSums, &blockSums[blockIdx.x]);
+    for (int k = 0; k < 4; k++) {
+        if (j + k < n) prefix[j + k] = run;
+        run += v[k];
+    }
+    scanTotalsLast(blockSums, (int)gridDim.x, &counters[5]);
+}
+// The consumer adds both levels: prefix(j) = data[j] + sums[j / kScanBlock].
 
 __global__ void scatterKernel(const int* order, const int* posTask, const Task* tasks, const Split* splits,
                               const unsigned* flags, const unsigned* prefix, const unsigned* blockSums, int nPos,
-                              int* orderNext, int* posTaskNext, int* error) {
+                              int* orderNext, int* posTaskNext, const int* taskCount, int* error) {
+    if (!taskCount[0]) return;
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nPos) return;
     int t = posTask[j];
@@ -631,37 +692,254 @@ __global__ void scatterKernel(const int* order, const int* posTask, const Task* 
     posTaskNext[dst] = S.childTask[left ? 0 : 1];
 }
 
-// Node count after a level's splits: the first node of the next depth.
-__global__ void recordLevelKernel(const int* counters, int* levelStart) { *levelStart = counters[0]; }
+// ---- subtrees of at most kSubtree primitives ----
+constexpr int kSubtreeWarps = 4;
+struct SubtreeEntry { unsigned mask; int first, depth, slot; float lo[3], hi[3], clo[3], chi[3]; };
+struct SubtreeShared {
+    float4 lo[kSubtree], hi[kSubtree];    // primitive boxes; lo.w: the bins of the three axes, 4 bits each
+    BinNode nodes[2 * (kSubtree - 1)];    // all nodes but the root, in depth-first order (children in pairs)
+    SubtreeEntry stack[kSubtree];         // right siblings not yet visited
+};
+
+// One warp builds the whole subtree of a small task; lane l holds primitive l
+// of the task's range and a node is a mask of lanes. The partition is stable,
+// so a node's primitives are its lanes in order and nothing moves until the
+// leaves write the range. The split search is the reference's over its 33
+// candidates (3 axes x 11 bins): candidate j on lane j, which unites the
+// boxes on both sides over the node's primitives (minima and maxima, the
+// same values as uniting bins), the 33rd by warp reductions; the first
+// minimum wins as in splitTask. Nodes are visited depth first, left before
+// right, so a split's rank among the subtree's splits is the reference's
+// numbering of its children.
+// This replaces about 12 levels of global binning, splitting and partitioning
+// (3.0 of the 9.2 ms of the 1.3M-piece tree, 0.9 of 1.4 ms at 8,000 triangles).
+// Bound by instructions, about 300 per split and 20 more per primitive.
+__global__ void __launch_bounds__(32 * kSubtreeWarps) subtreeKernel(int* order, const float4* cent, const float4* plo,
+                                                                    const float4* phi, const Task* tasks, int* counters,
+                                                                    BinNode* nodes, int nodeCapacity, int leafSize,
+                                                                    int* interiorOf, Subtree* done) {
+    __shared__ SubtreeShared shared[kSubtreeWarps];
+    const unsigned full = 0xFFFFFFFFu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    SubtreeShared& S = shared[warp];
+    const int count = counters[4];
+    const int axis = lane / 11, cut = lane % 11;  // this lane's candidate
+    auto axisOf = [](float x, float y, float z, int a) { return a == 0 ? x : (a == 1 ? y : z); };
+    for (int t = blockIdx.x * kSubtreeWarps + warp; t < count; t += gridDim.x * kSubtreeWarps) {
+        const Task T = tasks[t];
+        const bool have = lane < T.count;
+        int prim = 0;
+        float4 lo = make_float4(0, 0, 0, 0), hi = lo, c = lo;
+        if (have) {
+            prim = order[T.first + lane];
+            lo = plo[prim]; hi = phi[prim]; c = cent[prim];
+        }
+        __syncwarp();
+        S.lo[lane] = lo;
+        S.hi[lane] = hi;
+        SubtreeEntry N;
+        N.mask = __ballot_sync(full, have);
+        N.first = T.first; N.depth = T.depth; N.slot = -1;
+        for (int a = 0; a < 3; a++) { N.lo[a] = T.lo[a]; N.hi[a] = T.hi[a]; N.clo[a] = T.clo[a]; N.chi[a] = T.chi[a]; }
+        BinNode root;
+        int interior = 0, top = 0, depth = T.depth;
+        // Writes a node's record (children by their place in S.nodes).
+        auto record = [&](int slot, const float* l, const float* h, int first, int n) {
+            const BinNode r{v3(l[0], l[1], l[2]), first, v3(h[0], h[1], h[2]), n};
+            if (slot < 0) root = r;
+            else if (lane == 0) S.nodes[slot] = r;
+        };
+        auto leaf = [&](unsigned mask, int first) {
+            if ((mask >> lane) & 1u) order[first + __popc(mask & below)] = prim;
+        };
+        auto reduceMin = [&](float v, bool in) { return keyFloat(__reduce_min_sync(full, in ? orderedKey(v) : 0x7FFFFFFF)); };
+        auto reduceMax = [&](float v, bool in) { return keyFloat(__reduce_max_sync(full, in ? orderedKey(v) : (int)0x80000000)); };
+        for (;;) {
+            const int n = __popc(N.mask);
+            const bool mine = (N.mask >> lane) & 1u;
+            int bestAxis = -1, bestCut = 0;
+            float side[2][6];  // the winning candidate's boxes: low, high
+            if (n > leafSize && N.depth != kBinaryMaxDepth) {
+                const float nodeArea = halfArea(N.lo, N.hi), unsplit = nodeArea * n;
+                int bin[3] = {0, 0, 0};
+                bool valid[3];
+                for (int a = 0; a < 3; a++) {
+                    const float extent = N.chi[a] - N.clo[a];
+                    valid[a] = !(extent <= 1e-12f);
+                    if (valid[a]) bin[a] = binOf(axisOf(c.x, c.y, c.z, a), N.clo[a], kBins / extent);
+                }
+                __syncwarp();
+                reinterpret_cast<int*>(&S.lo[lane])[3] = bin[0] | bin[1] << 4 | bin[2] << 8;
+                __syncwarp();
+                float L[6], R[6];
+                for (int k = 0; k < 3; k++) { L[k] = R[k] = FLT_MAX; L[3 + k] = R[3 + k] = -FLT_MAX; }
+                int nl = 0;
+                for (unsigned m = N.mask; m; m &= m - 1u) {
+                    const int i = __ffs(m) - 1;
+                    const float4 pl = S.lo[i], ph = S.hi[i];
+                    if (((__float_as_int(pl.w) >> (4 * axis)) & 15) <= cut) {
+                        L[0] = fminf(L[0], pl.x); L[1] = fminf(L[1], pl.y); L[2] = fminf(L[2], pl.z);
+                        L[3] = fmaxf(L[3], ph.x); L[4] = fmaxf(L[4], ph.y); L[5] = fmaxf(L[5], ph.z);
+                        nl++;
+                    } else {
+                        R[0] = fminf(R[0], pl.x); R[1] = fminf(R[1], pl.y); R[2] = fminf(R[2], pl.z);
+                        R[3] = fmaxf(R[3], ph.x); R[4] = fmaxf(R[4], ph.y); R[5] = fmaxf(R[5], ph.z);
+                    }
+                }
+                const int nr = n - nl;
+                const bool usable = (axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]) && nl && nr;
+                const float cost = nodeArea + halfArea(L, L + 3) * nl + halfArea(R, R + 3) * nr;
+                // Costs are sums of areas, not negative: their bits order like them.
+                const unsigned bits = usable && cost < unsplit ? __float_as_uint(cost) : full;
+                unsigned best = __reduce_min_sync(full, bits);
+                if (best != full) {
+                    const int winner = __ffs(__ballot_sync(full, bits == best)) - 1;
+                    bestAxis = winner / 11;
+                    bestCut = winner % 11;
+                    for (int k = 0; k < 6; k++) {
+                        side[0][k] = __shfl_sync(full, L[k], winner);
+                        side[1][k] = __shfl_sync(full, R[k], winner);
+                    }
+                }
+                // Candidate 32: the last cut of the z axis.
+                const unsigned low = __ballot_sync(full, mine && bin[2] <= kBins - 2), high = N.mask & ~low;
+                if (valid[2] && low && high) {
+                    float l[6], r[6];
+                    const bool inLow = (low >> lane) & 1u, inHigh = (high >> lane) & 1u;
+                    l[0] = reduceMin(lo.x, inLow); l[1] = reduceMin(lo.y, inLow); l[2] = reduceMin(lo.z, inLow);
+                    l[3] = reduceMax(hi.x, inLow); l[4] = reduceMax(hi.y, inLow); l[5] = reduceMax(hi.z, inLow);
+                    r[0] = reduceMin(lo.x, inHigh); r[1] = reduceMin(lo.y, inHigh); r[2] = reduceMin(lo.z, inHigh);
+                    r[3] = reduceMax(hi.x, inHigh); r[4] = reduceMax(hi.y, inHigh); r[5] = reduceMax(hi.z, inHigh);
+                    const float last = nodeArea + halfArea(l, l + 3) * __popc(low) + halfArea(r, r + 3) * __popc(high);
+                    if (last < unsplit && __float_as_uint(last) < best) {
+                        bestAxis = 2;
+                        bestCut = kBins - 2;
+                        for (int k = 0; k < 6; k++) { side[0][k] = l[k]; side[1][k] = r[k]; }
+                    }
+                }
+                if (bestAxis >= 0) {
+                    const int b = bestAxis == 0 ? bin[0] : bestAxis == 1 ? bin[1] : bin[2];
+                    const unsigned left = __ballot_sync(full, mine && b <= bestCut);
+                    const int pair = 2 * interior++;
+                    record(N.slot, N.lo, N.hi, pair, 0);
+                    const int childDepth = N.depth + 1;
+                    depth = max(depth, childDepth);
+                    const unsigned masks[2] = {left, N.mask & ~left};
+                    const int firsts[2] = {N.first, N.first + __popc(left)};
+                    bool go = false;
+                    SubtreeEntry next;
+                    for (int s = 1; s >= 0; s--) {
+                        const int k = __popc(masks[s]);
+                        if (k <= leafSize || childDepth == kBinaryMaxDepth) {
+                            record(pair + s, side[s], side[s] + 3, firsts[s], k);
+                            leaf(masks[s], firsts[s]);
+                            continue;
+                        }
+                        SubtreeEntry E;
+                        const bool in = (masks[s] >> lane) & 1u;
+                        E.mask = masks[s]; E.first = firsts[s]; E.depth = childDepth; E.slot = pair + s;
+                        for (int a = 0; a < 3; a++) { E.lo[a] = side[s][a]; E.hi[a] = side[s][3 + a]; }
+                        E.clo[0] = reduceMin(c.x, in); E.clo[1] = reduceMin(c.y, in); E.clo[2] = reduceMin(c.z, in);
+                        E.chi[0] = reduceMax(c.x, in); E.chi[1] = reduceMax(c.y, in); E.chi[2] = reduceMax(c.z, in);
+                        if (s == 1) {
+                            if (lane == 0) S.stack[top] = E;
+                            top++;
+                        } else {
+                            next = E;
+                            go = true;
+                        }
+                    }
+                    if (go) { N = next; continue; }
+                }
+            }
+            if (bestAxis < 0) {
+                record(N.slot, N.lo, N.hi, N.first, n);
+                leaf(N.mask, N.first);
+            }
+            if (!top) break;
+            top--;
+            __syncwarp();
+            N = S.stack[top];
+            __syncwarp();
+        }
+        int base = 0;
+        if (lane == 0) {
+            if (interior) base = atomicAdd(&counters[0], 2 * interior);
+            atomicMax(&counters[2], depth);
+        }
+        base = __shfl_sync(full, base, 0);
+        __syncwarp();
+        if (base + 2 * interior > nodeCapacity) {
+            if (lane == 0) atomicExch(&counters[3], 1);
+            continue;
+        }
+        if (lane == 0) {
+            if (root.count == 0) root.first += base;
+            nodes[T.node] = root;
+            if (interiorOf) interiorOf[T.node] = interior;
+            if (done) done[t] = Subtree{T.node, base, interior};
+        }
+        for (int i = lane; i < 2 * interior; i += 32) {
+            BinNode r = S.nodes[i];
+            if (r.count == 0) r.first += base;
+            nodes[base + i] = r;
+        }
+    }
+}
 
 // ---- renumbering into the reference's depth-first numbering ----
-__global__ void subtreeInteriorKernel(const BinNode* nodes, int begin, int end, int* interior) {
+// Nodes below topNodes were made level by level; an interior one whose
+// children lie above is the root of a finished subtree, whose interior count
+// subtreeKernel has set and whose other nodes keep their order.
+__global__ void subtreeInteriorKernel(const BinNode* nodes, int begin, int end, int topNodes, int* interior) {
     int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= end) return;
     const BinNode& n = nodes[i];
-    interior[i] = n.count > 0 ? 0 : 1 + interior[n.first] + interior[n.first + 1];
+    if (n.count > 0) interior[i] = 0;
+    else if (n.first < topNodes) interior[i] = 1 + interior[n.first] + interior[n.first + 1];
 }
-__global__ void preorderKernel(const BinNode* nodes, int begin, int end, int count, const int* interior, int* rank,
-                               int* newIndex, int* error) {
+__global__ void preorderKernel(const BinNode* nodes, int begin, int end, int topNodes, int count, const int* interior,
+                               int* rank, int* newIndex, int* error) {
     int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= end) return;
     const BinNode& n = nodes[i];
-    if (n.count > 0) return;
+    if (n.count > 0 || n.first >= topNodes) return;
     int c = n.first, r = rank[i];
-    if (c < 1 || c + 1 >= count || r < 0 || 2 + 2 * r >= count) { atomicExch(error, 6); return; }
+    if (c < 1 || c + 1 >= topNodes || r < 0 || 2 + 2 * r >= count) { atomicExch(error, 6); return; }
     newIndex[c] = 1 + 2 * r;
     newIndex[c + 1] = 2 + 2 * r;
     rank[c] = r + 1;
     rank[c + 1] = r + 1 + interior[c];
 }
-__global__ void renumberKernel(const BinNode* nodes, int count, const int* newIndex, BinNode* out, int* error) {
+__global__ void renumberKernel(const BinNode* nodes, int topNodes, int count, const int* newIndex, const int* rank,
+                               BinNode* out, int* error) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    if (i >= topNodes) return;
     BinNode n = nodes[i];
-    if (n.count == 0) n.first = newIndex[n.first];
+    if (n.count == 0) n.first = n.first < topNodes ? newIndex[n.first] : 1 + 2 * rank[i];
     int dst = newIndex[i];
     if (dst < 0 || dst >= count || (n.count == 0 && (n.first < 1 || n.first + 1 >= count))) { atomicExch(error, 7); return; }
     out[dst] = n;
+}
+// The nodes of the finished subtrees, a warp each: those of a root of rank r
+// follow from 1 + 2 r.
+__global__ void placeSubtreesKernel(const BinNode* nodes, const Subtree* done, const int* counters, const int* rank, int count,
+                                    BinNode* out, int* error) {
+    const int warps = (int)(gridDim.x * blockDim.x) >> 5, lane = threadIdx.x & 31;
+    for (int t = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < counters[4]; t += warps) {
+        const Subtree S = done[t];
+        const int to = 1 + 2 * rank[S.root];
+        if (to < 1 || to + 2 * S.interior > count) {
+            if (lane == 0 && S.interior) atomicExch(error, 7);
+            continue;
+        }
+        for (int i = lane; i < 2 * S.interior; i += 32) {
+            BinNode n = nodes[S.base + i];
+            if (n.count == 0) n.first += to - S.base;
+            out[to + i] = n;
+        }
+    }
 }
 
 // ---- collapse into wide nodes (logic in rt_collapse.cuh) ----
@@ -734,15 +1012,15 @@ cudaError_t pieceMap(const SceneTri* tris, int triCount, int maxPieces, cudaStre
     cudaError_t err = alloc(counts, triCount);
     if (err == cudaSuccess) err = alloc(pfx, triCount);
     if (err == cudaSuccess) err = alloc(sums, nb);
-    if (err == cudaSuccess) err = alloc(dTotal, 1);
+    if (err == cudaSuccess) err = alloc(dTotal, 2);  // the total, and the scan's count of finished blocks
     if (err == cudaSuccess && primTri) err = alloc(map, (size_t)triCount * maxPieces);
     if (err == cudaSuccess) err = cudaEventCreate(&t0);
     if (err == cudaSuccess) err = cudaEventCreate(&t1);
+    if (err == cudaSuccess) err = cudaMemsetAsync(dTotal, 0, 2 * sizeof(int), stream);
     if (err == cudaSuccess) err = cudaEventRecord(t0, stream);
     if (err == cudaSuccess) {
         pieceCountKernel<<<blocksFor(triCount, 256), 256, 0, stream>>>(tris, triCount, maxPieces, counts);
-        scanBlocksKernel<<<nb, 256, 0, stream>>>(counts, pfx, triCount, sums);
-        scanTotalsKernel<<<1, 1024, 0, stream>>>(sums, nb);
+        scanBlocksKernel<<<nb, 256, 0, stream>>>(counts, pfx, triCount, sums, dTotal + 1);
         pieceFillKernel<<<blocksFor(triCount, 256), 256, 0, stream>>>(counts, pfx, sums, triCount, map, dTotal);
         err = cudaGetLastError();
     }
@@ -788,27 +1066,30 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         n = total;
     }
     const int nodeCapacity = 2 * n + 2;
-    const int taskCapacity = n / (leafSize + 1) + 2;
+    const int taskCapacity = n / (kSubtree + 1) + 2;
+    const int subtreeCapacity = n / (leafSize + 1) + 2;
     const int wideCapacity = 2 * n + 8;
     // Temporaries.
     float4* cent = nullptr; int* orderB = nullptr; int* posTask = nullptr; int* posTaskB = nullptr;
-    Task* tasks = nullptr; Task* tasksB = nullptr; BinAcc* bins = nullptr; Split* splits = nullptr;
+    Task* tasks = nullptr; Task* tasksB = nullptr; Task* subtrees = nullptr; Subtree* done = nullptr; BinAcc* bins = nullptr; Split* splits = nullptr;
     unsigned* flags = nullptr; unsigned* prefix = nullptr; unsigned* blockSums = nullptr; int* counters = nullptr;
     BinNode* rawNodes = nullptr; int* interior = nullptr; int* rank = nullptr; int* newIndex = nullptr;
     Job* jobs = nullptr; Job* jobsB = nullptr;
     int* levelCounts = nullptr; int* levelStartDev = nullptr; int* jobCounts = nullptr;
-    int hostCounters[8] = {}, hostLevels[2 * (kBinaryMaxDepth + 2 + kLevelBatch)], hostStarts[kBinaryMaxDepth + 4 + kLevelBatch];
+    int hostCounters[kCounters] = {}, hostLevels[2 * (kBinaryMaxDepth + 2 + kLevelBatch)], hostStarts[kBinaryMaxDepth + 4 + kLevelBatch];
     int hostJobs[kStackCapacity + 2 + kLevelBatch];
     std::vector<int> levelStart;
+    // A tree over pieces is only traced: its nodes stay as they are numbered.
+    const bool renumber = pieces == 1;
     int nScanBlocks = blocksFor(n, kScanBlock);
 
 #define RT_TRY(x) do { err = (x); if (err != cudaSuccess) goto done; } while (0)
     RT_TRY(alloc(out.primLo, n)); RT_TRY(alloc(out.primHi, n)); RT_TRY(alloc(cent, n));
     RT_TRY(alloc(out.order, n)); RT_TRY(alloc(orderB, n)); RT_TRY(alloc(posTask, n)); RT_TRY(alloc(posTaskB, n));
-    RT_TRY(alloc(tasks, taskCapacity)); RT_TRY(alloc(tasksB, taskCapacity));
+    RT_TRY(alloc(tasks, taskCapacity)); RT_TRY(alloc(tasksB, taskCapacity)); RT_TRY(alloc(subtrees, subtreeCapacity));
     RT_TRY(alloc(bins, (size_t)taskCapacity * 3 * kBins)); RT_TRY(alloc(splits, taskCapacity));
     RT_TRY(alloc(flags, n)); RT_TRY(alloc(prefix, n)); RT_TRY(alloc(blockSums, nScanBlocks));
-    RT_TRY(alloc(counters, 8)); RT_TRY(alloc(rawNodes, nodeCapacity));
+    RT_TRY(alloc(counters, kCounters)); RT_TRY(alloc(rawNodes, nodeCapacity));
     {
         const int levelSlots = kBinaryMaxDepth + 2 + kLevelBatch, jobSlots = kStackCapacity + 2 + kLevelBatch;
         RT_TRY(alloc(levelCounts, 2 * levelSlots)); RT_TRY(alloc(levelStartDev, levelSlots + 2));
@@ -817,8 +1098,10 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     // Renumbering and collapse buffers at their upper bounds (node count <=
     // nodeCapacity, wide nodes and jobs <= 2n + 8), so no allocation falls
     // inside the timed spans.
-    RT_TRY(alloc(interior, nodeCapacity)); RT_TRY(alloc(rank, nodeCapacity)); RT_TRY(alloc(newIndex, nodeCapacity));
-    RT_TRY(alloc(out.binNodes, nodeCapacity));
+    if (renumber) {
+        RT_TRY(alloc(interior, nodeCapacity)); RT_TRY(alloc(rank, nodeCapacity)); RT_TRY(alloc(newIndex, nodeCapacity));
+        RT_TRY(alloc(out.binNodes, nodeCapacity)); RT_TRY(alloc(done, subtreeCapacity));
+    }
     RT_TRY(alloc(out.wideNodes, (size_t)wideCapacity * 5));
     RT_TRY(alloc(out.packedTris, (size_t)n * 3));
     RT_TRY(alloc(jobs, wideCapacity)); RT_TRY(alloc(jobsB, wideCapacity));
@@ -829,7 +1112,9 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         root.node = 0; root.first = 0; root.count = n; root.depth = 0;
         for (int a = 0; a < 3; a++) { root.lo[a] = root.clo[a] = FLT_MAX; root.hi[a] = root.chi[a] = -FLT_MAX; }
         RT_TRY(cudaMemcpyAsync(tasks, &root, sizeof(Task), cudaMemcpyHostToDevice, stream));
-        int init[8] = {1, 0, 0, 0, 0, 0, 0, 0};
+        // A root of few primitives is a subtree task itself.
+        const bool smallRoot = n <= kSubtree;
+        int init[kCounters] = {1, 0, 0, 0, smallRoot ? 1 : 0, 0, 0, 0};
         RT_TRY(cudaMemcpyAsync(counters, init, sizeof(init), cudaMemcpyHostToDevice, stream));
         if (!primTri)
             primBoxesKernel<<<blocksFor(n, 256), 256, 0, stream>>>(tris, n, out.primLo, out.primHi, cent, tasks);
@@ -849,65 +1134,82 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         RT_TRY(cudaMemsetAsync(levelCounts, 0, sizeof(int) * 2 * levelSlots, stream));
         RT_TRY(cudaMemsetAsync(levelStartDev, 0, sizeof(int) * (levelSlots + 2), stream));
         {
-            int rootCounts[2] = {1, n > kSmallTask ? 1 : 0};
+            int rootCounts[2] = {smallRoot ? 0 : 1, n > kSmallTask ? 1 : 0};
             int starts[2] = {0, 1};  // depth 0 holds node 0
             RT_TRY(cudaMemcpyAsync(levelCounts, rootCounts, sizeof(rootCounts), cudaMemcpyHostToDevice, stream));
             RT_TRY(cudaMemcpyAsync(levelStartDev, starts, sizeof(starts), cudaMemcpyHostToDevice, stream));
         }
-        const int perTaskBlocks = std::max(1, std::min(blocksFor(taskCapacity, 8), 1184));
+        if (smallRoot) RT_TRY(cudaMemcpyAsync(subtrees, tasks, sizeof(Task), cudaMemcpyDeviceToDevice, stream));
+        const int largeBlocks = n > kSmallTask ? blocksFor(n, kBinBlock * kBinPer) : 0;
+        const int smallBlocks = std::max(1, std::min(blocksFor(taskCapacity, 8), 1184));
         const int splitBlocks = std::max(1, std::min(blocksFor(taskCapacity, 128), 592));
         const int clearBlocks = std::max(1, std::min(blocksFor((long long)taskCapacity * 3 * kBins, 256), 1184));
-        int level = 0;
-        for (;;) {
-            for (int b = 0; b < kLevelBatch && level < levelSlots - 1; b++, level++) {
-                const int* tc = levelCounts + 2 * level;
-                int* nc = levelCounts + 2 * (level + 1);
-                clearBinsKernel<<<clearBlocks, 256, 0, stream>>>(bins, tc, tasks);
-                binKernel<<<blocksFor(n, kBinBlock * kBinPer), kBinBlock, 0, stream>>>(out.order, posTask, cent, out.primLo,
-                                                                                        out.primHi, tasks, n, bins, tc);
-                binSmallKernel<<<perTaskBlocks, 256, 0, stream>>>(out.order, cent, out.primLo, out.primHi, tasks, tc, bins);
-                splitKernel<<<splitBlocks, 128, 0, stream>>>(tasks, tc, bins, splits, rawNodes, counters, nc, tasksB,
-                                                             nodeCapacity, taskCapacity, leafSize);
-                recordLevelKernel<<<1, 1, 0, stream>>>(counters, levelStartDev + level + 2);
-                flagKernel<<<blocksFor(n, 256), 256, 0, stream>>>(out.order, posTask, cent, tasks, splits, n, flags);
-                scanBlocksKernel<<<nScanBlocks, 256, 0, stream>>>(flags, prefix, n, blockSums);
-                scanTotalsKernel<<<1, 1024, 0, stream>>>(blockSums, nScanBlocks);
-                scatterKernel<<<blocksFor(n, 256), 256, 0, stream>>>(out.order, posTask, tasks, splits, flags, prefix,
-                                                                     blockSums, n, orderB, posTaskB, counters + 3);
-                std::swap(out.order, orderB); std::swap(posTask, posTaskB); std::swap(tasks, tasksB);
+        clearBinsKernel<<<clearBlocks, 256, 0, stream>>>(bins, levelCounts, tasks);
+        int level = 0, used = 0;  // levels queued, and those that held tasks
+        if (!smallRoot)
+            for (int batch = kLevelBatch;; batch = kNextLevels) {
+                for (int b = 0; b < batch && level < levelSlots - 1; b++, level++) {
+                    const int* tc = levelCounts + 2 * level;
+                    int* nc = levelCounts + 2 * (level + 1);
+                    binKernel<<<largeBlocks + smallBlocks, kBinBlock, 0, stream>>>(out.order, posTask, cent, out.primLo, out.primHi,
+                                                                                   tasks, n, bins, tc, largeBlocks);
+                    splitKernel<<<splitBlocks, 128, 0, stream>>>(tasks, tc, bins, splits, rawNodes, counters, nc, tasksB, subtrees,
+                                                                 nodeCapacity, taskCapacity, subtreeCapacity, leafSize);
+                    partitionKernel<<<nScanBlocks, 256, 0, stream>>>(out.order, posTask, cent, tasks, splits, n, flags, prefix,
+                                                                     blockSums, counters, levelStartDev + level + 2, tc, nc,
+                                                                     tasksB, bins);
+                    scatterKernel<<<blocksFor(n, 256), 256, 0, stream>>>(out.order, posTask, tasks, splits, flags, prefix,
+                                                                         blockSums, n, orderB, posTaskB, tc, counters + 3);
+                    std::swap(out.order, orderB); std::swap(posTask, posTaskB); std::swap(tasks, tasksB);
+                }
+                RT_TRY(cudaGetLastError());
+                RT_TRY(cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream));
+                RT_TRY(cudaMemcpyAsync(hostLevels, levelCounts, sizeof(int) * 2 * levelSlots, cudaMemcpyDeviceToHost, stream));
+                RT_TRY(cudaStreamSynchronize(stream));
+                if (hostCounters[3]) { *failure = "BVH build ran out of node or task capacity"; err = cudaErrorMemoryAllocation; goto done; }
+                if (hostLevels[2 * level] == 0) break;  // the next level has no task
+                if (level >= levelSlots - 1) { *failure = "BVH build exceeded the depth limit"; err = cudaErrorUnknown; goto done; }
             }
-            RT_TRY(cudaGetLastError());
-            RT_TRY(cudaMemcpyAsync(hostCounters, counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-            RT_TRY(cudaMemcpyAsync(hostLevels, levelCounts, sizeof(int) * 2 * levelSlots, cudaMemcpyDeviceToHost, stream));
-            RT_TRY(cudaStreamSynchronize(stream));
-            if (hostCounters[3]) { *failure = "BVH build ran out of node or task capacity"; err = cudaErrorMemoryAllocation; goto done; }
-            if (hostLevels[2 * level] == 0) break;  // the next level has no task
-            if (level >= levelSlots - 1) { *failure = "BVH build exceeded the depth limit"; err = cudaErrorUnknown; goto done; }
-        }
+        while (used < level && hostLevels[2 * used] > 0) used++;
+        if ((level - used) & 1) std::swap(out.order, orderB);  // levels past the last moved nothing
+        // Subtrees of small tasks. Few are known before the levels end; the
+        // kernel loops over the device count.
+        const int topNodes = smallRoot ? 1 : hostCounters[0];
+        subtreeKernel<<<std::max(1, std::min(blocksFor(subtreeCapacity, kSubtreeWarps), 148 * 8)), 32 * kSubtreeWarps, 0, stream>>>(
+            out.order, cent, out.primLo, out.primHi, subtrees, counters, rawNodes, nodeCapacity, leafSize, interior, done);
+        RT_TRY(cudaGetLastError());
+        RT_TRY(cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream));
         RT_TRY(cudaMemcpyAsync(hostStarts, levelStartDev, sizeof(int) * (level + 2), cudaMemcpyDeviceToHost, stream));
         RT_TRY(cudaStreamSynchronize(stream));
+        if (hostCounters[3]) { *failure = "BVH build ran out of node or task capacity"; err = cudaErrorMemoryAllocation; goto done; }
         levelStart.assign(hostStarts, hostStarts + level + 2);
         int nodeCount = hostCounters[0];
         result.binaryNodes = nodeCount;
         result.binaryDepth = hostCounters[2];
-        // levelStart[d] .. levelStart[d+1] are the nodes of depth d.
-        while (levelStart.size() > 2 && levelStart.back() == levelStart[levelStart.size() - 2]) levelStart.pop_back();
-        int depths = (int)levelStart.size() - 1;
-        for (int d = depths - 1; d >= 0; d--) {
-            int b = levelStart[d], e = levelStart[d + 1];
-            subtreeInteriorKernel<<<blocksFor(e - b, 256), 256, 0, stream>>>(rawNodes, b, e, interior);
+        if (renumber) {
+            // levelStart[d] .. levelStart[d+1] are the nodes of depth d made level by level.
+            while (levelStart.size() > 2 && levelStart.back() == levelStart[levelStart.size() - 2]) levelStart.pop_back();
+            int depths = (int)levelStart.size() - 1;
+            for (int d = depths - 1; d >= 0; d--) {
+                int b = levelStart[d], e = levelStart[d + 1];
+                subtreeInteriorKernel<<<blocksFor(e - b, 256), 256, 0, stream>>>(rawNodes, b, e, topNodes, interior);
+            }
+            RT_TRY(cudaMemsetAsync(rank, 0xFF, sizeof(int) * topNodes, stream));
+            RT_TRY(cudaMemsetAsync(newIndex, 0xFF, sizeof(int) * topNodes, stream));
+            RT_TRY(cudaMemsetAsync(rank, 0, sizeof(int), stream));
+            RT_TRY(cudaMemsetAsync(newIndex, 0, sizeof(int), stream));
+            for (int d = 0; d < depths; d++) {
+                int b = levelStart[d], e = levelStart[d + 1];
+                preorderKernel<<<blocksFor(e - b, 256), 256, 0, stream>>>(rawNodes, b, e, topNodes, nodeCount, interior, rank,
+                                                                          newIndex, counters + 3);
+            }
+            renumberKernel<<<blocksFor(topNodes, 256), 256, 0, stream>>>(rawNodes, topNodes, nodeCount, newIndex, rank,
+                                                                         out.binNodes, counters + 3);
+            placeSubtreesKernel<<<std::max(1, std::min(blocksFor(subtreeCapacity, 8), 1184)), 256, 0, stream>>>(
+                rawNodes, done, counters, rank, nodeCount, out.binNodes, counters + 3);
+        } else {
+            std::swap(out.binNodes, rawNodes);
         }
-        RT_TRY(cudaMemsetAsync(rank, 0xFF, sizeof(int) * nodeCount, stream));
-        RT_TRY(cudaMemsetAsync(newIndex, 0xFF, sizeof(int) * nodeCount, stream));
-        RT_TRY(cudaMemsetAsync(rank, 0, sizeof(int), stream));
-        RT_TRY(cudaMemsetAsync(newIndex, 0, sizeof(int), stream));
-        for (int d = 0; d < depths; d++) {
-            int b = levelStart[d], e = levelStart[d + 1];
-            preorderKernel<<<blocksFor(e - b, 256), 256, 0, stream>>>(rawNodes, b, e, nodeCount, interior, rank,
-                                                                      newIndex, counters + 3);
-        }
-        renumberKernel<<<blocksFor(nodeCount, 256), 256, 0, stream>>>(rawNodes, nodeCount, newIndex, out.binNodes,
-                                                                      counters + 3);
         RT_TRY(cudaGetLastError());
         RT_TRY(cudaEventRecord(e1, stream));
 
@@ -961,7 +1263,8 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     }
 done:
 #undef RT_TRY
-    rt::deviceFree(cent); rt::deviceFree(orderB); rt::deviceFree(posTask); rt::deviceFree(posTaskB); rt::deviceFree(tasks); rt::deviceFree(tasksB);
+    rt::deviceFree(cent); rt::deviceFree(orderB); rt::deviceFree(posTask); rt::deviceFree(posTaskB); rt::deviceFree(tasks); rt::deviceFree(tasksB); rt::deviceFree(subtrees);
+    rt::deviceFree(done);
     rt::deviceFree(bins); rt::deviceFree(splits); rt::deviceFree(flags); rt::deviceFree(prefix); rt::deviceFree(blockSums); rt::deviceFree(counters);
     rt::deviceFree(rawNodes); rt::deviceFree(interior); rt::deviceFree(rank); rt::deviceFree(newIndex); rt::deviceFree(jobs); rt::deviceFree(jobsB);
     rt::deviceFree(primTri);

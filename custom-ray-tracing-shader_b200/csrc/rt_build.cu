@@ -38,10 +38,12 @@ constexpr int kBins = 12;          // bvh.cuh:29
 constexpr int kLeafSize = 4;       // bvh.cuh:64
 constexpr int kScanBlock = 1024;   // elements per scan block
 constexpr int kBinBlock = 256;
-constexpr int kBinPer = 8;         // positions per thread in the binning pass
-// Tasks of at most kSmallTask primitives are binned by one warp each
-// (binSmallKernel); larger ones by position blocks (binKernel).
+constexpr int kBinPer = 8;         // most positions per thread in the binning pass
+// Tasks of at most kSmallTask primitives are binned by one
+// block, or up to kWarpTask by one warp (binKernel); larger ones by position
+// blocks (binLarge).
 constexpr int kSmallTask = 2048;
+constexpr int kWarpTask = 128;
 // Tasks of at most this many primitives are finished by one warp each, down to
 // their leaves (subtreeKernel).
 constexpr int kSubtree = 32;
@@ -249,14 +251,6 @@ __device__ __forceinline__ void clearBins(BinAcc* bins, const int* taskCount, co
 }
 __global__ void clearBinsKernel(BinAcc* bins, const int* taskCount, const Task* tasks) { clearBins(bins, taskCount, tasks); }
 
-__device__ __forceinline__ void accumulateBin(BinAcc* dst, float4 lo, float4 hi, float4 c) {
-    atomicAdd(&dst->count, 1u);
-    atomicMinFloat(&dst->lo[0], lo.x); atomicMinFloat(&dst->lo[1], lo.y); atomicMinFloat(&dst->lo[2], lo.z);
-    atomicMaxFloat(&dst->hi[0], hi.x); atomicMaxFloat(&dst->hi[1], hi.y); atomicMaxFloat(&dst->hi[2], hi.z);
-    atomicMinFloat(&dst->clo[0], c.x); atomicMinFloat(&dst->clo[1], c.y); atomicMinFloat(&dst->clo[2], c.z);
-    atomicMaxFloat(&dst->chi[0], c.x); atomicMaxFloat(&dst->chi[1], c.y); atomicMaxFloat(&dst->chi[2], c.z);
-}
-
 // Floats as integers of the same order (-0 below +0, as the atomics above
 // order them), so warp reductions can use the integer min/max instructions.
 __device__ __forceinline__ int orderedKey(float f) {
@@ -265,295 +259,302 @@ __device__ __forceinline__ int orderedKey(float f) {
 }
 __device__ __forceinline__ float keyFloat(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7FFFFFFF); }
 
-// accumulateBin for a whole warp (every lane calls it; dst null: no
-// primitive). Spatially coherent primitives put most of a warp's lanes into
-// one bin, where per-lane atomics would serialise on one address: the lanes
-// of the first two destinations are reduced with warp instructions and
-// their leaders add the results; the lanes left over use per-lane atomics.
-// Counts and minima/maxima do not depend on the order of accumulation.
-__device__ void warpAccumulate(BinAcc* dst, float4 lo, float4 hi, float4 c) {
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    unsigned pending = __ballot_sync(full, dst != nullptr);
-    for (int round = 0; round < 2 && pending; round++) {
-        const int leader = __ffs(pending) - 1;
-        BinAcc* first = reinterpret_cast<BinAcc*>(__shfl_sync(full, reinterpret_cast<unsigned long long>(dst), leader));
-        const bool mine = dst != nullptr && dst == first;
-        const unsigned group = __ballot_sync(full, mine);
-        const int kMin = 0x7FFFFFFF, kMax = (int)0x80000000;
-        const int l0 = __reduce_min_sync(full, mine ? orderedKey(lo.x) : kMin);
-        const int l1 = __reduce_min_sync(full, mine ? orderedKey(lo.y) : kMin);
-        const int l2 = __reduce_min_sync(full, mine ? orderedKey(lo.z) : kMin);
-        const int h0 = __reduce_max_sync(full, mine ? orderedKey(hi.x) : kMax);
-        const int h1 = __reduce_max_sync(full, mine ? orderedKey(hi.y) : kMax);
-        const int h2 = __reduce_max_sync(full, mine ? orderedKey(hi.z) : kMax);
-        const int c0 = __reduce_min_sync(full, mine ? orderedKey(c.x) : kMin);
-        const int c1 = __reduce_min_sync(full, mine ? orderedKey(c.y) : kMin);
-        const int c2 = __reduce_min_sync(full, mine ? orderedKey(c.z) : kMin);
-        const int d0 = __reduce_max_sync(full, mine ? orderedKey(c.x) : kMax);
-        const int d1 = __reduce_max_sync(full, mine ? orderedKey(c.y) : kMax);
-        const int d2 = __reduce_max_sync(full, mine ? orderedKey(c.z) : kMax);
-        if (lane == leader) {
-            atomicAdd(&first->count, (unsigned)__popc(group));
-            atomicMinFloat(&first->lo[0], keyFloat(l0)); atomicMinFloat(&first->lo[1], keyFloat(l1));
-            atomicMinFloat(&first->lo[2], keyFloat(l2));
-            atomicMaxFloat(&first->hi[0], keyFloat(h0)); atomicMaxFloat(&first->hi[1], keyFloat(h1));
-            atomicMaxFloat(&first->hi[2], keyFloat(h2));
-            atomicMinFloat(&first->clo[0], keyFloat(c0)); atomicMinFloat(&first->clo[1], keyFloat(c1));
-            atomicMinFloat(&first->clo[2], keyFloat(c2));
-            atomicMaxFloat(&first->chi[0], keyFloat(d0)); atomicMaxFloat(&first->chi[1], keyFloat(d1));
-            atomicMaxFloat(&first->chi[2], keyFloat(d2));
-        }
-        pending &= ~group;
+// A bin in shared memory, its values as ordered keys. A value that does not
+// improve the bin costs a read and a comparison: after the first few
+// primitives nearly all of them, where adding each with atomics (13 per
+// primitive and axis, the lanes of one bin one after another) bound binning
+// (110-200 us a level for 1.3M primitives, 2.5 of the 6.1 ms build). Counts
+// and minima/maxima do not depend on the order of accumulation, and a stale
+// read only makes an atomic that changes nothing.
+struct BinKeys { unsigned count; int lo[3], hi[3], clo[3], chi[3]; };
+struct PrimKeys { int lo[3], hi[3], c[3]; };
+__device__ __forceinline__ PrimKeys primKeys(float4 lo, float4 hi, float4 c) {
+    return PrimKeys{{orderedKey(lo.x), orderedKey(lo.y), orderedKey(lo.z)},
+                    {orderedKey(hi.x), orderedKey(hi.y), orderedKey(hi.z)},
+                    {orderedKey(c.x), orderedKey(c.y), orderedKey(c.z)}};
+}
+__device__ __forceinline__ void clearKeys(BinKeys& b) {
+    b.count = 0;
+    for (int a = 0; a < 3; a++) {
+        b.lo[a] = b.clo[a] = orderedKey(FLT_MAX);
+        b.hi[a] = b.chi[a] = orderedKey(-FLT_MAX);
     }
-    if ((pending >> lane) & 1u) accumulateBin(dst, lo, hi, c);
+}
+__device__ __forceinline__ void lower(int* at, int v) {
+    if (v < *reinterpret_cast<volatile int*>(at)) atomicMin(at, v);
+}
+__device__ __forceinline__ void raise(int* at, int v) {
+    if (v > *reinterpret_cast<volatile int*>(at)) atomicMax(at, v);
+}
+__device__ __forceinline__ void addToBin(BinKeys& b, const PrimKeys& p) {
+    atomicAdd(&b.count, 1u);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        lower(&b.lo[a], p.lo[a]);
+        raise(&b.hi[a], p.hi[a]);
+        lower(&b.clo[a], p.c[a]);
+        raise(&b.chi[a], p.c[a]);
+    }
+}
+__device__ __forceinline__ BinAcc toBin(const BinKeys& k) {
+    BinAcc b;
+    b.count = k.count;
+    for (int a = 0; a < 3; a++) {
+        b.lo[a] = keyFloat(k.lo[a]); b.hi[a] = keyFloat(k.hi[a]);
+        b.clo[a] = keyFloat(k.clo[a]); b.chi[a] = keyFloat(k.chi[a]);
+    }
+    return b;
 }
 
-// Bins every primitive of the open tasks above kSmallTask. The task owning the
-// first position of a block's chunk is aggregated in shared memory (sb, 3 *
-// kBins); others go to global bins.
+// Bins every primitive of the open tasks above kSmallTask. A block takes a
+// chunk of at most kSmallTask positions, which therefore meets at most two of
+// them, at its ends: their bins are two sets of shared ones (sb, 2 x 3 kBins),
+// added to the global bins at the end.
 __device__ void binLarge(const int* order, const int* posTask, const float4* cent, const float4* plo, const float4* phi,
-                         const Task* tasks, int nPos, BinAcc* bins, const int* taskCount, BinAcc* sb) {
-    __shared__ int sTask;
+                         const Task* tasks, int nPos, BinAcc* bins, const int* taskCount, BinKeys* sb, int perThread) {
+    __shared__ int ends[2];
     if (!taskCount[1]) return;  // no task above kSmallTask at this level
-    int base = blockIdx.x * kBinBlock * kBinPer;
-    if (threadIdx.x == 0) sTask = base < nPos ? posTask[base] : -1;
-    if (threadIdx.x < 3 * kBins) {
-        BinAcc& b = sb[threadIdx.x];
-        b.count = 0;
-        for (int a = 0; a < 3; a++) { b.lo[a] = FLT_MAX; b.hi[a] = -FLT_MAX; b.clo[a] = FLT_MAX; b.chi[a] = -FLT_MAX; }
+    const int base = blockIdx.x * kBinBlock * perThread, end = min(base + kBinBlock * perThread, nPos);
+    if (threadIdx.x < 2) {
+        const int t = posTask[threadIdx.x ? end - 1 : base];
+        ends[threadIdx.x] = t >= 0 && tasks[t].count > kSmallTask ? t : -1;
     }
+    for (int i = threadIdx.x; i < 2 * 3 * kBins; i += kBinBlock) clearKeys(sb[i]);
     __syncthreads();
-    int st = sTask;
-    // Every lane walks all kBinPer positions (warpAccumulate needs the whole
-    // warp); positions past the end or of finished or small tasks add nothing.
-    for (int k = 0; k < kBinPer; k++) {
+    for (int k = 0; k < perThread; k++) {
         const int j = base + k * kBinBlock + threadIdx.x;
-        const int t = j < nPos ? posTask[j] : -1;
-        const Task* T = t >= 0 ? &tasks[t] : nullptr;
-        const bool valid = T && T->count > kSmallTask;  // small tasks: binned by binSmallKernel
-        float4 c = make_float4(0, 0, 0, 0), lo = c, hi = c;
-        if (valid) {
-            const int prim = order[j];
-            c = cent[prim]; lo = plo[prim]; hi = phi[prim];
-        }
-        if (!__any_sync(0xFFFFFFFFu, valid)) continue;
+        if (j >= end) break;
+        const int t = posTask[j];
+        if (t < 0 || (t != ends[0] && t != ends[1])) continue;
+        BinKeys* set = sb + (t == ends[0] ? 0 : 3 * kBins);
+        const Task& T = tasks[t];
+        const int prim = order[j];
+        const float4 c = cent[prim];
+        const PrimKeys keys = primKeys(plo[prim], phi[prim], c);
         for (int a = 0; a < 3; a++) {
-            BinAcc* dst = nullptr;
-            if (valid) {
-                const float extent = T->chi[a] - T->clo[a];
-                if (extent > 1e-12f) {
-                    const float s = kBins / extent;
-                    const float ca = a == 0 ? c.x : (a == 1 ? c.y : c.z);
-                    const int b = binOf(ca, T->clo[a], s);
-                    dst = t == st ? &sb[a * kBins + b] : &bins[((size_t)t * 3 + a) * kBins + b];
-                }
-            }
-            warpAccumulate(dst, lo, hi, c);
+            const float extent = T.chi[a] - T.clo[a];
+            if (extent <= 1e-12f) continue;
+            const float ca = a == 0 ? c.x : (a == 1 ? c.y : c.z);
+            addToBin(set[a * kBins + binOf(ca, T.clo[a], kBins / extent)], keys);
         }
     }
     __syncthreads();
-    if (st >= 0 && threadIdx.x < 3 * kBins) {
-        const BinAcc& s = sb[threadIdx.x];
-        if (s.count) {
-            BinAcc* d = &bins[(size_t)st * 3 * kBins + threadIdx.x];
-            atomicAdd(&d->count, s.count);
-            for (int a = 0; a < 3; a++) {
-                atomicMinFloat(&d->lo[a], s.lo[a]); atomicMaxFloat(&d->hi[a], s.hi[a]);
-                atomicMinFloat(&d->clo[a], s.clo[a]); atomicMaxFloat(&d->chi[a], s.chi[a]);
-            }
+    for (int i = threadIdx.x; i < 2 * 3 * kBins; i += kBinBlock) {
+        const int s = i / (3 * kBins), t = ends[s];
+        if (t < 0 || !sb[i].count) continue;
+        const BinAcc b = toBin(sb[i]);
+        BinAcc* d = &bins[(size_t)t * 3 * kBins + i % (3 * kBins)];
+        atomicAdd(&d->count, b.count);
+        for (int a = 0; a < 3; a++) {
+            atomicMinFloat(&d->lo[a], b.lo[a]); atomicMaxFloat(&d->hi[a], b.hi[a]);
+            atomicMinFloat(&d->clo[a], b.clo[a]); atomicMaxFloat(&d->chi[a], b.chi[a]);
         }
     }
 }
 
-__device__ void binSmallTask(const int* order, const float4* cent, const float4* plo, const float4* phi,
-                             const Task T, int t, BinAcc* bins, BinAcc* my, int lane) {
-    if (T.count > kSmallTask) return;
-    for (int i = lane; i < 3 * kBins; i += 32) {
-        BinAcc& b = my[i];
-        b.count = 0;
-        for (int a = 0; a < 3; a++) { b.lo[a] = FLT_MAX; b.hi[a] = -FLT_MAX; b.clo[a] = FLT_MAX; b.chi[a] = -FLT_MAX; }
-    }
+// Adds primitives first + lane, first + lane + step, ... of task T to a warp's
+// own bins.
+__device__ __forceinline__ void binRange(const int* order, const float4* cent, const float4* plo, const float4* phi,
+                                         const Task& T, int first, int step, BinKeys* my, int lane) {
+    for (int i = lane; i < 3 * kBins; i += 32) clearKeys(my[i]);
     __syncwarp();
     float scale[3];
     for (int a = 0; a < 3; a++) {
         float extent = T.chi[a] - T.clo[a];
         scale[a] = extent <= 1e-12f ? 0.0f : kBins / extent;
     }
-    // Per-lane atomics: small tasks are deep in the tree, where a warp's
-    // primitives spread over the bins (warpAccumulate measured slower here).
-    for (int j = T.first + lane; j < T.first + T.count; j += 32) {
+    for (int j = T.first + first + lane; j < T.first + T.count; j += step) {
         const int prim = order[j];
-        const float4 c = cent[prim], lo = plo[prim], hi = phi[prim];
+        const float4 c = cent[prim];
+        const PrimKeys keys = primKeys(plo[prim], phi[prim], c);
         for (int a = 0; a < 3; a++) {
             if (scale[a] == 0.0f) continue;
             const float ca = a == 0 ? c.x : (a == 1 ? c.y : c.z);
-            accumulateBin(&my[a * kBins + binOf(ca, T.clo[a], scale[a])], lo, hi, c);
+            addToBin(my[a * kBins + binOf(ca, T.clo[a], scale[a])], keys);
         }
     }
-    __syncwarp();
-    for (int i = lane; i < 3 * kBins; i += 32) bins[(size_t)t * 3 * kBins + i] = my[i];
     __syncwarp();
 }
 
 // The bins of a level's tasks in one launch. Blocks below largeBlocks: position
-// chunks of the large tasks. The others: one warp per small task, with
-// warp-private bins in shared memory (atomics only within the warp), written
-// out with plain stores, so these bins need no clearing and no global atomics.
-// Bins hold a count and minima/maxima, so the order of accumulation does not
-// change them.
+// chunks of the large tasks. The others take 8 small tasks: one warp each, or
+// all eight warps one after another for tasks above kWarpTask (a warp alone
+// walked 2,048 primitives in 100 us and more), with warp-private bins in
+// shared memory, written out with plain stores, so these bins need no clearing and no global atomics. Bins hold a count and
+// minima/maxima, so the order of accumulation does not change them.
 __global__ void __launch_bounds__(kBinBlock) binKernel(const int* order, const int* posTask, const float4* cent,
                                                        const float4* plo, const float4* phi, const Task* tasks,
-                                                       int nPos, BinAcc* bins, const int* taskCount, int largeBlocks) {
-    __shared__ BinAcc sb[8][3 * kBins];
+                                                       int nPos, BinAcc* bins, const int* taskCount, int largeBlocks,
+                                                       int perThread) {
+    __shared__ BinKeys sb[8][3 * kBins];
     if ((int)blockIdx.x < largeBlocks) {
-        binLarge(order, posTask, cent, plo, phi, tasks, nPos, bins, taskCount, sb[0]);
+        binLarge(order, posTask, cent, plo, phi, tasks, nPos, bins, taskCount, sb[0], perThread);
         return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nTasks = taskCount[0], first = (int)blockIdx.x - largeBlocks, stride = ((int)gridDim.x - largeBlocks) * 8;
-    for (int t = first * 8 + warp; t < nTasks; t += stride)
-        binSmallTask(order, cent, plo, phi, tasks[t], t, bins, sb[warp], lane);
+    for (int base = first * 8; base < nTasks; base += stride) {
+        // Tasks for the whole block, one by one.
+        for (int t = base; t < min(base + 8, nTasks); t++) {
+            const int n = tasks[t].count;
+            if (n <= kWarpTask || n > kSmallTask) continue;
+            const Task T = tasks[t];
+            binRange(order, cent, plo, phi, T, warp * 32, 256, sb[warp], lane);
+            __syncthreads();
+            for (int i = threadIdx.x; i < 3 * kBins; i += kBinBlock) {
+                BinKeys b = sb[0][i];
+                for (int w = 1; w < 8; w++) {
+                    const BinKeys& o = sb[w][i];
+                    b.count += o.count;
+                    for (int a = 0; a < 3; a++) {
+                        b.lo[a] = min(b.lo[a], o.lo[a]); b.hi[a] = max(b.hi[a], o.hi[a]);
+                        b.clo[a] = min(b.clo[a], o.clo[a]); b.chi[a] = max(b.chi[a], o.chi[a]);
+                    }
+                }
+                bins[(size_t)t * 3 * kBins + i] = toBin(b);
+            }
+            __syncthreads();
+        }
+        const int t = base + warp;
+        if (t < nTasks && tasks[t].count <= kWarpTask) {
+            const Task T = tasks[t];
+            binRange(order, cent, plo, phi, T, 0, 32, sb[warp], lane);
+            for (int i = lane; i < 3 * kBins; i += 32) bins[(size_t)t * 3 * kBins + i] = toBin(sb[warp][i]);
+        }
+        __syncthreads();
+    }
 }
 
-// One thread per open task: the reference's SAH sweep, then node records.
-// The counters every task updates (maximum depth, node and task allocation)
-// are aggregated per warp first: one atomic per warp instead of one per
-// task on a single address, which serialised the deep levels (hundreds of
-// thousands of tasks). Node and task numbers within a level are assigned in
-// lane order instead of atomic order; nodes are renumbered to the
-// reference's order after the build, and tasks carry their own ranges.
-// taskCount: this level's counts; nextCount: the next level's (open tasks,
-// tasks above kSmallTask); counters: 0 nodes, 2 maximum depth, 3 error.
-__device__ void splitTask(bool have, const Task& T, int t, const BinAcc* bins, Split* splits, BinNode* nodes,
-                          int* counters, int* nextCount, Task* nextTasks, Task* subtrees, int nodeCapacity,
-                          int taskCapacity, int subtreeCapacity, int leafSize) {
+// Raises the maximum depth; most calls find it there and leave the address alone.
+__device__ __forceinline__ void deepen(int* counters, int depth) {
+    if (*reinterpret_cast<volatile int*>(&counters[2]) < depth) atomicMax(&counters[2], depth);
+}
+
+// A level's splits, one warp per open task: the reference's SAH sweep, then
+// node records and the children's tasks. Candidate j = (axis, cut) sits on
+// lane j, which unites the boxes of its axis's 12 bins on both sides; the
+// 33rd (the z axis's last cut) on lane 0 of a second, uniform step. The first
+// minimum in (axis, cut) order wins, as in the reference's loop. (One thread
+// per task walked the 36 bins in about 11 us whatever the level held.)
+// Node and task numbers within a level come in atomic order; nodes are
+// renumbered to the reference's order after the build, and tasks carry their
+// own ranges. nextCount: the next level's open tasks and those above
+// kSmallTask; counters as listed at kCounters.
+__global__ void __launch_bounds__(128) splitKernel(const Task* tasks, const int* taskCount, const BinAcc* bins, Split* splits,
+                                                   BinNode* nodes, int* counters, int* nextCount, Task* nextTasks,
+                                                   Task* subtrees, int nodeCapacity, int taskCapacity, int subtreeCapacity,
+                                                   int leafSize) {
+    __shared__ BinAcc sb[4][3 * kBins];
     const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    int bestAxis = -1, bestBin = -1;
-    if (have && T.count > leafSize && T.depth != kBinaryMaxDepth) {
-        const float nodeArea = halfArea(T.lo, T.hi);
-        float bestCost = nodeArea * T.count;
-        for (int a = 0; a < 3; a++) {
-            float extent = T.chi[a] - T.clo[a];
-            if (extent <= 1e-12f) continue;
-            const BinAcc* B = &bins[((size_t)t * 3 + a) * kBins];
-            float sufLo[kBins][3], sufHi[kBins][3];
-            int sufN[kBins];
-            float accLo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, accHi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            int accN = 0;
-            for (int b = kBins - 1; b >= 0; b--) {
-                if (B[b].count) growBox(accLo, accHi, B[b].lo, B[b].hi);
-                accN += (int)B[b].count;
-                for (int k = 0; k < 3; k++) { sufLo[b][k] = accLo[k]; sufHi[b][k] = accHi[k]; }
-                sufN[b] = accN;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nTasks = taskCount[0], warps = (int)gridDim.x * 4;
+    BinAcc* B = sb[warp];
+    for (int t = (int)blockIdx.x * 4 + warp; t < nTasks; t += warps) {
+        const Task T = tasks[t];
+        // Every open task has more than leafSize primitives and is above the
+        // depth limit.
+        constexpr int kWords = 3 * kBins * (int)(sizeof(BinAcc) / 4);
+        __syncwarp();
+        for (int i = lane; i < kWords; i += 32)
+            reinterpret_cast<unsigned*>(B)[i] = reinterpret_cast<const unsigned*>(bins + (size_t)t * 3 * kBins)[i];
+        __syncwarp();
+        const float nodeArea = halfArea(T.lo, T.hi), unsplit = nodeArea * T.count;
+        bool valid[3];
+        for (int a = 0; a < 3; a++) valid[a] = !(T.chi[a] - T.clo[a] <= 1e-12f);
+        // Boxes and counts on both sides of a candidate.
+        float box[2][6];
+        int count[2];
+        auto sweep = [&](int axis, int cut) {
+            for (int s = 0; s < 2; s++) {
+                for (int k = 0; k < 3; k++) { box[s][k] = FLT_MAX; box[s][3 + k] = -FLT_MAX; }
+                count[s] = 0;
             }
-            float preLo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, preHi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            int preN = 0;
-            for (int b = 0; b < kBins - 1; b++) {
-                if (B[b].count) growBox(preLo, preHi, B[b].lo, B[b].hi);
-                preN += (int)B[b].count;
-                if (!preN || !sufN[b + 1]) continue;
-                float cost = nodeArea + halfArea(preLo, preHi) * preN + halfArea(sufLo[b + 1], sufHi[b + 1]) * sufN[b + 1];
-                if (cost < bestCost) { bestCost = cost; bestAxis = a; bestBin = b; }
+            for (int b = 0; b < kBins; b++) {
+                const BinAcc& o = B[axis * kBins + b];
+                if (!o.count) continue;
+                if (b <= cut) { growBox(box[0], box[0] + 3, o.lo, o.hi); count[0] += (int)o.count; }
+                else { growBox(box[1], box[1] + 3, o.lo, o.hi); count[1] += (int)o.count; }
             }
+        };
+        auto candidateCost = [&](bool axisValid) {
+            if (!axisValid || !count[0] || !count[1]) return FLT_MAX;
+            return nodeArea + halfArea(box[0], box[0] + 3) * count[0] + halfArea(box[1], box[1] + 3) * count[1];
+        };
+        sweep(2, kBins - 2);
+        const float last = candidateCost(valid[2]);
+        const int axis = lane / 11, cut = lane % 11;
+        sweep(axis, cut);
+        const float cost = candidateCost(axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]);
+        // Costs are sums of areas, not negative: their bits order like them.
+        const unsigned bits = cost < unsplit ? __float_as_uint(cost) : full;
+        const unsigned best = __reduce_min_sync(full, bits);
+        int bestAxis = -1, bestBin = -1;
+        if (best != full) {
+            const int winner = __ffs(__ballot_sync(full, bits == best)) - 1;
+            bestAxis = winner / 11;
+            bestBin = winner % 11;
         }
-    }
-    const bool split = bestAxis >= 0;
-    // Children's boxes, centroid boxes and counts are unions over the bins.
-    Task C[2];
-    bool open[2] = {false, false}, small[2] = {false, false};  // small: finished by subtreeKernel
-    if (split) {
-        for (int side = 0; side < 2; side++) {
-            for (int k = 0; k < 3; k++) { C[side].lo[k] = C[side].clo[k] = FLT_MAX; C[side].hi[k] = C[side].chi[k] = -FLT_MAX; }
-            C[side].count = 0;
-        }
-        const BinAcc* B = &bins[((size_t)t * 3 + bestAxis) * kBins];
-        for (int b = 0; b < kBins; b++) {
-            if (!B[b].count) continue;
-            Task& c = C[b <= bestBin ? 0 : 1];
-            growBox(c.lo, c.hi, B[b].lo, B[b].hi);
-            growBox(c.clo, c.chi, B[b].clo, B[b].chi);
-            c.count += (int)B[b].count;
-        }
-        for (int side = 0; side < 2; side++) {
-            C[side].depth = T.depth + 1;
-            open[side] = !(C[side].count <= leafSize || C[side].depth == kBinaryMaxDepth);
-            small[side] = open[side] && C[side].count <= kSubtree;
-            open[side] = open[side] && !small[side];
-        }
-    }
-    // Maximum depth: a task's own, its children's when it splits.
-    const int depth = __reduce_max_sync(full, have ? T.depth + (split ? 1 : 0) : -1);
-    if (lane == 0 && depth >= 0) atomicMax(&counters[2], depth);
-    // Two nodes per split task.
-    const unsigned splitMask = __ballot_sync(full, split);
-    const unsigned below = (1u << lane) - 1u;
-    int childBase = 0;
-    if (lane == 0 && splitMask) childBase = atomicAdd(&counters[0], 2 * __popc(splitMask));
-    childBase = __shfl_sync(full, childBase, 0);
-    // Next-level tasks: the open children, side 0 before side 1.
-    const unsigned open0 = __ballot_sync(full, open[0]), open1 = __ballot_sync(full, open[1]);
-    const unsigned big0 = __ballot_sync(full, open[0] && C[0].count > kSmallTask);
-    const unsigned big1 = __ballot_sync(full, open[1] && C[1].count > kSmallTask);
-    int taskBase = 0;
-    if (lane == 0 && (open0 | open1)) taskBase = atomicAdd(&nextCount[0], __popc(open0) + __popc(open1));
-    if (lane == 0 && (big0 | big1)) atomicAdd(&nextCount[1], __popc(big0) + __popc(big1));
-    taskBase = __shfl_sync(full, taskBase, 0);
-    const unsigned small0 = __ballot_sync(full, small[0]), small1 = __ballot_sync(full, small[1]);
-    int subtreeBase = 0;
-    if (lane == 0 && (small0 | small1)) subtreeBase = atomicAdd(&counters[4], __popc(small0) + __popc(small1));
-    subtreeBase = __shfl_sync(full, subtreeBase, 0);
-    if (!have) return;
-
-    Split S;
-    S.axis = bestAxis; S.bin = bestBin; S.leftCount = 0; S.childTask[0] = S.childTask[1] = -1;
-    if (!split) {
-        nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), T.first, v3(T.hi[0], T.hi[1], T.hi[2]), T.count};
-        splits[t] = S;
-        return;
-    }
-    const int child = childBase + 2 * __popc(splitMask & below);
-    if (child + 2 > nodeCapacity) { atomicExch(&counters[3], 1); splits[t] = Split{-1, -1, 0, {-1, -1}}; return; }
-    nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), child, v3(T.hi[0], T.hi[1], T.hi[2]), 0};
-    C[0].first = T.first;
-    C[1].first = T.first + C[0].count;
-    S.leftCount = C[0].count;
-    int k = taskBase + __popc(open0 & below) + __popc(open1 & below);
-    int m = subtreeBase + __popc(small0 & below) + __popc(small1 & below);
-    for (int side = 0; side < 2; side++) {
-        Task& c = C[side];
-        c.node = child + side;
-        if (small[side]) {
-            if (m >= subtreeCapacity) atomicExch(&counters[3], 2);
-            else subtrees[m] = c;
-            m++;
+        if (last < unsplit && __float_as_uint(last) < best) { bestAxis = 2; bestBin = kBins - 2; }
+        if (bestAxis < 0) {
+            if (lane == 0) {
+                nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), T.first, v3(T.hi[0], T.hi[1], T.hi[2]), T.count};
+                splits[t] = Split{-1, -1, 0, {-1, -1}};
+                deepen(counters, T.depth);
+            }
             continue;
         }
-        if (!open[side]) {
-            nodes[c.node] = BinNode{v3(c.lo[0], c.lo[1], c.lo[2]), c.first, v3(c.hi[0], c.hi[1], c.hi[2]), c.count};
+        // Lane s < 2 makes child s: its boxes, centroid boxes and count are
+        // unions over its bins.
+        int child = 0, leftCount = 0;
+        Task C;
+        C.count = 0;
+        bool open = false, small = false;
+        if (lane < 2) {
+            for (int k = 0; k < 3; k++) { C.lo[k] = C.clo[k] = FLT_MAX; C.hi[k] = C.chi[k] = -FLT_MAX; }
+            for (int b = 0; b < kBins; b++) {
+                const BinAcc& o = B[bestAxis * kBins + b];
+                if (!o.count || (b <= bestBin) != (lane == 0)) continue;
+                growBox(C.lo, C.hi, o.lo, o.hi);
+                growBox(C.clo, C.chi, o.clo, o.chi);
+                C.count += (int)o.count;
+            }
+            C.depth = T.depth + 1;
+            open = !(C.count <= leafSize || C.depth == kBinaryMaxDepth);
+            small = open && C.count <= kSubtree;
+            open = open && !small;
+        }
+        if (lane == 0) {
+            child = atomicAdd(&counters[0], 2);
+            deepen(counters, T.depth + 1);
+        }
+        child = __shfl_sync(full, child, 0);
+        leftCount = __shfl_sync(full, C.count, 0);
+        if (child + 2 > nodeCapacity) {
+            if (lane == 0) { atomicExch(&counters[3], 1); splits[t] = Split{-1, -1, 0, {-1, -1}}; }
             continue;
         }
-        if (k >= taskCapacity) { atomicExch(&counters[3], 2); k++; continue; }
-        nextTasks[k] = c;
-        S.childTask[side] = k;
-        k++;
-    }
-    splits[t] = S;
-}
-__global__ void splitKernel(const Task* tasks, const int* taskCount, const BinAcc* bins, Split* splits, BinNode* nodes,
-                            int* counters, int* nextCount, Task* nextTasks, Task* subtrees, int nodeCapacity,
-                            int taskCapacity, int subtreeCapacity, int leafSize) {
-    const int nTasks = taskCount[0];
-    // Whole warps walk the tasks (splitTask uses warp collectives).
-    for (int base = blockIdx.x * blockDim.x; base < nTasks; base += gridDim.x * blockDim.x) {
-        const int t = base + (int)threadIdx.x;
-        const bool have = t < nTasks;
-        Task T;
-        if (have) T = tasks[t];
-        else T.count = 0, T.depth = 0;
-        splitTask(have, T, t, bins, splits, nodes, counters, nextCount, nextTasks, subtrees, nodeCapacity, taskCapacity,
-                  subtreeCapacity, leafSize);
+        int taskIndex = -1;
+        if (lane < 2) {
+            C.node = child + lane;
+            C.first = T.first + (lane ? leftCount : 0);
+            if (small) {
+                const int m = atomicAdd(&counters[4], 1);
+                if (m >= subtreeCapacity) atomicExch(&counters[3], 2);
+                else subtrees[m] = C;
+            } else if (open) {
+                const int k = atomicAdd(&nextCount[0], 1);
+                if (C.count > kSmallTask) atomicAdd(&nextCount[1], 1);
+                if (k >= taskCapacity) atomicExch(&counters[3], 2);
+                else { nextTasks[k] = C; taskIndex = k; }
+            } else {
+                nodes[C.node] = BinNode{v3(C.lo[0], C.lo[1], C.lo[2]), C.first, v3(C.hi[0], C.hi[1], C.hi[2]), C.count};
+            }
+        }
+        const int rightTask = __shfl_sync(full, taskIndex, 1);
+        if (lane == 0) {
+            nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), child, v3(T.hi[0], T.hi[1], T.hi[2]), 0};
+            splits[t] = Split{bestAxis, bestBin, leftCount, {taskIndex, rightTask}};
+        }
     }
 }
 
@@ -866,7 +867,7 @@ __global__ void __launch_bounds__(32 * kSubtreeWarps) subtreeKernel(int* order, 
         int base = 0;
         if (lane == 0) {
             if (interior) base = atomicAdd(&counters[0], 2 * interior);
-            atomicMax(&counters[2], depth);
+            deepen(counters, depth);
         }
         base = __shfl_sync(full, base, 0);
         __syncwarp();
@@ -943,44 +944,259 @@ __global__ void placeSubtreesKernel(const BinNode* nodes, const Subtree* done, c
 }
 
 // ---- collapse into wide nodes (logic in rt_collapse.cuh) ----
+// planCollapse and emitCollapse with eight lanes per job (four jobs a warp):
+// a lane holds one candidate while the node's children are opened, then one
+// kid: its box, triangles, slot and quantised planes. One thread per job
+// walked some hundred dependent loads one after another (65 us a level even
+// for a few jobs). The choices, their order and the arithmetic are
+// planCollapse's; within a level storage comes in job order per warp.
 // jobCount: this wide level's jobs; nextCount receives the next level's.
-__global__ void collapseKernel(const BinNode* bn, const int* order, const float4* plo, const float4* phi,
+struct CollapseShared { WideNode node[4]; };
+__global__ void __launch_bounds__(64) collapseKernel(const BinNode* bn, const int* order, const float4* plo, const float4* phi,
                                const SceneTri* tris, const Job* jobs, const int* jobCount, Job* nextJobs,
                                int* nextCount, WideNode* wide, float4* packed, int* counters, int wideCapacity,
                                int jobCapacity, int triCapacity, int group, int width, const int* primTri) {
-    // Whole warps walk the jobs: each plans its node, then the warp's wide
-    // children, packed triangles and next-level jobs are allocated with one
-    // atomic each (in lane order) instead of one per job on a single address.
-    const int nJobs = *jobCount;
+    __shared__ CollapseShared shared[2];
     const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x; base < nJobs; base += gridDim.x * blockDim.x) {
-        const int j = base + (int)threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, slotOfJob = lane >> 3;
+    const int nJobs = *jobCount;
+    auto get = [&](auto v, int from) { return __shfl_sync(full, v, from, 8); };
+    auto sumAll = [&](int v) { for (int o = 4; o; o >>= 1) v += __shfl_xor_sync(full, v, o, 8); return v; };
+    auto orAll = [&](unsigned v) { for (int o = 4; o; o >>= 1) v |= __shfl_xor_sync(full, v, o, 8); return v; };
+    auto minAll = [&](float v) { for (int o = 4; o; o >>= 1) v = fminf(v, __shfl_xor_sync(full, v, o, 8)); return v; };
+    auto maxAll = [&](float v) { for (int o = 4; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(full, v, o, 8)); return v; };
+    // The lane of the best key (the larger where MAX, the lower lane of
+    // equals), or -1 when no lane takes part.
+    auto pick = [&](float key, bool in, bool largest) {
+        int at = in ? sub : -1;
+        for (int o = 4; o; o >>= 1) {
+            const float k = __shfl_xor_sync(full, key, o, 8);
+            const int l = __shfl_xor_sync(full, at, o, 8);
+            const bool better = l >= 0 && (at < 0 || (largest ? k > key : k < key) || (k == key && l < at));
+            if (better) { key = k; at = l; }
+        }
+        return at;
+    };
+    for (int base = ((int)blockIdx.x * 2 + warp) * 4; base < nJobs; base += (int)gridDim.x * 8) {
+        const int j = base + slotOfJob;
         const bool have = j < nJobs;
-        CollapsePlan P;
-        int ni = 0, nt = 0;
-        if (have) {
-            planCollapse(jobs[j], bn, order, plo, phi, group, width, primTri, P);
-            ni = P.nInterior;
-            nt = P.nTris;
+        Job J = have ? jobs[j] : Job{1, 0, 0, 0, 0};
+        if (have && J.kind == 0 && bn[J.node].count > 0) { J.kind = 1; J.first = bn[J.node].first; J.count = bn[J.node].count; }
+        const bool inner = have && J.kind == 0;
+        // Candidates: lane i holds the i-th.
+        BinNode cand{};
+        int node = -1, slots = 0, opened = 0, nc = inner ? 2 : 0;
+        float area = -1.0f;
+        auto place = [&](int n) {
+            node = n;
+            cand = bn[n];
+            slots = slotsOf(cand, group, width);
+            area = -1.0f;
+            opened = 0;
+            if (cand.count == 0) {
+                const float lo[3] = {cand.low.x, cand.low.y, cand.low.z}, hi[3] = {cand.high.x, cand.high.y, cand.high.z};
+                area = collapseHalfArea(lo, hi);
+                opened = slotsOf(bn[cand.first], group, width) + slotsOf(bn[cand.first + 1], group, width);
+            }
+        };
+        if (inner && sub < 2) place(bn[J.node].first + sub);
+        for (bool more = inner;;) {
+            const int total = sumAll(slots);
+            const bool can = more && node >= 0 && area > -1.0f && nc < width && total - 1 + opened <= width;
+            const int best = pick(area, can, true);
+            more = more && best >= 0;
+            if (!__any_sync(full, more)) break;
+            const int first = get(cand.first, best < 0 ? 0 : best);
+            if (more) {
+                if (sub == best) place(first);
+                else if (sub == nc) place(first + 1);
+                nc++;
+            }
         }
-        int si = ni, st = nt;  // inclusive prefix sums over the warp
-        for (int off = 1; off < 32; off <<= 1) {
-            const int a = __shfl_up_sync(full, si, off), b = __shfl_up_sync(full, st, off);
-            if (lane >= off) { si += a; st += b; }
+        // Leaves that do not fit inline become wide children of their own,
+        // the largest first (the first of equals).
+        bool asNode = false;
+        for (bool more = inner;;) {
+            const int total = sumAll(asNode ? 1 : slots);
+            const bool over = more && total > width;
+            const int at = pick((float)cand.count, over && node >= 0 && !asNode && cand.count > group, true);
+            more = over && at >= 0;
+            if (!__any_sync(full, more)) break;
+            if (more && sub == at) asNode = true;
         }
-        const int ti = __shfl_sync(full, si, 31), tt = __shfl_sync(full, st, 31);
+        // Kids: lane k takes the k-th.
+        int kind = -1, kidNode = -1, first = 0, count = 0;
+        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        {
+            const bool range = node >= 0 && cand.count > 0 && (asNode || cand.count > width * group);
+            const int mine = node < 0 ? 0 : cand.count == 0 || range ? 1 : (cand.count + group - 1) / group;
+            int before = 0;
+            for (int i = 0; i < 8; i++) {
+                const int n = get(mine, i), r = get(range ? 1 : 0, i), cn = get(node, i), cf = get(cand.first, i), cc = get(cand.count, i);
+                const float l[3] = {get(cand.low.x, i), get(cand.low.y, i), get(cand.low.z, i)};
+                const float h[3] = {get(cand.high.x, i), get(cand.high.y, i), get(cand.high.z, i)};
+                if (sub >= before && sub < before + n && sub < width) {
+                    if (cc == 0 || r) {
+                        kind = cc == 0 ? 0 : 1;
+                        kidNode = cc == 0 ? cn : -1;
+                        first = cc == 0 ? 0 : cf;
+                        count = cc;
+                        if (kind == 0)
+                            for (int a = 0; a < 3; a++) { lo[a] = l[a]; hi[a] = h[a]; }
+                    } else {
+                        kind = 2;
+                        first = cf + (sub - before) * group;
+                        count = imin(group, cc - (sub - before) * group);
+                    }
+                }
+                before += n;
+            }
+        }
+        if (have && !inner) {
+            const int chunk = J.count <= width * group ? group : (J.count + width - 1) / width;
+            const int g = sub * chunk;
+            if (g < J.count && sub < width) {
+                first = J.first + g;
+                count = imin(chunk, J.count - g);
+                kind = chunk == group || count <= group ? 2 : 1;
+            }
+        }
+        // Boxes of primitive ranges, and each triangle group's triangles once.
+        int tri[3] = {-1, -1, -1}, nTri = 0;
+        if (kind > 0) {
+            for (int i = 0; i < count; i++) {
+                const int p = order[first + i];
+                const float4 a = plo[p], b = phi[p];
+                lo[0] = fminf(lo[0], a.x); lo[1] = fminf(lo[1], a.y); lo[2] = fminf(lo[2], a.z);
+                hi[0] = fmaxf(hi[0], b.x); hi[1] = fmaxf(hi[1], b.y); hi[2] = fmaxf(hi[2], b.z);
+                if (kind == 2) {
+                    const int t = primTri ? primTri[p] : p;
+                    if (t != tri[0] && t != tri[1] && t != tri[2]) {
+                        if (nTri == 0) tri[0] = t;
+                        else if (nTri == 1) tri[1] = t;
+                        else tri[2] = t;
+                        nTri++;
+                    }
+                }
+            }
+        }
+        float nlo[3], nhi[3];
+        for (int a = 0; a < 3; a++) { nlo[a] = minAll(lo[a]); nhi[a] = maxAll(hi[a]); }
+        // Slots: greedily the cheapest (kid, slot) pair.
+        float ck[3];
+        for (int a = 0; a < 3; a++) ck[a] = 0.5f * (lo[a] + hi[a]) - 0.5f * (nlo[a] + nhi[a]);
+        int slot = -1;
+        {
+            unsigned freeSlots = 0xFFu;
+            const int nk = __popc((__ballot_sync(full, kind >= 0) >> (slotOfJob * 8)) & 0xFFu);
+            const int rounds = __reduce_max_sync(full, nk);
+            float cost = FLT_MAX;
+            int at = -1;
+            auto cheapest = [&]() {
+                cost = FLT_MAX;
+                at = -1;
+                for (int s = 0; s < 8; s++) {
+                    if (!((freeSlots >> s) & 1u)) continue;
+                    const float c = ((s & 4) ? -ck[0] : ck[0]) + ((s & 2) ? -ck[1] : ck[1]) + ((s & 1) ? -ck[2] : ck[2]);
+                    if (c < cost) { cost = c; at = s; }
+                }
+            };
+            if (kind >= 0) cheapest();
+            for (int round = 0; round < rounds; round++) {
+                const bool waiting = kind >= 0 && slot < 0;
+                int winner = pick(cost, waiting && at >= 0, false);
+                const int next = pick(0.0f, waiting, false);
+                int taken = get(at, winner < 0 ? 0 : winner);
+                if (winner < 0) {  // non-finite costs: the first waiting kid into the first free slot
+                    winner = next;
+                    taken = __ffs(freeSlots) - 1;
+                }
+                if (winner >= 0) {
+                    if (sub == winner) slot = taken;
+                    freeSlots &= ~(1u << taken);
+                    if (waiting && sub != winner && at == taken) cheapest();
+                }
+            }
+        }
+        // Storage: the warp's jobs in order.
+        const unsigned innerSlots = orAll(kind == 0 || kind == 1 ? 1u << slot : 0u);
+        const unsigned triCounts = orAll(kind == 2 ? (unsigned)nTri << (2 * slot) : 0u);  // 2 bits per slot
+        const int ni = __popc(innerSlots), nt = __popc(triCounts & 0x5555u) + 2 * __popc(triCounts & 0xAAAAu);
+        int si = 0, st = 0, ti = 0, tt = 0;
+        for (int g = 0; g < 4; g++) {
+            const int a = __shfl_sync(full, ni, g * 8), b = __shfl_sync(full, nt, g * 8);
+            if (g < slotOfJob) { si += a; st += b; }
+            ti += a;
+            tt += b;
+        }
         int childBase = 0, triBase = 0, jobBase = 0;
         if (lane == 0) {
             if (ti) { childBase = atomicAdd(&counters[0], ti); jobBase = atomicAdd(nextCount, ti); }
             if (tt) triBase = atomicAdd(&counters[1], tt);
         }
-        childBase = __shfl_sync(full, childBase, 0);
-        triBase = __shfl_sync(full, triBase, 0);
-        jobBase = __shfl_sync(full, jobBase, 0);
-        if (have)
-            emitCollapse(P, childBase + si - ni, triBase + st - nt, jobBase + si - ni, tris, nextJobs, wide, packed,
-                         counters, wideCapacity, jobCapacity, triCapacity);
+        childBase = __shfl_sync(full, childBase, 0) + si;
+        jobBase = __shfl_sync(full, jobBase, 0) + si;
+        triBase = __shfl_sync(full, triBase, 0) + st;
+        const bool fits = childBase + ni <= wideCapacity && triBase + nt <= triCapacity;
+        if (have && !fits && sub == 0) atomicExch(&counters[3], 3);
+        // The node record in shared memory: lane 0 the header, then each kid
+        // its slot's bytes.
+        WideNode& W = shared[warp].node[slotOfJob];
+        float sc[3];
+        unsigned char ebits[3];
+        for (int a = 0; a < 3; a++) {
+            float extent = nhi[a] - nlo[a];
+            int ex = -126;
+            if (extent > 0.0f) { frexpf(extent / 255.0f, &ex); }
+            ex = imax(-126, imin(127, ex));
+            ebits[a] = (unsigned char)(ex + 127);
+            sc[a] = bitsToFloat((unsigned)ebits[a] << 23);
+        }
+        __syncwarp();
+        if (sub < 5) reinterpret_cast<uint4*>(&W)[sub] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+        if (sub == 0) {
+            W.px = nlo[0]; W.py = nlo[1]; W.pz = nlo[2];
+            W.ex = ebits[0]; W.ey = ebits[1]; W.ez = ebits[2];
+            W.imask = (unsigned char)innerSlots;
+            W.childBase = (unsigned)childBase;
+            W.triBase = (unsigned)triBase;
+        }
+        if (kind >= 0 && fits) {
+            for (int a = 0; a < 3; a++) {
+                const float p = nlo[a];
+                int ql = (int)floorf((lo[a] - p) / sc[a]);
+                int qh = (int)ceilf((hi[a] - p) / sc[a]);
+                ql = imax(0, imin(255, ql));
+                qh = imax(0, imin(255, qh));
+                while (ql > 0 && fmaRn((float)ql, sc[a], p) > lo[a]) ql--;
+                while (qh < 255 && fmaRn((float)qh, sc[a], p) < hi[a]) qh++;
+                W.qlo[a][slot] = (unsigned char)ql;
+                W.qhi[a][slot] = (unsigned char)qh;
+            }
+            const unsigned lower = (1u << slot) - 1u, lower2 = (1u << (2 * slot)) - 1u;
+            if (kind == 2) {
+                const unsigned below = triCounts & lower2;
+                const int offset = __popc(below & 0x5555u) + 2 * __popc(below & 0xAAAAu);
+                W.meta[slot] = (unsigned char)((((1u << nTri) - 1u) << 5) | (unsigned)offset);
+                for (int i = 0; i < nTri; i++) {
+                    const int p = i == 0 ? tri[0] : i == 1 ? tri[1] : tri[2];
+                    const SceneTri& t = tris[p];
+                    float4* dst = packed + (size_t)(triBase + offset + i) * 3;
+                    dst[0] = make_float4(t.origin.x, t.origin.y, t.origin.z, t.edge1.x);
+                    dst[1] = make_float4(t.edge1.y, t.edge1.z, t.edge2.x, t.edge2.y);
+                    dst[2] = make_float4(t.edge2.z, bitsToFloat(t.oneSided != 0 ? 1u : 0u), bitsToFloat((unsigned)p), 0.0f);
+                }
+            } else {
+                W.meta[slot] = (unsigned char)(0x20u | (24u + (unsigned)slot));
+                const int rank = __popc(innerSlots & lower), q = jobBase + rank;
+                if (q >= jobCapacity) atomicExch(&counters[3], 4);
+                else nextJobs[q] = Job{kind, kidNode, first, count, childBase + rank};
+            }
+        }
+        __syncwarp();
+        if (have && fits && sub < 5) reinterpret_cast<uint4*>(wide + J.wide)[sub] = reinterpret_cast<const uint4*>(&W)[sub];
+        __syncwarp();
     }
 }
 
@@ -1140,9 +1356,11 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
             RT_TRY(cudaMemcpyAsync(levelStartDev, starts, sizeof(starts), cudaMemcpyHostToDevice, stream));
         }
         if (smallRoot) RT_TRY(cudaMemcpyAsync(subtrees, tasks, sizeof(Task), cudaMemcpyDeviceToDevice, stream));
-        const int largeBlocks = n > kSmallTask ? blocksFor(n, kBinBlock * kBinPer) : 0;
+        // Enough position blocks for the SMs where there are few positions.
+        const int perThread = std::max(1, std::min(kBinPer, n / (148 * kBinBlock)));
+        const int largeBlocks = n > kSmallTask ? blocksFor(n, kBinBlock * perThread) : 0;
         const int smallBlocks = std::max(1, std::min(blocksFor(taskCapacity, 8), 1184));
-        const int splitBlocks = std::max(1, std::min(blocksFor(taskCapacity, 128), 592));
+        const int splitBlocks = std::max(1, std::min(blocksFor(taskCapacity, 4), 1184));
         const int clearBlocks = std::max(1, std::min(blocksFor((long long)taskCapacity * 3 * kBins, 256), 1184));
         clearBinsKernel<<<clearBlocks, 256, 0, stream>>>(bins, levelCounts, tasks);
         int level = 0, used = 0;  // levels queued, and those that held tasks
@@ -1152,7 +1370,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
                     const int* tc = levelCounts + 2 * level;
                     int* nc = levelCounts + 2 * (level + 1);
                     binKernel<<<largeBlocks + smallBlocks, kBinBlock, 0, stream>>>(out.order, posTask, cent, out.primLo, out.primHi,
-                                                                                   tasks, n, bins, tc, largeBlocks);
+                                                                                   tasks, n, bins, tc, largeBlocks, perThread);
                     splitKernel<<<splitBlocks, 128, 0, stream>>>(tasks, tc, bins, splits, rawNodes, counters, nc, tasksB, subtrees,
                                                                  nodeCapacity, taskCapacity, subtreeCapacity, leafSize);
                     partitionKernel<<<nScanBlocks, 256, 0, stream>>>(out.order, posTask, cent, tasks, splits, n, flags, prefix,
@@ -1223,7 +1441,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         const int jobSlots = kStackCapacity + 2 + kLevelBatch;
         RT_TRY(cudaMemsetAsync(jobCounts, 0, sizeof(int) * jobSlots, stream));
         RT_TRY(cudaMemcpyAsync(jobCounts, cinit, sizeof(int), cudaMemcpyHostToDevice, stream));  // one root job
-        const int collapseBlocks = std::max(1, std::min(blocksFor(jobCapacity, 64), 2368));
+        const int collapseBlocks = std::max(1, std::min(blocksFor(jobCapacity, 8), 2368));
         int wideLevel = 0, wideDepth = 0;
         for (;;) {
             for (int b = 0; b < kLevelBatch && wideLevel < jobSlots - 1; b++, wideLevel++) {

@@ -72,26 +72,35 @@ RT_HD void planCollapse(Job J, const BinNode* bn, const int* order, const float4
     Kid* kids = P.kids;
     int nk = 0;
     if (J.kind == 0) {
-        int cand[8], nc = 2;
+        // Candidates with what opening one needs, read once each: its slots,
+        // and for an interior one its area and the slots after opening it.
+        int cand[8], slots[8], opened[8], nc = 0, total = 0;
+        float area[8];
         bool asNode[8] = {false, false, false, false, false, false, false, false};
-        cand[0] = bn[J.node].first; cand[1] = cand[0] + 1;
-        for (;;) {
-            int total = 0;
-            for (int i = 0; i < nc; i++) total += slotsOf(bn[cand[i]], group, width);
-            int best = -1; float bestArea = -1.0f;
-            for (int i = 0; i < nc; i++) {
-                const BinNode& c = bn[cand[i]];
-                if (c.count != 0 || nc >= width) continue;
-                int after = total - 1 + slotsOf(bn[c.first], group, width) + slotsOf(bn[c.first + 1], group, width);
-                if (after > width) continue;
+        auto place = [&](int i, int node) {
+            const BinNode& c = bn[node];
+            cand[i] = node;
+            slots[i] = slotsOf(c, group, width);
+            area[i] = -1.0f;
+            if (c.count == 0) {
                 float lo[3] = {c.low.x, c.low.y, c.low.z}, hi[3] = {c.high.x, c.high.y, c.high.z};
-                float a = collapseHalfArea(lo, hi);
-                if (a > bestArea) { bestArea = a; best = i; }
+                area[i] = collapseHalfArea(lo, hi);
+                opened[i] = slotsOf(bn[c.first], group, width) + slotsOf(bn[c.first + 1], group, width);
             }
+            total += slots[i];
+        };
+        const int children = bn[J.node].first;
+        place(nc++, children);
+        place(nc++, children + 1);
+        for (;;) {
+            int best = -1; float bestArea = -1.0f;
+            for (int i = 0; i < nc; i++)
+                if (area[i] > bestArea && nc < width && total - 1 + opened[i] <= width) { bestArea = area[i]; best = i; }
             if (best < 0) break;
-            int opened = cand[best];
-            cand[best] = bn[opened].first;
-            cand[nc++] = bn[opened].first + 1;
+            const int first = bn[cand[best]].first;
+            total -= slots[best];
+            place(best, first);
+            place(nc++, first + 1);
         }
         // Leaves that do not fit inline become wide children of their own.
         for (;;) {
@@ -152,22 +161,35 @@ RT_HD void planCollapse(Job J, const BinNode* bn, const int* order, const float4
         for (int a = 0; a < 3; a++) cn[a] = 0.5f * (nlo[a] + nhi[a]);
         for (int k = 0; k < nk; k++)
             for (int a = 0; a < 3; a++) ck[k][a] = 0.5f * (kids[k].lo[a] + kids[k].hi[a]) - cn[a];
-        bool kidUsed[8] = {false, false, false, false, false, false, false, false};
+        // Greedy: the cheapest (kid, slot) pair first, the lower kid and slot
+        // of equals. Each kid keeps its cheapest free slot, looked up again only
+        // when that slot is taken.
+        float cost[8];
+        int at[8];
+        unsigned freeSlots = 0xFFu, left = (1u << nk) - 1u;
+        auto cheapest = [&](int k) {
+            cost[k] = FLT_MAX;
+            at[k] = -1;
+            for (int s = 0; s < 8; s++) {
+                if (!((freeSlots >> s) & 1u)) continue;
+                float c = ((s & 4) ? -ck[k][0] : ck[k][0]) + ((s & 2) ? -ck[k][1] : ck[k][1]) + ((s & 1) ? -ck[k][2] : ck[k][2]);
+                if (c < cost[k]) { cost[k] = c; at[k] = s; }
+            }
+        };
+        for (int k = 0; k < nk; k++) cheapest(k);
         for (int round = 0; round < nk; round++) {
             float best = FLT_MAX; int bk = -1, bs = -1;
-            for (int k = 0; k < nk; k++) {
-                if (kidUsed[k]) continue;
-                for (int s = 0; s < 8; s++) {
-                    if (slotKid[s] >= 0) continue;
-                    float c = ((s & 4) ? -ck[k][0] : ck[k][0]) + ((s & 2) ? -ck[k][1] : ck[k][1]) + ((s & 1) ? -ck[k][2] : ck[k][2]);
-                    if (c < best) { best = c; bk = k; bs = s; }
-                }
-            }
+            for (int k = 0; k < nk; k++)
+                if (((left >> k) & 1u) && cost[k] < best) { best = cost[k]; bk = k; bs = at[k]; }
             if (bk < 0) {  // non-finite costs: first free kid into the first free slot
-                for (int k = 0; k < nk && bk < 0; k++) if (!kidUsed[k]) bk = k;
-                for (int s = 0; s < 8 && bs < 0; s++) if (slotKid[s] < 0) bs = s;
+                for (int k = 0; k < nk && bk < 0; k++) if ((left >> k) & 1u) bk = k;
+                for (int s = 0; s < 8 && bs < 0; s++) if ((freeSlots >> s) & 1u) bs = s;
             }
-            kidUsed[bk] = true; slotKid[bs] = bk;
+            left &= ~(1u << bk);
+            freeSlots &= ~(1u << bs);
+            slotKid[bs] = bk;
+            for (int k = 0; k < nk; k++)
+                if (((left >> k) & 1u) && at[k] == bs) cheapest(k);
         }
     }
     // Triangles of each triangle group, once each: pieces of one triangle in

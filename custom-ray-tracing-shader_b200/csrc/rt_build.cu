@@ -40,10 +40,12 @@ constexpr int kScanBlock = 1024;   // elements per scan block
 constexpr int kBinBlock = 256;
 constexpr int kBinPer = 8;         // most positions per thread in the binning pass
 // Tasks of at most kSmallTask primitives are binned by one
-// block, or up to kWarpTask by one warp (binKernel); larger ones by position
-// blocks (binLarge).
+// block (binKernel); larger ones by position blocks (binLarge).
 constexpr int kSmallTask = 2048;
-constexpr int kWarpTask = 128;
+// Tasks of at most kSearchTask are searched by splitKernel straight from their
+// primitives and need no bins (1.3M primitives in tasks of 128-500: 110-190 us
+// of binning a level against about 25 for the search).
+constexpr int kSearchTask = 512;
 // Tasks of at most this many primitives are finished by one warp each, down to
 // their leaves (subtreeKernel).
 constexpr int kSubtree = 32;
@@ -377,10 +379,9 @@ __device__ __forceinline__ void binRange(const int* order, const float4* cent, c
 }
 
 // The bins of a level's tasks in one launch. Blocks below largeBlocks: position
-// chunks of the large tasks. The others take 8 small tasks: one warp each, or
-// all eight warps one after another for tasks above kWarpTask (a warp alone
-// walked 2,048 primitives in 100 us and more), with warp-private bins in
-// shared memory, written out with plain stores, so these bins need no clearing and no global atomics. Bins hold a count and
+// chunks of the large tasks. The others go over the tasks of kSearchTask to
+// kSmallTask primitives, a block each with warp-private bins in shared
+// memory, written out with plain stores, so these bins need no clearing and no global atomics. Bins hold a count and
 // minima/maxima, so the order of accumulation does not change them.
 __global__ void __launch_bounds__(kBinBlock) binKernel(const int* order, const int* posTask, const float4* cent,
                                                        const float4* plo, const float4* phi, const Task* tasks,
@@ -392,34 +393,24 @@ __global__ void __launch_bounds__(kBinBlock) binKernel(const int* order, const i
         return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nTasks = taskCount[0], first = (int)blockIdx.x - largeBlocks, stride = ((int)gridDim.x - largeBlocks) * 8;
-    for (int base = first * 8; base < nTasks; base += stride) {
-        // Tasks for the whole block, one by one.
-        for (int t = base; t < min(base + 8, nTasks); t++) {
-            const int n = tasks[t].count;
-            if (n <= kWarpTask || n > kSmallTask) continue;
-            const Task T = tasks[t];
-            binRange(order, cent, plo, phi, T, warp * 32, 256, sb[warp], lane);
-            __syncthreads();
-            for (int i = threadIdx.x; i < 3 * kBins; i += kBinBlock) {
-                BinKeys b = sb[0][i];
-                for (int w = 1; w < 8; w++) {
-                    const BinKeys& o = sb[w][i];
-                    b.count += o.count;
-                    for (int a = 0; a < 3; a++) {
-                        b.lo[a] = min(b.lo[a], o.lo[a]); b.hi[a] = max(b.hi[a], o.hi[a]);
-                        b.clo[a] = min(b.clo[a], o.clo[a]); b.chi[a] = max(b.chi[a], o.chi[a]);
-                    }
+    const int nTasks = taskCount[0], first = (int)blockIdx.x - largeBlocks, stride = (int)gridDim.x - largeBlocks;
+    for (int t = first; t < nTasks; t += stride) {
+        const int n = tasks[t].count;
+        if (n <= kSearchTask || n > kSmallTask) continue;
+        const Task T = tasks[t];
+        binRange(order, cent, plo, phi, T, warp * 32, 256, sb[warp], lane);
+        __syncthreads();
+        for (int i = threadIdx.x; i < 3 * kBins; i += kBinBlock) {
+            BinKeys b = sb[0][i];
+            for (int w = 1; w < 8; w++) {
+                const BinKeys& o = sb[w][i];
+                b.count += o.count;
+                for (int a = 0; a < 3; a++) {
+                    b.lo[a] = min(b.lo[a], o.lo[a]); b.hi[a] = max(b.hi[a], o.hi[a]);
+                    b.clo[a] = min(b.clo[a], o.clo[a]); b.chi[a] = max(b.chi[a], o.chi[a]);
                 }
-                bins[(size_t)t * 3 * kBins + i] = toBin(b);
             }
-            __syncthreads();
-        }
-        const int t = base + warp;
-        if (t < nTasks && tasks[t].count <= kWarpTask) {
-            const Task T = tasks[t];
-            binRange(order, cent, plo, phi, T, 0, 32, sb[warp], lane);
-            for (int i = lane; i < 3 * kBins; i += 32) bins[(size_t)t * 3 * kBins + i] = toBin(sb[warp][i]);
+            bins[(size_t)t * 3 * kBins + i] = toBin(b);
         }
         __syncthreads();
     }
@@ -432,69 +423,117 @@ __device__ __forceinline__ void deepen(int* counters, int depth) {
 
 // A level's splits, one warp per open task: the reference's SAH sweep, then
 // node records and the children's tasks. Candidate j = (axis, cut) sits on
-// lane j, which unites the boxes of its axis's 12 bins on both sides; the
-// 33rd (the z axis's last cut) on lane 0 of a second, uniform step. The first
-// minimum in (axis, cut) order wins, as in the reference's loop. (One thread
-// per task walked the 36 bins in about 11 us whatever the level held.)
+// lane j, which unites the boxes on both sides: of its axis's 12 bins, or for
+// tasks of at most kSearchTask of the primitives themselves (the same minima
+// and maxima), staged 32 at a time in shared memory. The 33rd candidate (the
+// z axis's last cut) is a uniform second step or a reduction over the lanes.
+// The first minimum in (axis, cut) order wins, as in the reference's loop.
+// (One thread per task walked the 36 bins in about 11 us whatever the level
+// held.)
 // Node and task numbers within a level come in atomic order; nodes are
 // renumbered to the reference's order after the build, and tasks carry their
 // own ranges. nextCount: the next level's open tasks and those above
 // kSmallTask; counters as listed at kCounters.
-__global__ void __launch_bounds__(128) splitKernel(const Task* tasks, const int* taskCount, const BinAcc* bins, Split* splits,
+__global__ void __launch_bounds__(128) splitKernel(const int* order, const float4* cent, const float4* plo, const float4* phi,
+                                                   const Task* tasks, const int* taskCount, const BinAcc* bins, Split* splits,
                                                    BinNode* nodes, int* counters, int* nextCount, Task* nextTasks,
                                                    Task* subtrees, int nodeCapacity, int taskCapacity, int subtreeCapacity,
                                                    int leafSize) {
-    __shared__ BinAcc sb[4][3 * kBins];
+    __shared__ __align__(16) BinAcc sb[4][3 * kBins];
     const unsigned full = 0xFFFFFFFFu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nTasks = taskCount[0], warps = (int)gridDim.x * 4;
     BinAcc* B = sb[warp];
     for (int t = (int)blockIdx.x * 4 + warp; t < nTasks; t += warps) {
         const Task T = tasks[t];
-        // Every open task has more than leafSize primitives and is above the
-        // depth limit.
-        constexpr int kWords = 3 * kBins * (int)(sizeof(BinAcc) / 4);
-        __syncwarp();
-        for (int i = lane; i < kWords; i += 32)
-            reinterpret_cast<unsigned*>(B)[i] = reinterpret_cast<const unsigned*>(bins + (size_t)t * 3 * kBins)[i];
-        __syncwarp();
         const float nodeArea = halfArea(T.lo, T.hi), unsplit = nodeArea * T.count;
         bool valid[3];
         for (int a = 0; a < 3; a++) valid[a] = !(T.chi[a] - T.clo[a] <= 1e-12f);
-        // Boxes and counts on both sides of a candidate.
-        float box[2][6];
-        int count[2];
-        auto sweep = [&](int axis, int cut) {
-            for (int s = 0; s < 2; s++) {
-                for (int k = 0; k < 3; k++) { box[s][k] = FLT_MAX; box[s][3 + k] = -FLT_MAX; }
-                count[s] = 0;
-            }
-            for (int b = 0; b < kBins; b++) {
-                const BinAcc& o = B[axis * kBins + b];
-                if (!o.count) continue;
-                if (b <= cut) { growBox(box[0], box[0] + 3, o.lo, o.hi); count[0] += (int)o.count; }
-                else { growBox(box[1], box[1] + 3, o.lo, o.hi); count[1] += (int)o.count; }
-            }
-        };
-        auto candidateCost = [&](bool axisValid) {
-            if (!axisValid || !count[0] || !count[1]) return FLT_MAX;
-            return nodeArea + halfArea(box[0], box[0] + 3) * count[0] + halfArea(box[1], box[1] + 3) * count[1];
-        };
-        sweep(2, kBins - 2);
-        const float last = candidateCost(valid[2]);
+        // Boxes (low, high) and counts on both sides of this lane's candidate,
+        // and of the last one.
         const int axis = lane / 11, cut = lane % 11;
-        sweep(axis, cut);
-        const float cost = candidateCost(axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]);
+        float box[2][6], lastBox[2][6];
+        int count[2], lastCount[2];
+        auto reset = [](float (&b)[2][6], int (&n)[2]) {
+            for (int s = 0; s < 2; s++) {
+                for (int k = 0; k < 3; k++) { b[s][k] = FLT_MAX; b[s][3 + k] = -FLT_MAX; }
+                n[s] = 0;
+            }
+        };
+        auto reduceMin = [&](float v) { return keyFloat(__reduce_min_sync(full, orderedKey(v))); };
+        auto reduceMax = [&](float v) { return keyFloat(__reduce_max_sync(full, orderedKey(v))); };
+        const bool search = T.count <= kSearchTask;
+        float scale[3];
+        for (int a = 0; a < 3; a++) scale[a] = valid[a] ? kBins / (T.chi[a] - T.clo[a]) : 0.0f;
+        auto axisOf = [](float x, float y, float z, int a) { return a == 0 ? x : (a == 1 ? y : z); };
+        auto binAt = [&](float4 c, int a) { return valid[a] ? binOf(axisOf(c.x, c.y, c.z, a), T.clo[a], scale[a]) : 0; };
+        __syncwarp();
+        reset(box, count);
+        reset(lastBox, lastCount);
+        if (search) {
+            float4* stage = reinterpret_cast<float4*>(B);  // 32 low corners (w: the three bins), 32 high
+            for (int base = 0; base < T.count; base += 32) {
+                const int n = min(32, T.count - base);
+                __syncwarp();
+                if (lane < n) {
+                    const int prim = order[T.first + base + lane];
+                    const float4 c = cent[prim];
+                    float4 lo = plo[prim], hi = phi[prim];
+                    const int b2 = binAt(c, 2);
+                    lo.w = __int_as_float(binAt(c, 0) | binAt(c, 1) << 4 | b2 << 8);
+                    stage[lane] = lo;
+                    stage[32 + lane] = hi;
+                    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+                    if (b2 <= kBins - 2) { growBox(lastBox[0], lastBox[0] + 3, l, h); lastCount[0]++; }
+                    else { growBox(lastBox[1], lastBox[1] + 3, l, h); lastCount[1]++; }
+                }
+                __syncwarp();
+                for (int i = 0; i < n; i++) {
+                    const float4 lo = stage[i], hi = stage[32 + i];
+                    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+                    if (((__float_as_int(lo.w) >> (4 * axis)) & 15) <= cut) { growBox(box[0], box[0] + 3, l, h); count[0]++; }
+                    else { growBox(box[1], box[1] + 3, l, h); count[1]++; }
+                }
+            }
+            for (int s = 0; s < 2; s++) {
+                for (int k = 0; k < 3; k++) {
+                    lastBox[s][k] = reduceMin(lastBox[s][k]);
+                    lastBox[s][3 + k] = reduceMax(lastBox[s][3 + k]);
+                }
+                lastCount[s] = __reduce_add_sync(full, lastCount[s]);
+            }
+        } else {
+            constexpr int kWords = 3 * kBins * (int)(sizeof(BinAcc) / 4);
+            for (int i = lane; i < kWords; i += 32)
+                reinterpret_cast<unsigned*>(B)[i] = reinterpret_cast<const unsigned*>(bins + (size_t)t * 3 * kBins)[i];
+            __syncwarp();
+            auto sweep = [&](float (&to)[2][6], int (&n)[2], int a, int c) {
+                for (int b = 0; b < kBins; b++) {
+                    const BinAcc& o = B[a * kBins + b];
+                    if (!o.count) continue;
+                    if (b <= c) { growBox(to[0], to[0] + 3, o.lo, o.hi); n[0] += (int)o.count; }
+                    else { growBox(to[1], to[1] + 3, o.lo, o.hi); n[1] += (int)o.count; }
+                }
+            };
+            sweep(box, count, axis, cut);
+            sweep(lastBox, lastCount, 2, kBins - 2);
+        }
+        auto candidateCost = [&](const float (&b)[2][6], const int (&n)[2], bool axisValid) {
+            if (!axisValid || !n[0] || !n[1]) return FLT_MAX;
+            return nodeArea + halfArea(b[0], b[0] + 3) * n[0] + halfArea(b[1], b[1] + 3) * n[1];
+        };
+        const float last = candidateCost(lastBox, lastCount, valid[2]);
+        const float cost = candidateCost(box, count, axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]);
         // Costs are sums of areas, not negative: their bits order like them.
         const unsigned bits = cost < unsplit ? __float_as_uint(cost) : full;
         const unsigned best = __reduce_min_sync(full, bits);
-        int bestAxis = -1, bestBin = -1;
+        int bestAxis = -1, bestBin = -1, winner = -1;
         if (best != full) {
-            const int winner = __ffs(__ballot_sync(full, bits == best)) - 1;
+            winner = __ffs(__ballot_sync(full, bits == best)) - 1;
             bestAxis = winner / 11;
             bestBin = winner % 11;
         }
-        if (last < unsplit && __float_as_uint(last) < best) { bestAxis = 2; bestBin = kBins - 2; }
+        if (last < unsplit && __float_as_uint(last) < best) { bestAxis = 2; bestBin = kBins - 2; winner = -1; }
         if (bestAxis < 0) {
             if (lane == 0) {
                 nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), T.first, v3(T.hi[0], T.hi[1], T.hi[2]), T.count};
@@ -503,21 +542,48 @@ __global__ void __launch_bounds__(128) splitKernel(const Task* tasks, const int*
             }
             continue;
         }
-        // Lane s < 2 makes child s: its boxes, centroid boxes and count are
-        // unions over its bins.
+        // Lane s < 2 makes child s: the winning candidate's box and count, and
+        // its centroid box over its bins or primitives.
         int child = 0, leftCount = 0;
         Task C;
         C.count = 0;
         bool open = false, small = false;
-        if (lane < 2) {
-            for (int k = 0; k < 3; k++) { C.lo[k] = C.clo[k] = FLT_MAX; C.hi[k] = C.chi[k] = -FLT_MAX; }
+        for (int s = 0; s < 2; s++) {
+            float w[6];
+            for (int k = 0; k < 6; k++) w[k] = winner < 0 ? lastBox[s][k] : __shfl_sync(full, box[s][k], winner);
+            const int n = winner < 0 ? lastCount[s] : __shfl_sync(full, count[s], winner);
+            if (lane == s) {
+                for (int k = 0; k < 3; k++) { C.lo[k] = w[k]; C.hi[k] = w[3 + k]; }
+                C.count = n;
+            }
+        }
+        float cen[2][6];
+        {
+            int unused[2];
+            reset(cen, unused);
+        }
+        if (search) {
+            for (int i = lane; i < T.count; i += 32) {
+                const float4 c = cent[order[T.first + i]];
+                const float p[3] = {c.x, c.y, c.z};
+                if (binAt(c, bestAxis) <= bestBin) growBox(cen[0], cen[0] + 3, p, p);
+                else growBox(cen[1], cen[1] + 3, p, p);
+            }
+            for (int s = 0; s < 2; s++)
+                for (int k = 0; k < 3; k++) {
+                    cen[s][k] = reduceMin(cen[s][k]);
+                    cen[s][3 + k] = reduceMax(cen[s][3 + k]);
+                }
+        } else {
             for (int b = 0; b < kBins; b++) {
                 const BinAcc& o = B[bestAxis * kBins + b];
-                if (!o.count || (b <= bestBin) != (lane == 0)) continue;
-                growBox(C.lo, C.hi, o.lo, o.hi);
-                growBox(C.clo, C.chi, o.clo, o.chi);
-                C.count += (int)o.count;
+                if (!o.count) continue;
+                if (b <= bestBin) growBox(cen[0], cen[0] + 3, o.clo, o.chi);
+                else growBox(cen[1], cen[1] + 3, o.clo, o.chi);
             }
+        }
+        if (lane < 2) {
+            for (int k = 0; k < 3; k++) { C.clo[k] = lane ? cen[1][k] : cen[0][k]; C.chi[k] = lane ? cen[1][3 + k] : cen[0][3 + k]; }
             C.depth = T.depth + 1;
             open = !(C.count <= leafSize || C.depth == kBinaryMaxDepth);
             small = open && C.count <= kSubtree;
@@ -1359,7 +1425,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         // Enough position blocks for the SMs where there are few positions.
         const int perThread = std::max(1, std::min(kBinPer, n / (148 * kBinBlock)));
         const int largeBlocks = n > kSmallTask ? blocksFor(n, kBinBlock * perThread) : 0;
-        const int smallBlocks = std::max(1, std::min(blocksFor(taskCapacity, 8), 1184));
+        const int smallBlocks = std::max(1, std::min(n / kSearchTask, 1184));
         const int splitBlocks = std::max(1, std::min(blocksFor(taskCapacity, 4), 1184));
         const int clearBlocks = std::max(1, std::min(blocksFor((long long)taskCapacity * 3 * kBins, 256), 1184));
         clearBinsKernel<<<clearBlocks, 256, 0, stream>>>(bins, levelCounts, tasks);
@@ -1371,7 +1437,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
                     int* nc = levelCounts + 2 * (level + 1);
                     binKernel<<<largeBlocks + smallBlocks, kBinBlock, 0, stream>>>(out.order, posTask, cent, out.primLo, out.primHi,
                                                                                    tasks, n, bins, tc, largeBlocks, perThread);
-                    splitKernel<<<splitBlocks, 128, 0, stream>>>(tasks, tc, bins, splits, rawNodes, counters, nc, tasksB, subtrees,
+                    splitKernel<<<splitBlocks, 128, 0, stream>>>(out.order, cent, out.primLo, out.primHi, tasks, tc, bins, splits, rawNodes, counters, nc, tasksB, subtrees,
                                                                  nodeCapacity, taskCapacity, subtreeCapacity, leafSize);
                     partitionKernel<<<nScanBlocks, 256, 0, stream>>>(out.order, posTask, cent, tasks, splits, n, flags, prefix,
                                                                      blockSums, counters, levelStartDev + level + 2, tc, nc,

@@ -299,26 +299,28 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
                     if (a.outF) {
                         float4* o = reinterpret_cast<float4*>(a.outF + pix * a.coutTotal + nBase + c);
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            float4 s = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                            if (a.accumulate) {
-                                const float4 old = o[q];
-                                s = make_float4(old.x + s.x, old.y + s.y, old.z + s.z, old.w + s.w);
+                        for (int q = 0; q < 2; q++) {
+                            uint32_t words[8];
+#pragma unroll
+                            for (int j = 0; j < 8; j += 4) {
+                                float4 s = make_float4(v[8 * q + j], v[8 * q + j + 1], v[8 * q + j + 2], v[8 * q + j + 3]);
+                                if (a.accumulate) {
+                                    const float4 old = o[2 * q + j / 4];
+                                    s = make_float4(old.x + s.x, old.y + s.y, old.z + s.z, old.w + s.w);
+                                }
+                                words[j] = __float_as_uint(s.x); words[j + 1] = __float_as_uint(s.y);
+                                words[j + 2] = __float_as_uint(s.z); words[j + 3] = __float_as_uint(s.w);
                             }
-                            o[q] = s;
+                            storeWords8(o + 2 * q, words);
                         }
                     } else {
-                        uint4* o = reinterpret_cast<uint4*>(a.outB + pix * a.coutTotal + nBase + c);
+                        uint32_t words[8];
 #pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            uint32_t words[4];
-#pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                __nv_bfloat162 pair = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
-                                words[j] = *reinterpret_cast<uint32_t*>(&pair);
-                            }
-                            o[q] = make_uint4(words[0], words[1], words[2], words[3]);
+                        for (int j = 0; j < 8; j++) {
+                            __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                            words[j] = *reinterpret_cast<uint32_t*>(&pair);
                         }
+                        storeWords8(a.outB + pix * a.coutTotal + nBase + c, words);
                     }
                 }
                 tcFenceBefore();

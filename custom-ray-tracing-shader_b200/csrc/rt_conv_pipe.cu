@@ -439,26 +439,34 @@ __device__ __forceinline__ void epilogueStore16(const PipeArgs& a, const uint32_
     if (a.outF) {
         float4* o = reinterpret_cast<float4*>(a.outF + pix * a.coutTotal + nBase + c0);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            float4 x = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            if (a.accumulate) {
-                const float4 old = o[q];
-                x = make_float4(old.x + x.x, old.y + x.y, old.z + x.z, old.w + x.w);
+        for (int q = 0; q < 2; q++) {
+            uint32_t words[8];
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                float4 x = make_float4(v[8 * q + j], v[8 * q + j + 1], v[8 * q + j + 2], v[8 * q + j + 3]);
+                if (a.accumulate) {
+                    const float4 old = o[2 * q + j / 4];
+                    x = make_float4(old.x + x.x, old.y + x.y, old.z + x.z, old.w + x.w);
+                }
+                words[j] = __float_as_uint(x.x); words[j + 1] = __float_as_uint(x.y);
+                words[j + 2] = __float_as_uint(x.z); words[j + 3] = __float_as_uint(x.w);
             }
-            o[q] = x;
+            storeWords8(o + 2 * q, words);
         }
     } else {
+        uint32_t words[8];
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            uint32_t words[4];
+        for (int j = 0; j < 8; j++) {
+            __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            words[j] = *reinterpret_cast<uint32_t*>(&pair);
+        }
+        if (a.outPixels) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                __nv_bfloat162 pair = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
-                words[j] = *reinterpret_cast<uint32_t*>(&pair);
-            }
-            uint4* o = a.outPixels ? reinterpret_cast<uint4*>(a.outB) + ((size_t)(nBase + c0) / 8 + q) * (size_t)a.outPixels + pix
-                                   : reinterpret_cast<uint4*>(a.outB + pix * a.coutTotal + nBase + c0) + q;
-            *o = make_uint4(words[0], words[1], words[2], words[3]);
+            for (int q = 0; q < 2; q++)
+                reinterpret_cast<uint4*>(a.outB)[((size_t)(nBase + c0) / 8 + q) * (size_t)a.outPixels + pix] =
+                    make_uint4(words[4 * q], words[4 * q + 1], words[4 * q + 2], words[4 * q + 3]);
+        } else {
+            storeWords8(a.outB + pix * a.coutTotal + nBase + c0, words);
         }
     }
 }

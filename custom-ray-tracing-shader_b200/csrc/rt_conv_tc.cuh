@@ -37,6 +37,16 @@ __host__ __device__ constexpr uint64_t ummaSmemDesc(uint32_t address, uint32_t l
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+#ifdef __CUDACC__
+// 32 bytes to a 32-byte boundary in one store: a pixel's 16 BF16 channels fill
+// a whole sector (two 16-byte stores wrote each sector in two halves).
+__device__ __forceinline__ void storeWords8(void* to, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+#endif
+
 // out[p][n] = act(bias[n] + sum_tap,k in[p + off(tap)][k] * w[tap'][n][k]) over
 // NHWC BF16 input with Cin channels; w is [9][Cout][Cin] BF16 (K-major) and
 // tap' = 8 - tap when reverseTaps (the data gradient reads the forward

@@ -16,8 +16,16 @@
 // all nine taps: ceil(3 cin / 128) blocks x 3 column taps of accumulators in
 // tensor memory. (One block per row tap, each padding its cin rows to M =
 // 128 and staging x and dY again as planes of 8 channels, took 125 us for
-// 32 -> 32 channels at 32 x 128 x 128 pixels; this form 31 us. Its floors:
-// 67 MB of operands, 10 us; 4096 rows x 24 MMAs of ~42 cycles, 15 us.)
+// 32 -> 32 channels at 32 x 128 x 128 pixels; this form 29 us. Its floors:
+// 67 MB of operands, 10 us; 32,768 MMAs of N = 96, 10 us.)
+//
+// Where dY's channels are one slab (32 or 64 output channels), the column taps
+// sit side by side along N as well: a shift by one pixel is one pixel row of
+// the slab, so with a group stride of one pixel row N covers dY shifted by 0,
+// 1 and 2 pixels, and one MMA does all nine taps of a block (N = 96 takes ~80
+// cycles, three of N = 32 ~42 each and three issues). Then x is staged without
+// and dY with the one-pixel halo, and group g holds tap dx = 2 - g. Else the
+// tap shifts x's start address.
 // Where the accumulators pass 512 columns, blocks of the grid take slices of
 // the M blocks. Split K over the blocks; each adds its accumulators to dw
 // with 16-byte FP32 reductions at the end. Rows of the last M block beyond 3 cin
@@ -56,6 +64,7 @@ __host__ __device__ constexpr uint32_t slabBytes(int px, int s) {
 
 struct WgradArgs {
     int h, w, cin, cout;
+    int xHalo, dHalo;              // pixels staged on each side of a segment (one of them 1)
     int px;                        // pixels per segment (K per row): 16..128, a multiple of 16
     int tilesPerRow, strips, units, rows;
     int xSlabs, dSlabs;            // slabs per row
@@ -90,32 +99,32 @@ __device__ __forceinline__ uint64_t slabDescriptor(uint32_t addr, uint32_t slab)
     return ummaSmemDesc(addr, slab, 16u * S) | slabLayout(S);
 }
 
-// The MMAs of one dY row and one M block: 3 column taps x KK steps of 16
-// pixels, descriptors as compile-time offsets from two bases (one thread
-// issues; computing descriptors per MMA is several times slower than the
-// tensor pipe).
-template <int SX, int SD, int KK>
+// The MMAs of one dY row and one M block: KK steps of 16 pixels, for all
+// column taps at once (WIDE) or for each, descriptors as compile-time offsets
+// from two bases (one thread issues; computing descriptors per MMA is several
+// times slower than the tensor pipe).
+template <int SX, int SD, bool WIDE, int KK>
 __device__ __forceinline__ void issueRow(uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
                                          uint32_t first) {
 #pragma unroll
-    for (int dx = 0; dx < 3; dx++)
+    for (int dx = 0; dx < (WIDE ? 1 : 3); dx++)
 #pragma unroll
         for (int kk = 0; kk < KK; kk++)
             mma(acc + (uint32_t)dx * accStep, x + (uint64_t)(dx * (SX / 8) + kk * 2 * SX), d + (uint64_t)(kk * 2 * SD),
                 idesc, (first || kk > 0) ? 1u : 0u);
 }
-template <int SX, int SD>
+template <int SX, int SD, bool WIDE>
 __device__ __forceinline__ void issueRowK(int kk, uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
                                           uint32_t first) {
     switch (kk) {
-        case 1: issueRow<SX, SD, 1>(acc, accStep, x, d, idesc, first); break;
-        case 2: issueRow<SX, SD, 2>(acc, accStep, x, d, idesc, first); break;
-        case 3: issueRow<SX, SD, 3>(acc, accStep, x, d, idesc, first); break;
-        case 4: issueRow<SX, SD, 4>(acc, accStep, x, d, idesc, first); break;
-        case 5: issueRow<SX, SD, 5>(acc, accStep, x, d, idesc, first); break;
-        case 6: issueRow<SX, SD, 6>(acc, accStep, x, d, idesc, first); break;
-        case 7: issueRow<SX, SD, 7>(acc, accStep, x, d, idesc, first); break;
-        default: issueRow<SX, SD, 8>(acc, accStep, x, d, idesc, first); break;
+        case 1: issueRow<SX, SD, WIDE, 1>(acc, accStep, x, d, idesc, first); break;
+        case 2: issueRow<SX, SD, WIDE, 2>(acc, accStep, x, d, idesc, first); break;
+        case 3: issueRow<SX, SD, WIDE, 3>(acc, accStep, x, d, idesc, first); break;
+        case 4: issueRow<SX, SD, WIDE, 4>(acc, accStep, x, d, idesc, first); break;
+        case 5: issueRow<SX, SD, WIDE, 5>(acc, accStep, x, d, idesc, first); break;
+        case 6: issueRow<SX, SD, WIDE, 6>(acc, accStep, x, d, idesc, first); break;
+        case 7: issueRow<SX, SD, WIDE, 7>(acc, accStep, x, d, idesc, first); break;
+        default: issueRow<SX, SD, WIDE, 8>(acc, accStep, x, d, idesc, first); break;
     }
 }
 
@@ -127,7 +136,7 @@ __device__ __forceinline__ Unit unitOf(const WgradArgs& a, int u) {
     return Unit{img, xt * a.px, y0, min(a.rows, a.h - y0)};
 }
 
-template <int SX, int SD>
+template <int SX, int SD, bool WIDE>
 __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant__ CUtensorMap xMap,
                                                          const __grid_constant__ CUtensorMap dMap, WgradArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -173,32 +182,37 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         for (int u = (int)blockIdx.x; u < a.units; u += (int)gridDim.x, k++) {
             const int st = k % S;
             if (!waitPhaseWarp(base + Header::empty + 8 * st, (uint32_t)(((k / S) & 1) ^ 1), abortFlag, limit)) { ok = false; break; }
-            if (lane == 0) {
-                const Unit U = unitOf(a, u);
-                const uint32_t fb = base + Header::full + 8 * st;
-                const uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
-                // Staged row j (image row y0 - 1 + j) slab c is slab (j - r) xSlabs
-                // + c of dY row r's stack: loaded when some r's M blocks cover it.
-                auto needed = [&](int j, int c) {
-                    const int rLo = max(0, j - 2), rHi = min(U.rows - 1, j);
-                    for (int r = rLo; r <= rHi; r++) {
-                        const int q = (j - r) * a.xSlabs + c;
-                        if (q >= slab0 && q < slab1) return true;
-                    }
-                    return false;
-                };
-                uint32_t boxes = 0;
-                for (int j = 0; j < U.rows + 2; j++)
-                    for (int c = 0; c < a.xSlabs; c++) boxes += needed(j, c) ? 1u : 0u;
-                barExpectTx(fb, boxes * (uint32_t)(a.px + 2) * 2u * SX + (uint32_t)(U.rows * a.dSlabs * a.px) * 2u * SD);
-                for (int r = 0; r < U.rows; r++)
-                    for (int c = 0; c < a.dSlabs; c++)
-                        tmaLoad4(ds + (uint32_t)(r * a.dSlabs + c) * a.dSlab, &dMap, c * SD, U.x0, U.y0 + r, U.img, fb);
-                for (int j = 0; j < U.rows + 2; j++)
-                    for (int c = 0; c < a.xSlabs; c++)
-                        if (needed(j, c))
-                            tmaLoad4(xs + (uint32_t)(j * a.xSlabs + c) * a.xSlab, &xMap, c * SX, U.x0 - 1, U.y0 - 1 + j,
-                                     U.img, fb);
+            // The lanes issue the boxes: first dY's, then x's.
+            const Unit U = unitOf(a, u);
+            const uint32_t fb = base + Header::full + 8 * st;
+            const uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
+            const int dBoxes = U.rows * a.dSlabs, xBoxes = (U.rows + 2) * a.xSlabs;
+            // Staged row j (image row y0 - 1 + j) slab c is slab (j - r) xSlabs
+            // + c of dY row r's stack: loaded when some r's M blocks cover it.
+            auto needed = [&](int i) {
+                if (gridDim.y == 1) return true;
+                const int j = i / a.xSlabs, c = i - j * a.xSlabs;
+                const int rLo = max(0, j - 2), rHi = min(U.rows - 1, j);
+                for (int r = rLo; r <= rHi; r++) {
+                    const int q = (j - r) * a.xSlabs + c;
+                    if (q >= slab0 && q < slab1) return true;
+                }
+                return false;
+            };
+            int mine = 0;
+            for (int i = lane; i < xBoxes; i += 32) mine += needed(i) ? 1 : 0;
+            const uint32_t boxes = (uint32_t)__reduce_add_sync(0xFFFFFFFFu, mine);
+            if (lane == 0)
+                barExpectTx(fb, boxes * (uint32_t)(a.px + 2 * a.xHalo) * 2u * SX +
+                                    (uint32_t)(dBoxes * (a.px + 2 * a.dHalo)) * 2u * SD);
+            __syncwarp();
+            for (int i = lane; i < dBoxes; i += 32) {
+                const int r = i / a.dSlabs, c = i - r * a.dSlabs;
+                tmaLoad4(ds + (uint32_t)i * a.dSlab, &dMap, c * SD, U.x0 - a.dHalo, U.y0 + r, U.img, fb);
+            }
+            for (int i = lane; i < xBoxes; i += 32) {
+                const int j = i / a.xSlabs, c = i - j * a.xSlabs;
+                if (needed(i)) tmaLoad4(xs + (uint32_t)i * a.xSlab, &xMap, c * SX, U.x0 - a.xHalo, U.y0 - 1 + j, U.img, fb);
             }
             __syncwarp();
         }
@@ -213,7 +227,7 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         // ---- MMA issuer ----
         if (lane == 0) {
             bool ok = true;
-            const uint32_t idesc = idescMnMajor(kM, a.cout);
+            const uint32_t idesc = idescMnMajor(kM, WIDE ? 3 * a.cout : a.cout);
             const uint32_t cols = (uint32_t)a.cout;
             int k = 0, st = 0;
             uint32_t parity = 0, started = 0;
@@ -224,9 +238,9 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
                 const int rows = unitOf(a, u).rows;
                 uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
                 for (int r = 0; r < rows; r++) {
-                    const uint64_t dDesc = slabDescriptor<SD>(ds, a.dSlab);
+                    const uint64_t dDesc = slabDescriptor<SD>(ds, WIDE ? 2u * SD : a.dSlab);
                     for (int b = b0; b < b1; b++)
-                        issueRowK<SX, SD>(a.px / 16, tmem + (uint32_t)(b - b0) * 3u * cols, cols,
+                        issueRowK<SX, SD, WIDE>(a.px / 16, tmem + (uint32_t)(b - b0) * 3u * cols, cols,
                                           slabDescriptor<SX>(xs + (uint32_t)(b * (kM / SX)) * a.xSlab, a.xSlab), dDesc, idesc,
                                           started);
                     started = 1u;
@@ -258,7 +272,7 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
                 const int q = b * kM + quarter * 32 + lane;  // (dy, ci) of this thread's accumulator row
                 const int dy = q / a.cin, ci = q % a.cin;
                 for (int dx = 0; dx < 3; dx++) {
-                    float* out = a.dw + ((size_t)(dy * 3 + dx) * a.cin + ci) * a.cout;
+                    float* out = a.dw + ((size_t)(dy * 3 + (WIDE ? 2 - dx : dx)) * a.cin + ci) * a.cout;
                     for (int c = 0; c < a.cout; c += 16) {
                         uint32_t v[16];
                         __syncwarp();  // the load needs converged lanes; the additions below may diverge
@@ -298,24 +312,28 @@ bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, i
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int SX, int SD>
+template <int SX, int SD, bool WIDE>
 cudaError_t launch(const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid, uint32_t smemBytes,
                    cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel<SX, SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel<SX, SD, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    wgradTcKernel<SX, SD><<<grid, kThreads, smemBytes, stream>>>(xMap, dMap, a);
+    wgradTcKernel<SX, SD, WIDE><<<grid, kThreads, smemBytes, stream>>>(xMap, dMap, a);
     return cudaGetLastError();
 }
 template <int SX>
 cudaError_t launchD(int sd, const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid,
                     uint32_t smemBytes, cudaStream_t stream) {
-    return sd == 64   ? launch<SX, 64>(xMap, dMap, a, grid, smemBytes, stream)
-           : sd == 32 ? launch<SX, 32>(xMap, dMap, a, grid, smemBytes, stream)
-                      : launch<SX, 16>(xMap, dMap, a, grid, smemBytes, stream);
+    if (a.dHalo)
+        return sd == 64   ? launch<SX, 64, true>(xMap, dMap, a, grid, smemBytes, stream)
+               : sd == 32 ? launch<SX, 32, true>(xMap, dMap, a, grid, smemBytes, stream)
+                          : launch<SX, 16, true>(xMap, dMap, a, grid, smemBytes, stream);
+    return sd == 64   ? launch<SX, 64, false>(xMap, dMap, a, grid, smemBytes, stream)
+           : sd == 32 ? launch<SX, 32, false>(xMap, dMap, a, grid, smemBytes, stream)
+                      : launch<SX, 16, false>(xMap, dMap, a, grid, smemBytes, stream);
 }
 
 }  // namespace
@@ -332,6 +350,8 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
     WgradArgs a{};
     a.h = h; a.w = w; a.cin = cin; a.cout = cout;
     a.xSlabs = cin / sx; a.dSlabs = cout / sd;
+    a.dHalo = a.dSlabs == 1 ? 1 : 0;  // the column taps along N (3 cout <= 192)
+    a.xHalo = 1 - a.dHalo;
     a.mBlocks = (3 * cin + kM - 1) / kM;
     // As many M blocks per grid slice as 512 columns of accumulators hold,
     // evenly over the slices.
@@ -344,15 +364,21 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
     int sms = 0, device = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int splits = std::max(1, std::max(1, sms) / slices);
-    // Segment width and rows per stage: two stages have to fit; the busiest
-    // block's staged rows (each unit costs its rows and about one row's
-    // latency) decide. Segments of 128 pixels fit up to about 100 channels in
-    // all, wide layers on wide images take narrower ones.
-    long long bestCost = -1, bestUnits = 0;
+    const int most = std::max(1, std::max(1, sms) / slices);
+    // Segment width, rows per stage and blocks per slice, by estimated cycles:
+    // two stages have to fit; a block's units each cost the larger of their
+    // MMAs (about 60 cycles each for N up to 64, 0.85 N above) and loads (20
+    // bytes a cycle) and about 1,200 of latency; and every block adds its
+    // accumulators to dw, about 800 bytes a cycle over all of them, which is what
+    // limits the deep levels (128 -> 128 channels at 8 x 8: 29 MB from 147 blocks).
+    const int n0 = a.dHalo ? 3 * cout : cout;
+    const double mmaCycles = std::max(60.0, 0.85 * n0);
+    const double addCycles = 36.0 * cin * cout / 800.0;
+    double bestCost = -1.0;
+    int splits = 1;
     for (int px = std::min(kM, (w + 15) / 16 * 16), next = 0; px >= 16; px = next) {
         next = px > 64 ? 64 : px > 32 ? 32 : px > 16 ? 16 : 0;
-        const uint32_t xSlab = slabBytes(px + 2, sx), dSlab = slabBytes(px, sd);
+        const uint32_t xSlab = slabBytes(px + 2 * a.xHalo, sx), dSlab = slabBytes(px + 2 * a.dHalo, sd);
         const int tiles = (w + px - 1) / px;
         // A stage: rows + 2 rows of x, then the dY rows. The last M block may
         // read past the stacked rows, at most `over` bytes past x's part.
@@ -362,14 +388,21 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
             const uint32_t stage = (xPart + std::max(over, (uint32_t)(rows * a.dSlabs) * dSlab) + 1023u) & ~1023u;
             if (kHeader + 2u * stage > kSmemMax) break;
             const long long strips = (h + rows - 1) / rows, units = (long long)n * tiles * strips;
-            const long long cost = (units + splits - 1) / splits * (rows + 1) * (px + 16);
-            if (units > 0x7FFFFFFFll || (bestCost >= 0 && cost > bestCost)) continue;
-            bestCost = cost;
-            bestUnits = units;
-            a.px = px; a.rows = rows;
-            a.tilesPerRow = tiles; a.strips = (int)strips; a.units = (int)units;
-            a.xSlab = xSlab; a.dSlab = dSlab;
-            a.xBytes = xPart; a.stageBytes = stage;
+            if (units > 0x7FFFFFFFll) continue;
+            const double mmas = (double)rows * a.blocksPerSlice * (a.dHalo ? 1 : 3) * (px / 16) * mmaCycles;
+            const double loads = ((rows + 2.0) * (px + 2) * cin / slices + (double)rows * px * cout) * 2.0 / 20.0;
+            const double unit = std::max(mmas, loads) + 1200.0;
+            for (int s = most; s >= 1; s = s > 8 ? s * 3 / 4 : s - 1) {
+                const long long per = (units + s - 1) / s;
+                const double cost = (double)per * unit + s * addCycles;
+                if (bestCost >= 0.0 && cost >= bestCost) continue;
+                bestCost = cost;
+                splits = (int)std::min<long long>(s, units);
+                a.px = px; a.rows = rows;
+                a.tilesPerRow = tiles; a.strips = (int)strips; a.units = (int)units;
+                a.xSlab = xSlab; a.dSlab = dSlab;
+                a.xBytes = xPart; a.stageBytes = stage;
+            }
         }
     }
     if (bestCost < 0) return cudaErrorNotSupported;
@@ -379,10 +412,10 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
     a.errorFlag = errorFlag;
     a.waitLimitNs = 1000000000ull;
     CUtensorMap xMap{}, dMap{};
-    if (!makeActivationMap(&xMap, x, n, h, w, cin, sx, (uint32_t)(a.px + 2)) ||
-        !makeActivationMap(&dMap, dy, n, h, w, cout, sd, (uint32_t)a.px))
+    if (!makeActivationMap(&xMap, x, n, h, w, cin, sx, (uint32_t)(a.px + 2 * a.xHalo)) ||
+        !makeActivationMap(&dMap, dy, n, h, w, cout, sd, (uint32_t)(a.px + 2 * a.dHalo)))
         return cudaErrorNotSupported;
-    const dim3 grid((unsigned)std::min<long long>(splits, bestUnits), (unsigned)slices);
+    const dim3 grid((unsigned)splits, (unsigned)slices);
     const uint32_t smemBytes = kHeader + (uint32_t)a.stages * a.stageBytes;
     return sx == 64   ? launchD<64>(sd, xMap, dMap, a, grid, smemBytes, stream)
            : sx == 32 ? launchD<32>(sd, xMap, dMap, a, grid, smemBytes, stream)

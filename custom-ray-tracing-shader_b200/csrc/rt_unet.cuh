@@ -90,6 +90,8 @@ private:
     int n_ = 0, h_ = 0, w_ = 0;
     bool training_ = false;
     cudaStream_t stream_ = nullptr;
+    cudaStream_t side_ = nullptr;    // the backward pass's weight gradients
+    cudaEvent_t fork_ = nullptr, join_ = nullptr;
 };
 
 }  // namespace rt

@@ -1,5 +1,6 @@
-// 3x3 convolutions of the denoiser on narrow images (up to 64 pixels wide:
-// the deep levels of training crops) on the fifth-generation tensor cores.
+// 3x3 convolutions of the denoiser on narrow or small images (the deep levels
+// of training crops and of 1080p frames) and of layers whose weights don't fit
+// shared memory, on the fifth-generation tensor cores.
 //
 // The pipelined kernel's tile is 128 pixels of one image row, so an image 8,
 // 16, 32 or 64 pixels wide leaves most of every MMA to padding and makes a
@@ -10,7 +11,8 @@
 // operand layout, 8-pixel groups a constant stride apart across the row
 // ends), and tap (dy, dx) is the same line shifted by dy (w + 2) + dx pixels.
 // The two padding positions of each row (2 / (w + 2) of a tile) compute
-// values that are not stored.
+// values that are not stored. Wider images are cut into equal column segments
+// of up to 64 pixels, each staged with its own halo.
 //
 // A block owns a slice of the output channels (its weights stay in shared
 // memory, three TMA boxes per slab, one per kernel row, each with its own
@@ -19,15 +21,21 @@
 // up to two sets of accumulators, warps 2-9 drain them (alternate tiles).
 // Hand-offs are mbarriers; waits are bounded as in rt_conv_pipe.cu.
 //
+// Streamed layers (224 -> 96 and its data gradient: 387 KB of weights) fill a
+// stage with one slab of a strip and that slab of the weights, up to four in
+// flight, and keep the accumulators of a strip over its slabs: the weights are
+// read once per strip, and the block computes all or half of the channels.
+//
 // Measured at 32 images (ncu, cold): 128 -> 128 channels at 8 x 8 36 -> 10 us,
-// 224 -> 96 at 16 x 16 122 -> 27, 64 -> 64 at 32 x 32 30 -> 13, 48 -> 48 at
+// 224 -> 96 at 16 x 16 122 -> 27 (resident
+// slices of 16 channels; streamed, 240 x 136: 111 -> 21), 64 -> 64 at 32 x 32 30 -> 13, 48 -> 48 at
 // 64 x 64 32 -> 22; all 28 such convolutions of a training step 1.21 -> 0.57 ms.
 // What is left is launch, the weights' first load and one to five strips per block.
 //
 // The products are accumulated in the order of the kernel that runs the
 // layer on wide images, so results are bit-identical to it: taps outer and
-// channels inner, or for layers whose channels rt_conv_tc.cu takes in chunks
-// of 16, chunks outer and taps inner.
+// channels inner, or for the streamed layers, whose channels rt_conv_tc.cu
+// takes in chunks of 16, chunks outer and taps inner.
 #include <algorithm>
 #include <cstdint>
 
@@ -42,11 +50,13 @@ constexpr int kTile = 128;
 constexpr int kEpilogueWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kMaxTiles = 16;            // tiles per strip
+constexpr int kMaxStages = 4;
 constexpr uint32_t kHeader = 2048;
 constexpr uint32_t kSmemMax = 227u * 1024u;
 
 struct NarrowArgs {
     int n, h, w, pitch, cin;
+    int segments, segWidth;           // column segments of the image (pitch = segWidth + 2)
     int coutTotal, cout, slices;      // output channels of the layer, of a block, and slices
     int rows, strips, units;
     int slabs;
@@ -62,10 +72,10 @@ struct NarrowArgs {
 };
 
 struct Header {
-    static constexpr uint32_t full = 0;         // 2 stages
-    static constexpr uint32_t empty = 16;       // 2
-    static constexpr uint32_t weights = 32;     // 3 kernel rows
-    static constexpr uint32_t accFull = 64;     // 2 sets x kMaxTiles
+    static constexpr uint32_t full = 0;         // kMaxStages
+    static constexpr uint32_t empty = 8 * kMaxStages;
+    static constexpr uint32_t weights = 16 * kMaxStages;  // 3 kernel rows
+    static constexpr uint32_t accFull = weights + 32;     // 2 sets x kMaxTiles
     static constexpr uint32_t accEmpty = accFull + 16 * kMaxTiles;  // 2 sets x kMaxTiles
     static constexpr uint32_t drain = accEmpty + 16 * kMaxTiles;
     static constexpr uint32_t tmemSlot = drain + 8;
@@ -82,43 +92,47 @@ __device__ __forceinline__ uint64_t rowsDescriptor(uint32_t addr) {
 
 // The 9 x K MMAs of one tile; a: descriptors of the tile's start in the three
 // kernel rows' lines (first slab), aSlab and bSlab descriptor units between
-// slabs, bTap between taps. CHUNKED: K steps outer, else taps outer.
-template <int S, int K, bool CHUNKED>
+// slabs, bTap between taps.
+template <int S>
+__device__ __forceinline__ void issueStep(uint32_t acc, const uint64_t (&a)[3], uint64_t b, uint32_t aSlab, int bSlab,
+                                          int bTap, uint32_t idesc, int t, int k, bool fresh) {
+    mma(acc, a[t / 3] + (uint64_t)((t % 3) * (S / 8) + (k % (S / 16)) * 2 + (k / (S / 16)) * aSlab),
+        b + (uint64_t)(int64_t)((k % (S / 16)) * 2 + (k / (S / 16)) * bSlab + t * bTap), idesc, fresh ? 0u : 1u);
+}
+template <int S, int K>
 __device__ __forceinline__ void issueTile(uint32_t acc, const uint64_t (&a)[3], uint64_t b, uint32_t aSlab, int bSlab,
                                           int bTap, uint32_t idesc) {
-    auto step = [&](int t, int k, bool fresh) {
-        mma(acc, a[t / 3] + (uint64_t)((t % 3) * (S / 8) + (k % (S / 16)) * 2 + (k / (S / 16)) * aSlab),
-            b + (uint64_t)(int64_t)((k % (S / 16)) * 2 + (k / (S / 16)) * bSlab + t * bTap), idesc, fresh ? 0u : 1u);
-    };
-    if (CHUNKED) {
 #pragma unroll
-        for (int k = 0; k < K; k++)
+    for (int t = 0; t < 9; t++)
 #pragma unroll
-            for (int t = 0; t < 9; t++) step(t, k, t == 0 && k == 0);
-    } else {
+        for (int k = 0; k < K; k++) issueStep<S>(acc, a, b, aSlab, bSlab, bTap, idesc, t, k, t == 0 && k == 0);
+}
+// The same for one slab of a streamed layer: chunks of 16 channels outer.
+template <int S>
+__device__ __forceinline__ void issueSlab(uint32_t acc, const uint64_t (&a)[3], uint64_t b, int bTap, uint32_t idesc,
+                                          bool first) {
 #pragma unroll
-        for (int t = 0; t < 9; t++)
+    for (int k = 0; k < S / 16; k++)
 #pragma unroll
-            for (int k = 0; k < K; k++) step(t, k, t == 0 && k == 0);
-    }
+        for (int t = 0; t < 9; t++) issueStep<S>(acc, a, b, 0u, 0, bTap, idesc, t, k, first && t == 0 && k == 0);
 }
 // The K steps a slab width occurs with (cin / 16 of the network's layers).
-template <int S, bool CHUNKED>
+template <int S>
 __device__ __forceinline__ void issueTileK(int k, uint32_t acc, const uint64_t (&a)[3], uint64_t b, uint32_t aSlab,
                                            int bSlab, int bTap, uint32_t idesc) {
     if constexpr (S == 16) {
-        if (k == 1) issueTile<S, 1, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else if (k == 3) issueTile<S, 3, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else if (k == 5) issueTile<S, 5, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else issueTile<S, 7, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        if (k == 1) issueTile<S, 1>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else if (k == 3) issueTile<S, 3>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else if (k == 5) issueTile<S, 5>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else issueTile<S, 7>(acc, a, b, aSlab, bSlab, bTap, idesc);
     } else if constexpr (S == 32) {
-        if (k == 2) issueTile<S, 2, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else if (k == 6) issueTile<S, 6, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else if (k == 10) issueTile<S, 10, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else issueTile<S, 14, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        if (k == 2) issueTile<S, 2>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else if (k == 6) issueTile<S, 6>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else if (k == 10) issueTile<S, 10>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else issueTile<S, 14>(acc, a, b, aSlab, bSlab, bTap, idesc);
     } else {
-        if (k == 4) issueTile<S, 4, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
-        else issueTile<S, 8, CHUNKED>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        if (k == 4) issueTile<S, 4>(acc, a, b, aSlab, bSlab, bTap, idesc);
+        else issueTile<S, 8>(acc, a, b, aSlab, bSlab, bTap, idesc);
     }
 }
 inline bool knownCin(int cin) {
@@ -127,14 +141,17 @@ inline bool knownCin(int cin) {
     return false;
 }
 
-// Unit u: image, first row and rows of a strip, and its tiles.
-struct Unit { int img, y0, rows, tiles; };
+// Unit u: image, first column and row and rows of a strip of a segment, and its tiles.
+struct Unit { int img, x0, y0, rows, tiles; };
 __device__ __forceinline__ Unit unitOf(const NarrowArgs& a, int u) {
-    const int img = u / a.strips, y0 = (u % a.strips) * a.rows, rows = min(a.rows, a.h - y0);
-    return Unit{img, y0, rows, (rows * a.pitch + kTile - 1) / kTile};
+    const int column = u / a.strips, img = column / a.segments, x0 = (column - img * a.segments) * a.segWidth;
+    const int y0 = (u - column * a.strips) * a.rows, rows = min(a.rows, a.h - y0);
+    return Unit{img, x0, y0, rows, (rows * a.pitch + kTile - 1) / kTile};
 }
 
-template <int S, bool CHUNKED>
+// STREAM: a stage is one slab of a strip and of the block's weights; else all
+// slabs of a strip, with the weights resident.
+template <int S, bool STREAM>
 __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_constant__ CUtensorMap inMap,
                                                             const __grid_constant__ CUtensorMap wMap, NarrowArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -151,7 +168,7 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
     const int firstUnit = (int)(blockIdx.x / (unsigned)a.slices), unitStride = (int)(gridDim.x / (unsigned)a.slices);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < kMaxStages; s++) {
             barInit(base + Header::full + 8 * s, 1);
             barInit(base + Header::empty + 8 * s, 1);
         }
@@ -166,7 +183,7 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
         // The weights before the wait for the previous kernel: it does not
         // write them (see rt_conv_pipe.cu). Kernel row r's taps as they are
         // used (the data gradient reads the taps reversed).
-        for (int r = 0; r < 3; r++) {
+        for (int r = 0; r < 3 && !STREAM; r++) {
             const int row = a.reverseTaps ? 2 - r : r;
             barExpectTx(base + Header::weights + 8 * r, a.weightBytes / 3u);
             for (int j = 0; j < a.slabs; j++)
@@ -194,25 +211,31 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
 
     if (warp == 0) {
         // ---- producer ----
+        // Fill k: a strip (STREAM: a slab of one) in stage k % stages.
         int k = 0;
         bool ok = true;
-        for (int u = firstUnit; u < a.units; u += unitStride, k++) {
-            const int st = k % a.stages;
-            if (!waitPhaseWarp(base + Header::empty + 8 * st, (uint32_t)(((k / a.stages) & 1) ^ 1), abortFlag, limit)) { ok = false; break; }
-            if (lane == 0) {
-                const Unit U = unitOf(a, u);
-                const uint32_t fb = base + Header::full + 8 * st;
-                barExpectTx(fb, (uint32_t)(a.slabs * (a.rows + 2) * a.pitch) * 2u * S);
-                for (int j = 0; j < a.slabs; j++)
-                    tmaLoad4(stage0 + (uint32_t)st * a.stageBytes + (uint32_t)j * a.slabBytes, &inMap, j * S, -1, U.y0 - 1,
-                             U.img, fb);
+        const int perFill = STREAM ? 1 : a.slabs;
+        for (int u = firstUnit; u < a.units && ok; u += unitStride) {
+            const Unit U = unitOf(a, u);
+            for (int first = 0; first < a.slabs; first += perFill, k++) {
+                const int st = k % a.stages;
+                if (!waitPhaseWarp(base + Header::empty + 8 * st, (uint32_t)(((k / a.stages) & 1) ^ 1), abortFlag, limit)) { ok = false; break; }
+                if (lane == 0) {
+                    const uint32_t fb = base + Header::full + 8 * st, stage = stage0 + (uint32_t)st * a.stageBytes;
+                    barExpectTx(fb, (uint32_t)(perFill * (a.rows + 2) * a.pitch) * 2u * S + (STREAM ? a.weightBytes : 0u));
+                    for (int j = 0; j < perFill; j++)
+                        tmaLoad4(stage + (uint32_t)j * a.slabBytes, &inMap, (first + j) * S, U.x0 - 1, U.y0 - 1, U.img, fb);
+                    if (STREAM)
+                        for (int r = 0; r < 3; r++)
+                            tmaLoad3(stage + a.slabBytes + (uint32_t)(r * 3 * a.cout) * 2u * S, &wMap, first * S, nBase, r * 3, fb);
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
         if (!ok) *abortFlag = 1;
         // Every issued load lands before the block exits.
         if (lane == 0) {
-            for (int r = 0; r < 3; r++) pollPhase(base + Header::weights + 8 * r, 0u, limit);
+            for (int r = 0; r < 3 && !STREAM; r++) pollPhase(base + Header::weights + 8 * r, 0u, limit);
             for (int e = k > a.stages ? k - a.stages : 0; e < k; e++)
                 pollPhase(base + Header::full + 8 * (e % a.stages), (uint32_t)((e / a.stages) & 1), limit);
         }
@@ -226,33 +249,40 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
             const uint32_t aSlab = a.slabBytes >> 4;
             const int wTap = a.cout * 2 * S / 16, bTap = a.reverseTaps ? -wTap : wTap;
             const uint64_t b = a.reverseTaps ? wDesc + (uint64_t)(8 * wTap) : wDesc;
-            int k = 0;
+            int k = 0, strip = 0;  // fills and strips so far
             uint32_t used[2] = {0u, 0u};  // per set, bit i: parity of tile i's uses so far
-            for (int u = firstUnit; u < a.units && ok; u += unitStride, k++) {
-                const int st = k % a.stages, set = a.sets == 2 ? k & 1 : 0;
+            for (int u = firstUnit; u < a.units && ok; u += unitStride, strip++) {
+                const int set = a.sets == 2 ? strip & 1 : 0;
                 const Unit U = unitOf(a, u);
-                ok = waitPhase(base + Header::full + 8 * st, (uint32_t)((k / a.stages) & 1), abortFlag, limit);
-                for (int r = 0; r < 3 && ok && k == 0; r++)
-                    ok = waitPhase(base + Header::weights + 8 * r, 0u, abortFlag, limit);
-                if (!ok) break;
-                uint32_t line = stage0 + (uint32_t)st * a.stageBytes;
-                for (int i = 0; i < U.tiles; i++, line += kTile * 2 * S) {
-                    // The tile's accumulator drained since its last use.
-                    ok = waitPhase(base + Header::accEmpty + 8 * (set * kMaxTiles + i), (((set ? used[1] : used[0]) >> i) & 1u) ^ 1u,
-                                   abortFlag, limit);
+                const uint32_t pitch = (uint32_t)a.pitch * 2u * S;
+                for (int j = 0; j < (STREAM ? a.slabs : 1) && ok; j++, k++) {
+                    const int st = k % a.stages;
+                    ok = waitPhase(base + Header::full + 8 * st, (uint32_t)((k / a.stages) & 1), abortFlag, limit);
+                    for (int r = 0; r < 3 && ok && k == 0 && !STREAM; r++)
+                        ok = waitPhase(base + Header::weights + 8 * r, 0u, abortFlag, limit);
                     if (!ok) break;
-                    if (set) used[1] ^= 1u << i;
-                    else used[0] ^= 1u << i;
-                    tcFenceAfter();
-                    const uint32_t pitch = (uint32_t)a.pitch * 2u * S;
-                    const uint64_t rows[3] = {rowsDescriptor<S>(line), rowsDescriptor<S>(line + pitch),
-                                              rowsDescriptor<S>(line + 2 * pitch)};
-                    issueTileK<S, CHUNKED>(a.cin / 16, tmem + (uint32_t)set * a.setCols + (uint32_t)(i * a.cout), rows, b, aSlab,
-                                           9 * wTap, bTap, idesc);
-                    commit(base + Header::accFull + 8 * (set * kMaxTiles + i));
+                    uint32_t line = stage0 + (uint32_t)st * a.stageBytes;
+                    const uint64_t bSlab = STREAM ? b + (uint64_t)((line + a.slabBytes - wAddr) >> 4) : b;
+                    for (int i = 0; i < U.tiles; i++, line += kTile * 2 * S) {
+                        if (j == 0) {
+                            // The tile's accumulator drained since its last use.
+                            ok = waitPhase(base + Header::accEmpty + 8 * (set * kMaxTiles + i),
+                                           (((set ? used[1] : used[0]) >> i) & 1u) ^ 1u, abortFlag, limit);
+                            if (!ok) break;
+                            if (set) used[1] ^= 1u << i;
+                            else used[0] ^= 1u << i;
+                        }
+                        tcFenceAfter();
+                        const uint64_t rows[3] = {rowsDescriptor<S>(line), rowsDescriptor<S>(line + pitch),
+                                                  rowsDescriptor<S>(line + 2 * pitch)};
+                        const uint32_t acc = tmem + (uint32_t)set * a.setCols + (uint32_t)(i * a.cout);
+                        if (STREAM) issueSlab<S>(acc, rows, bSlab, bTap, idesc, j == 0);
+                        else issueTileK<S>(a.cin / 16, acc, rows, b, aSlab, 9 * wTap, bTap, idesc);
+                        if (!STREAM || j == a.slabs - 1) commit(base + Header::accFull + 8 * (set * kMaxTiles + i));
+                    }
+                    if (!ok) break;
+                    commit(base + Header::empty + 8 * st);
                 }
-                if (!ok) break;
-                commit(base + Header::empty + 8 * st);
             }
             if (ok) {
                 // The commits' arrivals land before shared memory goes away.
@@ -282,8 +312,8 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
                 if (set) phases[1] ^= 1u << i;
                 else phases[0] ^= 1u << i;
                 tcFenceAfter();
-                const int m = i * kTile + quarter * 32 + lane, row = m / a.pitch, x = m - row * a.pitch;
-                const bool inside = x < a.w && row < U.rows;
+                const int m = i * kTile + quarter * 32 + lane, row = m / a.pitch, col = m - row * a.pitch, x = U.x0 + col;
+                const bool inside = col < a.segWidth && x < a.w && row < U.rows;
                 const size_t pix = ((size_t)U.img * a.h + U.y0 + row) * a.w + x;
                 for (int c = 0; c < a.cout; c += 16) {
                     uint32_t r[16];
@@ -339,12 +369,12 @@ __global__ void __launch_bounds__(kThreads) convNarrowKernel(const __grid_consta
     }
 }
 
-template <int S, bool CHUNKED>
+template <int S, bool STREAM>
 cudaError_t launch(const CUtensorMap& inMap, const CUtensorMap& wMap, const NarrowArgs& a, int grid, uint32_t smemBytes,
                    cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(convNarrowKernel<S, CHUNKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(convNarrowKernel<S, STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
         if (e != cudaSuccess) return e;
         configured = true;
     }
@@ -358,7 +388,7 @@ cudaError_t launch(const CUtensorMap& inMap, const CUtensorMap& wMap, const Narr
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, convNarrowKernel<S, CHUNKED>, inMap, wMap, a);
+    return cudaLaunchKernelEx(&cfg, convNarrowKernel<S, STREAM>, inMap, wMap, a);
 }
 template <int S>
 cudaError_t launchC(bool chunked, const CUtensorMap& inMap, const CUtensorMap& wMap, const NarrowArgs& a, int grid,
@@ -372,11 +402,15 @@ cudaError_t launchC(bool chunked, const CUtensorMap& inMap, const CUtensorMap& w
 cudaError_t convNarrow(const bf16* in, int n, int h, int w, int cin, const bf16* weights, bool reverseTaps,
                        const float* bias, int cout, bf16* outB, float* outF, bool relu, bool accumulate, bool chunked,
                        int* errorFlag, cudaStream_t stream) {
-    if (n < 1 || h < 1 || w < 1 || w > kNarrowWidth || !knownCin(cin) || cout < 16 || cout % 16 || (!outB && !outF) || !errorFlag)
+    if (n < 1 || h < 1 || w < 1 || !knownCin(cin) || cout < 16 || cout % 16 || (!outB && !outF) || !errorFlag)
         return cudaErrorNotSupported;
     const int S = slabChannels(cin);
     NarrowArgs a{};
-    a.n = n; a.h = h; a.w = w; a.pitch = w + 2; a.cin = cin; a.coutTotal = cout;
+    a.n = n; a.h = h; a.w = w; a.cin = cin; a.coutTotal = cout;
+    // Columns in equal segments of up to kNarrowWidth, each with its own halo.
+    a.segments = (w + kNarrowWidth - 1) / kNarrowWidth;
+    a.segWidth = (w + a.segments - 1) / a.segments;
+    a.pitch = a.segWidth + 2;
     a.slabs = cin / S;
     int sms = 0, device = 0;
     cudaGetDevice(&device);
@@ -388,37 +422,51 @@ cudaError_t convNarrow(const bf16* in, int n, int h, int w, int cin, const bf16*
     // the weights and the first strip, and the larger of the two per strip
     // after that (their sum where only one stage fits).
     double best = -1.0;
+    long long bestPer = 0;
     for (int s = 1; s <= cout / 16; s++) {
         const int slice = cout / s;
         if (cout % s || slice % 16 || slice > 128) continue;
-        const uint32_t weightBytes = 9u * (uint32_t)cin * (uint32_t)slice * 2u, space = (weightBytes + 1023u) & ~1023u;
+        const int held = chunked ? S : cin;  // input channels whose weights are held at a time
+        const uint32_t weightBytes = 9u * (uint32_t)held * (uint32_t)slice * 2u, space = (weightBytes + 1023u) & ~1023u;
         const int perSlice = std::max(1, sms / s);
         for (int rows = 1; rows <= std::min(h, 254); rows++) {
             const int tiles = (rows * a.pitch + kTile - 1) / kTile;
             if (tiles > kMaxTiles || tiles * slice > 512) break;
             // The last tile reads up to 2 rows and 2 pixels past its start + 128.
             const int line = std::max((rows + 2) * a.pitch, tiles * kTile + 2 * a.pitch + 2);
-            const uint32_t slabBytes = ((uint32_t)line * 2u * (uint32_t)S + 1023u) & ~1023u, stage = (uint32_t)a.slabs * slabBytes;
-            if (kHeader + space + stage > kSmemMax) break;
+            const uint32_t slabBytes = ((uint32_t)line * 2u * (uint32_t)S + 1023u) & ~1023u;
+            const uint32_t stage = chunked ? slabBytes + space : (uint32_t)a.slabs * slabBytes;
+            const uint32_t fixed = kHeader + (chunked ? 0u : space);
+            if (fixed + stage > kSmemMax) break;
             const int strips = (h + rows - 1) / rows;
-            const long long units = (long long)n * strips;
+            const long long units = (long long)n * a.segments * strips;
             if (units * s > 0x7FFFFFFFll) continue;
-            const long long per = (units + perSlice - 1) / perSlice;
-            const int stages = per > 1 && kHeader + space + 2 * stage <= kSmemMax ? 2 : 1;
-            const double mmas = tiles * 9.0 * (cin / 16) * std::max(60.0, slice * 0.55), load = stage / 24.0;
-            const double cost = 3000.0 + weightBytes / 24.0 + load + mmas + tiles * 150.0 +
-                                (double)(per - 1) * (stages == 2 ? std::max(mmas, load) + 300.0 : mmas + load + 1000.0);
+            const long long per = (units + perSlice - 1) / perSlice, fills = chunked ? per * a.slabs : per;
+            const int stages = (int)std::min<long long>({fills, chunked ? kMaxStages : 2, (kSmemMax - fixed) / stage});
+            const double mmas = tiles * 9.0 * (held / 16) * std::max(60.0, slice * 0.55), load = stage / 24.0;
+            const double cost = 3000.0 + (chunked ? 0.0 : weightBytes / 24.0) + load + mmas + tiles * 150.0 +
+                                (double)(fills - 1) * (stages >= 2 ? std::max(mmas, load) + 300.0 : mmas + load + 1000.0);
             if (best >= 0.0 && cost >= best) continue;
             best = cost;
+            bestPer = per;
             a.cout = slice; a.slices = s;
             a.rows = rows; a.strips = strips; a.units = (int)units;
-            a.slabBytes = slabBytes; a.stageBytes = stage; a.weightBytes = weightBytes; a.weightSpace = space;
+            a.slabBytes = slabBytes; a.stageBytes = stage; a.weightBytes = weightBytes; a.weightSpace = chunked ? 0u : space;
             a.stages = stages;
             a.setCols = (uint32_t)(tiles * slice);
             a.sets = per > 1 && 2u * a.setCols <= 512u ? 2 : 1;
         }
     }
     if (best < 0.0) return cudaErrorNotSupported;
+    // Wider images whose weights stay resident: only small ones, whose strips
+    // load behind the MMAs. One 1080p inference, this kernel against the
+    // pipelined one (us): 64 -> 64 at 480 x 272 25 / 33, 48 -> 64 22 / 30,
+    // 64 -> 96 at 240 x 136 12 / 19, 128 -> 128 at 120 x 68 11 / 23; but
+    // 96 -> 96 at 240 x 136, one stage and two strips per block, 30 / 25, and
+    // 48 -> 48 at 960 x 544 61 / 48. Streamed layers at any size: 224 -> 96 at
+    // 240 x 136 21 us against 74 in the single-role kernel.
+    if (!chunked && w > kNarrowWidth && ((long long)n * h * w > 1024ll * sms || (bestPer > 1 && a.stages < 2)))
+        return cudaErrorNotSupported;
     a.tmemCols = 32;
     while (a.tmemCols < a.setCols * (uint32_t)a.sets) a.tmemCols <<= 1;
     a.bias = bias; a.outB = outB; a.outF = outF;

@@ -543,16 +543,17 @@ cudaError_t convTc(const bf16* in, const bf16* low, int lowChannels, int n, int 
         if (e == cudaSuccess) g_pipeLaunches++;
         return e;
     }
-    // Narrow images: the kernel whose tiles span rows, accumulating in the
-    // order of the kernel below that would take the layer.
+    // The kernel whose tiles span rows where it takes the layer (narrow or
+    // small images, streamed weights), accumulating in the order of the kernel
+    // below that would take it otherwise.
     const bool piped = convPipePreferred(cin, cout, low ? lowChannels : 0);
-    if (g_convPath.load() == 0 && !g_convPipeReference.load() && !low && w <= kNarrowWidth) {
+    if (g_convPath.load() == 0 && !g_convPipeReference.load() && !low) {
         const int kc = piped ? cin : singleRoleForm(cin, cout).kc;
         cudaError_t e = kc != cin && kc != 16 ? cudaErrorNotSupported
                                               : convNarrow(in, n, h, w, cin, weights, reverseTaps, bias, cout, outB, outF, relu,
                                                            accumulate, kc != cin, errorFlag, stream);
         if (e != cudaErrorNotSupported) {
-            g_pipeLaunches++;
+            (kc != cin ? g_singleLaunches : g_pipeLaunches)++;
             return e;
         }
     }

@@ -159,11 +159,12 @@ cudaError_t convPipe(const __nv_bfloat16* in, const __nv_bfloat16* low, int lowC
                      cudaStream_t stream, const ConvPipeTest* test = nullptr,
                      const __nv_bfloat16* upAddend = nullptr, const ConvHead* head = nullptr, bool planarOut = false);
 
-// The same convolution on images of up to kNarrowWidth pixels (rt_conv_narrow
-// .cu): tiles of 128 positions over several rows. chunked: products
+// The same convolution with tiles of 128 positions over several rows of column
+// segments of up to kNarrowWidth pixels (rt_conv_narrow.cu). chunked: products
 // accumulated in chunks of 16 input channels (the single-role kernel's order
-// for layers whose weights it stages in chunks), else tap by tap. Returns
-// cudaErrorNotSupported (before any launch) for shapes it does not take.
+// for layers whose weights it stages in chunks) with streamed weights, else
+// tap by tap. Returns cudaErrorNotSupported (before any launch) for shapes it
+// does not take and for those the pipelined kernel runs faster.
 // Above 64 pixels a row-wide tile of 128 is more than half full and the
 // pipelined kernel's ring stages every row once.
 constexpr int kNarrowWidth = 64;

@@ -716,7 +716,7 @@ cudaError_t Unet::ensure(int n, int h, int w, bool training) {
             if ((e = A.make(A.upWeights[j], (size_t)9 * 4 * L.cout * Cl)) != cudaSuccess) return e;
             if ((e = A.make(A.skipWeights[j], (size_t)9 * L.cout * (L.cin - Cl))) != cudaSuccess) return e;
         }
-        if (training && (e = A.make(A.cat[j], px(level) * layers_[10 + 2 * j].cin)) != cudaSuccess) return e;
+        if ((training || !A.upWeights[j]) && (e = A.make(A.cat[j], px(level) * layers_[10 + 2 * j].cin)) != cudaSuccess) return e;
         if (training && (e = A.make(A.dCat[j], px(level) * layers_[10 + 2 * j].cin)) != cudaSuccess) return e;
     }
     if (upHalf && (e = A.make(A.upHalf, upHalf)) != cudaSuccess) return e;
@@ -756,8 +756,10 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
         const bf16* skip = A.a[2 * level + 1];
         for (int r = 0; r < 2; r++, k++) {
             const UnetLayer& L = layers_[k];
-            if (r == 0 && training) {
-                // The weight gradient reads the concatenated input: keep it.
+            if (r == 0 && (training || (A.cat[j] && convPath() == 0))) {
+                // The weight gradient reads the concatenated input; at inference
+                // the streamed convolution does (8 + 21 us against 74 for the
+                // single-role kernel reading its halves in place, 240 x 136).
                 upConcatKernel<<<blocksFor((long long)n * H * W * ((Cl + Cs) / 8), 256), 256, 0, s>>>(low, Cl, skip, Cs, n, H, W, A.cat[j]);
                 e = convTc(A.cat[j], nullptr, 0, n, H, W, L.cin, wT_ + L.wOffset, false, master_ + L.bOffset, L.cout, A.a[k], nullptr, true, false, convError_, s);
             } else if (r == 0 && A.upWeights[j] && convPath() == 0) {

@@ -401,12 +401,14 @@ __global__ void aovKernel(const Accum* sums, const float* depthSums, unsigned sa
     o[6] = n.x; o[7] = n.y; o[8] = n.z;
     o[9] = depthSums[i] * inv;
 }
-__global__ void presentRadianceKernel(const Accum* sums, const float* radiance, int count, float exposure,
+// Coverage as bytes from the network's input kernel: the 40-byte sums' flag cost
+// their 83 MB again at 1080p (26 us, now 14).
+__global__ void presentRadianceKernel(const unsigned char* coverage, const float* radiance, int count, float exposure,
                                       uchar4* pixels) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const float* r = radiance + (size_t)i * 3;
-    float3 c = sums[i].covered ? v3(r[0], r[1], r[2]) : v3(0, 0, 0);
+    float3 c = coverage[i] ? v3(r[0], r[1], r[2]) : v3(0, 0, 0);
     pixels[i] = make_uchar4(tonemap(c.x, exposure), tonemap(c.y, exposure), tonemap(c.z, exposure), 255);
 }
 
@@ -678,9 +680,9 @@ cudaError_t launchAovs(const Accum* sums, const float* depthSums, unsigned sampl
     aovKernel<<<blocks(count, 256), 256, 0, stream>>>(sums, depthSums, samples, count, aov);
     return cudaGetLastError();
 }
-cudaError_t launchPresentRadiance(const Accum* sums, const float* radiance, int count, float exposure, uchar4* pixels,
+cudaError_t launchPresentRadiance(const unsigned char* coverage, const float* radiance, int count, float exposure, uchar4* pixels,
                                   cudaStream_t stream) {
-    presentRadianceKernel<<<blocks(count, 256), 256, 0, stream>>>(sums, radiance, count, exposure, pixels);
+    presentRadianceKernel<<<blocks(count, 256), 256, 0, stream>>>(coverage, radiance, count, exposure, pixels);
     return cudaGetLastError();
 }
 

@@ -106,7 +106,7 @@ cudaError_t launchAovs(const Accum* sums, const float* depthSums, unsigned sampl
                        cudaStream_t stream);
 // Tonemap linear radiance (3 floats per pixel) into the display image;
 // uncovered pixels stay black (renderer.cu:429-435).
-cudaError_t launchPresentRadiance(const Accum* sums, const float* radiance, int count, float exposure, uchar4* pixels,
+cudaError_t launchPresentRadiance(const unsigned char* coverage, const float* radiance, int count, float exposure, uchar4* pixels,
                                   cudaStream_t stream);
 
 }  // namespace rt

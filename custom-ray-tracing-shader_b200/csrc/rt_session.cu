@@ -578,9 +578,10 @@ int RtDenoise(void* p, unsigned char* output, int outputBytes, float* millisecon
         // Learned denoiser: running sums -> U-Net (AOVs formed in its input
         // kernel, as RtxReadAovs forms them) -> display, on the session stream.
         float* radiance = reinterpret_cast<float*>(s->dDenoise) + 10 * count;
+        unsigned char* coverage = reinterpret_cast<unsigned char*>(radiance + 3 * count);
         if ((e = s->denoiser->net.inferFromSums(reinterpret_cast<const float*>(s->dSum), s->dDepth, s->samples,
-                                                s->height, s->width, radiance, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
-        if ((e = launchPresentRadiance(s->dSum, radiance, (int)count, s->lastSettings.exposure, s->dPixels, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+                                                s->height, s->width, radiance, coverage, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+        if ((e = launchPresentRadiance(coverage, radiance, (int)count, s->lastSettings.exposure, s->dPixels, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
         s->denoisedOffset = 10 * count;
         s->denoisedStride = 3;
     } else {

@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(128) weightsKernel(const WeightTable T, float*
 // transform of inputKernel, for every pixel of the padded frame (beyond w x h
 // the edge pixels repeat).
 __global__ void sumsInputKernel(const float* sums, const float* depthSums, unsigned samples, int h, int w, int H,
-                                int W, bf16* x0) {
+                                int W, bf16* x0, unsigned char* coverage) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)H * W) return;
     const int X = (int)(i % W), Y = (int)(i / W);
@@ -457,6 +457,7 @@ __global__ void sumsInputKernel(const float* sums, const float* depthSums, unsig
     const float3 c = scale(v3(a[0], a[1], a[2]), inv), al = scale(v3(a[3], a[4], a[5]), inv);
     const float3 nr = normalize(v3(a[6], a[7], a[8]));
     const float depth = depthSums[src] * inv;
+    if (X < w && Y < h) coverage[src] = __float_as_uint(a[9]) != 0u;
     float v[kInputPadded] = {};
     v[0] = log1pf(fmaxf(c.x, 0.0f)); v[1] = log1pf(fmaxf(c.y, 0.0f)); v[2] = log1pf(fmaxf(c.z, 0.0f));
     v[3] = al.x; v[4] = al.y; v[5] = al.z;
@@ -736,6 +737,31 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
     cudaError_t e;
     const bf16* x = A.x0;
     int k = 0;
+    // The decoders' combined weights, 14 us of small kernels at 1080p that
+    // only the decoders need, beside the encoder.
+    const bool combine = !training && convPath() == 0;
+    struct Join {  // the side stream's work never outlives the call's order on s
+        cudaStream_t s;
+        cudaEvent_t pending;
+        ~Join() {
+            if (pending) cudaStreamWaitEvent(s, pending, 0);
+        }
+    } join{s, nullptr};
+    if (combine) {
+        if ((e = cudaEventRecord(fork_, s)) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(side_, fork_, 0)) != cudaSuccess) return e;
+        cudaError_t made = cudaSuccess;
+        for (int j = 0; j < 4; j++) {
+            const UnetLayer& L = layers_[10 + 2 * j];
+            if (A.upWeights[j] && made == cudaSuccess)
+                made = combineUpsampledWeights(wT_ + L.wOffset, L.cout, L.cin, layers_[9 + 2 * j].cout, A.upWeights[j],
+                                               A.skipWeights[j], side_);
+        }
+        e = cudaEventRecord(join_, side_);
+        join.pending = join_;
+        if (made != cudaSuccess) e = made;
+        if (e != cudaSuccess) return e;
+    }
     for (int l = 0; l < 5; l++) {
         int H = A.H >> l, W = A.W >> l;
         if (l > 0) {
@@ -749,6 +775,8 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
             x = A.a[k];
         }
     }
+    if (combine && (e = cudaStreamWaitEvent(s, join_, 0)) != cudaSuccess) return e;
+    join.pending = nullptr;
     for (int j = 0; j < 4; j++) {
         int level = 3 - j, H = A.H >> level, W = A.W >> level;
         int Cl = layers_[k - 1].cout, Cs = kWidths[level];
@@ -762,13 +790,11 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
                 // single-role kernel reading its halves in place, 240 x 136).
                 upConcatKernel<<<blocksFor((long long)n * H * W * ((Cl + Cs) / 8), 256), 256, 0, s>>>(low, Cl, skip, Cs, n, H, W, A.cat[j]);
                 e = convTc(A.cat[j], nullptr, 0, n, H, W, L.cin, wT_ + L.wOffset, false, master_ + L.bOffset, L.cout, A.a[k], nullptr, true, false, convError_, s);
-            } else if (r == 0 && A.upWeights[j] && convPath() == 0) {
+            } else if (r == 0 && A.upWeights[j] && combine) {
                 // Inference, two passes: the upsampled half at half
                 // resolution (4 parity blocks), then the skip half adding it.
-                e = combineUpsampledWeights(wT_ + L.wOffset, L.cout, L.cin, Cl, A.upWeights[j], A.skipWeights[j], s);
-                if (e == cudaSuccess)
-                    e = convTc(low, nullptr, 0, n, H / 2, W / 2, Cl, A.upWeights[j], false, nullptr, 4 * L.cout, A.upHalf,
-                               nullptr, false, false, convError_, s, nullptr, nullptr, true);
+                e = convTc(low, nullptr, 0, n, H / 2, W / 2, Cl, A.upWeights[j], false, nullptr, 4 * L.cout, A.upHalf,
+                           nullptr, false, false, convError_, s, nullptr, nullptr, true);
                 if (e == cudaSuccess)
                     e = convTc(skip, nullptr, 0, n, H, W, Cs, A.skipWeights[j], false, master_ + L.bOffset, L.cout, A.a[k],
                                nullptr, true, false, convError_, s, A.upHalf);
@@ -929,11 +955,12 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
 }
 
 cudaError_t Unet::inferFromSums(const float* sums, const float* depthSums, unsigned samples, int h, int w,
-                                float* radiance, cudaStream_t s) {
+                                float* radiance, unsigned char* coverage, cudaStream_t s) {
     cudaError_t e = ensure(1, h, w, false);
     if (e != cudaSuccess) return e;
     Activations& A = *act_;
-    sumsInputKernel<<<blocksFor((long long)A.H * A.W, 256), 256, 0, s>>>(sums, depthSums, samples, h, w, A.H, A.W, A.x0);
+    sumsInputKernel<<<blocksFor((long long)A.H * A.W, 256), 256, 0, s>>>(sums, depthSums, samples, h, w, A.H, A.W, A.x0,
+                                                                        coverage);
     const UnetLayer& O = layers_[18];
     const ConvHead head{master_ + O.wOffset, master_ + O.bOffset, radiance, h, w};
     bool fused = false;

@@ -52,9 +52,10 @@ public:
     // byte fields per pixel: radiance, albedo and normal sums, coverage) and
     // first-hit distance sums after `samples` paths per pixel: the AOVs are
     // formed inside the input kernel with the expressions of RtxReadAovs, and
-    // the output layer writes the cropped radiance directly.
+    // the output layer writes the cropped radiance directly. coverage (h x w
+    // bytes): whether a path of the pixel hit anything, for the display.
     cudaError_t inferFromSums(const float* sums, const float* depthSums, unsigned samples, int h, int w,
-                              float* radiance, cudaStream_t stream);
+                              float* radiance, unsigned char* coverage, cudaStream_t stream);
     // Checkpoint file: parameters, and the Adam state when optimizerState.
     cudaError_t save(const char* path, bool optimizerState, std::string& error) const;
     // After the work has finished: an error if a tensor-core convolution gave

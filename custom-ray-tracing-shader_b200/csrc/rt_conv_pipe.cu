@@ -1138,8 +1138,11 @@ cudaError_t convPipe(const bf16* in, const bf16* low, int lowChannels, int n, in
     // Measured per layer: the stacked form is faster for unsplit 32-channel
     // layers (1080p 16 -> 32: 78.6 -> 74.2 us, 32 -> 32: 98.9 -> 94.0), slower
     // for 64 output channels (64 -> 64 at 480x272: 31.4 -> 36.9) and for a
-    // 32-channel slice of a split layer (128 -> 128 at 120x68: 19.2 -> 23.0).
-    const bool stackDefault = cout == 32 && nSplits == 1;
+    // 32-channel slice of a split layer (128 -> 128 at 120x68: 19.2 -> 23.0), and
+    // where one block fits per SM: there two issuers of the tap-per-tile form
+    // issue faster than the stacked form's one (1080p 80 -> 32: 165 us against
+    // 228; with two blocks, 48 -> 32 at 960x544, 36 against 35).
+    const bool stackDefault = cout == 32 && nSplits == 1 && perSm > 1;
     if (stackMode == 2 && !stackFits) return cudaErrorNotSupported;
     const bool stacked = stackFits && (stackMode == 2 || (stackMode == 0 && stackDefault));
     const int issuers = !stacked && (force == 2 || (force == 0 && perSm == 1 && twoFit)) ? 2 : 1;

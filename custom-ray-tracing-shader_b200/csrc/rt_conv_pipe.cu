@@ -905,6 +905,7 @@ __global__ void __launch_bounds__(pipeThreads(ISS, EPI), ISS > 1 ? 1 : (COUT <= 
 #pragma unroll
                     for (int g = 0; g < kChunks; g += kGroup) {
                         uint32_t r[kGroup][16];
+                        __syncwarp();  // the loads need converged lanes; the stores below diverge
 #pragma unroll
                         for (int c = 0; c < kGroup; c++) tmemLoad16(taddr + (uint32_t)(16 * (chunk0 + g + c)), r[c]);
                         tmemWaitLoads();

@@ -168,7 +168,7 @@ def test_convolutions_identical(lib, net, h, w):
         lib.RtxSetConvPath(0)
 
 
-@pytest.mark.parametrize('n,h,w', ((1, 16, 16), (3, 16, 176), (1, 144, 16), (2, 80, 112), (1, 32, 272)))
+@pytest.mark.parametrize('n,h,w', ((1, 16, 16), (3, 16, 176), (1, 144, 16), (2, 80, 112), (1, 32, 272), (5, 128, 256)))
 def test_gradients_at_edges(net, n, h, w):
     """Weight gradients (segments of 16 to 128 pixels, column taps along N or
     not), the head, the pre-activation gradients and the data gradients against

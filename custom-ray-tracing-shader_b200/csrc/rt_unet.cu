@@ -400,7 +400,10 @@ __global__ void outForwardKernel(const bf16* d, long long pixels, int C, const f
 // owns 16 input channels of one tap of one layer (16 * cout consecutive
 // parameters, transposed through shared memory into 32-byte runs of wT), or a
 // layer's bias, or the output layer. One launch of ~830 blocks replaces Adam,
-// the conversion and 18 transposes (73 us, launch-bound).
+// the conversion and 18 transposes (73 us, launch-bound). Bound by the latency
+// of a thread's parameters one after another: 24 us in blocks of 128 threads,
+// 12 in blocks of 512 (32 MB of traffic: 5 us).
+constexpr int kWeightThreads = 512;
 struct WeightTable {
     int blocks[19];               // first block of each layer's entries (taps x cin / 16, then its bias)
     int cin[19], cout[19];
@@ -408,7 +411,7 @@ struct WeightTable {
     int total;                    // blocks in all
 };
 template <bool ADAM>
-__global__ void __launch_bounds__(128) weightsKernel(const WeightTable T, float* p, const float* g, float* m, float* v,
+__global__ void __launch_bounds__(kWeightThreads) weightsKernel(const WeightTable T, float* p, const float* g, float* m, float* v,
                                                      float lr, float b1, float b2, float eps, float c1, float c2,
                                                      bf16* wbf, bf16* wT) {
     __shared__ bf16 tile[16 * 129];  // [ci][co], padded against bank conflicts
@@ -658,7 +661,7 @@ WeightTable weightTable(const std::vector<UnetLayer>& layers) {
 
 cudaError_t Unet::syncWeights(cudaStream_t s) {
     const WeightTable T = weightTable(layers_);
-    weightsKernel<false><<<T.total, 128, 0, s>>>(T, master_, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f,
+    weightsKernel<false><<<T.total, kWeightThreads, 0, s>>>(T, master_, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f,
                                                  1.0f, wbf_, wT_);
     return cudaGetLastError();
 }
@@ -941,7 +944,7 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
         adamStep_++;
         const float b1 = 0.9f, b2 = 0.999f;
         float c1 = 1.0f - std::pow(b1, (float)adamStep_), c2 = 1.0f - std::pow(b2, (float)adamStep_);
-        weightsKernel<true><<<table.total, 128, 0, stream_>>>(table, master_, grad_, adamM_, adamV_, lr, b1, b2, 1e-8f, c1,
+        weightsKernel<true><<<table.total, kWeightThreads, 0, stream_>>>(table, master_, grad_, adamM_, adamV_, lr, b1, b2, 1e-8f, c1,
                                                               c2, wbf_, wT_);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         // The tiny host copies above wait for the stream; keep them ordered.

@@ -16,25 +16,29 @@
 // all nine taps: ceil(3 cin / 128) blocks x 3 column taps of accumulators in
 // tensor memory. (One block per row tap, each padding its cin rows to M =
 // 128 and staging x and dY again as planes of 8 channels, took 125 us for
-// 32 -> 32 channels at 32 x 128 x 128 pixels; this form 29 us. Its floors:
-// 67 MB of operands, 10 us; 32,768 MMAs of N = 96, 10 us.)
-//
-// Where dY's channels are one slab (32 or 64 output channels), the column taps
-// sit side by side along N as well: a shift by one pixel is one pixel row of
-// the slab, so with a group stride of one pixel row N covers dY shifted by 0,
-// 1 and 2 pixels, and one MMA does all nine taps of a block (N = 96 takes ~80
-// cycles, three of N = 32 ~42 each and three issues). Then x is staged without
-// and dY with the one-pixel halo, and group g holds tap dx = 2 - g. Else the
-// tap shifts x's start address.
+// 32 -> 32 channels at 32 x 128 x 128 pixels; this form 50 us. Its floors:
+// 67 MB of operands, 10 us; 98,304 MMAs of N = 32, 14 us.)
 // Where the accumulators pass 512 columns, blocks of the grid take slices of
-// the M blocks. Split K over the blocks; each adds its accumulators to dw
-// with 16-byte FP32 reductions at the end. Rows of the last M block beyond 3 cin
-// read the next staged row and are dropped (a row of D depends on its row of
-// A only).
+// the M blocks. Rows of the last M block beyond 3 cin read the next staged row
+// and are dropped (a row of D depends on its row of A only).
 //
-// Segments are as wide as the image rounded up to 16 pixels (at most 128), so the narrow
-// deep levels do no work for padding; a stage holds `rows` dY rows and
-// rows + 2 x rows.
+// K is split over the blocks: each takes a group of consecutive row segments
+// (of 128 pixels) in order and adds its accumulators to dw with 16-byte FP32
+// reductions at the end. Which products share an accumulator, and in what
+// order, decides the rounding of the gradient (2e-6 to 5e-6 of a layer's between
+// two groupings, against 1e-7 from the order of the blocks' additions), and
+// Adam from fresh moments turns such differences into whole steps of weights
+// whose gradient is near zero. So the grouping is part of the training's result
+// and is fixed (see wgradTc): not by what balances best, and with the column
+// tap as a shift of x, never of dY, whose products would pair up otherwise.
+// Spread over all multiprocessors with dY shifted where its channels are one
+// slab (all column taps in one MMA of N = 3 cout) the 18 layers of a step took
+// 473 us instead of 659 and the layer above 29; beside the backward pass, on a
+// stream of its own, that is 1.69 ms a step instead of 1.84.
+//
+// Segments are staged as wide as the image rounded up to 16 pixels (at most
+// 128), so the narrow deep levels do no work for padding; a stage holds up to
+// `rows` dY rows and rows + 2 x rows.
 //
 // Roles: warp 0 issues the TMA loads into two or more stages, warp 1 issues
 // the MMAs and owns the tensor memory, warps 2-5 drain the accumulators at
@@ -64,9 +68,9 @@ __host__ __device__ constexpr uint32_t slabBytes(int px, int s) {
 
 struct WgradArgs {
     int h, w, cin, cout;
-    int xHalo, dHalo;              // pixels staged on each side of a segment (one of them 1)
-    int px;                        // pixels per segment (K per row): 16..128, a multiple of 16
-    int tilesPerRow, strips, units, rows;
+    int px;                        // pixels of a segment that are staged (K per row): 16..128, a multiple of 16
+    int tilesPerRow, segments, perGroup;
+    int rows;                      // most dY rows per stage
     int xSlabs, dSlabs;            // slabs per row
     uint32_t xSlab, dSlab;         // bytes of one
     uint32_t xBytes, stageBytes;   // x part of a stage, and the whole stage
@@ -99,44 +103,45 @@ __device__ __forceinline__ uint64_t slabDescriptor(uint32_t addr, uint32_t slab)
     return ummaSmemDesc(addr, slab, 16u * S) | slabLayout(S);
 }
 
-// The MMAs of one dY row and one M block: KK steps of 16 pixels, for all
-// column taps at once (WIDE) or for each, descriptors as compile-time offsets
-// from two bases (one thread issues; computing descriptors per MMA is several
-// times slower than the tensor pipe).
-template <int SX, int SD, bool WIDE, int KK>
+// The MMAs of one dY row and one M block: KK steps of 16 pixels for each
+// column tap, descriptors as compile-time offsets from two bases (one thread
+// issues; computing descriptors per MMA is several times slower than the
+// tensor pipe).
+template <int SX, int SD, int KK>
 __device__ __forceinline__ void issueRow(uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
                                          uint32_t first) {
 #pragma unroll
-    for (int dx = 0; dx < (WIDE ? 1 : 3); dx++)
+    for (int dx = 0; dx < 3; dx++)
 #pragma unroll
         for (int kk = 0; kk < KK; kk++)
             mma(acc + (uint32_t)dx * accStep, x + (uint64_t)(dx * (SX / 8) + kk * 2 * SX), d + (uint64_t)(kk * 2 * SD),
                 idesc, (first || kk > 0) ? 1u : 0u);
 }
-template <int SX, int SD, bool WIDE>
+template <int SX, int SD>
 __device__ __forceinline__ void issueRowK(int kk, uint32_t acc, uint32_t accStep, uint64_t x, uint64_t d, uint32_t idesc,
                                           uint32_t first) {
     switch (kk) {
-        case 1: issueRow<SX, SD, WIDE, 1>(acc, accStep, x, d, idesc, first); break;
-        case 2: issueRow<SX, SD, WIDE, 2>(acc, accStep, x, d, idesc, first); break;
-        case 3: issueRow<SX, SD, WIDE, 3>(acc, accStep, x, d, idesc, first); break;
-        case 4: issueRow<SX, SD, WIDE, 4>(acc, accStep, x, d, idesc, first); break;
-        case 5: issueRow<SX, SD, WIDE, 5>(acc, accStep, x, d, idesc, first); break;
-        case 6: issueRow<SX, SD, WIDE, 6>(acc, accStep, x, d, idesc, first); break;
-        case 7: issueRow<SX, SD, WIDE, 7>(acc, accStep, x, d, idesc, first); break;
-        default: issueRow<SX, SD, WIDE, 8>(acc, accStep, x, d, idesc, first); break;
+        case 1: issueRow<SX, SD, 1>(acc, accStep, x, d, idesc, first); break;
+        case 2: issueRow<SX, SD, 2>(acc, accStep, x, d, idesc, first); break;
+        case 3: issueRow<SX, SD, 3>(acc, accStep, x, d, idesc, first); break;
+        case 4: issueRow<SX, SD, 4>(acc, accStep, x, d, idesc, first); break;
+        case 5: issueRow<SX, SD, 5>(acc, accStep, x, d, idesc, first); break;
+        case 6: issueRow<SX, SD, 6>(acc, accStep, x, d, idesc, first); break;
+        case 7: issueRow<SX, SD, 7>(acc, accStep, x, d, idesc, first); break;
+        default: issueRow<SX, SD, 8>(acc, accStep, x, d, idesc, first); break;
     }
 }
 
-// Unit u: image, first pixel and first row, and its dY rows.
-struct Unit { int img, x0, y0, rows; };
-__device__ __forceinline__ Unit unitOf(const WgradArgs& a, int u) {
-    const int strip = u % a.strips, xt = (u / a.strips) % a.tilesPerRow, img = u / (a.strips * a.tilesPerRow);
-    const int y0 = strip * a.rows;
-    return Unit{img, xt * a.px, y0, min(a.rows, a.h - y0)};
+// The stage that begins at segment s of a group that ends before `end`: image,
+// first pixel and first row, and its dY rows (consecutive segments of one
+// image where a row is one segment, else one).
+struct Strip { int img, x0, y0, rows; };
+__device__ __forceinline__ Strip stripAt(const WgradArgs& a, int s, int end) {
+    const int row = s / a.tilesPerRow, xt = s - row * a.tilesPerRow, img = row / a.h, y0 = row - img * a.h;
+    return Strip{img, xt * kM, y0, a.tilesPerRow == 1 ? min(min(a.rows, a.h - y0), end - s) : 1};
 }
 
-template <int SX, int SD, bool WIDE>
+template <int SX, int SD>
 __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant__ CUtensorMap xMap,
                                                          const __grid_constant__ CUtensorMap dMap, WgradArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -153,6 +158,7 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
     // This block's M blocks, and the slabs of the stacked rows they cover.
     const int b0 = (int)blockIdx.y * a.blocksPerSlice, b1 = min(a.mBlocks, b0 + a.blocksPerSlice);
     const int slab0 = b0 * (kM / SX), slab1 = min(b1 * (kM / SX), 3 * a.xSlabs);
+    const int seg0 = (int)blockIdx.x * a.perGroup, seg1 = min(a.segments, seg0 + a.perGroup);  // its group
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
@@ -176,14 +182,15 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + Header::tmemSlot);
 
     if (warp == 0) {
-        // ---- producer: one stage per unit ----
+        // ---- producer: one stage per strip ----
         int k = 0;
         bool ok = true;
-        for (int u = (int)blockIdx.x; u < a.units; u += (int)gridDim.x, k++) {
+        for (int s = seg0; s < seg1; k++) {
             const int st = k % S;
             if (!waitPhaseWarp(base + Header::empty + 8 * st, (uint32_t)(((k / S) & 1) ^ 1), abortFlag, limit)) { ok = false; break; }
             // The lanes issue the boxes: first dY's, then x's.
-            const Unit U = unitOf(a, u);
+            const Strip U = stripAt(a, s, seg1);
+            s += U.rows;
             const uint32_t fb = base + Header::full + 8 * st;
             const uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
             const int dBoxes = U.rows * a.dSlabs, xBoxes = (U.rows + 2) * a.xSlabs;
@@ -203,16 +210,15 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
             for (int i = lane; i < xBoxes; i += 32) mine += needed(i) ? 1 : 0;
             const uint32_t boxes = (uint32_t)__reduce_add_sync(0xFFFFFFFFu, mine);
             if (lane == 0)
-                barExpectTx(fb, boxes * (uint32_t)(a.px + 2 * a.xHalo) * 2u * SX +
-                                    (uint32_t)(dBoxes * (a.px + 2 * a.dHalo)) * 2u * SD);
+                barExpectTx(fb, boxes * (uint32_t)(a.px + 2) * 2u * SX + (uint32_t)(dBoxes * a.px) * 2u * SD);
             __syncwarp();
             for (int i = lane; i < dBoxes; i += 32) {
                 const int r = i / a.dSlabs, c = i - r * a.dSlabs;
-                tmaLoad4(ds + (uint32_t)i * a.dSlab, &dMap, c * SD, U.x0 - a.dHalo, U.y0 + r, U.img, fb);
+                tmaLoad4(ds + (uint32_t)i * a.dSlab, &dMap, c * SD, U.x0, U.y0 + r, U.img, fb);
             }
             for (int i = lane; i < xBoxes; i += 32) {
                 const int j = i / a.xSlabs, c = i - j * a.xSlabs;
-                if (needed(i)) tmaLoad4(xs + (uint32_t)i * a.xSlab, &xMap, c * SX, U.x0 - a.xHalo, U.y0 - 1 + j, U.img, fb);
+                if (needed(i)) tmaLoad4(xs + (uint32_t)i * a.xSlab, &xMap, c * SX, U.x0 - 1, U.y0 - 1 + j, U.img, fb);
             }
             __syncwarp();
         }
@@ -227,22 +233,22 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         // ---- MMA issuer ----
         if (lane == 0) {
             bool ok = true;
-            const uint32_t idesc = idescMnMajor(kM, WIDE ? 3 * a.cout : a.cout);
+            const uint32_t idesc = idescMnMajor(kM, a.cout);
             const uint32_t cols = (uint32_t)a.cout;
             int k = 0, st = 0;
             uint32_t parity = 0, started = 0;
-            for (int u = (int)blockIdx.x; u < a.units && ok; u += (int)gridDim.x, k++) {
+            for (int s = seg0; s < seg1 && ok; k++) {
                 ok = waitPhase(base + Header::full + 8 * st, parity, abortFlag, limit);
                 if (!ok) break;
                 tcFenceAfter();
-                const int rows = unitOf(a, u).rows;
+                const int rows = stripAt(a, s, seg1).rows;
+                s += rows;
                 uint32_t xs = stage0 + (uint32_t)st * a.stageBytes, ds = xs + a.xBytes;
                 for (int r = 0; r < rows; r++) {
-                    const uint64_t dDesc = slabDescriptor<SD>(ds, WIDE ? 2u * SD : a.dSlab);
+                    const uint64_t dDesc = slabDescriptor<SD>(ds, a.dSlab);
                     for (int b = b0; b < b1; b++)
-                        issueRowK<SX, SD, WIDE>(a.px / 16, tmem + (uint32_t)(b - b0) * 3u * cols, cols,
-                                          slabDescriptor<SX>(xs + (uint32_t)(b * (kM / SX)) * a.xSlab, a.xSlab), dDesc, idesc,
-                                          started);
+                        issueRowK<SX, SD>(a.px / 16, tmem + (uint32_t)(b - b0) * 3u * cols, cols,
+                                          slabDescriptor<SX>(xs + (uint32_t)(b * (kM / SX)) * a.xSlab, a.xSlab), dDesc, idesc, started);
                     started = 1u;
                     xs += (uint32_t)a.xSlabs * a.xSlab;
                     ds += (uint32_t)a.dSlabs * a.dSlab;
@@ -266,13 +272,13 @@ __global__ void __launch_bounds__(kThreads) wgradTcKernel(const __grid_constant_
         // ---- epilogue: add the accumulators to dw ----
         const int quarter = warp & 3;
         const bool ok = waitPhaseWarp(base + Header::done, 0u, abortFlag, limit);
-        if (ok && (int)blockIdx.x < a.units) {
+        if (ok && seg0 < seg1) {
             tcFenceAfter();
             for (int b = b0; b < b1; b++) {
                 const int q = b * kM + quarter * 32 + lane;  // (dy, ci) of this thread's accumulator row
                 const int dy = q / a.cin, ci = q % a.cin;
                 for (int dx = 0; dx < 3; dx++) {
-                    float* out = a.dw + ((size_t)(dy * 3 + (WIDE ? 2 - dx : dx)) * a.cin + ci) * a.cout;
+                    float* out = a.dw + ((size_t)(dy * 3 + dx) * a.cin + ci) * a.cout;
                     for (int c = 0; c < a.cout; c += 16) {
                         uint32_t v[16];
                         __syncwarp();  // the load needs converged lanes; the additions below may diverge
@@ -312,28 +318,24 @@ bool makeActivationMap(CUtensorMap* map, const bf16* ptr, int n, int h, int w, i
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int SX, int SD, bool WIDE>
+template <int SX, int SD>
 cudaError_t launch(const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid, uint32_t smemBytes,
                    cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel<SX, SD, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(wgradTcKernel<SX, SD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    wgradTcKernel<SX, SD, WIDE><<<grid, kThreads, smemBytes, stream>>>(xMap, dMap, a);
+    wgradTcKernel<SX, SD><<<grid, kThreads, smemBytes, stream>>>(xMap, dMap, a);
     return cudaGetLastError();
 }
 template <int SX>
 cudaError_t launchD(int sd, const CUtensorMap& xMap, const CUtensorMap& dMap, const WgradArgs& a, dim3 grid,
                     uint32_t smemBytes, cudaStream_t stream) {
-    if (a.dHalo)
-        return sd == 64   ? launch<SX, 64, true>(xMap, dMap, a, grid, smemBytes, stream)
-               : sd == 32 ? launch<SX, 32, true>(xMap, dMap, a, grid, smemBytes, stream)
-                          : launch<SX, 16, true>(xMap, dMap, a, grid, smemBytes, stream);
-    return sd == 64   ? launch<SX, 64, false>(xMap, dMap, a, grid, smemBytes, stream)
-           : sd == 32 ? launch<SX, 32, false>(xMap, dMap, a, grid, smemBytes, stream)
-                      : launch<SX, 16, false>(xMap, dMap, a, grid, smemBytes, stream);
+    return sd == 64   ? launch<SX, 64>(xMap, dMap, a, grid, smemBytes, stream)
+           : sd == 32 ? launch<SX, 32>(xMap, dMap, a, grid, smemBytes, stream)
+                      : launch<SX, 16>(xMap, dMap, a, grid, smemBytes, stream);
 }
 
 }  // namespace
@@ -350,8 +352,6 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
     WgradArgs a{};
     a.h = h; a.w = w; a.cin = cin; a.cout = cout;
     a.xSlabs = cin / sx; a.dSlabs = cout / sd;
-    a.dHalo = a.dSlabs == 1 ? 1 : 0;  // the column taps along N (3 cout <= 192)
-    a.xHalo = 1 - a.dHalo;
     a.mBlocks = (3 * cin + kM - 1) / kM;
     // As many M blocks per grid slice as 512 columns of accumulators hold,
     // evenly over the slices.
@@ -364,58 +364,53 @@ cudaError_t wgradTc(const bf16* x, const bf16* dy, int n, int h, int w, int cin,
     int sms = 0, device = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int most = std::max(1, std::max(1, sms) / slices);
-    // Segment width, rows per stage and blocks per slice, by estimated cycles:
-    // two stages have to fit; a block's units each cost the larger of their
-    // MMAs (about 60 cycles each for N up to 64, 0.85 N above) and loads (20
-    // bytes a cycle) and about 1,200 of latency; and every block adds its
-    // accumulators to dw, about 800 bytes a cycle over all of them, which is what
-    // limits the deep levels (128 -> 128 channels at 8 x 8: 29 MB from 147 blocks).
-    const int n0 = a.dHalo ? 3 * cout : cout;
-    const double mmaCycles = std::max(60.0, 0.85 * n0);
-    const double addCycles = 36.0 * cin * cout / 800.0;
+    // The groups of segments that are summed in one accumulator. A weight's
+    // gradient is rounded as its group sums are, and the first Adam steps carry
+    // such roundings on (an update is close to the gradient's sign), so the
+    // groups follow from the layer and the image sizes alone: two for every
+    // three multiprocessors, fewer where a row tap's input channels pass 128.
+    a.tilesPerRow = (w + kM - 1) / kM;
+    const long long segments = (long long)n * h * a.tilesPerRow;
+    if (segments > 0x7FFFFFFFll) return cudaErrorNotSupported;
+    a.segments = (int)segments;
+    const int most = std::max(1, 2 * std::max(1, sms) / (3 * (cin >= cout ? (cin + kM - 1) / kM : 1)));
+    const int wanted = std::min(a.segments, most);
+    a.perGroup = (a.segments + wanted - 1) / wanted;
+    const int groups = (a.segments + a.perGroup - 1) / a.perGroup;
+    // Rows per stage, by estimated cycles: two stages have to fit; a strip costs
+    // the larger of its MMAs (about 60 cycles each for N up to 64, 0.85 N above)
+    // and its loads (20 bytes a cycle) and about 1,200 of latency.
+    a.px = std::min(kM, (w + 15) / 16 * 16);
+    a.xSlab = slabBytes(a.px + 2, sx);
+    a.dSlab = slabBytes(a.px, sd);
+    // A stage: rows + 2 rows of x, then the dY rows. The last M block may
+    // read past the stacked rows, at most `over` bytes past x's part.
+    const uint32_t over = (uint32_t)(a.mBlocks * (kM / sx) - 3 * a.xSlabs) * a.xSlab;
+    const double mmaCycles = std::max(60.0, 0.85 * cout);
     double bestCost = -1.0;
-    int splits = 1;
-    for (int px = std::min(kM, (w + 15) / 16 * 16), next = 0; px >= 16; px = next) {
-        next = px > 64 ? 64 : px > 32 ? 32 : px > 16 ? 16 : 0;
-        const uint32_t xSlab = slabBytes(px + 2 * a.xHalo, sx), dSlab = slabBytes(px + 2 * a.dHalo, sd);
-        const int tiles = (w + px - 1) / px;
-        // A stage: rows + 2 rows of x, then the dY rows. The last M block may
-        // read past the stacked rows, at most `over` bytes past x's part.
-        const uint32_t over = (uint32_t)(a.mBlocks * (kM / sx) - 3 * a.xSlabs) * xSlab;
-        for (int rows = 1; rows <= std::min(kMaxRows, h); rows++) {
-            const uint32_t xPart = ((uint32_t)((rows + 2) * a.xSlabs) * xSlab + 1023u) & ~1023u;
-            const uint32_t stage = (xPart + std::max(over, (uint32_t)(rows * a.dSlabs) * dSlab) + 1023u) & ~1023u;
-            if (kHeader + 2u * stage > kSmemMax) break;
-            const long long strips = (h + rows - 1) / rows, units = (long long)n * tiles * strips;
-            if (units > 0x7FFFFFFFll) continue;
-            const double mmas = (double)rows * a.blocksPerSlice * (a.dHalo ? 1 : 3) * (px / 16) * mmaCycles;
-            const double loads = ((rows + 2.0) * (px + 2) * cin / slices + (double)rows * px * cout) * 2.0 / 20.0;
-            const double unit = std::max(mmas, loads) + 1200.0;
-            for (int s = most; s >= 1; s = s > 8 ? s * 3 / 4 : s - 1) {
-                const long long per = (units + s - 1) / s;
-                const double cost = (double)per * unit + s * addCycles;
-                if (bestCost >= 0.0 && cost >= bestCost) continue;
-                bestCost = cost;
-                splits = (int)std::min<long long>(s, units);
-                a.px = px; a.rows = rows;
-                a.tilesPerRow = tiles; a.strips = (int)strips; a.units = (int)units;
-                a.xSlab = xSlab; a.dSlab = dSlab;
-                a.xBytes = xPart; a.stageBytes = stage;
-            }
-        }
+    for (int rows = 1; rows <= std::min({kMaxRows, h, a.perGroup, a.tilesPerRow == 1 ? kMaxRows : 1}); rows++) {
+        const uint32_t xPart = ((uint32_t)((rows + 2) * a.xSlabs) * a.xSlab + 1023u) & ~1023u;
+        const uint32_t stage = (xPart + std::max(over, (uint32_t)(rows * a.dSlabs) * a.dSlab) + 1023u) & ~1023u;
+        if (kHeader + 2u * stage > kSmemMax) break;
+        const double mmas = (double)rows * a.blocksPerSlice * 3 * (a.px / 16) * mmaCycles;
+        const double loads = ((rows + 2.0) * (a.px + 2) * cin / slices + (double)rows * a.px * cout) * 2.0 / 20.0;
+        const double cost = ((a.perGroup + rows - 1) / rows) * (std::max(mmas, loads) + 1200.0);
+        if (bestCost >= 0.0 && cost >= bestCost) continue;
+        bestCost = cost;
+        a.rows = rows;
+        a.xBytes = xPart; a.stageBytes = stage;
     }
-    if (bestCost < 0) return cudaErrorNotSupported;
+    if (bestCost < 0.0) return cudaErrorNotSupported;
     a.stages = 2;
     while (a.stages < kMaxStages && kHeader + (uint32_t)(a.stages + 1) * a.stageBytes <= kSmemMax) a.stages++;
     a.dw = dw;
     a.errorFlag = errorFlag;
     a.waitLimitNs = 1000000000ull;
     CUtensorMap xMap{}, dMap{};
-    if (!makeActivationMap(&xMap, x, n, h, w, cin, sx, (uint32_t)(a.px + 2 * a.xHalo)) ||
-        !makeActivationMap(&dMap, dy, n, h, w, cout, sd, (uint32_t)(a.px + 2 * a.dHalo)))
+    if (!makeActivationMap(&xMap, x, n, h, w, cin, sx, (uint32_t)(a.px + 2)) ||
+        !makeActivationMap(&dMap, dy, n, h, w, cout, sd, (uint32_t)a.px))
         return cudaErrorNotSupported;
-    const dim3 grid((unsigned)splits, (unsigned)slices);
+    const dim3 grid((unsigned)groups, (unsigned)slices);
     const uint32_t smemBytes = kHeader + (uint32_t)a.stages * a.stageBytes;
     return sx == 64   ? launchD<64>(sd, xMap, dMap, a, grid, smemBytes, stream)
            : sx == 32 ? launchD<32>(sd, xMap, dMap, a, grid, smemBytes, stream)

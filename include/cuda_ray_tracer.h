@@ -271,6 +271,9 @@ int RtxSetEnvironment(void* session, int mode, float r, float g, float b);
  *   RtxUnetLossGrad   one forward/backward over n crops (h, w multiples of 16):
  *                     L1 loss on log(1 + radiance) and its gradient
  *   RtxUnetTrain      Adam steps over random batches (with flips) of a data set
+ *                     (gradients are summed with atomics: two runs agree to
+ *                     FP32 summation order, not to the bit, and parameters
+ *                     whose gradient is near zero may end two steps apart)
  *   RtxUnetInfer      host-to-host inference for any h, w
  *   RtxUnetSave / RtxUnetLoad  checkpoint: parameters, and the Adam state
  *                     when optimizerState is non-zero

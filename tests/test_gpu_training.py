@@ -1,0 +1,85 @@
+"""Training (RtxUnetLossGrad, RtxUnetTrain) beyond one layer's tolerance: which
+sums are taken together. Needs a GPU.
+
+A network of unit weights makes every product exact: channel 0 of the input's
+albedo passes unchanged through layers 0, 1, 16 and 17, channel 1 drives the
+prediction, and the gradient at layer 17's pre-activation is +1 or -1 as the
+target lies below or above it. The weight gradient between the two channels is
+then a sum of chosen numbers over the pixels."""
+import numpy as np
+import pytest
+import torch
+
+from native_api import Unet
+from test_gpu_unet import layer_table
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def net(lib):
+    n = Unet(lib, seed=3)
+    yield n
+    n.close()
+
+
+def offsets():
+    """Flat offset of each 3x3 layer's weights, then the output layer's."""
+    out, at = [], 0
+    for ci, co in layer_table():
+        out.append(at)
+        at += 9 * ci * co + co
+    return out + [at]
+
+
+CENTRE = 4  # tap (0, 0)
+
+
+def unit_network(net, pixels):
+    """Sets the parameters described above for a batch of `pixels` pixels."""
+    table, at = layer_table(), offsets()
+    flat = np.zeros(net.param_count, np.float32)
+    for layer, first in ((0, 3), (1, 0), (16, 48), (17, 0)):  # albedo is input channels 3-5; layer 16 reads [up 48, skip 32]
+        ci, co = table[layer]
+        for c in range(2):
+            flat[at[layer] + (CENTRE * ci + first + c) * co + c] = 1.0
+    # The gradient at the prediction is +-1 / (3 pixels): a weight of 3 pixels
+    # makes it +-1 below, and the bias brings the prediction back to 1.
+    assert 3 * pixels < 1 << 24
+    flat[at[18] + 1 * 3 + 0] = 3 * pixels
+    flat[at[18] + 96 + 0] = 1 - 3 * pixels
+    net.set_params(flat)
+
+
+def weight_between(net, values, sign):
+    """The gradient of layer 17's centre weight from channel 0 to 1: the sum of
+    values * sign over the pixels, as the kernel adds it."""
+    n, h, w = values.shape
+    unit_network(net, values.size)
+    aovs = np.zeros((n, h, w, 10), np.float32)
+    aovs[..., 3], aovs[..., 4] = values, 1.0
+    target = np.zeros((n, h, w, 3), np.float32)
+    target[..., 0] = np.where(sign > 0, 0.0, 1e30)
+    _, grads = net.loss_grad(aovs, target)
+    return float(grads[offsets()[17] + (CENTRE * 32 + 0) * 32 + 1])
+
+
+@pytest.mark.parametrize('n,h,w', ((4, 128, 128), (32, 32, 32), (3, 80, 112), (2, 16, 16)))
+def test_weight_gradient_groups(net, n, h, w):
+    """A weight gradient's pixels are summed in groups of whole image rows in
+    order, as many rows each as make two groups for three multiprocessors.
+    Training from fresh Adam moments carries the rounding of these sums on, so
+    they are part of its result. A number that swallows every 1 added between
+    it and its negative shows which rows share a sum."""
+    rows = n * h
+    groups = min(rows, 2 * torch.cuda.get_device_properties(0).multi_processor_count // 3)
+    per = -(-rows // groups)
+    groups = -(-rows // per)
+    for g in sorted({0, groups // 2, groups - 1}):
+        first, last = g * per, min(rows, (g + 1) * per) - 1
+        values = np.ones((rows, w), np.float32)
+        sign = np.ones((rows, w), np.float32)
+        values[first, 0] = values[last, w - 1] = 2.0 ** 40
+        sign[last, w - 1] = -1.0
+        got = weight_between(net, values.reshape(n, h, w), sign.reshape(n, h, w))
+        assert got == (rows - (last - first + 1)) * w, (g, got)

@@ -518,14 +518,16 @@ __global__ void __launch_bounds__(128) splitKernel(const int* order, const float
             sweep(box, count, axis, cut);
             sweep(lastBox, lastCount, 2, kBins - 2);
         }
-        auto candidateCost = [&](const float (&b)[2][6], const int (&n)[2], bool axisValid) {
-            if (!axisValid || !n[0] || !n[1]) return FLT_MAX;
-            return nodeArea + halfArea(b[0], b[0] + 3) * n[0] + halfArea(b[1], b[1] + 3) * n[1];
+        // Costs are sums of areas, not negative: their bits order like them. A
+        // candidate that is out (no extent, an empty side, not below the leaf's
+        // cost) is above every cost, infinite ones among them.
+        auto candidateBits = [&](const float (&b)[2][6], const int (&n)[2], bool axisValid) {
+            if (!axisValid || !n[0] || !n[1]) return full;
+            const float cost = nodeArea + halfArea(b[0], b[0] + 3) * n[0] + halfArea(b[1], b[1] + 3) * n[1];
+            return cost < unsplit ? __float_as_uint(cost) : full;
         };
-        const float last = candidateCost(lastBox, lastCount, valid[2]);
-        const float cost = candidateCost(box, count, axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]);
-        // Costs are sums of areas, not negative: their bits order like them.
-        const unsigned bits = cost < unsplit ? __float_as_uint(cost) : full;
+        const unsigned last = candidateBits(lastBox, lastCount, valid[2]);
+        const unsigned bits = candidateBits(box, count, axis == 0 ? valid[0] : axis == 1 ? valid[1] : valid[2]);
         const unsigned best = __reduce_min_sync(full, bits);
         int bestAxis = -1, bestBin = -1, winner = -1;
         if (best != full) {
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(128) splitKernel(const int* order, const float
             bestAxis = winner / 11;
             bestBin = winner % 11;
         }
-        if (last < unsplit && __float_as_uint(last) < best) { bestAxis = 2; bestBin = kBins - 2; winner = -1; }
+        if (last < best) { bestAxis = 2; bestBin = kBins - 2; winner = -1; }
         if (bestAxis < 0) {
             if (lane == 0) {
                 nodes[T.node] = BinNode{v3(T.lo[0], T.lo[1], T.lo[2]), T.first, v3(T.hi[0], T.hi[1], T.hi[2]), T.count};

@@ -63,6 +63,25 @@ def test_build_sizes(session, oracle, sphere, n):
     assert session.query(q).tobytes() == oracle.query(scene, q, False)[0].tobytes()
 
 
+@pytest.mark.parametrize('far', (1e25, np.inf))
+@pytest.mark.parametrize('n', (20, 40, 600, 3000))
+def test_build_with_unbounded_boxes(session, oracle, sphere, n, far):
+    """A vertex so far out that a box's area is infinite: no split is cheaper
+    than the leaf, in the subtree, search and binned forms alike, so the nodes
+    are the reference's. Nothing is asked of rays through an infinite box."""
+    tris = some_triangles(sphere, n).copy()
+    for axis in 'xyz':
+        tris['origin'][axis][n // 2] = far
+    scene = oracle.scene(tris)
+    session.initialize(tris, 8, 8)
+    nodes, order = session.export_bvh(n)
+    assert nodes.tobytes() == scene.nodes().tobytes()
+    assert _leaf_sets(nodes, order) == _leaf_sets(scene.nodes(), scene.order())
+    if np.isfinite(far):
+        q = rays(257)
+        assert session.query(q).tobytes() == oracle.query(scene, q, False)[0].tobytes()
+
+
 @pytest.mark.parametrize('offset', (-1, 0, 1))
 def test_query_counts(session, oracle, sphere, offset):
     """Around a warp, a block and the count from which queries run as blocks

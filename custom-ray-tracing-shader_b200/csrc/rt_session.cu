@@ -757,7 +757,8 @@ int RtxSetIntegrator(void* p, int mode) {
 
 void* RtxUnetCreate(unsigned seed) {
     UnetHandle* h = new UnetHandle(seed);
-    if (cudaGetLastError() != cudaSuccess) { delete h; return nullptr; }
+    const bool failed = cudaGetLastError() != cudaSuccess;
+    if (failed || h->net.status() != cudaSuccess) { delete h; return nullptr; }
     return h;
 }
 void RtxUnetDestroy(void* p) { delete static_cast<UnetHandle*>(p); }

@@ -613,25 +613,27 @@ Unet::Unet(unsigned seed) {
             host[L.wOffset + i] = v;
         }
     }
-    rt::deviceAlloc(&master_, sizeof(float) * params_);
-    rt::deviceAlloc(&grad_, sizeof(float) * params_);
-    rt::deviceAlloc(&adamM_, sizeof(float) * params_);
-    rt::deviceAlloc(&adamV_, sizeof(float) * params_);
-    rt::deviceAlloc(&wbf_, sizeof(bf16) * params_);
-    rt::deviceAlloc(&wT_, sizeof(bf16) * params_);
-    rt::deviceAlloc(&convError_, sizeof(int));
     // Every copy and fill goes through stream_: it is non-blocking, so it is
-    // not ordered after work on the legacy default stream.
-    cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
-    cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking);
-    cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&join_, cudaEventDisableTiming);
-    cudaMemsetAsync(convError_, 0, sizeof(int), stream_);
-    cudaMemcpyAsync(master_, host.data(), sizeof(float) * params_, cudaMemcpyHostToDevice, stream_);
-    cudaMemsetAsync(adamM_, 0, sizeof(float) * params_, stream_);
-    cudaMemsetAsync(adamV_, 0, sizeof(float) * params_, stream_);
-    syncWeights(stream_);
-    cudaStreamSynchronize(stream_);
+    // not ordered after work on the legacy default stream. Nothing is launched
+    // once a step has failed.
+    auto attempt = [&](auto step) { if (status_ == cudaSuccess) status_ = step(); };
+    attempt([&] { return rt::deviceAlloc(&master_, sizeof(float) * params_); });
+    attempt([&] { return rt::deviceAlloc(&grad_, sizeof(float) * params_); });
+    attempt([&] { return rt::deviceAlloc(&adamM_, sizeof(float) * params_); });
+    attempt([&] { return rt::deviceAlloc(&adamV_, sizeof(float) * params_); });
+    attempt([&] { return rt::deviceAlloc(&wbf_, sizeof(bf16) * params_); });
+    attempt([&] { return rt::deviceAlloc(&wT_, sizeof(bf16) * params_); });
+    attempt([&] { return rt::deviceAlloc(&convError_, sizeof(int)); });
+    attempt([&] { return cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking); });
+    attempt([&] { return cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking); });
+    attempt([&] { return cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming); });
+    attempt([&] { return cudaEventCreateWithFlags(&join_, cudaEventDisableTiming); });
+    attempt([&] { return cudaMemsetAsync(convError_, 0, sizeof(int), stream_); });
+    attempt([&] { return cudaMemcpyAsync(master_, host.data(), sizeof(float) * params_, cudaMemcpyHostToDevice, stream_); });
+    attempt([&] { return cudaMemsetAsync(adamM_, 0, sizeof(float) * params_, stream_); });
+    attempt([&] { return cudaMemsetAsync(adamV_, 0, sizeof(float) * params_, stream_); });
+    attempt([&] { return syncWeights(stream_); });
+    attempt([&] { return cudaStreamSynchronize(stream_); });
 }
 
 Unet::~Unet() {

@@ -31,6 +31,8 @@ public:
     Unet(const Unet&) = delete;
     Unet& operator=(const Unet&) = delete;
 
+    // Whether the network was made: the error of the first step that failed.
+    cudaError_t status() const { return status_; }
     size_t paramCount() const { return params_; }
     // Host copies of the FP32 master parameters, in the flat layout (per 3x3
     // layer: weights [tap][cin][cout] then bias [cout]; the 1x1 output layer:
@@ -77,6 +79,7 @@ private:
                                 cudaStream_t stream);
     cudaError_t syncWeights(cudaStream_t stream);
 
+    cudaError_t status_ = cudaSuccess;
     std::vector<UnetLayer> layers_;
     size_t params_ = 0;
     float* master_ = nullptr;     // FP32 parameters

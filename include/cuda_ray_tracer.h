@@ -247,8 +247,8 @@ int RtxConvLaunchCounts(long long* pipelined, long long* singleRole);
 int RtxDebugConvWaitProbe(void);
 
 /* Failure injection on the host, no counterpart in the reference: the n-th
- * next device allocation made by the renderer (sessions, scene upload, BVH
- * build, wave buffers, batches) fails with cudaErrorMemoryAllocation without
+ * next device allocation made by the library (sessions, scene upload, BVH
+ * build, wave buffers, batches, networks) fails with cudaErrorMemoryAllocation without
  * calling cudaMalloc, as if the device were out of memory; n = 0 disarms it.
  * Process-wide; for testing the error paths (each must return 0, report the
  * error through RtLastError and leave the session usable). Returns 0 for
@@ -266,7 +266,8 @@ int RtxSetEnvironment(void* session, int mode, float r, float g, float b);
  * 32-48-64-96-128, about 1.01M parameters) on BF16 tensor cores with FP32
  * accumulation. Input per pixel: the 10 floats RtxReadAovs returns; output:
  * linear radiance RGB. Returns 1 on success, 0 on failure (RtxUnetLastError).
- *   RtxUnetCreate     new network, He-normal initialisation from seed
+ *   RtxUnetCreate     new network, He-normal initialisation from seed; NULL
+ *                     when it could not be made (no device memory)
  *   RtxUnetGetParams / RtxUnetSetParams  FP32 parameters, RtxUnetParamCount floats
  *   RtxUnetLossGrad   one forward/backward over n crops (h, w multiples of 16):
  *                     L1 loss on log(1 + radiance) and its gradient

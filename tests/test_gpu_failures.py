@@ -238,3 +238,26 @@ def test_invalid_arguments_rejected(lib, session):
     lib.RtShutdown(session.handle)
     assert not lib.RtRender(session.handle, c.byref(cam), c.byref(st), po, out.size, 2, c.byref(ms))
     assert b'not initialised' in lib.RtLastError(session.handle)
+
+
+def test_out_of_memory_every_allocation_of_a_network(lib):
+    """RtxUnetCreate with each of its allocations failing in turn returns NULL
+    and launches nothing; the network made after that is the usual one."""
+    made = []
+
+    def create():
+        handle = lib.RtxUnetCreate(7)
+        if handle:
+            made.append(handle)
+        return bool(handle)
+    count = _count_allocations(lib, create)
+    assert count >= 7 and len(made) == 1  # parameters, gradient, two moments, two BF16 copies, the error flag
+    expect = lib.RtxUnetCreate(7)
+    try:
+        n = lib.RtxUnetParamCount(expect)
+        a, b = np.zeros(n, np.float32), np.zeros(n, np.float32)
+        assert lib.RtxUnetGetParams(made[0], a.ctypes.data) and lib.RtxUnetGetParams(expect, b.ctypes.data)
+        assert np.array_equal(a, b) and np.abs(a).max() > 0
+    finally:
+        lib.RtxUnetDestroy(expect)
+        lib.RtxUnetDestroy(made[0])

@@ -697,8 +697,18 @@ cudaError_t Unet::ensure(int n, int h, int w, bool training) {
     if (act_ && act_->n == n && act_->H == H && act_->W == W && (act_->training || !training)) return cudaSuccess;
     delete act_;
     act_ = new Activations();
-    Activations& A = *act_;
-    A.n = n; A.H = H; A.W = W; A.training = training;
+    act_->n = n; act_->H = H; act_->W = W; act_->training = training;
+    const cudaError_t e = allocate(*act_);
+    if (e != cudaSuccess) {  // nothing half made is found by the next call of this size
+        delete act_;
+        act_ = nullptr;
+    }
+    return e;
+}
+
+cudaError_t Unet::allocate(Activations& A) const {
+    const int n = A.n, H = A.H, W = A.W;
+    const bool training = A.training;
     cudaError_t e = cudaSuccess;
     auto px = [&](int level) { return (size_t)n * (H >> level) * (W >> level); };
     if ((e = A.make(A.x0, px(0) * kInputPadded)) != cudaSuccess) return e;

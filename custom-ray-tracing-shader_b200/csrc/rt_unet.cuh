@@ -68,6 +68,7 @@ public:
 private:
     struct Activations;
     cudaError_t ensure(int n, int h, int w, bool training);
+    cudaError_t allocate(Activations& A) const;
     // head (inference): the output head to fuse into the last convolution;
     // *headDone tells whether it was (else A.a[17] holds that layer's output).
     cudaError_t forward(cudaStream_t stream, bool training, bool outputLayer = true, const ConvHead* head = nullptr,

@@ -261,3 +261,45 @@ def test_out_of_memory_every_allocation_of_a_network(lib):
     finally:
         lib.RtxUnetDestroy(expect)
         lib.RtxUnetDestroy(made[0])
+
+
+@pytest.mark.parametrize('what', ('grad', 'train', 'infer'))
+def test_out_of_memory_in_network_calls(lib, what):
+    """Every allocation of a network's call failing in turn: 0 with a message
+    each time, and the same call at the same size then gives what a network
+    that never failed gives (gradients to the order of their sums)."""
+    from native_api import Unet
+    from test_gpu_unet import synthetic
+    aovs, target = synthetic(np.random.default_rng(8), 2, 32, 48)
+    loss, grads, out = np.zeros(1, np.float32), np.zeros(1_017_379, np.float32), np.zeros((32, 48, 3), np.float32)
+    losses = np.zeros(2, np.float32)
+    ptr = [a.ctypes.data for a in (aovs, target)]
+    calls = {
+        'grad': lambda h: lib.RtxUnetLossGrad(h, *ptr, 2, 32, 48, loss.ctypes.data, grads.ctypes.data),
+        'train': lambda h: lib.RtxUnetTrain(h, *ptr, 2, 32, 48, 2, 2, 1e-4, 1, losses.ctypes.data),
+        'infer': lambda h: lib.RtxUnetInfer(h, aovs[0].ctypes.data, 32, 48, out.ctypes.data),
+    }
+    nets = [Unet(lib, seed=5), Unet(lib, seed=5)]
+    try:
+        messages = []
+
+        def call():
+            ok = calls[what](nets[0].handle)
+            if not ok:
+                messages.append(lib.RtxUnetLastError(nets[0].handle).decode())
+            return ok
+        count = _count_allocations(lib, call)
+        assert count >= 20 and len(messages) == count and all('memory' in m for m in messages)
+        got = loss[0], grads.copy(), losses.copy(), out.copy(), nets[0].params()
+        assert calls[what](nets[1].handle)
+        if what == 'infer':
+            assert np.array_equal(got[3], out) and out.max() > 0
+        elif what == 'grad':
+            assert abs(got[0] - loss[0]) <= 1e-5 * loss[0]
+            assert np.linalg.norm(got[1] - grads) <= 1e-5 * np.linalg.norm(grads) > 0
+        else:
+            assert np.abs(got[2] - losses).max() <= 1e-4 * losses.max()
+            assert np.abs(got[4] - nets[1].params()).max() <= 4.1e-4  # two steps of 1e-4 either way
+    finally:
+        for n in nets:
+            n.close()

@@ -799,10 +799,12 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
         const bf16* skip = A.a[2 * level + 1];
         for (int r = 0; r < 2; r++, k++) {
             const UnetLayer& L = layers_[k];
-            if (r == 0 && (training || (A.cat[j] && convPath() == 0))) {
+            if (r == 0 && (training || (!A.upWeights[j] && A.cat[j] && convPath() == 0))) {
                 // The weight gradient reads the concatenated input; at inference
                 // the streamed convolution does (8 + 21 us against 74 for the
-                // single-role kernel reading its halves in place, 240 x 136).
+                // single-role kernel reading its halves in place, 240 x 136),
+                // and no other: buffers left by a training call of this size
+                // hold a concatenation for every level.
                 upConcatKernel<<<blocksFor((long long)n * H * W * ((Cl + Cs) / 8), 256), 256, 0, s>>>(low, Cl, skip, Cs, n, H, W, A.cat[j]);
                 e = convTc(A.cat[j], nullptr, 0, n, H, W, L.cin, wT_ + L.wOffset, false, master_ + L.bOffset, L.cout, A.a[k], nullptr, true, false, convError_, s);
             } else if (r == 0 && A.upWeights[j] && combine) {

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 from native_api import Unet
-from test_gpu_unet import layer_table
+from test_gpu_unet import layer_table, synthetic
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +83,18 @@ def test_weight_gradient_groups(net, n, h, w):
         sign[last, w - 1] = -1.0
         got = weight_between(net, values.reshape(n, h, w), sign.reshape(n, h, w))
         assert got == (rows - (last - first + 1)) * w, (g, got)
+
+
+@pytest.mark.parametrize('h,w', ((64, 96), (37, 23)))
+def test_inference_after_training_is_the_same(lib, h, w):
+    """A gradient of one image leaves buffers that inference of the same padded
+    size uses: its result is a fresh network's, byte for byte."""
+    aovs, target = synthetic(np.random.default_rng(h), 1, -(-h // 16) * 16, -(-w // 16) * 16)
+    nets = [Unet(lib, seed=5), Unet(lib, seed=5)]
+    try:
+        nets[0].loss_grad(aovs, target)
+        got, expect = (n.infer(np.ascontiguousarray(aovs[0, :h, :w])) for n in nets)
+        assert np.array_equal(got, expect) and expect.max() > 0
+    finally:
+        for n in nets:
+            n.close()

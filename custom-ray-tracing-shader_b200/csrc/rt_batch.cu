@@ -421,7 +421,15 @@ void dropGraph(Batch* b) {
     b->graphValid = false;
 }
 
+// Nothing of the batch is left in flight after this.
+void settleBatch(Batch* b) {
+    for (cudaStream_t lane : b->laneStreams)
+        if (lane) settle(lane);
+    if (b->stream) settle(b->stream);
+}
+
 void freeArena(Batch* b) {
+    settleBatch(b);
     void* owned[] = {b->aTris, b->aShade, b->aWide, b->aPacked, b->aLights, b->dScenes};
     for (void* p : owned)
         if (p) rt::deviceFree(p);
@@ -431,6 +439,7 @@ void freeArena(Batch* b) {
 }
 
 void freeViews(Batch* b) {
+    settleBatch(b);
     void* owned[] = {b->dViews, b->dSum, b->dDepth, b->dPixels, b->dTiles};
     for (void* p : owned)
         if (p) rt::deviceFree(p);
@@ -587,6 +596,7 @@ int waveCapacity(const Batch* b, int raysPerPixel) {
 }
 
 void freeLanes(Batch* b) {
+    settleBatch(b);
     for (int k = 0; k < kMaxLanes - 1; k++) {
         freeWavefront(b->laneWaves[k]);
         if (b->laneStreams[k]) cudaStreamDestroy(b->laneStreams[k]);
@@ -604,6 +614,7 @@ bool ensureWave(Batch* b, int raysPerPixel) {
     const int cap = waveCapacity(b, raysPerPixel);
     cudaError_t e;
     if (b->wave.capacity != cap) {
+        settleBatch(b);
         dropGraph(b);
         if ((e = allocWavefront(b->wave, cap)) != cudaSuccess) return failB(b, e, "wavefront buffers");
     }
@@ -616,6 +627,7 @@ bool ensureWave(Batch* b, int raysPerPixel) {
     }
     for (int k = 0; k < b->lanes - 1; k++) {
         if (b->laneWaves[k].capacity != cap) {
+            settleBatch(b);
             dropGraph(b);
             if ((e = allocWavefront(b->laneWaves[k], cap)) != cudaSuccess) { freeLanes(b); return failB(b, e, "wavefront buffers"); }
         }
@@ -796,6 +808,7 @@ void RtxBatchDestroy(void* p) {
     Batch* b = static_cast<Batch*>(p);
     if (!b) return;
     if (b->device >= 0) (void)cudaSetDevice(b->device);  // freeing goes on regardless
+    settleBatch(b);
     freeArena(b);
     freeViews(b);
     freeWavefront(b->wave);

@@ -1314,6 +1314,7 @@ cudaError_t pieceMap(const SceneTri* tris, int triCount, int maxPieces, cudaStre
     if (err == cudaSuccess && ms) err = cudaEventElapsedTime(ms, t0, t1);
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
+    if (err != cudaSuccess) settle(stream);
     rt::deviceFree(counts); rt::deviceFree(pfx); rt::deviceFree(sums); rt::deviceFree(dTotal);
     if (err == cudaSuccess && (hostTotal < triCount || hostTotal > triCount * maxPieces)) err = cudaErrorUnknown;
     if (err != cudaSuccess) { rt::deviceFree(map); return err; }
@@ -1549,6 +1550,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
     }
 done:
 #undef RT_TRY
+    if (err != cudaSuccess) settle(stream);
     rt::deviceFree(cent); rt::deviceFree(orderB); rt::deviceFree(posTask); rt::deviceFree(posTaskB); rt::deviceFree(tasks); rt::deviceFree(tasksB); rt::deviceFree(subtrees);
     rt::deviceFree(done);
     rt::deviceFree(bins); rt::deviceFree(splits); rt::deviceFree(flags); rt::deviceFree(prefix); rt::deviceFree(blockSums); rt::deviceFree(counters);

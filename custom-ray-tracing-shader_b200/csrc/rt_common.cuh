@@ -24,11 +24,12 @@ constexpr float kPi = 3.14159265358979323846f;
 // ---- device allocation ----
 // The library's device allocations go through deviceAlloc and deviceFree
 // (rt_memory.cu). Freed blocks are kept, up to a bound per device, for later
-// allocations of about their size, and handed out again only after a device
-// synchronisation that follows the free, so any stream may use them (freeing
-// waits for the device with cudaFree as well). The cache is given back when
-// the last DeviceMemoryUser (session, batch, network) goes, at RtShutdown, and
-// when the device runs out of memory. Safe with several threads and devices.
+// allocations of about their size on any stream: deviceFree is called when no
+// work uses the block any more. The owner's calls end with its streams drained;
+// where one may have ended early (an error) it settles them first. The cache is
+// given back when the last DeviceMemoryUser (session, batch, network) goes, at
+// RtShutdown, and when the device runs out of memory. Safe with several threads
+// and devices, and beside another thread's stream capture.
 // setFailAllocation makes the n-th next allocation fail on the host, as an
 // out-of-memory cudaMalloc would, without touching the GPU
 // (RtxDebugFailAllocation).
@@ -38,6 +39,8 @@ inline cudaError_t deviceAlloc(T** p, size_t bytes) {
     return deviceAllocBytes(reinterpret_cast<void**>(p), bytes);
 }
 void deviceFree(void* p);
+// Waits for a stream's work before blocks that it may use are freed.
+inline void settle(cudaStream_t stream) { (void)cudaStreamSynchronize(stream); }
 void trimDeviceMemory();
 void setFailAllocation(int n);
 struct DeviceMemoryUser {

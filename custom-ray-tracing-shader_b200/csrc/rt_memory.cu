@@ -3,7 +3,10 @@
 //
 // A scene load makes about 70 allocations and frees, a ray query or gradient
 // call a handful; each cudaMalloc, cudaFree or cudaMallocHost costs 10 us to
-// several hundred and cudaFree waits for the device every time. Measured:
+// several hundred and cudaFree waits for the device every time. No work uses a
+// block that is freed here (deviceFree), so handing it out again waits for
+// nothing: waiting for the whole device would also fail, and break the capture,
+// while another thread records a CUDA graph. Measured:
 // loading 8,000 triangles took 20 ms of which the kernels 2, the million-
 // triangle scene 54 ms of which upload and kernels 21.
 #include <cuda_runtime.h>
@@ -25,9 +28,8 @@ constexpr size_t kCacheBytes = 4ull << 30;
 
 struct Block { void* p; size_t bytes; };
 struct DeviceCache {
-    std::list<Block> ready;    // oldest first; no GPU work uses them
-    std::list<Block> pending;  // freed since the last device synchronisation
-    size_t bytes = 0;          // of both
+    std::list<Block> ready;  // oldest first
+    size_t bytes = 0;
 };
 struct Owned { int device; size_t bytes; };
 
@@ -46,14 +48,13 @@ size_t stepped(size_t bytes) {
     return (bytes + step - 1) / step * step;
 }
 
-// With g_lock held. cudaFree waits for the work that uses the block.
+// With g_lock held.
 void evict(DeviceCache& c, size_t keep) {
-    for (std::list<Block>* l : {&c.ready, &c.pending})
-        while (c.bytes > keep && !l->empty()) {
-            cudaFree(l->front().p);
-            c.bytes -= l->front().bytes;
-            l->pop_front();
-        }
+    while (c.bytes > keep && !c.ready.empty()) {
+        cudaFree(c.ready.front().p);
+        c.bytes -= c.ready.front().bytes;
+        c.ready.pop_front();
+    }
 }
 
 }  // namespace
@@ -74,25 +75,14 @@ cudaError_t deviceAllocBytes(void** p, size_t bytes) {
     DeviceCache& c = caches()[device];
     // The smallest block that fits without wasting more than a quarter.
     auto fits = [&](const Block& b) { return b.bytes >= want && b.bytes - want <= (want / 4 > 65536 ? want / 4 : 65536); };
-    auto find = [&](std::list<Block>& l) {
-        auto best = l.end();
-        for (auto it = l.begin(); it != l.end(); ++it)
-            if (fits(*it) && (best == l.end() || it->bytes < best->bytes)) best = it;
-        return best;
-    };
-    auto it = find(c.ready);
-    if (it == c.ready.end() && find(c.pending) != c.pending.end()) {
-        // As cudaFree would have done at the free: wait for all work on the
-        // device, then every pending block is free to use on any stream.
-        if ((e = cudaDeviceSynchronize()) != cudaSuccess) return e;
-        c.ready.splice(c.ready.end(), c.pending);
-        it = find(c.ready);
-    }
-    if (it != c.ready.end()) {
-        *p = it->p;
-        owned()[it->p] = Owned{device, it->bytes};
-        c.bytes -= it->bytes;
-        c.ready.erase(it);
+    auto best = c.ready.end();
+    for (auto it = c.ready.begin(); it != c.ready.end(); ++it)
+        if (fits(*it) && (best == c.ready.end() || it->bytes < best->bytes)) best = it;
+    if (best != c.ready.end()) {
+        *p = best->p;
+        owned()[best->p] = Owned{device, best->bytes};
+        c.bytes -= best->bytes;
+        c.ready.erase(best);
         return cudaSuccess;
     }
     e = cudaMalloc(p, want);
@@ -115,7 +105,7 @@ void deviceFree(void* p) {
     owned().erase(it);
     if (g_users == 0 || o.bytes > kCacheBytes) { cudaFree(p); return; }
     DeviceCache& c = caches()[o.device];
-    c.pending.push_back(Block{p, o.bytes});
+    c.ready.push_back(Block{p, o.bytes});
     c.bytes += o.bytes;
     evict(c, kCacheBytes);
 }

@@ -165,8 +165,17 @@ const uint4* travWide(const Session* s) { return s->pieceBvh.wideNodes ? s->piec
 const float4* travPacked(const Session* s) { return s->pieceBvh.wideNodes ? s->pieceBvh.packedTris : s->bvh.packedTris; }
 const BuildResult& travBuild(const Session* s) { return s->pieceBvh.wideNodes ? s->pieceBuild : s->build; }
 
+// Nothing of the session is left in flight after this.
+void settleSession(Session* s) {
+    if (!s->stream) return;
+    for (cudaStream_t lane : s->overlap.streams)
+        if (lane) settle(lane);
+    settle(s->stream);
+}
+
 void releaseOverlap(Session* s) {
     WaveOverlap& o = s->overlap;
+    settleSession(s);
     for (int k = 0; k < kMaxLanes - 1; k++) {
         freeWavefront(s->laneWaves[k]);
         if (o.streams[k]) cudaStreamDestroy(o.streams[k]);
@@ -178,6 +187,7 @@ void releaseOverlap(Session* s) {
 }
 
 void releaseScene(Session* s) {
+    settleSession(s);
     freeBvh(s->bvh);
     freeBvh(s->pieceBvh);
     s->pieceBuild = BuildResult{};
@@ -242,6 +252,7 @@ bool ensureWave(Session* s, int raysPerPixel) {
     const int limit = (int)std::min<long long>(setting, pixels * 16);
     const int cap = (s->wave.capacity >= need && s->wave.capacity <= limit) ? s->wave.capacity : need;
     cudaError_t e;
+    if (s->wave.capacity != cap) settleSession(s);
     if (s->wave.capacity != cap && (e = allocWavefront(s->wave, cap)) != cudaSuccess)
         return fail(s, e, "could not allocate wavefront buffers");
     const int lanes = s->tuning.lanes;
@@ -254,6 +265,7 @@ bool ensureWave(Session* s, int raysPerPixel) {
         return fail(s, e, "could not create the wave lane events");
     }
     for (int k = 0; k < lanes - 1; k++) {
+        if (s->laneWaves[k].capacity != cap) settleSession(s);
         if ((s->laneWaves[k].capacity != cap && (e = allocWavefront(s->laneWaves[k], cap)) != cudaSuccess) ||
             (!o.streams[k] && (e = cudaStreamCreateWithFlags(&o.streams[k], cudaStreamNonBlocking)) != cudaSuccess) ||
             (!o.joins[k] && (e = cudaEventCreateWithFlags(&o.joins[k], cudaEventDisableTiming)) != cudaSuccess)) {
@@ -566,30 +578,37 @@ int RtDenoise(void* p, unsigned char* output, int outputBytes, float* millisecon
     s->hostError.clear();
     size_t count = (size_t)s->width * s->height;
     cudaError_t e;
-    if (!s->dDenoise && (e = rt::deviceAlloc(&s->dDenoise, sizeof(float4) * 4 * count)) != cudaSuccess) { fail(s, e); return 0; }
+    // The network's buffers belong to the network: nothing of a call that fails
+    // stays in flight over them.
+    auto abandon = [&](cudaError_t error, const char* what = nullptr) {
+        settle(s->stream);
+        fail(s, error, what);
+        return 0;
+    };
+    if (!s->dDenoise && (e = rt::deviceAlloc(&s->dDenoise, sizeof(float4) * 4 * count)) != cudaSuccess) return abandon(e);
     if (s->lastBackend != 2) {
-        if ((e = cudaMemcpyAsync(s->dSum, s->hostSum.data(), count * sizeof(Accum), cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+        if ((e = cudaMemcpyAsync(s->dSum, s->hostSum.data(), count * sizeof(Accum), cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) return abandon(e);
     }
     if (s->lastBackend != 2 && s->hostDepth.size() == count) {
-        if ((e = cudaMemcpyAsync(s->dDepth, s->hostDepth.data(), count * sizeof(float), cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+        if ((e = cudaMemcpyAsync(s->dDepth, s->hostDepth.data(), count * sizeof(float), cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) return abandon(e);
     }
-    if ((e = cudaEventRecord(s->start, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+    if ((e = cudaEventRecord(s->start, s->stream)) != cudaSuccess) return abandon(e);
     if (s->denoiser) {
         // Learned denoiser: running sums -> U-Net (AOVs formed in its input
         // kernel, as RtxReadAovs forms them) -> display, on the session stream.
         float* radiance = reinterpret_cast<float*>(s->dDenoise) + 10 * count;
         unsigned char* coverage = reinterpret_cast<unsigned char*>(radiance + 3 * count);
         if ((e = s->denoiser->net.inferFromSums(reinterpret_cast<const float*>(s->dSum), s->dDepth, s->samples,
-                                                s->height, s->width, radiance, coverage, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
-        if ((e = launchPresentRadiance(coverage, radiance, (int)count, s->lastSettings.exposure, s->dPixels, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+                                                s->height, s->width, radiance, coverage, s->stream)) != cudaSuccess) return abandon(e);
+        if ((e = launchPresentRadiance(coverage, radiance, (int)count, s->lastSettings.exposure, s->dPixels, s->stream)) != cudaSuccess) return abandon(e);
         s->denoisedOffset = 10 * count;
         s->denoisedStride = 3;
     } else {
-        if ((e = launchDenoise(s->dSum, s->samples, s->width, s->height, s->lastSettings.exposure, s->dDenoise, s->dPixels, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+        if ((e = launchDenoise(s->dSum, s->samples, s->width, s->height, s->lastSettings.exposure, s->dDenoise, s->dPixels, s->stream)) != cudaSuccess) return abandon(e);
         s->denoisedOffset = 4 * 3 * count;  // region 3 of the filter's work buffer
         s->denoisedStride = 4;
     }
-    if ((e = cudaEventRecord(s->stop, s->stream)) != cudaSuccess) { fail(s, e); return 0; }
+    if ((e = cudaEventRecord(s->stop, s->stream)) != cudaSuccess) return abandon(e);
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) { fail(s, e); return 0; }
     if ((e = cudaEventElapsedTime(&s->stats.denoiseMs, s->start, s->stop)) != cudaSuccess) { fail(s, e); return 0; }
     if (s->denoiser) {
@@ -626,6 +645,7 @@ int RtxQueryRays(void* p, const RtxQuery* queries, int count, int any, RtxHit* h
         e = cudaMemcpyAsync(hits, dh, sizeof(RtxHit) * (size_t)count, cudaMemcpyDeviceToHost, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     }
+    if (e != cudaSuccess) settle(s->stream);
     rt::deviceFree(dq); rt::deviceFree(dh);
     if (e != cudaSuccess) { fail(s, e); return 0; }
     if (overflow) { s->hostError = "BVH traversal stack overflow"; return 0; }
@@ -652,6 +672,7 @@ int RtxSobolSamples(const unsigned* pixel, const unsigned* sample, const unsigne
     if (e == cudaSuccess) e = cudaMemcpy(dseed, seed, sizeof(unsigned) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launchSobolSamples(dd, dp, ds, dseed, count, ndim, dout, 0);
     if (e == cudaSuccess) e = cudaMemcpy(out, dout, sizeof(float) * n * ndim, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) settle(0);
     rt::deviceFree(dd); rt::deviceFree(dp); rt::deviceFree(ds); rt::deviceFree(dseed); rt::deviceFree(dout);
     return e == cudaSuccess ? 1 : 0;
 }
@@ -804,6 +825,7 @@ int RtxUnetInfer(void* p, const float* aovs, int h, int w, float* radiance) {
     if (e == cudaSuccess) e = u->net.inferDevice(dIn, h, w, dOut, 0, why);
     if (e == cudaSuccess) e = cudaMemcpy(radiance, dOut, sizeof(float) * px * 3, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = u->net.checkConvolutions(why);
+    if (e != cudaSuccess) settle(0);
     rt::deviceFree(dIn); rt::deviceFree(dOut);
     return unetResult(u, e, why);
 }

@@ -637,6 +637,7 @@ Unet::Unet(unsigned seed) {
 }
 
 Unet::~Unet() {
+    settleStreams();
     delete act_;
     rt::deviceFree(master_); rt::deviceFree(grad_); rt::deviceFree(adamM_); rt::deviceFree(adamV_); rt::deviceFree(wbf_); rt::deviceFree(wT_); rt::deviceFree(convError_);
     if (fork_) cudaEventDestroy(fork_);
@@ -692,9 +693,15 @@ cudaError_t Unet::setParams(const float* host) {
     return cudaStreamSynchronize(stream_);
 }
 
+void Unet::settleStreams() {
+    if (stream_) settle(stream_);
+    if (side_) settle(side_);
+}
+
 cudaError_t Unet::ensure(int n, int h, int w, bool training) {
     int H = (h + 15) / 16 * 16, W = (w + 15) / 16 * 16;
     if (act_ && act_->n == n && act_->H == H && act_->W == W && (act_->training || !training)) return cudaSuccess;
+    settleStreams();
     delete act_;
     act_ = new Activations();
     act_->n = n; act_->H = H; act_->W = W; act_->training = training;
@@ -922,6 +929,7 @@ cudaError_t Unet::lossAndGradient(const float* aovs, const float* targets, int n
     if (e == cudaSuccess && grads) e = cudaMemcpyAsync(grads, grad_, sizeof(float) * params_, cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
     if (e == cudaSuccess) e = checkConvolutions(error);
+    if (e != cudaSuccess) settleStreams();
     rt::deviceFree(dA); rt::deviceFree(dT);
     return e;
 }
@@ -944,7 +952,11 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     std::vector<unsigned char> flips(batch);
     std::vector<float> lossHost(steps, 0.0f);
     float* dLosses = nullptr;
-    if ((e = rt::deviceAlloc(&dLosses, sizeof(float) * std::max(steps, 1))) != cudaSuccess) { rt::deviceFree(dA); rt::deviceFree(dT); return e; }
+    if ((e = rt::deviceAlloc(&dLosses, sizeof(float) * std::max(steps, 1))) != cudaSuccess) {
+        settleStreams();
+        rt::deviceFree(dA); rt::deviceFree(dT);
+        return e;
+    }
     cudaMemsetAsync(dLosses, 0, sizeof(float) * std::max(steps, 1), stream_);
     const size_t bpx = (size_t)batch * h * w;
     const WeightTable table = weightTable(layers_);
@@ -967,6 +979,7 @@ cudaError_t Unet::train(const float* aovs, const float* targets, int count, int 
     if (e == cudaSuccess && losses) e = cudaMemcpyAsync(losses, dLosses, sizeof(float) * steps, cudaMemcpyDeviceToHost, stream_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
     if (e == cudaSuccess) e = checkConvolutions(error);
+    if (e != cudaSuccess) settleStreams();
     rt::deviceFree(dA); rt::deviceFree(dT); rt::deviceFree(dLosses);
     return e;
 }

@@ -67,6 +67,9 @@ public:
 
 private:
     struct Activations;
+    // Waits for the network's own streams. Inference runs on its caller's: who
+    // abandons one waits for that stream.
+    void settleStreams();
     cudaError_t ensure(int n, int h, int w, bool training);
     cudaError_t allocate(Activations& A) const;
     // head (inference): the output head to fuse into the last convolution;

@@ -251,6 +251,7 @@ cudaError_t uploadScene(const void* triangles, int count, cudaStream_t stream, S
     R.lightArea = area;
 #undef RT_TRY
 done:
+    if (e != cudaSuccess) settle(stream);
     rt::deviceFree(table); rt::deviceFree(slotIndex); rt::deviceFree(values); rt::deviceFree(counters); rt::deviceFree(blockCounts);
     rt::deviceFree(decoded); rt::deviceFree(emitterArea); rt::deviceFree(emitterTri);
     if (e != cudaSuccess) {

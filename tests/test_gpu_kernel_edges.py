@@ -239,3 +239,61 @@ def test_device_memory_is_shared_and_given_back(lib, sphere):
         t.join()
     assert len(results) == 16 and all(results)
     assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)
+
+
+def test_queries_beside_a_graph_capture(lib, sphere):
+    """A batch that records a CUDA graph for every frame (its settings change)
+    in one thread, and queries, scene loads and gradients, whose buffers come
+    and go, in others: every call succeeds with its usual result."""
+    from native_api import Batch, NativeError, Settings
+    _, cam, _, _, _ = scenes.cornell_sphere()
+    cam.aspect = 1.0
+    q = rays(1500)
+    aovs, target = synthetic(np.random.default_rng(1), 1, 32, 32)
+
+    def images(batch, view, frames):
+        out = []
+        for k in range(frames):
+            batch.render(Settings(2, 1.0, 0.0, 1.0, 0.5, 1 + k % 2, 1))
+            out.append(batch.image(view).tobytes())
+        return out
+
+    def frames(count):
+        batch = Batch(lib)
+        try:
+            view = batch.add_view(batch.add_scene(sphere), cam, 48, 48)
+            return images(batch, view, count)
+        finally:
+            batch.close()
+
+    def queries(count):
+        out = []
+        for _ in range(count):
+            with Session(lib) as s:
+                s.initialize(sphere, 8, 8)
+                out += [s.query(q).tobytes() for _ in range(8)]
+        return out
+
+    def gradients(count):
+        n = Unet(lib, seed=2)
+        try:
+            losses = [n.loss_grad(aovs, target)[0] for _ in range(count)]  # equal to the order of their sums
+            return [max(losses) - min(losses) <= 1e-5 * min(losses)]
+        finally:
+            n.close()
+    jobs = ((frames, 2, 150), (queries, 1, 30), (gradients, 1, 100))
+    expect = {job: set(job(few)) for job, few, _ in jobs}
+    results, errors = {}, []
+
+    def work(job, many):
+        try:
+            results[job] = set(job(many))
+        except NativeError as e:
+            errors.append((job.__name__, str(e)))
+    threads = [threading.Thread(target=work, args=(job, many)) for job, _, many in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert results == expect

@@ -303,3 +303,36 @@ def test_out_of_memory_in_network_calls(lib, what):
     finally:
         for n in nets:
             n.close()
+
+
+def test_scene_after_a_device_reset():
+    """cudaDeviceReset, called through a runtime of the host's own while a
+    session exists and freed blocks are kept, ends the context and its memory:
+    a new session in the new context allocates afresh and answers as before.
+    In a process of its own, which leaves the old session alone."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = '''
+import ctypes, os, sys
+sys.path[:0] = [sys.argv[1] + '/custom-ray-tracing-shader_b200']
+import numpy as np
+import scenes
+from native_api import Session, load_library
+lib = load_library()
+tris, q = scenes.cornell_sphere()[0], scenes.random_rays(np.random.Generator(np.random.PCG64(3)), 2000)
+
+def answers():
+    s = Session(lib)
+    s.initialize(tris, 64, 64)
+    return s, s.query(q).tobytes()
+old, expect = answers()
+with Session(lib) as other:  # leaves its blocks to the next
+    other.initialize(tris, 64, 64)
+assert ctypes.CDLL('libcudart.so.12').cudaDeviceReset() == 0
+new, got = answers()
+os._exit(0 if got == expect else 3)
+'''
+    env = dict(__import__('os').environ)
+    env['LD_LIBRARY_PATH'] = '/usr/local/cuda/lib64:' + env.get('LD_LIBRARY_PATH', '')
+    assert subprocess.run([sys.executable, '-c', code, str(ROOT)], env=env, timeout=120).returncode == 0

@@ -336,3 +336,49 @@ os._exit(0 if got == expect else 3)
     env = dict(__import__('os').environ)
     env['LD_LIBRARY_PATH'] = '/usr/local/cuda/lib64:' + env.get('LD_LIBRARY_PATH', '')
     assert subprocess.run([sys.executable, '-c', code, str(ROOT)], env=env, timeout=120).returncode == 0
+
+
+def test_kept_memory_is_bounded_and_returned():
+    """What the library keeps of freed device memory: something while another
+    object exists (a scene and its path buffers of 64 MB each come and go), at
+    most 4 GiB of it (also after path buffers of 256 MB each), nothing after
+    RtShutdown or with the last object. In a process of its own, so that no other
+    object exists; 32 MB of allowance for what the driver keeps."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = '''
+import sys
+sys.path[:0] = [sys.argv[1] + '/custom-ray-tracing-shader_b200']
+import torch
+import scenes
+from native_api import Session, load_library
+lib = load_library()
+tris, cam, st, _, _ = scenes.cornell_sphere()
+st.raysPerPixel = 16
+free = lambda: torch.cuda.mem_get_info()[0]
+MB = 1 << 20
+
+def come_and_go(w, h):
+    with Session(lib) as s:
+        s.initialize(tris, w, h)
+        s.render_device(cam, st)
+come_and_go(512, 512)
+come_and_go(1920, 1080)
+base = free()
+keeper = Session(lib)
+come_and_go(512, 512)
+kept = base - free()
+assert 500 * MB <= kept <= 4096 * MB, kept
+come_and_go(512, 512)
+assert base - free() <= kept + 32 * MB, (kept, base - free())
+come_and_go(1920, 1080)
+assert base - free() <= 4128 * MB, base - free()
+lib.RtShutdown(keeper.handle)
+assert base - free() <= 32 * MB, base - free()
+come_and_go(512, 512)
+assert base - free() >= 500 * MB
+keeper.close()
+assert base - free() <= 32 * MB, base - free()
+'''
+    assert subprocess.run([sys.executable, '-c', code, str(ROOT)], timeout=120).returncode == 0

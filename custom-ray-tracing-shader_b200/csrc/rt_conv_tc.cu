@@ -455,7 +455,7 @@ int deviceSms() {
 }  // namespace
 
 static std::atomic<int> g_convPath{0};
-static std::atomic<long long> g_pipeLaunches{0}, g_singleLaunches{0};
+static std::atomic<long long> g_pipeLaunches{0}, g_singleLaunches{0}, g_narrowLaunches{0};
 void setConvPath(int mode) { g_convPath.store(mode); }
 int convPath() { return g_convPath.load(); }
 static std::atomic<bool> g_convPipeReference{false};
@@ -465,6 +465,7 @@ void convLaunchCounts(long long* pipe, long long* single) {
     if (pipe) *pipe = g_pipeLaunches.load();
     if (single) *single = g_singleLaunches.load();
 }
+long long convNarrowLaunches() { return g_narrowLaunches.load(); }
 
 namespace {
 // Low-resolution tap (a, b) of output parity (py, px) collects the full taps
@@ -554,6 +555,7 @@ cudaError_t convTc(const bf16* in, const bf16* low, int lowChannels, int n, int 
                                                            accumulate, kc != cin, errorFlag, stream);
         if (e != cudaErrorNotSupported) {
             (kc != cin ? g_singleLaunches : g_pipeLaunches)++;
+            g_narrowLaunches++;
             return e;
         }
     }

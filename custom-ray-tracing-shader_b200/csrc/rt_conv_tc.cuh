@@ -122,8 +122,10 @@ int convPath();
 // identical, for comparison.
 void setConvPipeReference(bool on);
 bool convPipeReference();
-// Convolutions run so far by the pipelined and by the single-role kernel.
+// Convolutions run so far in the pipelined and in the single-role kernel's order.
 void convLaunchCounts(long long* pipe, long long* single);
+// Those of both counts that convNarrow ran.
+long long convNarrowLaunches();
 
 // Test hooks of the pipelined form (convPipe): zero values keep the defaults.
 struct ConvPipeTest {

@@ -923,6 +923,7 @@ int RtxConvLaunchCounts(long long* pipelined, long long* singleRole) {
     rt::convLaunchCounts(pipelined, singleRole);
     return 1;
 }
+long long RtxConvRowSpanLaunches(void) { return rt::convNarrowLaunches(); }
 
 int RtxDebugFailAllocation(int n) {
     if (n < 0) return 0;

@@ -108,6 +108,7 @@ EXPORTS = ('RtCreate', 'RtDestroy', 'RtShutdown', 'RtInitialize', 'RtRender', 'R
            'RtBvhInfo', 'RtLastError', 'RtxQueryRays', 'RtxSobolSamples', 'RtxExportBvh', 'RtxBvhStatsGet',
            'RtxReadAccumulation', 'RtxRenderStatsGet', 'RtxRenderDevice', 'RtxSetIntegrator', 'RtxSetTuning',
            'RtxDebugFailAllocation', 'RtxSetConvPath', 'RtxDebugConvWaitProbe', 'RtxConvLaunchCounts',
+           'RtxConvRowSpanLaunches',
            'RtxQueryRaysStatic', 'RtxSetEnvironment', 'RtxUnetCreate', 'RtxUnetDestroy', 'RtxUnetParamCount',
            'RtxUnetLastError', 'RtxUnetGetParams', 'RtxUnetSetParams', 'RtxUnetLossGrad', 'RtxUnetTrain',
            'RtxUnetInfer', 'RtxUnetSave', 'RtxUnetLoad', 'RtxSetDenoiser', 'RtxReadAovs', 'RtxReadDenoised',
@@ -152,6 +153,8 @@ def load_library(path=None):
     lib.RtxSetConvPath.argtypes = [c.c_int]
     lib.RtxDebugConvWaitProbe.argtypes = []
     lib.RtxConvLaunchCounts.argtypes = [c.c_void_p, c.c_void_p]
+    lib.RtxConvRowSpanLaunches.argtypes = []
+    lib.RtxConvRowSpanLaunches.restype = c.c_longlong
     lib.RtxQueryRaysStatic.argtypes = [vp, c.c_void_p, c.c_int, c.c_int, c.c_void_p]
     lib.RtxSetEnvironment.argtypes = [vp, c.c_int, c.c_float, c.c_float, c.c_float]
     lib.RtxUnetCreate.restype = vp

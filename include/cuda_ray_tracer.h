@@ -229,22 +229,33 @@ int RtxSetIntegrator(void* session, int mode);
 #define RTX_TUNE_STACK_LIMIT 7
 int RtxSetTuning(void* session, int key, int value);
 
-/* Which tensor-core convolution kernel the learned denoiser runs, no
- * counterpart in the reference: 0 (default) the warp-specialised TMA-fed
- * kernel wherever its shared memory allows (inference then also runs the
- * decoders' concatenated layers as two passes and fuses the output head
- * into the last layer; input rows are staged as swizzled slabs of 16-64
- * channels, and unsplit 32-channel layers issue one MMA per input row and
- * column tap over the three kernel rows' weights side by side), 1 the
- * single-role kernel for every layer, one pass each, 2 as 0 with every
- * layer's MMAs issued tap by tap per output tile over rows staged as planes
- * of 8 channels. Process-wide; 0 and 2 give identical results, 1 agrees with
- * them to BF16 rounding. */
+/* Which tensor-core convolution kernels the learned denoiser runs, no
+ * counterpart in the reference.
+ *   0  (default) the warp-specialised TMA-fed kernel wherever its shared
+ *      memory allows. Inference then also runs the decoders' concatenated
+ *      layers as two passes and fuses the output head into the last layer;
+ *      input rows are staged as swizzled slabs of 16-64 channels, and unsplit
+ *      32-channel layers issue one MMA per input row and column tap over the
+ *      three kernel rows' weights side by side where two blocks share a
+ *      multiprocessor. Images up to 64 pixels wide, small wider ones, and the
+ *      layer whose weights do not fit (224 -> 96, streamed) go to a kernel whose
+ *      tiles span image rows.
+ *   1  the single-role kernel for every layer, one pass each
+ *   2  as 0 without the row-spanning kernel (224 -> 96 on the single-role
+ *      kernel), every layer's MMAs issued tap by tap per output tile over rows
+ *      staged as planes of 8 channels
+ * Process-wide; 0 and 2 give identical results, 1 agrees with them to BF16
+ * rounding. */
 int RtxSetConvPath(int mode);
-/* Convolutions launched so far in this process by the warp-specialised
- * kernel and by the single-role kernel (either pointer may be null); no
- * counterpart in the reference. */
+/* Convolutions launched so far in this process, by the order in which they
+ * accumulate (either pointer may be null); no counterpart in the reference.
+ * pipelined: tap by tap over all input channels, the order of the
+ * warp-specialised kernel; singleRole: as the single-role kernel (whose order
+ * for 224 -> 96 is by chunks of 16 channels). The row-spanning kernel stands in
+ * for either and is counted there. */
 int RtxConvLaunchCounts(long long* pipelined, long long* singleRole);
+/* Those of both counts that the row-spanning kernel ran. */
+long long RtxConvRowSpanLaunches(void);
 /* Failure path of the warp-specialised convolution, no counterpart in the
  * reference: one launch whose wait on a barrier that nothing completes runs
  * out (2 ms limit) must report it through its error flag and free its

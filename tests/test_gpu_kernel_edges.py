@@ -297,3 +297,28 @@ def test_queries_beside_a_graph_capture(lib, sphere):
         t.join()
     assert not errors, errors
     assert results == expect
+
+
+def test_convolution_counts_name_the_kernel(lib, net):
+    """The counts go by order of accumulation; the row-spanning kernel's own say
+    how many of them it ran: none where a path switch leaves it out."""
+    import ctypes
+    aovs, _ = synthetic(np.random.default_rng(4), 1, 64, 256)
+
+    def counts():
+        pipe, single = ctypes.c_longlong(), ctypes.c_longlong()
+        lib.RtxConvLaunchCounts(ctypes.byref(pipe), ctypes.byref(single))
+        return np.array((pipe.value, single.value, lib.RtxConvRowSpanLaunches()))
+    try:
+        got = {}
+        for mode in (0, 1, 2):
+            assert lib.RtxSetConvPath(mode)
+            before = counts()
+            net.infer(aovs[0])
+            got[mode] = tuple(counts() - before)
+    finally:
+        lib.RtxSetConvPath(0)
+    assert got[1] == (0, 18, 0) and got[2] == (20, 1, 0)
+    # Levels 2 to 4 (64, 32 and 16 pixels wide) and 224 -> 96: 6 layers down, 4 up,
+    # one of them in two passes, at least.
+    assert got[0][:2] == (20, 1) and 11 <= got[0][2] <= 21, got[0]

@@ -64,7 +64,9 @@ struct Split { int axis, bin, leftCount, childTask[2]; };
 // 2 * interior) in the reference's depth-first order.
 struct Subtree { int root, base, interior; };
 // counters: [0] raw nodes, [1] (unused), [2] maximum depth, [3] error, [4]
-// subtree tasks, [5] finished blocks of a scan.
+// subtree tasks, [5] finished blocks of a scan. Errors: 1 nodes, 2 tasks, 3
+// wide nodes or triangles, 4 jobs past their capacity; 5 a position, 6 and 7 a
+// node outside its range (nothing is written there).
 constexpr int kCounters = 8;
 
 __device__ __forceinline__ void atomicMinFloat(float* a, float v) {
@@ -1270,6 +1272,14 @@ __global__ void __launch_bounds__(64) collapseKernel(const BinNode* bn, const in
 
 inline int blocksFor(long long n, int block) { return (int)((n + block - 1) / block); }
 
+// What an error of the kernels (counters[3]) means to the caller.
+cudaError_t buildError(int code, const char** failure) {
+    if (!code) return cudaSuccess;
+    *failure = code <= 2 ? "BVH build ran out of node or task capacity"
+             : code <= 4 ? "wide BVH collapse ran out of capacity" : "BVH build met an index out of its range";
+    return code <= 4 ? cudaErrorMemoryAllocation : cudaErrorUnknown;
+}
+
 template <class T>
 cudaError_t alloc(T*& p, size_t count) { return rt::deviceAlloc(reinterpret_cast<void**>(&p), sizeof(T) * (count ? count : 1)); }
 
@@ -1453,7 +1463,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
                 RT_TRY(cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream));
                 RT_TRY(cudaMemcpyAsync(hostLevels, levelCounts, sizeof(int) * 2 * levelSlots, cudaMemcpyDeviceToHost, stream));
                 RT_TRY(cudaStreamSynchronize(stream));
-                if (hostCounters[3]) { *failure = "BVH build ran out of node or task capacity"; err = cudaErrorMemoryAllocation; goto done; }
+                if ((err = buildError(hostCounters[3], failure)) != cudaSuccess) goto done;
                 if (hostLevels[2 * level] == 0) break;  // the next level has no task
                 if (level >= levelSlots - 1) { *failure = "BVH build exceeded the depth limit"; err = cudaErrorUnknown; goto done; }
             }
@@ -1468,7 +1478,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         RT_TRY(cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream));
         RT_TRY(cudaMemcpyAsync(hostStarts, levelStartDev, sizeof(int) * (level + 2), cudaMemcpyDeviceToHost, stream));
         RT_TRY(cudaStreamSynchronize(stream));
-        if (hostCounters[3]) { *failure = "BVH build ran out of node or task capacity"; err = cudaErrorMemoryAllocation; goto done; }
+        if ((err = buildError(hostCounters[3], failure)) != cudaSuccess) goto done;
         levelStart.assign(hostStarts, hostStarts + level + 2);
         int nodeCount = hostCounters[0];
         result.binaryNodes = nodeCount;
@@ -1505,7 +1515,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
         const int jobCapacity = wideCapacity;
         Job rootJob{0, 0, 0, 0, 0};
         RT_TRY(cudaMemcpyAsync(jobs, &rootJob, sizeof(Job), cudaMemcpyHostToDevice, stream));
-        int cinit[8] = {1, 0, 0, 0, 0, 0, 0, 0};
+        int cinit[3] = {1, 0, 0};  // the error stays: the renumbering may have set it
         RT_TRY(cudaMemcpyAsync(counters, cinit, sizeof(cinit), cudaMemcpyHostToDevice, stream));
         const int jobSlots = kStackCapacity + 2 + kLevelBatch;
         RT_TRY(cudaMemsetAsync(jobCounts, 0, sizeof(int) * jobSlots, stream));
@@ -1526,7 +1536,7 @@ cudaError_t buildBvh(const SceneTri* tris, int triCount, cudaStream_t stream, Bu
             RT_TRY(cudaMemcpyAsync(hostCounters, counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, stream));
             RT_TRY(cudaMemcpyAsync(hostJobs, jobCounts, sizeof(int) * jobSlots, cudaMemcpyDeviceToHost, stream));
             RT_TRY(cudaStreamSynchronize(stream));
-            if (hostCounters[3]) { *failure = "wide BVH collapse ran out of capacity"; err = cudaErrorMemoryAllocation; goto done; }
+            if ((err = buildError(hostCounters[3], failure)) != cudaSuccess) goto done;
             if (hostJobs[wideLevel] == 0) break;
             if (wideLevel >= jobSlots - 1) break;
         }

@@ -453,8 +453,23 @@ void resetSamples(Batch* b) {
     if (b->dSample) cudaMemsetAsync(b->dSample, 0, sizeof(unsigned), b->stream);
 }
 
-bool ensureBase(Batch* b) {
-    if (b->stream) return true;
+// The stream, events and sampler tables that every frame uses.
+void releaseBase(Batch* b) {
+    settleBatch(b);
+    void* owned[] = {b->dDirs, b->dPassXor, b->dSeedHash, b->dSample, b->dCounters, b->dError};
+    for (void* q : owned)
+        if (q) rt::deviceFree(q);
+    b->dDirs = b->dPassXor = b->dSeedHash = b->dSample = nullptr;
+    b->dCounters = nullptr;
+    b->dError = nullptr;
+    if (b->start) cudaEventDestroy(b->start);
+    if (b->stop) cudaEventDestroy(b->stop);
+    if (b->stream) cudaStreamDestroy(b->stream);
+    b->start = b->stop = nullptr;
+    b->stream = nullptr;
+}
+
+bool makeBase(Batch* b) {
     cudaError_t e;
     if ((e = cudaGetDevice(&b->device)) != cudaSuccess) return failB(b, e);
     std::string why;
@@ -476,6 +491,12 @@ bool ensureBase(Batch* b) {
     if ((e = rt::deviceAlloc(&b->dCounters, 4 * sizeof(unsigned long long))) != cudaSuccess) return failB(b, e);
     if ((e = rt::deviceAlloc(&b->dError, 2 * sizeof(int))) != cudaSuccess) return failB(b, e);
     return true;
+}
+bool ensureBase(Batch* b) {
+    if (b->stream) return true;
+    if (makeBase(b)) return true;
+    releaseBase(b);  // nothing half made is found by the next call
+    return false;
 }
 
 // Traversal tree of a scene at the batch's BVH width and pieces per triangle
@@ -817,12 +838,7 @@ void RtxBatchDestroy(void* p) {
         freeBvh(S.bvh);
         if (S.dTris) rt::deviceFree(S.dTris);
     }
-    void* owned[] = {b->dDirs, b->dPassXor, b->dSeedHash, b->dSample, b->dCounters, b->dError};
-    for (void* q : owned)
-        if (q) rt::deviceFree(q);
-    if (b->start) cudaEventDestroy(b->start);
-    if (b->stop) cudaEventDestroy(b->stop);
-    if (b->stream) cudaStreamDestroy(b->stream);
+    releaseBase(b);
     delete b;
 }
 

@@ -382,3 +382,37 @@ keeper.close()
 assert base - free() <= 32 * MB, base - free()
 '''
     assert subprocess.run([sys.executable, '-c', code, str(ROOT)], timeout=120).returncode == 0
+
+
+def test_out_of_memory_every_allocation_of_a_batch(lib):
+    """Every allocation of a batch's first scene and frame failing in turn: an
+    error with a message each time, and the same batch then renders the usual
+    image."""
+    from native_api import Batch
+    tris, cam, st, w, h = small_scene()
+    expect_rgba, expect_sums = reference_pass(lib, tris, cam, st, w, h)
+    failed = 0
+    for n in range(1, 200):
+        batch = Batch(lib)
+        try:
+            lib.RtxDebugFailAllocation(n)
+            steps = [lambda: batch.add_scene(tris), lambda: batch.add_view(0, cam, w, h), lambda: batch.render(st)]
+            errors = []
+            for step in steps:
+                try:
+                    step()
+                except NativeError as e:
+                    errors.append(str(e))
+                    lib.RtxDebugFailAllocation(0)
+                    step()
+            lib.RtxDebugFailAllocation(0)
+            assert batch.image(0).tobytes() == expect_rgba.tobytes(), n
+            assert batch.accumulation(0).tobytes() == expect_sums.tobytes(), n
+            if not errors:
+                break
+            assert len(errors) == 1 and errors[0]
+            failed += 1
+        finally:
+            lib.RtxDebugFailAllocation(0)
+            batch.close()
+    assert failed >= 40  # tables, upload, build, arenas, views, path buffers of two lanes

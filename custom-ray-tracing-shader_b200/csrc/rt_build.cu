@@ -1167,7 +1167,7 @@ __global__ void __launch_bounds__(64) collapseKernel(const BinNode* bn, const in
                 at = -1;
                 for (int s = 0; s < 8; s++) {
                     if (!((freeSlots >> s) & 1u)) continue;
-                    const float c = ((s & 4) ? -ck[0] : ck[0]) + ((s & 2) ? -ck[1] : ck[1]) + ((s & 1) ? -ck[2] : ck[2]);
+                    const float c = slotCost(ck, s);
                     if (c < cost) { cost = c; at = s; }
                 }
             };
@@ -1212,16 +1212,8 @@ __global__ void __launch_bounds__(64) collapseKernel(const BinNode* bn, const in
         // The node record in shared memory: lane 0 the header, then each kid
         // its slot's bytes.
         WideNode& W = shared[warp].node[slotOfJob];
-        float sc[3];
         unsigned char ebits[3];
-        for (int a = 0; a < 3; a++) {
-            float extent = nhi[a] - nlo[a];
-            int ex = -126;
-            if (extent > 0.0f) { frexpf(extent / 255.0f, &ex); }
-            ex = imax(-126, imin(127, ex));
-            ebits[a] = (unsigned char)(ex + 127);
-            sc[a] = bitsToFloat((unsigned)ebits[a] << 23);
-        }
+        for (int a = 0; a < 3; a++) ebits[a] = gridExponent(nhi[a] - nlo[a]);
         __syncwarp();
         if (sub < 5) reinterpret_cast<uint4*>(&W)[sub] = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
@@ -1233,32 +1225,18 @@ __global__ void __launch_bounds__(64) collapseKernel(const BinNode* bn, const in
             W.triBase = (unsigned)triBase;
         }
         if (kind >= 0 && fits) {
-            for (int a = 0; a < 3; a++) {
-                const float p = nlo[a];
-                int ql = (int)floorf((lo[a] - p) / sc[a]);
-                int qh = (int)ceilf((hi[a] - p) / sc[a]);
-                ql = imax(0, imin(255, ql));
-                qh = imax(0, imin(255, qh));
-                while (ql > 0 && fmaRn((float)ql, sc[a], p) > lo[a]) ql--;
-                while (qh < 255 && fmaRn((float)qh, sc[a], p) < hi[a]) qh++;
-                W.qlo[a][slot] = (unsigned char)ql;
-                W.qhi[a][slot] = (unsigned char)qh;
-            }
+            for (int a = 0; a < 3; a++) quantise(lo[a], hi[a], nlo[a], gridStep(ebits[a]), W.qlo[a][slot], W.qhi[a][slot]);
             const unsigned lower = (1u << slot) - 1u, lower2 = (1u << (2 * slot)) - 1u;
             if (kind == 2) {
                 const unsigned below = triCounts & lower2;
                 const int offset = __popc(below & 0x5555u) + 2 * __popc(below & 0xAAAAu);
-                W.meta[slot] = (unsigned char)((((1u << nTri) - 1u) << 5) | (unsigned)offset);
+                W.meta[slot] = groupMeta(nTri, offset);
                 for (int i = 0; i < nTri; i++) {
                     const int p = i == 0 ? tri[0] : i == 1 ? tri[1] : tri[2];
-                    const SceneTri& t = tris[p];
-                    float4* dst = packed + (size_t)(triBase + offset + i) * 3;
-                    dst[0] = make_float4(t.origin.x, t.origin.y, t.origin.z, t.edge1.x);
-                    dst[1] = make_float4(t.edge1.y, t.edge1.z, t.edge2.x, t.edge2.y);
-                    dst[2] = make_float4(t.edge2.z, bitsToFloat(t.oneSided != 0 ? 1u : 0u), bitsToFloat((unsigned)p), 0.0f);
+                    packTriangle(tris[p], p, packed + (size_t)(triBase + offset + i) * 3);
                 }
             } else {
-                W.meta[slot] = (unsigned char)(0x20u | (24u + (unsigned)slot));
+                W.meta[slot] = innerMeta(slot);
                 const int rank = __popc(innerSlots & lower), q = jobBase + rank;
                 if (q >= jobCapacity) atomicExch(&counters[3], 4);
                 else nextJobs[q] = Job{kind, kidNode, first, count, childBase + rank};

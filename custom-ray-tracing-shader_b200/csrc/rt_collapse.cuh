@@ -1,4 +1,8 @@
-// Collapse of the binary BVH into 8-wide compressed nodes (host and device).
+// Collapse of the binary BVH into 8-wide compressed nodes: the rules, and what
+// both forms compute with. The library's form is collapseKernel (rt_build.cu),
+// eight lanes per job; planCollapse, emitCollapse and collapseJob below are the
+// same rules one job after another on the host, which the tests check against
+// the reference's fixtures and hold the kernel's nodes against.
 //
 // One job per wide node. A job is either a binary node (interior or leaf) or
 // a range of primitives (a leaf too large for one node). For a binary node,
@@ -17,20 +21,6 @@ namespace rt {
 
 RT_HD int imin(int a, int b) { return a < b ? a : b; }
 RT_HD int imax(int a, int b) { return a > b ? a : b; }
-RT_HD int portableAdd(int* p, int v) {
-#ifdef __CUDA_ARCH__
-    return atomicAdd(p, v);
-#else
-    int old = *p; *p += v; return old;
-#endif
-}
-RT_HD void portableSet(int* p, int v) {
-#ifdef __CUDA_ARCH__
-    atomicExch(p, v);
-#else
-    *p = v;
-#endif
-}
 RT_HD float collapseHalfArea(const float lo[3], const float hi[3]) {
     float x = fmaxf(0.0f, hi[0] - lo[0]), y = fmaxf(0.0f, hi[1] - lo[1]), z = fmaxf(0.0f, hi[2] - lo[2]);
     return x * y + x * z + y * z;
@@ -49,6 +39,41 @@ RT_HD int slotsOf(const BinNode& n, int group, int width) {
     return n.count <= width * group ? (n.count + group - 1) / group : 1;
 }
 
+// Cost of a child whose centre lies at c from the node's in slot s: how late
+// rays whose direction signs are s meet it.
+RT_HD float slotCost(const float c[3], int s) {
+    return ((s & 4) ? -c[0] : c[0]) + ((s & 2) ? -c[1] : c[1]) + ((s & 1) ? -c[2] : c[2]);
+}
+// Exponent byte of a node's grid along an axis (steps of 2^(byte - 127), 255 of
+// them at least the extent), and the step.
+RT_HD unsigned char gridExponent(float extent) {
+    int ex = -126;
+    if (extent > 0.0f) { frexpf(extent / 255.0f, &ex); }
+    return (unsigned char)(imax(-126, imin(127, ex)) + 127);
+}
+RT_HD float gridStep(unsigned char exponent) { return bitsToFloat((unsigned)exponent << 23); }
+// A child's planes on the grid at p, rounded outward and checked with the
+// traversal's arithmetic.
+RT_HD void quantise(float lo, float hi, float p, float step, unsigned char& qlo, unsigned char& qhi) {
+    int ql = (int)floorf((lo - p) / step);
+    int qh = (int)ceilf((hi - p) / step);
+    ql = imax(0, imin(255, ql));
+    qh = imax(0, imin(255, qh));
+    while (ql > 0 && fmaRn((float)ql, step, p) > lo) ql--;
+    while (qh < 255 && fmaRn((float)qh, step, p) < hi) qh++;
+    qlo = (unsigned char)ql;
+    qhi = (unsigned char)qh;
+}
+// Meta bytes: a group of `count` triangles from `offset`, an interior child.
+RT_HD unsigned char groupMeta(int count, int offset) { return (unsigned char)((((1u << count) - 1u) << 5) | (unsigned)offset); }
+RT_HD unsigned char innerMeta(int slot) { return (unsigned char)(0x20u | (24u + (unsigned)slot)); }
+// Triangle `index` as traversal reads it.
+RT_HD void packTriangle(const SceneTri& t, int index, float4* dst) {
+    dst[0] = make_float4(t.origin.x, t.origin.y, t.origin.z, t.edge1.x);
+    dst[1] = make_float4(t.edge1.y, t.edge1.z, t.edge2.x, t.edge2.y);
+    dst[2] = make_float4(t.edge2.z, bitsToFloat(t.oneSided != 0 ? 1u : 0u), bitsToFloat((unsigned)index), 0.0f);
+}
+
 // A job's wide node before its storage is allocated: the children, their
 // slots and boxes, and the triangles of each triangle group.
 struct CollapsePlan {
@@ -65,7 +90,7 @@ struct CollapsePlan {
 // per node; the node format keeps eight slots either way. primTri: the
 // triangle of each primitive when primitives are triangle pieces (null:
 // primitive p is triangle p).
-RT_HD void planCollapse(Job J, const BinNode* bn, const int* order, const float4* plo, const float4* phi, int group,
+inline void planCollapse(Job J, const BinNode* bn, const int* order, const float4* plo, const float4* phi, int group,
                         int width, const int* primTri, CollapsePlan& P) {
     if (J.kind == 0 && bn[J.node].count > 0) { J.kind = 1; J.first = bn[J.node].first; J.count = bn[J.node].count; }
     P.wide = J.wide;
@@ -172,7 +197,7 @@ RT_HD void planCollapse(Job J, const BinNode* bn, const int* order, const float4
             at[k] = -1;
             for (int s = 0; s < 8; s++) {
                 if (!((freeSlots >> s) & 1u)) continue;
-                float c = ((s & 4) ? -ck[k][0] : ck[k][0]) + ((s & 2) ? -ck[k][1] : ck[k][1]) + ((s & 1) ? -ck[k][2] : ck[k][2]);
+                float c = slotCost(ck[k], s);
                 if (c < cost[k]) { cost[k] = c; at[k] = s; }
             }
         };
@@ -219,7 +244,7 @@ RT_HD void planCollapse(Job J, const BinNode* bn, const int* order, const float4
 // from childBase, packed triangles from triBase, next-level jobs from
 // jobBase (nInterior of each). counters[3] receives an error code when an
 // allocation passes its capacity.
-RT_HD void emitCollapse(const CollapsePlan& P, int childBase, int triBase, int jobBase, const SceneTri* tris,
+inline void emitCollapse(const CollapsePlan& P, int childBase, int triBase, int jobBase, const SceneTri* tris,
                         Job* nextJobs, WideNode* wide, float4* packed, int* counters, int wideCapacity,
                         int jobCapacity, int triCapacity) {
     const Kid* kids = P.kids;
@@ -228,19 +253,11 @@ RT_HD void emitCollapse(const CollapsePlan& P, int childBase, int triBase, int j
     const int* groupCount = P.groupCount;
     const float* nlo = P.nlo;
     const float* nhi = P.nhi;
-    if (childBase + P.nInterior > wideCapacity || triBase + P.nTris > triCapacity) { portableSet(&counters[3], 3); return; }
+    if (childBase + P.nInterior > wideCapacity || triBase + P.nTris > triCapacity) { counters[3] = 3; return; }
     WideNode W;
     W.px = nlo[0]; W.py = nlo[1]; W.pz = nlo[2];
-    float sc[3];
     unsigned char ebits[3];
-    for (int a = 0; a < 3; a++) {
-        float extent = nhi[a] - nlo[a];
-        int ex = -126;
-        if (extent > 0.0f) { frexpf(extent / 255.0f, &ex); }
-        ex = imax(-126, imin(127, ex));
-        ebits[a] = (unsigned char)(ex + 127);
-        sc[a] = bitsToFloat((unsigned)ebits[a] << 23);
-    }
+    for (int a = 0; a < 3; a++) ebits[a] = gridExponent(nhi[a] - nlo[a]);
     W.ex = ebits[0]; W.ey = ebits[1]; W.ez = ebits[2];
     W.imask = 0;
     W.childBase = (unsigned)childBase;
@@ -254,34 +271,18 @@ RT_HD void emitCollapse(const CollapsePlan& P, int childBase, int triBase, int j
             continue;
         }
         const Kid& K = kids[k];
-        for (int a = 0; a < 3; a++) {
-            float p = a == 0 ? W.px : (a == 1 ? W.py : W.pz);
-            int ql = (int)floorf((K.lo[a] - p) / sc[a]);
-            int qh = (int)ceilf((K.hi[a] - p) / sc[a]);
-            ql = imax(0, imin(255, ql));
-            qh = imax(0, imin(255, qh));
-            while (ql > 0 && fmaRn((float)ql, sc[a], p) > K.lo[a]) ql--;
-            while (qh < 255 && fmaRn((float)qh, sc[a], p) < K.hi[a]) qh++;
-            W.qlo[a][s] = (unsigned char)ql;
-            W.qhi[a][s] = (unsigned char)qh;
-        }
+        for (int a = 0; a < 3; a++) quantise(K.lo[a], K.hi[a], nlo[a], gridStep(ebits[a]), W.qlo[a][s], W.qhi[a][s]);
         if (K.kind == 2) {
             const int count = groupCount[k];
-            W.meta[s] = (unsigned char)((((1u << count) - 1u) << 5) | (unsigned)triOffset);
-            for (int i = 0; i < count; i++) {
-                const int p = groupTris[k][i];  // the triangle
-                const SceneTri& t = tris[p];
-                float4* dst = packed + (size_t)(triBase + triOffset + i) * 3;
-                dst[0] = make_float4(t.origin.x, t.origin.y, t.origin.z, t.edge1.x);
-                dst[1] = make_float4(t.edge1.y, t.edge1.z, t.edge2.x, t.edge2.y);
-                dst[2] = make_float4(t.edge2.z, bitsToFloat(t.oneSided != 0 ? 1u : 0u), bitsToFloat((unsigned)p), 0.0f);
-            }
+            W.meta[s] = groupMeta(count, triOffset);
+            for (int i = 0; i < count; i++)
+                packTriangle(tris[groupTris[k][i]], groupTris[k][i], packed + (size_t)(triBase + triOffset + i) * 3);
             triOffset += count;
         } else {
-            W.meta[s] = (unsigned char)(0x20u | (24u + (unsigned)s));
+            W.meta[s] = innerMeta(s);
             W.imask |= (unsigned char)(1u << s);
             const int q = jobBase + interiorSeen;
-            if (q >= jobCapacity) { portableSet(&counters[3], 4); interiorSeen++; continue; }
+            if (q >= jobCapacity) { counters[3] = 4; interiorSeen++; continue; }
             nextJobs[q] = Job{K.kind == 0 ? 0 : 1, K.node, K.first, K.count, childBase + interiorSeen};
             interiorSeen++;
         }
@@ -292,18 +293,17 @@ RT_HD void emitCollapse(const CollapsePlan& P, int childBase, int triBase, int j
 // Builds wide node J.wide for one job: planCollapse, then allocation of its
 // wide children, packed triangles and next-level jobs, then emitCollapse.
 // counters: [0] wide nodes, [1] packed triangles, [2] next-level jobs,
-// [3] error code. Host and device (atomics through portableAdd), so the
-// collapse can be checked on the CPU. nextCount, when set, counts the
-// next-level jobs in place of counters[2].
-RT_HD void collapseJob(Job J, const BinNode* bn, const int* order, const float4* plo, const float4* phi,
+// [3] error code.
+inline void collapseJob(Job J, const BinNode* bn, const int* order, const float4* plo, const float4* phi,
                        const SceneTri* tris, Job* nextJobs, WideNode* wide, float4* packed, int* counters,
                        int wideCapacity, int jobCapacity, int triCapacity, int group, int width = 8,
-                       const int* primTri = nullptr, int* nextCount = nullptr) {
+                       const int* primTri = nullptr) {
     CollapsePlan P;
     planCollapse(J, bn, order, plo, phi, group, width, primTri, P);
-    const int childBase = P.nInterior ? portableAdd(&counters[0], P.nInterior) : 0;
-    const int triBase = P.nTris ? portableAdd(&counters[1], P.nTris) : 0;
-    const int jobBase = P.nInterior ? portableAdd(nextCount ? nextCount : &counters[2], P.nInterior) : 0;
+    const int childBase = counters[0], triBase = counters[1], jobBase = counters[2];
+    counters[0] += P.nInterior;
+    counters[1] += P.nTris;
+    counters[2] += P.nInterior;
     emitCollapse(P, childBase, triBase, jobBase, tris, nextJobs, wide, packed, counters, wideCapacity, jobCapacity,
                  triCapacity);
 }

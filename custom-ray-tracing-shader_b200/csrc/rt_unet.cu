@@ -743,7 +743,9 @@ cudaError_t Unet::allocate(Activations& A) const {
         if (training && (e = A.make(A.dCat[j], px(level) * layers_[10 + 2 * j].cin)) != cudaSuccess) return e;
     }
     if (upHalf && (e = A.make(A.upHalf, upHalf)) != cudaSuccess) return e;
-    if ((e = A.make(A.pred, px(0) * kOutChannels)) != cudaSuccess) return e;
+    // Inference writes it, of one image (also over the buffers of a training
+    // call of that size); training's output layer is headKernel's.
+    if (n == 1 && (e = A.make(A.pred, px(0) * kOutChannels)) != cudaSuccess) return e;
     if (training) {
         if ((e = A.make(A.loss, 1)) != cudaSuccess) return e;
         if ((e = A.make(A.batch, n)) != cudaSuccess) return e;

@@ -38,7 +38,7 @@ template <class T>
 inline cudaError_t deviceAlloc(T** p, size_t bytes) {
     return deviceAllocBytes(reinterpret_cast<void**>(p), bytes);
 }
-void deviceFree(void* p, bool keep = true);  // keep: false gives the block back to the device
+void deviceFree(void* p);
 // Waits for a stream's work before blocks that it may use are freed.
 inline void settle(cudaStream_t stream) { (void)cudaStreamSynchronize(stream); }
 void trimDeviceMemory();

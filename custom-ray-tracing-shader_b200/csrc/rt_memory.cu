@@ -26,7 +26,11 @@ namespace {
 // loads of a million triangles and their first full-HD frames free (about 1.5 GB
 // each, in blocks of up to 300 MB that find their next use within a quarter of
 // their size: with 2 GB kept such a load took 22.0 ms, with 4 GB 19.0) and is 2%
-// of the device's memory. A block of more than a quarter of it goes back at once.
+// of the device's memory. Of the path buffers of a 16-path full-HD pass (24
+// blocks of 256 MB, freed after the scene's) as many stay as fit: giving them all
+// back at once cost the next session's first such pass 3 to 390 ms, as the driver
+// hands out new memory. A block of more than a quarter of the bound goes back at
+// once.
 constexpr size_t kCacheBytes = 4ull << 30;
 
 // Blocks belong to the CUDA context they were allocated in. cudaDeviceReset
@@ -143,14 +147,14 @@ cudaError_t deviceAllocBytes(void** p, size_t bytes) {
     return cudaSuccess;
 }
 
-void deviceFree(void* p, bool keep) {
+void deviceFree(void* p) {
     if (!p) return;
     std::lock_guard<std::mutex> guard(g_lock);
     auto it = owned().find(p);
     if (it == owned().end()) { cudaFree(p); return; }
     const Owned o = it->second;
     owned().erase(it);
-    if (!keep || g_users == 0 || o.bytes > kCacheBytes / 4) { cudaFree(p); return; }
+    if (g_users == 0 || o.bytes > kCacheBytes / 4) { cudaFree(p); return; }
     DeviceCache& c = caches()[o.device];
     c.ready.push_back(Block{p, o.bytes, o.context});
     c.bytes += o.bytes;

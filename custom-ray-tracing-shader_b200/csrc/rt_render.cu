@@ -468,13 +468,10 @@ cudaError_t allocWavefront(WavefrontBuffers& b, int capacity) {
     return cudaSuccess;
 }
 void freeWavefront(WavefrontBuffers& b) {
-    // Those of a large pass (12 arrays of up to 256 MB per lane) are not kept:
-    // they would only push the scenes' blocks out.
-    const bool keep = sizeof(float4) * (size_t)b.capacity < 256ull << 20;
     void* owned[] = {b.pathA, b.pathB, b.pathC, b.radiance, b.albedo, b.normal, b.hits, b.queue[0], b.queue[1],
                      b.shadowRay, b.shadowDir, b.shadowContrib, b.counts};
     for (void* p : owned)
-        if (p) rt::deviceFree(p, keep);
+        if (p) rt::deviceFree(p);
     b = WavefrontBuffers{};
 }
 

@@ -17,8 +17,8 @@
  * All entry points use plain C types and pointers. A session is not
  * thread-safe; use one session per thread (the reference's rule).
  *
- * Device memory: up to 4 GiB of freed blocks per GPU (the path buffers of
- * passes of 2^24 paths not among them) are kept for later calls while any session, batch or network exists.
+ * Device memory: up to 4 GiB of freed blocks per GPU (none of more than
+ * 1 GiB) are kept for later calls while any session, batch or network exists.
  * They go back to the device at RtShutdown of any session, with the last of
  * those objects, and when an allocation of the library's own would fail; a host
  * that shares the GPU's memory calls RtShutdown where it wants them back.

@@ -27,9 +27,11 @@
 // read once per strip, and the block computes all or half of the channels.
 //
 // Measured at 32 images (ncu, cold): 128 -> 128 channels at 8 x 8 36 -> 10 us,
-// 224 -> 96 at 16 x 16 122 -> 27 (resident
-// slices of 16 channels; streamed, 240 x 136: 111 -> 21), 64 -> 64 at 32 x 32 30 -> 13, 48 -> 48 at
-// 64 x 64 32 -> 22; all 28 such convolutions of a training step 1.21 -> 0.57 ms.
+// 224 -> 96 at 16 x 16 122 -> 27 (resident slices of 16 channels), 64 -> 64 at
+// 32 x 32 30 -> 13, 48 -> 48 at 64 x 64 32 -> 22; all 28 such convolutions of a
+// training step 1.21 -> 0.49 ms. Streamed, 224 -> 96 at 240 x 136: 71 us in the
+// single-role kernel on the same concatenated input (73 reading its halves in
+// place), 22 here.
 // What is left is launch, the weights' first load and one to five strips per block.
 //
 // The products are accumulated in the order of the kernel that runs the
@@ -464,7 +466,7 @@ cudaError_t convNarrow(const bf16* in, int n, int h, int w, int cin, const bf16*
     // 64 -> 96 at 240 x 136 12 / 19, 128 -> 128 at 120 x 68 11 / 23; but
     // 96 -> 96 at 240 x 136, one stage and two strips per block, 30 / 25, and
     // 48 -> 48 at 960 x 544 61 / 48. Streamed layers at any size: 224 -> 96 at
-    // 240 x 136 21 us against 74 in the single-role kernel.
+    // 240 x 136 22 us against 71 in the single-role kernel.
     if (!chunked && w > kNarrowWidth && ((long long)n * h * w > 1024ll * sms || (bestPer > 1 && a.stages < 2)))
         return cudaErrorNotSupported;
     a.tmemCols = 32;

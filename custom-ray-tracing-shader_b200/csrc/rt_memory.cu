@@ -25,12 +25,12 @@ namespace {
 // Bytes of freed blocks kept per device; the oldest go first. It covers what
 // loads of a million triangles and their first full-HD frames free (about 1.5 GB
 // each, in blocks of up to 300 MB that find their next use within a quarter of
-// their size: with 2 GB kept such a load took 22.0 ms, with 4 GB 19.0) and is 2%
-// of the device's memory. Of the path buffers of a 16-path full-HD pass (24
-// blocks of 256 MB, freed after the scene's) as many stay as fit: giving them all
-// back at once cost the next session's first such pass 3 to 390 ms, as the driver
-// hands out new memory. A block of more than a quarter of the bound goes back at
-// once.
+// their size; with 2 GB kept a session's repeated loads took as long, a new
+// session's first 21.5 ms against 18.7) and is 2% of the device's memory. Of the
+// path buffers of a 16-path full-HD pass (20 blocks of 256 MB, freed after the
+// scene's) as many stay as fit: giving them all back at once cost the next
+// session's first such pass 3 to 390 ms, as the driver hands out new memory. A
+// block of more than a quarter of the bound goes back at once.
 constexpr size_t kCacheBytes = 4ull << 30;
 
 // Blocks belong to the CUDA context they were allocated in. cudaDeviceReset

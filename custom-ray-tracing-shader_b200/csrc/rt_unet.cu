@@ -810,7 +810,7 @@ cudaError_t Unet::forward(cudaStream_t s, bool training, bool outputLayer, const
             const UnetLayer& L = layers_[k];
             if (r == 0 && (training || (!A.upWeights[j] && A.cat[j] && convPath() == 0))) {
                 // The weight gradient reads the concatenated input; at inference
-                // the streamed convolution does (8 + 21 us against 74 for the
+                // the streamed convolution does (8 + 22 us against 73 for the
                 // single-role kernel reading its halves in place, 240 x 136),
                 // and no other: buffers left by a training call of this size
                 // hold a concatenation for every level.

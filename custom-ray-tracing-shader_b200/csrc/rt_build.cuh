@@ -33,8 +33,8 @@ struct BuiltBvh {
 };
 
 // Builds the BVH for n device triangles on `stream`. Returns a CUDA error code
-// (cudaSuccess on success) and fills `out`/`result`. `scratchBytes` is the
-// peak temporary memory used, for reporting. Timing uses events on `stream`.
+// (cudaSuccess on success) and fills `out`/`result`. Timing uses events on
+// `stream`, which is drained when it returns.
 // leafGroup (1..3): most triangles under one wide-node slot. width (4 or 8):
 // most children per wide node. pieces (1..8): with more than one, the tree is
 // built over triangle pieces for traversal only: triangles whose box holds

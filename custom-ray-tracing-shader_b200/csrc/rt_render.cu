@@ -1,17 +1,18 @@
 // Render, query, sampler and denoise kernels for sm_100a.
 //
 // Two integrators produce bit-identical accumulations:
-//  - wavefront (default): per wave of paths (one raysPerPixel row r over a
-//    range of pixels) a generate kernel writes camera rays, then for every
+//  - wavefront (default): per wave of paths (a slice of the pass's, which may
+//    span sample rows) a generate kernel writes camera rays, then for every
 //    bounce an extend kernel (closest hit) runs over the compacted queue of
 //    live paths, a shade kernel applies the bounce and compacts survivors and
 //    light-sample rays into queues with warp-aggregated atomics, and a shadow
 //    kernel (any hit) resolves the light samples; an accumulate kernel adds
-//    the wave's paths to the running sums in row order. Traversal kernels only
-//    hold a ray and its stack, so they run at high occupancy on coherent work.
+//    the wave's paths to the running sums in row order. A pass of one wave
+//    traces a bounce's shadow rays with the next bounce's closest hits. Traversal
+//    kernels only hold a ray and its stack, so they run at high occupancy.
 //  - one kernel per pixel (megakernel), the reference's launch shape with the
 //    same traversal and shading code.
-// Traversal stacks live in shared memory, one column per thread.
+// Traversal stacks start in shared memory, one column per thread (rt_trace.cuh).
 #include <algorithm>
 #include <vector>
 

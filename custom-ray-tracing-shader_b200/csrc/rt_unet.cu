@@ -444,7 +444,6 @@ __global__ void __launch_bounds__(kWeightThreads) weightsKernel(const WeightTabl
     for (int i = threadIdx.x; i < 16 * cout; i += blockDim.x)
         out[(size_t)(i / 16) * cin + i % 16] = tile[i % 16 * 129 + i / 16];
 }
-// Network output (log space, padded frame) to linear radiance (w x h x 3).
 // Network input straight from the running sums: the AOVs of RtxReadAovs
 // (sum / samples, normalised normal, distance / samples), then the input
 // transform of inputKernel, for every pixel of the padded frame (beyond w x h
@@ -499,6 +498,7 @@ __global__ void outputFusedKernel(const bf16* d, int H, int W, int h, int w, int
     for (int k = 0; k < kOutChannels; k++) out[(size_t)i * 3 + k] = fmaxf(expm1f(s[k]), 0.0f);
 }
 
+// Network output (log space, padded frame) to linear radiance (w x h x 3).
 __global__ void outputKernel(const float* pred, int H, int W, int h, int w, float* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= w * h) return;

@@ -201,9 +201,10 @@ int RtxSetIntegrator(void* session, int mode);
  *                             is built over the pieces' padded boxes, which
  *                             overlap less than the whole triangles' boxes; with
  *                             no such triangle, traversal uses the reference's
- *                             tree. The reference's tree is always built for
- *                             RtBvhInfo and RtxExportBvh; hits do not depend on
- *                             the tree
+ *                             tree. The reference's tree is built in any case
+ *                             for RtBvhInfo and RtxExportBvh (on their first
+ *                             call where it is not the traced one); hits do not
+ *                             depend on the tree
  *   RTX_TUNE_LEAF             leaf size of that traversal tree (1..8, default 2;
  *                             the reference tree keeps 4; applies from the next
  *                             RtInitialize)
